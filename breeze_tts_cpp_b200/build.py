@@ -1,4 +1,5 @@
-"""Builds libb200q.so (the CUDA kernels + C++ host layer + C ABI) in-tree for sm_100a.
+"""Builds libb200q.so (the CUDA kernels + C++ host layer + C ABI) in-tree for sm_100a, and beside it the
+CPython binding _native.so that ops.py calls per operation.
 
 Run as `python -m breeze_tts_cpp_b200.build`. Objects are rebuilt only when a source or header
 is newer; the producers are compiled with --fmad=false like the reference's own producers
@@ -10,6 +11,7 @@ import os
 import shutil
 import subprocess
 import sys
+import sysconfig
 from concurrent.futures import ThreadPoolExecutor
 from pathlib import Path
 
@@ -18,6 +20,8 @@ CSRC = HERE / "csrc"
 INCLUDE = HERE.parent / "include"
 OBJ = HERE / "build"
 LIB = HERE / "libb200q.so"
+BINDING_SOURCE = CSRC / "bindings" / "python.cpp"
+BINDING = HERE / "_native.so"  # the CPython side of ops.py, linked against libb200q.so beside it
 ARCH = ["-gencode", "arch=compute_100a,code=sm_100a"]
 
 # (source, extra flags)
@@ -76,15 +80,34 @@ def build(verbose: bool = False, force: bool = False) -> Path:
     stamp = _newest_header()
     with ThreadPoolExecutor(max_workers=min(8, len(sources))) as pool:
         objects = list(pool.map(lambda sf: _compile(nvcc, sf[0], sf[1], stamp, verbose), sources))
-    if LIB.exists() and all(LIB.stat().st_mtime >= o.stat().st_mtime for o in objects):
-        return LIB
-    cmd = [nvcc, "-shared", *ARCH, "-o", str(LIB), *map(str, objects), "-lcudart"]
+    if not LIB.exists() or any(LIB.stat().st_mtime < o.stat().st_mtime for o in objects):
+        cmd = [nvcc, "-shared", *ARCH, "-o", str(LIB), *map(str, objects), "-lcudart"]
+        if verbose:
+            print(" ".join(cmd), flush=True)
+        done = subprocess.run(cmd, capture_output=True, text=True)
+        if done.returncode:
+            raise RuntimeError(f"link failed:\n{done.stdout}\n{done.stderr}")
+    _build_binding(verbose)
+    return LIB
+
+
+def _build_binding(verbose: bool) -> None:
+    """The binding calls the C ABI only, so it is rebuilt for its own source and the ABI's header alone."""
+    stamp = max(p.stat().st_mtime for p in (BINDING_SOURCE, INCLUDE / "b200q.h"))
+    if BINDING.exists() and BINDING.stat().st_mtime >= stamp:
+        return
+    import torch
+    from torch.utils import cpp_extension
+    torch_lib = Path(torch.__file__).parent / "lib"
+    cmd = ["g++", "-std=c++17", "-O2", "-fPIC", "-shared", f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}",
+           f"-I{INCLUDE}", f"-I{sysconfig.get_paths()['include']}", *(f"-isystem{p}" for p in cpp_extension.include_paths()),
+           str(BINDING_SOURCE), "-o", str(BINDING), f"-L{HERE}", "-l:libb200q.so", "-Wl,-rpath,$ORIGIN",
+           f"-L{torch_lib}", "-ltorch_python", "-ltorch_cpu", "-lc10"]
     if verbose:
         print(" ".join(cmd), flush=True)
     done = subprocess.run(cmd, capture_output=True, text=True)
     if done.returncode:
-        raise RuntimeError(f"link failed:\n{done.stdout}\n{done.stderr}")
-    return LIB
+        raise RuntimeError(f"building the Python binding failed:\n{done.stdout}\n{done.stderr}")
 
 
 if __name__ == "__main__":

@@ -4,7 +4,9 @@ torch CUDA tensors (torch is only the owner of device memory and streams here).
 Names follow the reference: `quantize_rows`, `matmul`, `prepare_quantized`, `quantized_norm`,
 `quantized_gated`, `linear` (src/ops/storage.h:12, src/ops/basic.h:11,25-26,33-35,
 src/ops/linear.h:11-14) and `RowScaledView` (src/core/quantization.h:33-49). Every function ends in
-a call through the C ABI of libb200q.so.
+a call through the C ABI of libb200q.so: the per-step operations through the compiled binding `_native`
+(csrc/bindings/python.cpp), and through ctypes where that one declines an argument and for everything a
+program calls once.
 """
 from __future__ import annotations
 
@@ -13,7 +15,7 @@ from dataclasses import dataclass
 
 import torch
 
-from . import _lib
+from . import _lib, _native
 from ._lib import BF16, F16, F32, FP8, I8, I32, Epilogue, NormFusion, Path_, RowScaled, Tensor
 
 MODES = ("int8", "fp8", "group_int8", "group_fp8")
@@ -90,6 +92,9 @@ def _fusion(residual=None, projection_bias=None, raw=None, gate=None, shift=None
                       _tensor(scale), rows_per_sequence, rows_ptr)
 
 
+_native.bind(_lib.B200QError, RowScaledView.c)
+
+
 class Context:
     """Device + stream + GEMM workspace + plan cache (reference: CudaContext, src/runtime/cuda_context.h:13-35)."""
 
@@ -105,13 +110,13 @@ class Context:
         stream_ptr = C.c_void_p(stream.cuda_stream) if stream is not None else None
         _lib.call("b200q_context_create", device, stream_ptr, C.c_void_p(self._workspace.data_ptr()), workspace_bytes,
                   mode.encode(), C.byref(handle))
-        self._handle = handle
+        self._handle, self._address = handle, handle.value
         self.multiprocessors = _lib.load().b200q_multiprocessors(handle)
 
     def close(self):
         if getattr(self, "_handle", None):
             _lib.load().b200q_context_destroy(self._handle)
-            self._handle = None
+            self._handle, self._address = None, 0
 
     def __del__(self):
         try:
@@ -121,16 +126,19 @@ class Context:
 
     # ---- producers
     def quantize_rows(self, x: torch.Tensor, out: RowScaledView) -> RowScaledView:
-        _lib.call("b200q_row_quantize", self._handle, C.byref(_tensor(x)), C.byref(out.c()))
+        if _native.row_quantize(self._address, x, out) is NotImplemented:
+            _lib.call("b200q_row_quantize", self._handle, C.byref(_tensor(x)), C.byref(out.c()))
         return out
 
     def quantized_norm(self, residual, update, weight, out: RowScaledView, epsilon: float, gemma=False, update_scale=None):
-        _lib.call("b200q_quantized_norm", self._handle, C.byref(_tensor(residual)), C.byref(_tensor(update)),
-                  C.byref(_tensor(weight)), C.byref(out.c()), epsilon, int(gemma), C.byref(_tensor(update_scale)))
+        if _native.quantized_norm(self._address, residual, update, weight, out, epsilon, gemma, update_scale) is NotImplemented:
+            _lib.call("b200q_quantized_norm", self._handle, C.byref(_tensor(residual)), C.byref(_tensor(update)),
+                      C.byref(_tensor(weight)), C.byref(out.c()), epsilon, int(gemma), C.byref(_tensor(update_scale)))
         return out
 
     def quantized_gated(self, x: torch.Tensor, out: RowScaledView, kind: int = 0) -> RowScaledView:
-        _lib.call("b200q_quantized_gated", self._handle, C.byref(_tensor(x)), C.byref(out.c()), kind)
+        if _native.quantized_gated(self._address, x, out, kind) is NotImplemented:
+            _lib.call("b200q_quantized_gated", self._handle, C.byref(_tensor(x)), C.byref(out.c()), kind)
         return out
 
     # ---- GEMM
@@ -153,8 +161,9 @@ class Context:
         _lib.call("b200q_seal", self._handle)
 
     def matmul(self, x: RowScaledView, w: RowScaledView, out: torch.Tensor, **epilogue) -> torch.Tensor:
-        ep = C.byref(_epilogue(**epilogue)) if epilogue else None
-        _lib.call("b200q_linear", self._handle, C.byref(x.c()), C.byref(w.c()), C.byref(_tensor(out)), ep)
+        if _native.linear(self._address, x, w, out, epilogue) is NotImplemented:
+            ep = C.byref(_epilogue(**epilogue)) if epilogue else None
+            _lib.call("b200q_linear", self._handle, C.byref(x.c()), C.byref(w.c()), C.byref(_tensor(out)), ep)
         return out
 
     def quant_linear(self, path, x: RowScaledView, w: RowScaledView, out: torch.Tensor, **epilogue) -> torch.Tensor:
@@ -165,27 +174,31 @@ class Context:
 
     def linear(self, x: torch.Tensor, w: RowScaledView, scratch: RowScaledView, out: torch.Tensor,
                quantized_output: RowScaledView | None = None, **epilogue):
-        ep = C.byref(_epilogue(**epilogue)) if epilogue else None
-        qo = C.byref(quantized_output.c()) if quantized_output is not None else None
-        _lib.call("b200q_linear_forward", self._handle, C.byref(_tensor(x)), C.byref(w.c()), C.byref(scratch.c()),
-                  C.byref(_tensor(out)), ep, qo)
+        if _native.linear_forward(self._address, x, w, scratch, out, epilogue, quantized_output) is NotImplemented:
+            ep = C.byref(_epilogue(**epilogue)) if epilogue else None
+            qo = C.byref(quantized_output.c()) if quantized_output is not None else None
+            _lib.call("b200q_linear_forward", self._handle, C.byref(_tensor(x)), C.byref(w.c()), C.byref(scratch.c()),
+                      C.byref(_tensor(out)), ep, qo)
         return out
 
     # ---- row-wise operators around the projections
     def pointwise(self, x: torch.Tensor, y: torch.Tensor, **epilogue) -> torch.Tensor:
-        _lib.call("b200q_pointwise", self._handle, C.byref(_tensor(x)), C.byref(_tensor(y)), C.byref(_epilogue(**epilogue)))
+        if _native.pointwise(self._address, x, y, epilogue) is NotImplemented:
+            _lib.call("b200q_pointwise", self._handle, C.byref(_tensor(x)), C.byref(_tensor(y)), C.byref(_epilogue(**epilogue)))
         return y
 
     def pointwise_quantize(self, x: torch.Tensor, out: RowScaledView, retained: torch.Tensor | None = None,
                            **epilogue) -> RowScaledView:
-        _lib.call("b200q_pointwise_quantize", self._handle, C.byref(_tensor(x)), C.byref(out.c()),
-                  C.byref(_epilogue(**epilogue)), C.byref(_tensor(retained)))
+        if _native.pointwise_quantize(self._address, x, out, epilogue, retained) is NotImplemented:
+            _lib.call("b200q_pointwise_quantize", self._handle, C.byref(_tensor(x)), C.byref(out.c()),
+                      C.byref(_epilogue(**epilogue)), C.byref(_tensor(retained)))
         return out
 
     def layer_norm_quantize(self, x: torch.Tensor, out: RowScaledView, weight=None, bias=None, epsilon: float = 1e-5,
                             retained: torch.Tensor | None = None, **fusion) -> RowScaledView:
-        _lib.call("b200q_layer_norm_quantize", self._handle, C.byref(_tensor(x)), C.byref(out.c()), C.byref(_tensor(weight)),
-                  C.byref(_tensor(bias)), epsilon, C.byref(_fusion(**fusion)), C.byref(_tensor(retained)))
+        if _native.layer_norm_quantize(self._address, x, out, weight, bias, epsilon, fusion, retained) is NotImplemented:
+            _lib.call("b200q_layer_norm_quantize", self._handle, C.byref(_tensor(x)), C.byref(out.c()), C.byref(_tensor(weight)),
+                      C.byref(_tensor(bias)), epsilon, C.byref(_fusion(**fusion)), C.byref(_tensor(retained)))
         return out
 
     def normalized_linear(self, x: torch.Tensor, w: RowScaledView, out: torch.Tensor, norm_weight=None, norm_bias=None,
@@ -217,7 +230,7 @@ class Linear:
         array = (Tensor * len(parts))(*[_tensor(p) for p in parts])
         handle = C.c_void_p()
         _lib.call("b200q_linear_layer_create", ctx._handle, array, len(parts), C.byref(_tensor(bias)), C.byref(handle))
-        self._handle = handle
+        self._handle, self._address = handle, handle.value
         self.out_features = sum(p.shape[0] for p in parts)
         self.in_features = parts[0].shape[1]
         _lib.call("b200q_linear_layer_prepare", ctx._handle, self._handle, max_rows)
@@ -226,9 +239,10 @@ class Linear:
                 **epilogue) -> torch.Tensor:
         if out is None:
             out = torch.empty(x.shape[0], self.out_features, dtype=x.dtype, device=x.device)
-        ep = C.byref(_epilogue(**epilogue)) if epilogue else None
-        qo = C.byref(quantized_output.c()) if quantized_output is not None else None
-        _lib.call("b200q_linear_layer_forward", self.ctx._handle, self._handle, C.byref(_tensor(x)), C.byref(_tensor(out)), ep, qo)
+        if _native.layer_forward(self.ctx._address, self._address, x, out, epilogue, quantized_output) is NotImplemented:
+            ep = C.byref(_epilogue(**epilogue)) if epilogue else None
+            qo = C.byref(quantized_output.c()) if quantized_output is not None else None
+            _lib.call("b200q_linear_layer_forward", self.ctx._handle, self._handle, C.byref(_tensor(x)), C.byref(_tensor(out)), ep, qo)
         return out
 
     PLAN, PREPARE, CAPTURE, EXECUTE = 0, 1, 2, 3  # reference: ForwardContext::Mode (src/core/forward_context.h:58)
@@ -250,11 +264,13 @@ class Linear:
     def normalized_forward(self, x: torch.Tensor, out: torch.Tensor, norm_weight=None, norm_bias=None, epsilon: float = 1e-5,
                            normalized=None, fusion: dict | None = None, quantized_output: RowScaledView | None = None,
                            **epilogue) -> torch.Tensor:
-        ep = C.byref(_epilogue(**epilogue)) if epilogue else None
-        qo = C.byref(quantized_output.c()) if quantized_output is not None else None
-        _lib.call("b200q_linear_layer_normalized_forward", self.ctx._handle, self._handle, C.byref(_tensor(x)),
-                  C.byref(_tensor(normalized)), C.byref(_tensor(out)), C.byref(_tensor(norm_weight)),
-                  C.byref(_tensor(norm_bias)), epsilon, C.byref(_fusion(**(fusion or {}))), ep, qo)
+        if _native.layer_normalized_forward(self.ctx._address, self._address, x, normalized, out, norm_weight, norm_bias, epsilon,
+                                            fusion, epilogue, quantized_output) is NotImplemented:
+            ep = C.byref(_epilogue(**epilogue)) if epilogue else None
+            qo = C.byref(quantized_output.c()) if quantized_output is not None else None
+            _lib.call("b200q_linear_layer_normalized_forward", self.ctx._handle, self._handle, C.byref(_tensor(x)),
+                      C.byref(_tensor(normalized)), C.byref(_tensor(out)), C.byref(_tensor(norm_weight)),
+                      C.byref(_tensor(norm_bias)), epsilon, C.byref(_fusion(**(fusion or {}))), ep, qo)
         return out
 
     def weight(self) -> RowScaled:
@@ -265,7 +281,7 @@ class Linear:
     def close(self):
         if getattr(self, "_handle", None):
             _lib.load().b200q_linear_layer_destroy(self._handle)
-            self._handle = None
+            self._handle, self._address = None, 0
 
     def __del__(self):
         try:
