@@ -3,7 +3,6 @@
 // (src/ops/kernels/quant/quant_dispatch.cu:194-234, quant_grouped.cu:221-239).
 #include "kernels/quant_dispatch.h"
 #include "kernels/quant_linear_sm100.cuh"
-#include "kernels/quant_prefill_sm100.cuh"
 #include "kernels/quant_prefill_pair_sm100.cuh"
 #include "kernels/quant_prefill_grouped_sm100.cuh"
 #include "ops/epilogue.h"
@@ -77,6 +76,22 @@ CUtensorMap scale_map(const float *base, int rows, int groups) {
     return map;
 }
 
+// Row-major 16-bit matrix [rows, cols] (row stride `ld` elements) for the epilogue's TMA traffic: box = one slab, 128 token
+// rows x 64 channels, 128B swizzle. Boxes that reach past the matrix read zeros and store nothing there.
+CUtensorMap slab_map(const void *base, int rows, int cols, int ld, Type type) {
+    CUtensorMap map;
+    cuuint64_t dims[2] = {cuuint64_t(cols), cuuint64_t(rows)};
+    cuuint64_t strides[1] = {cuuint64_t(ld) * 2};
+    cuuint32_t box[2] = {cuuint32_t(kSlabChannels), cuuint32_t(kBlockChannels)};
+    cuuint32_t element_strides[2] = {1, 1};
+    CUresult status = encode_tiled()(&map, type == Type::F16 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT16 : CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2,
+                                     const_cast<void *>(base), dims, strides, box, element_strides, CU_TENSOR_MAP_INTERLEAVE_NONE,
+                                     CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+    if (status != CUDA_SUCCESS)
+        throw std::runtime_error("cuTensorMapEncodeTiled (rows) failed with code " + std::to_string(int(status)));
+    return map;
+}
+
 // Split-K launches group the `splits` CTAs of one output tile into a thread-block cluster (1,1,splits).
 template <Type F, bool Grouped, int BN>
 void launch_instance(const CUtensorMap &map_w, const CUtensorMap &map_x, const GemmArgs &args, dim3 grid,
@@ -124,7 +139,6 @@ template <Type F, bool Grouped, int BN> void raise_limit() {
                                int(kSmemBudget)),
           "cudaFuncSetAttribute(shared memory)");
 }
-constexpr size_t kPrefillSmem = 1024 + size_t(kPrefillStages) * (kBlockChannels + kPrefillTokens) * kBlockK + kPrefillPatchBytes;
 int multiprocessor_count() {
     static std::atomic<int> cached[64];
     int device = 0;
@@ -137,30 +151,15 @@ int multiprocessor_count() {
     }
     return count;
 }
+constexpr size_t kPairSmem = 1024 + kPairBytes;
+// CTA pairs: one cluster of two per tile, persistent over the tiles.
 template <Type F>
-void launch_prefill(const CUtensorMap &map_w, const CUtensorMap &map_x, const PrefillArgs &args, cudaStream_t stream) {
-    const int tiles = ((args.n + kBlockChannels - 1) / kBlockChannels) * ((args.m + kPrefillTokens - 1) / kPrefillTokens);
-    cudaLaunchConfig_t config{};
-    config.gridDim = dim3(unsigned(std::min(tiles, multiprocessor_count())));
-    config.blockDim = dim3(kGemmThreads);
-    config.dynamicSmemBytes = kPrefillSmem;
-    config.stream = stream;
-    cudaLaunchAttribute attribute{};
-    attribute.id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attribute.val.programmaticStreamSerializationAllowed = 1;
-    config.attrs = &attribute;
-    config.numAttrs = 1;
-    check(cudaLaunchKernelEx(&config, w8a8_tcgen05_prefill<F>, map_w, map_x, args), "quantized prefill GEMM launch");
-}
-
-constexpr size_t kPairSmem = 1024 + size_t(kPairStages) * (kBlockChannels + kPrefillTokens / 2) * kBlockK + kPrefillPatchBytes;
-// CTA pairs: one cluster of two per 256-channel x 256-token tile, persistent over the tiles.
-template <Type F>
-void launch_prefill_pair(const CUtensorMap &map_w, const CUtensorMap &map_x, const PrefillArgs &args, cudaStream_t stream) {
-    const int tiles = ((args.n + 2 * kBlockChannels - 1) / (2 * kBlockChannels)) * ((args.m + kPrefillTokens - 1) / kPrefillTokens);
+void launch_prefill_pair(const CUtensorMap &map_w, const CUtensorMap &map_x, const CUtensorMap &map_out,
+                         const CUtensorMap &map_residual, const PairArgs &args, Type output_type, cudaStream_t stream) {
+    const int tiles = ((args.n + args.channels - 1) / args.channels) * ((args.m + kPrefillTokens - 1) / kPrefillTokens);
     cudaLaunchConfig_t config{};
     config.gridDim = dim3(2u * unsigned(std::min(tiles, multiprocessor_count() / 2)));
-    config.blockDim = dim3(kGemmThreads);
+    config.blockDim = dim3(kPairThreads);
     config.dynamicSmemBytes = kPairSmem;
     config.stream = stream;
     cudaLaunchAttribute attribute{};
@@ -168,17 +167,16 @@ void launch_prefill_pair(const CUtensorMap &map_w, const CUtensorMap &map_x, con
     attribute.val.programmaticStreamSerializationAllowed = 1;
     config.attrs = &attribute;
     config.numAttrs = 1;
-    // Up to 4096 output channels the tile runs with the tokens as MMA rows (epilogue straight from registers).
-    if (args.n <= 4096)
-        check(cudaLaunchKernelEx(&config, w8a8_tcgen05_prefill_pair<F, true>, map_w, map_x, args), "quantized pair GEMM launch");
-    else
-        check(cudaLaunchKernelEx(&config, w8a8_tcgen05_prefill_pair<F, false>, map_w, map_x, args), "quantized pair GEMM launch");
+    const bool f16 = output_type == Type::F16;
+    auto *kernel = args.ep.chain ? (f16 ? w8a8_tcgen05_prefill_pair<F, true, true> : w8a8_tcgen05_prefill_pair<F, true, false>)
+                                 : (f16 ? w8a8_tcgen05_prefill_pair<F, false, true> : w8a8_tcgen05_prefill_pair<F, false, false>);
+    check(cudaLaunchKernelEx(&config, kernel, map_w, map_x, map_out, map_residual, args), "quantized pair GEMM launch");
 }
 
 // Persistent K-group kernel: one CTA per multiprocessor over 128x128 tiles.
 template <Type F>
 void launch_prefill_grouped(const CUtensorMap &map_w, const CUtensorMap &map_x, const CUtensorMap &map_sw,
-                            const CUtensorMap &map_sx, const PrefillArgs &args, cudaStream_t stream) {
+                            const CUtensorMap &map_sx, const GroupedArgs &args, cudaStream_t stream) {
     const int tiles = ((args.n + kBlockChannels - 1) / kBlockChannels) * ((args.m + kGroupedTokens - 1) / kGroupedTokens);
     cudaLaunchConfig_t config{};
     config.gridDim = dim3(unsigned(std::min(tiles, multiprocessor_count())));
@@ -197,12 +195,10 @@ void launch_prefill_grouped(const CUtensorMap &map_w, const CUtensorMap &map_x, 
 template <Type F> void raise_limits() {
     check(cudaFuncSetAttribute(w8a8_tcgen05_prefill_grouped<F>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(kGroupedSmem)),
           "cudaFuncSetAttribute(shared memory)");
-    check(cudaFuncSetAttribute(w8a8_tcgen05_prefill_pair<F>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(kPairSmem)),
-          "cudaFuncSetAttribute(shared memory)");
-    check(cudaFuncSetAttribute(w8a8_tcgen05_prefill_pair<F, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(kPairSmem)),
-          "cudaFuncSetAttribute(shared memory)");
-    check(cudaFuncSetAttribute(w8a8_tcgen05_prefill<F>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(kPrefillSmem)),
-          "cudaFuncSetAttribute(shared memory)");
+    for (auto *kernel : {w8a8_tcgen05_prefill_pair<F, false, false>, w8a8_tcgen05_prefill_pair<F, false, true>,
+                         w8a8_tcgen05_prefill_pair<F, true, false>, w8a8_tcgen05_prefill_pair<F, true, true>})
+        check(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(kPairSmem)),
+              "cudaFuncSetAttribute(shared memory)");
     raise_limit<F, false, 16>(); raise_limit<F, false, 32>(); raise_limit<F, false, 64>();
     raise_limit<F, false, 128>(); raise_limit<F, false, 256>();
     raise_limit<F, true, 16>(); raise_limit<F, true, 32>(); raise_limit<F, true, 64>(); raise_limit<F, true, 128>();
@@ -319,42 +315,49 @@ void launch_quant_linear(LinearPath config, KernelProblem shape, const void *inp
         args.ep.bias = e.bias.data;
         args.ep.residual = e.residual.data;
         args.ep.residual_ld = e.residual.data ? e.residual.ld() : 0;
+        args.ep.residual_vector = aligned16(e.residual.data) && args.ep.residual_ld % 8 == 0;
         args.ep.residual_f32 = e.residual_f32.ptr<const float>();
         args.ep.value_scale = e.value_scale; args.ep.residual_scale = e.residual_scale;
         args.ep.output_scale = e.output_scale; args.ep.alpha = e.alpha;
         args.ep.activation = int(e.activation);
+        args.ep.plain_residual = e.residual.data && e.value_scale == 1.f && e.residual_scale == 1.f;
         args.ep.chain = e.bias.data || e.residual.data || e.value_scale != 1.f || e.output_scale != 1.f ||
                         e.activation != ops::Activation::Identity;
         vector_io = vector_io && aligned16(e.residual_f32.data);
     }
     args.vector_io = vector_io;
+    // Compute-bound shapes take the persistent, double-buffered CTA-pair kernel (its epilogue moves whole aligned rows).
+    if (!grouped && bn == kPrefillTokens && splits == 1 && output_type != Type::I32 && args.vector_io &&
+        (!args.ep.residual || args.ep.residual_vector)) {
+        PairArgs pair{args.m, args.n, args.k, xs, ws, args.ep.residual_f32, args.status};
+        pair.ep = args.ep;
+        // Epilogue cycles per channel of 128 tokens, measured: plain 16, bias and residual 31, an activation 55 (tanh
+        // GELU) to 100 (SiLU).
+        const double column_cycles = args.ep.activation > 1 ? 75.0 : args.ep.residual || args.ep.residual_f32 ? 31.0
+                                                                  : args.ep.chain ? 20.0 : kPairColumnCycles;
+        pair.channels = pair_channel_tile(shape.rows, shape.channels, kb_total, multiprocessor_count() / 2, column_cycles).channels;
+        pair.stages = pair_stages(pair.channels, args.ep.residual != nullptr);
+        const CUtensorMap map_half = operand_map(weights, shape.channels, shape.reduction, pair.channels / 2, true);
+        const CUtensorMap map_x = operand_map(input, shape.rows, shape.reduction, kPrefillTokens / 2, false);
+        const CUtensorMap map_out = slab_map(y, shape.rows, shape.channels, shape.channels, output_type);
+        const CUtensorMap map_residual = args.ep.residual ? slab_map(args.ep.residual, shape.rows, shape.channels, args.ep.residual_ld, output_type)
+                                                          : map_out;
+        if (format == Type::I8) launch_prefill_pair<Type::I8>(map_half, map_x, map_out, map_residual, pair, output_type, stream);
+        else launch_prefill_pair<Type::FP8>(map_half, map_x, map_out, map_residual, pair, output_type, stream);
+        return;
+    }
     // The weight map is the caller's prepared one when it describes these weights, else built here.
     CUtensorMap local_w;
     const bool reuse = prepared && prepared->weights == weights && prepared->channels == shape.channels &&
                        prepared->reduction == shape.reduction;
     if (!reuse) local_w = operand_map(weights, shape.channels, shape.reduction, kBlockChannels, true);
     const CUtensorMap &map_w = reuse ? prepared->values : local_w;
-    // Compute-bound shapes with a plain epilogue take the persistent, double-buffered kernels:
-    // CTA pairs (each CTA loads half of the token tile) when there are at least two channel tiles.
-    if (!grouped && bn == kPrefillTokens && splits == 1 && !args.ep.chain && output_type != Type::I32 && args.vector_io) {
-        PrefillArgs prefill{args.m, args.n, args.k, xs, ws, y, int(output_type), args.ep.residual_f32, args.status};
-        if (shape.channels >= 2 * kBlockChannels) {
-            const CUtensorMap map_half = operand_map(input, shape.rows, shape.reduction, kPrefillTokens / 2, false);
-            if (format == Type::I8) launch_prefill_pair<Type::I8>(map_w, map_half, prefill, stream);
-            else launch_prefill_pair<Type::FP8>(map_w, map_half, prefill, stream);
-            return;
-        }
-        const CUtensorMap map_x = operand_map(input, shape.rows, shape.reduction, bn, false);
-        if (format == Type::I8) launch_prefill<Type::I8>(map_w, map_x, prefill, stream);
-        else launch_prefill<Type::FP8>(map_w, map_x, prefill, stream);
-        return;
-    }
     // Compute-bound K-group shapes (both operands grouped by 128, enough 128x128 tiles to fill most of
     // the GPU, plain epilogue, no split) take the persistent K-group kernel.
     if (grouped && shape.input_group == kBlockK && shape.weight_group == kBlockK && bn == kGroupedTokens && splits == 1 &&
         !args.ep.chain && args.vector_io && shape.rows % 4 == 0 &&
         int64_t(n_tiles) * ((shape.rows + kGroupedTokens - 1) / kGroupedTokens) >= int64_t(multiprocessor_count()) * 2 / 3) {
-        PrefillArgs prefill{args.m, args.n, args.k, xs, ws, y, int(output_type), args.ep.residual_f32, args.status};
+        GroupedArgs prefill{args.m, args.n, args.k, xs, ws, y, int(output_type), args.ep.residual_f32, args.status};
         const CUtensorMap map_x = operand_map(input, shape.rows, shape.reduction, kGroupedTokens, false);
         const CUtensorMap map_sw = scale_map(ws, shape.channels, kb_total);
         const CUtensorMap map_sx = scale_map(xs, shape.rows, kb_total);

@@ -3,6 +3,7 @@
 #pragma once
 #include <algorithm>
 #include <cstddef>
+#include <cstdint>
 
 namespace tts::b200 {
 constexpr int kBlockChannels = 128; // MMA M: weight rows per tile
@@ -10,9 +11,43 @@ constexpr int kBlockK = 128;        // bytes of K per pipeline stage (one 128B-s
 constexpr int kMaxStages = 12;
 constexpr int kRowsPerPass = 16;    // token rows the epilogue warps finish per pass (16 threads x 8 channels per row)
 constexpr int kMaxSplits = 8;       // portable thread-block cluster size
-constexpr int kPrefillTokens = 256; // token tile of the persistent per-row kernels
+constexpr int kPrefillTokens = 256; // token tile of the persistent per-row kernel
+constexpr int kWeightStreamTokens = 64; // up to here one token tile covers the batch and a decoder chain's plans apply
 constexpr int kGroupedTokens = 128; // token tile of the persistent K-group kernel
 constexpr size_t kSmemBudget = 224 * 1024; // dynamic part per CTA: all but 3 KiB of the SM, which is what the static barriers and a co-resident quantizer CTA of the next launch need
+// CTA-pair prefill kernel. Shared memory: a ring of stages (128 token rows + half of the tile's weight rows) and
+// 16 KiB slabs of finished 16-bit rows: two that alternate, or four when the epilogue adds a 16-bit residual (a
+// whole tile's residual is prefetched into them).
+constexpr int kPairMaxStages = 10, kPairSlabs = 2, kPairResidualSlabs = 4;
+constexpr size_t kPairSlabBytes = 16 * 1024, kPairBytes = 6 * 32 * 1024 + kPairSlabs * kPairSlabBytes;
+inline int pair_stages(int channels, bool residual) {
+    const size_t ring = kPairBytes - (residual ? kPairResidualSlabs : kPairSlabs) * kPairSlabBytes;
+    return std::min(kPairMaxStages, int(ring / (size_t(kBlockChannels + channels / 2) * kBlockK)));
+}
+// Channel tile of the CTA-pair kernel for `rows` tokens on `pairs` pairs: the width out of 64, 128, 192, 256 that
+// minimises the estimated cycles. Per 128-byte K block a tile of C channels takes the tensor pipe's 2C cycles and
+// never less than 325 (measured at 64 and 128 channels: operand arrival and hand-over), so the widest tile is the
+// most efficient one and narrower ones win only where they fill pairs that would idle. The epilogue
+// (`column_cycles` per channel) runs under the next tile's K loop where there is one. A launch on all pairs takes
+// about a microsecond longer than one on 32 of them, whatever K is. The constants are fitted to launches of 160 to
+// 8192 rows on K = 512 to 6144, N = 256 to 12288 (the choice is within 5 % of the best width on nearly all).
+constexpr double kPairColumnCycles = 16; // scale, round, store
+struct PairTile {
+    int channels;
+    double cycles;
+};
+inline PairTile pair_channel_tile(int rows, int channels, int kb_count, int pairs, double column_cycles) {
+    PairTile best{256, 0};
+    for (int c = 256; c >= kBlockChannels / 2; c -= kBlockChannels / 2) {
+        const int64_t tiles = int64_t((channels + c - 1) / c) * ((rows + kPrefillTokens - 1) / kPrefillTokens);
+        const int64_t waves = (tiles + pairs - 1) / pairs;
+        const double main_loop = double(kb_count) * std::max(2.1 * c, 325.0) + 800, epilogue = column_cycles * c + 800;
+        const double cycles = main_loop + epilogue + double(waves - 1) * std::max(main_loop, epilogue) +
+                              65.0 * double(std::max<int64_t>(0, std::min<int64_t>(tiles, pairs) - 32));
+        if (c == 256 || cycles < 0.97 * best.cycles) best = {c, cycles};
+    }
+    return best;
+}
 
 struct LaunchShape {
     bool fits = false;

@@ -35,6 +35,7 @@
 #include "core/tensor.h"
 #include <cuda_bf16.h>
 #include <cuda_fp16.h>
+#include <type_traits>
 
 namespace tts::b200 {
 
@@ -53,6 +54,8 @@ struct FusedEpilogue {
     float value_scale = 1.f, residual_scale = 1.f, output_scale = 1.f, alpha = .1f;
     int activation = 0;                 // ops::Activation
     int residual_ld = 0;
+    int residual_vector = 0;            // residual rows are 16-byte aligned
+    int plain_residual = 0;             // a residual with value_scale == residual_scale == 1
     int chain = 0;                      // nonzero when anything beyond residual_f32 is requested
 };
 
@@ -75,36 +78,94 @@ struct GemmArgs {
     FusedEpilogue ep;
 };
 
-__device__ __forceinline__ float round_to(float v, int type) {
-    return type == int(Type::F16) ? __half2float(__float2half_rn(v)) : __bfloat162float(__float2bfloat16_rn(v));
+// Two 16-bit values in one word -> fp32.
+template <bool F16> __device__ __forceinline__ float2 unpack16(uint32_t word) {
+    return F16 ? __half22float2(*reinterpret_cast<const __half2 *>(&word))
+               : make_float2(__uint_as_float(word << 16), __uint_as_float(word & 0xffff0000u));
 }
-__device__ __forceinline__ float load_as(const void *p, size_t i, int type) {
-    return type == int(Type::F16) ? __half2float(static_cast<const __half *>(p)[i])
-                                  : __bfloat162float(static_cast<const __nv_bfloat16 *>(p)[i]);
-}
-// Post-GEMM chain on one rounded value; rounding points follow the reference's separate pass
-// (src/ops/kernels/sequence/sequence_internal.cuh:52-74; the activations are the finishing pass's own
-// instruction sequences, so GEMM + fused chain equals GEMM followed by that pass bit for bit). `bias` and `skip` are already fp32
-// (0 when absent). Deliberately not inlined: the transcendental activations are large, and eight
-// inlined copies per row pushed the common no-chain path out of the instruction cache.
-__device__ __noinline__ float finish_chain(const FusedEpilogue &e, int type, float value, float bias, float skip) {
-    value = round_to(value, type);
-    if (e.bias) value = round_to(__fadd_rn(value, bias), type);
-    if (e.residual || e.value_scale != 1.f)
-        value = round_to(__fmaf_rn(e.value_scale, value, __fmul_rn(e.residual_scale, skip)), type); // contracted as in the reference's finishing pass
-    if (e.activation || e.output_scale != 1.f)
-        value = finish_activation(round_to(__fmul_rn(value, e.output_scale), type), e.activation, e.alpha);
-    return value;
-}
-__device__ __forceinline__ uint32_t pack16(float lo, float hi, int type) {
-    if (type == int(Type::F16)) {
+template <bool F16> __device__ __forceinline__ uint32_t pack2x16(float lo, float hi) {
+    if (F16) {
         __half2 h = __floats2half2_rn(lo, hi);
         return *reinterpret_cast<uint32_t *>(&h);
     }
     __nv_bfloat162 b = __floats2bfloat162_rn(lo, hi);
     return *reinterpret_cast<uint32_t *>(&b);
 }
-
+// Sum of two pairs, rounded once. Equal to the finishing pass's fp32 sum rounded to storage: fp32 carries more than
+// twice the storage type's precision plus two bits, so its intermediate rounding cannot show.
+template <bool F16> __device__ __forceinline__ uint32_t add2x16(uint32_t a, uint32_t b) {
+    if (F16) {
+        __half2 h = __hadd2(*reinterpret_cast<__half2 *>(&a), *reinterpret_cast<__half2 *>(&b));
+        return *reinterpret_cast<uint32_t *>(&h);
+    }
+    __nv_bfloat162 h = __hadd2(*reinterpret_cast<__nv_bfloat162 *>(&a), *reinterpret_cast<__nv_bfloat162 *>(&b));
+    return *reinterpret_cast<uint32_t *>(&h);
+}
+template <bool F16> __device__ __forceinline__ uint32_t relu2x16(uint32_t v) {
+    const float2 f = unpack16<F16>(v);
+    return pack2x16<F16>(fmaxf(f.x, 0.f), fmaxf(f.y, 0.f));
+}
+// Post-GEMM chain on eight consecutive channels of one row, already rounded to storage and packed, up to and
+// including ReLU; rounding points follow the reference's separate pass
+// (src/ops/kernels/sequence/sequence_internal.cuh:52-74), so GEMM + fused chain equals GEMM followed by that pass
+// bit for bit. Every step ends in a storage value, which is why the row can stay packed between them.
+template <bool F16> __device__ __forceinline__ uint4 chain8(const FusedEpilogue &e, uint4 row, uint4 bias, uint4 skip) {
+    uint32_t v[4] = {row.x, row.y, row.z, row.w};
+    const uint32_t b[4] = {bias.x, bias.y, bias.z, bias.w}, k[4] = {skip.x, skip.y, skip.z, skip.w};
+    if (e.bias) {
+#pragma unroll
+        for (int i = 0; i < 4; ++i) v[i] = add2x16<F16>(v[i], b[i]);
+    }
+    if (e.plain_residual) {
+#pragma unroll
+        for (int i = 0; i < 4; ++i) v[i] = add2x16<F16>(v[i], k[i]);
+    } else if (e.residual || e.value_scale != 1.f) { // contracted as in the reference's finishing pass
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            const float2 x = unpack16<F16>(v[i]), s = unpack16<F16>(k[i]);
+            v[i] = pack2x16<F16>(__fmaf_rn(e.value_scale, x.x, __fmul_rn(e.residual_scale, s.x)),
+                                 __fmaf_rn(e.value_scale, x.y, __fmul_rn(e.residual_scale, s.y)));
+        }
+    }
+    if (e.output_scale != 1.f) {
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            const float2 x = unpack16<F16>(v[i]);
+            v[i] = pack2x16<F16>(__fmul_rn(x.x, e.output_scale), __fmul_rn(x.y, e.output_scale));
+        }
+    }
+    if (e.activation == 1) {
+#pragma unroll
+        for (int i = 0; i < 4; ++i) v[i] = relu2x16<F16>(v[i]);
+    }
+    return make_uint4(v[0], v[1], v[2], v[3]);
+}
+// The finishing pass's other activations (its own instruction sequences) on eight packed values. Out of line because
+// they are large: one copy per kernel, eight independent evaluations per call, arguments and result in registers.
+template <bool F16> __device__ __noinline__ uint4 activate8(uint4 row, int kind, float alpha) {
+    uint32_t v[4] = {row.x, row.y, row.z, row.w};
+    switch (kind) {
+#define B200Q_ACTIVATION(K)                                                                                          \
+    case K:                                                                                                          \
+        _Pragma("unroll") for (int i = 0; i < 4; ++i) {                                                              \
+            const float2 x = unpack16<F16>(v[i]);                                                                    \
+            v[i] = pack2x16<F16>(finish_activation(x.x, K, alpha), finish_activation(x.y, K, alpha));                \
+        }                                                                                                            \
+        break;
+        B200Q_ACTIVATION(2)
+        B200Q_ACTIVATION(3)
+        B200Q_ACTIVATION(4)
+        B200Q_ACTIVATION(5)
+        B200Q_ACTIVATION(7)
+        B200Q_ACTIVATION(8)
+#undef B200Q_ACTIVATION
+    default: break;
+    }
+    return make_uint4(v[0], v[1], v[2], v[3]);
+}
+template <bool F16> __device__ __forceinline__ uint4 pack8x16(const float (&v)[8]) {
+    return make_uint4(pack2x16<F16>(v[0], v[1]), pack2x16<F16>(v[2], v[3]), pack2x16<F16>(v[4], v[5]), pack2x16<F16>(v[6], v[7]));
+}
 template <Type F, bool Grouped, int BN>
 __global__ void __launch_bounds__(kGemmThreads, (!Grouped && BN <= 64) ? 2 : 1)
 w8a8_tcgen05_gemm(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_x,
@@ -143,7 +204,7 @@ w8a8_tcgen05_gemm(const __grid_constant__ CUtensorMap map_w, const __grid_consta
     uint8_t *reduce_ptr = tiles_ptr + a.tile_region;
     float *scale_smem = reinterpret_cast<float *>(reduce_ptr + reduce_bytes);
 
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int warp = ptx::warp_index(), lane = threadIdx.x & 31;
     const int split = splits > 1 ? int(ptx::cluster_ctarank()) : 0; // cluster = (1,1,splits): rank == blockIdx.z
     const int n0 = blockIdx.x * kBlockChannels, m0 = blockIdx.y * BN;
     const int kb_total = (a.k + kBlockK - 1) / kBlockK;
@@ -175,7 +236,7 @@ w8a8_tcgen05_gemm(const __grid_constant__ CUtensorMap map_w, const __grid_consta
     ptx::tcgen05_fence_before();
     __syncthreads();
     ptx::tcgen05_fence_after();
-    const uint32_t tmem_base = tmem_slot;
+    const uint32_t tmem_base = ptx::warp_uniform(tmem_slot);
     volatile int *abort_ptr = &abort_flag;
     const long long wait_limit = a.wait_limit_cycles > 0 ? a.wait_limit_cycles : ptx::kWaitLimitCycles;
     // The next kernel in the stream may begin its own prologue; peers learn that this CTA is running.
@@ -184,38 +245,50 @@ w8a8_tcgen05_gemm(const __grid_constant__ CUtensorMap map_w, const __grid_consta
 
     if (warp == 0) {
         // ------------------------------------------------------------ TMA producer
-        if (lane == 0) {
+        // The whole warp runs the loops so that addresses and coordinates stay warp-uniform (a copy takes them from
+        // uniform registers; issued from a single-lane branch it took about 190 cycles, most of it moving operands
+        // there); one elected lane issues.
+        if (ptx::elect_one()) {
             ptx::prefetch_tensormap(&map_w);
             ptx::prefetch_tensormap(&map_x);
-            // Weights do not depend on the upstream kernel: fill the ring with weight tiles first
-            // (one barrier per stage), then wait for upstream and add the activation tiles of all
-            // those stages under ONE barrier. A barrier test between MMA issues costs the issuing
-            // thread about 200 cycles, so the burst over the prefetched stages must not need any.
-            // Weights are streamed once: they are marked first-to-evict so that the few megabytes of
-            // activations the chain keeps passing from kernel to kernel stay in L2.
-            const uint64_t stream_once = ptx::policy_evict_first();
-            const int ahead = min(a.stages, kb_count);
-            for (int i = 0; i < ahead; ++i) {
-                const uint32_t bar = ptx::smem_u32(&full_bar[i]);
+        }
+        // Weights do not depend on the upstream kernel: fill the ring with weight tiles first
+        // (one barrier per stage), then wait for upstream and add the activation tiles of all
+        // those stages under ONE barrier. A barrier test between MMA issues costs the issuing
+        // thread about 200 cycles, so the burst over the prefetched stages must not need any.
+        // Weights are streamed once: they are marked first-to-evict so that the few megabytes of
+        // activations the chain keeps passing from kernel to kernel stay in L2.
+        const uint64_t stream_once = ptx::policy_evict_first();
+        const int ahead = min(a.stages, kb_count);
+        for (int i = 0; i < ahead; ++i) {
+            const uint32_t bar = ptx::smem_u32(&full_bar[i]);
+            if (ptx::elect_one()) {
                 ptx::mbar_arrive_expect_tx(bar, kWeightBytes + (i == 0 ? uint32_t(a.expiry_extra_bytes) : 0u));
                 ptx::tma_load_2d_hint(tiles_base + uint32_t(i) * kStageBytes, &map_w, bar, (kb_begin + i) * kBlockK, n0, stream_once);
             }
-            ptx::wait_for_upstream();
-            ptx::mbar_arrive_expect_tx(ptx::smem_u32(&x_full), uint32_t(ahead) * kTokenBytes);
-            for (int i = 0; i < ahead; ++i)
+            __syncwarp();
+        }
+        ptx::wait_for_upstream();
+        if (ptx::elect_one()) ptx::mbar_arrive_expect_tx(ptx::smem_u32(&x_full), uint32_t(ahead) * kTokenBytes);
+        for (int i = 0; i < ahead; ++i) {
+            if (ptx::elect_one())
                 ptx::tma_load_2d(tiles_base + uint32_t(i) * kStageBytes + kWeightBytes, &map_x,
                                  ptx::smem_u32(&x_full), (kb_begin + i) * kBlockK, m0);
-            int stage = ahead == a.stages ? 0 : ahead;
-            uint32_t phase = ahead == a.stages ? 1u : 0u;
-            for (int kb = kb_begin + ahead; kb < kb_end; ++kb) {
-                if (!ptx::mbar_wait(ptx::smem_u32(&empty_bar[stage]), phase ^ 1u, abort_ptr, wait_limit)) break;
-                const uint32_t bar = ptx::smem_u32(&full_bar[stage]);
-                const uint32_t dst = tiles_base + uint32_t(stage) * kStageBytes;
+            __syncwarp();
+        }
+        int stage = ahead == a.stages ? 0 : ahead;
+        uint32_t phase = ahead == a.stages ? 1u : 0u;
+        for (int kb = kb_begin + ahead; kb < kb_end; ++kb) {
+            if (!__all_sync(0xffffffffu, ptx::mbar_wait(ptx::smem_u32(&empty_bar[stage]), phase ^ 1u, abort_ptr, wait_limit))) break;
+            const uint32_t bar = ptx::smem_u32(&full_bar[stage]);
+            const uint32_t dst = tiles_base + uint32_t(stage) * kStageBytes;
+            if (ptx::elect_one()) {
                 ptx::mbar_arrive_expect_tx(bar, kStageBytes);
                 ptx::tma_load_2d_hint(dst, &map_w, bar, kb * kBlockK, n0, stream_once);
                 ptx::tma_load_2d(dst + kWeightBytes, &map_x, bar, kb * kBlockK, m0);
-                if (++stage == a.stages) { stage = 0; phase ^= 1u; }
             }
+            __syncwarp();
+            if (++stage == a.stages) { stage = 0; phase ^= 1u; }
         }
         if (splits > 1) ptx::cluster_wait();
     } else if (warp == 1) {
@@ -325,12 +398,15 @@ w8a8_tcgen05_gemm(const __grid_constant__ CUtensorMap map_w, const __grid_consta
         const int passes = (valid_tokens + kRowsPerPass - 1) / kRowsPerPass;
         // Static operands (weights' scales, bias) are fetched before anything else so their latency
         // hides behind the main loop.
-        float sw8[8], bias8[8];
+        float sw8[8];
+        uint32_t bias_words[4]; // packed pairs
+        const uint16_t *bias16 = static_cast<const uint16_t *>(e.bias);
 #pragma unroll
-        for (int i = 0; i < 8; ++i) {
-            sw8[i] = (!Grouped && columns_ok) ? a.sw[n + i] : 1.f;
-            bias8[i] = (e.bias && columns_ok) ? load_as(e.bias, n + i, type) : 0.f;
-        }
+        for (int i = 0; i < 8; ++i) sw8[i] = (!Grouped && columns_ok) ? a.sw[n + i] : 1.f;
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+            bias_words[i] = (bias16 && columns_ok) ? uint32_t(bias16[n + 2 * i]) | (uint32_t(bias16[n + 2 * i + 1]) << 16) : 0u;
+        const uint4 bias8 = make_uint4(bias_words[0], bias_words[1], bias_words[2], bias_words[3]);
         // K-group mode: the weights' group scales of this CTA's K range are static too, one entry per
         // accumulation unit (a unit past the end of K, whose accumulator holds zeros, takes scale 1).
         const int unit_count = kb_count * units;
@@ -343,10 +419,14 @@ w8a8_tcgen05_gemm(const __grid_constant__ CUtensorMap map_w, const __grid_consta
         }
         ptx::wait_for_upstream(); // activation scales, residuals and the output buffer belong to upstream
         float first_residual[8];
+        uint4 first_skip = make_uint4(0, 0, 0, 0); // 16-bit residual of that pass
         {
             const int c = split * kRowsPerPass + row_in_pass; // first pass this CTA owns
 #pragma unroll
             for (int i = 0; i < 8; ++i) first_residual[i] = 0.f;
+            if (e.residual && e.residual_vector && columns_ok && c < valid_tokens)
+                first_skip = *reinterpret_cast<const uint4 *>(static_cast<const uint16_t *>(e.residual) +
+                                                              size_t(m0 + c) * e.residual_ld + n);
             if (e.residual_f32 && columns_ok && c < valid_tokens) {
                 const float *src = e.residual_f32 + size_t(m0 + c) * a.n + n;
                 if (a.vector_io) {
@@ -466,12 +546,13 @@ w8a8_tcgen05_gemm(const __grid_constant__ CUtensorMap map_w, const __grid_consta
         else asm volatile("bar.sync 1, 256;" ::: "memory");
 
         // ---- phase 2: finish token rows; every global access is a 16-byte vector on a 256-byte row.
-        // The common case (bf16 out, aligned rows, nothing but an optional fp32 residual) takes a lean
-        // loop; everything else takes the general loop below it.
-        const bool lean = type == int(Type::BF16) && a.vector_io && !e.chain;
-        if (ok && !*abort_ptr && columns_ok && lean) {
+        // Aligned 16-bit rows take a loop specialised for the output type and for whether the finishing chain
+        // follows; raw accumulators and unaligned rows take the general loop below it.
+        const bool lean = type != int(Type::I32) && a.vector_io && (!e.residual || e.residual_vector);
+        const auto finish_rows = [&](auto f16_tag, auto chain_tag) {
+            constexpr bool kF16 = decltype(f16_tag)::value, kChain = decltype(chain_tag)::value;
             const float *__restrict__ residual = e.residual_f32; // never aliases the output rows
-            uint16_t *__restrict__ out16 = static_cast<uint16_t *>(a.out);
+            uint16_t *out16 = static_cast<uint16_t *>(a.out);
             const size_t slot_stride = size_t(a.owned_passes) * kPassBytes;
 #pragma unroll 2
             for (int local_pass = 0;; ++local_pass) {
@@ -488,6 +569,10 @@ w8a8_tcgen05_gemm(const __grid_constant__ CUtensorMap map_w, const __grid_consta
 #pragma unroll
                     for (int i = 0; i < 8; ++i) r8[i] = first_residual[i];
                 }
+                uint4 skip16 = first_skip;
+                if (kChain && e.residual && local_pass > 0)
+                    skip16 = *reinterpret_cast<const uint4 *>(static_cast<const uint16_t *>(e.residual) +
+                                                              size_t(m0 + c) * e.residual_ld + n);
                 uint32_t raw[8];
                 if (splits == 1) {
                     const uint8_t *src = tiles_ptr + size_t(c * kBlockChannels + 8 * j) * 4;
@@ -515,14 +600,22 @@ w8a8_tcgen05_gemm(const __grid_constant__ CUtensorMap map_w, const __grid_consta
                     value[i] = Grouped ? acc : __fmul_rn(__fmul_rn(acc, scale_x), sw8[i]);
                     if (residual) value[i] = __fadd_rn(value[i], r8[i]);
                 }
-                uint4 packed;
-                {
-                    __nv_bfloat162 b0 = __floats2bfloat162_rn(value[0], value[1]), b1 = __floats2bfloat162_rn(value[2], value[3]);
-                    __nv_bfloat162 b2 = __floats2bfloat162_rn(value[4], value[5]), b3 = __floats2bfloat162_rn(value[6], value[7]);
-                    packed = make_uint4(*reinterpret_cast<uint32_t *>(&b0), *reinterpret_cast<uint32_t *>(&b1),
-                                        *reinterpret_cast<uint32_t *>(&b2), *reinterpret_cast<uint32_t *>(&b3));
+                uint4 packed = pack8x16<kF16>(value);
+                if (kChain) {
+                    packed = chain8<kF16>(e, packed, bias8, skip16);
+                    if (e.activation > 1) packed = activate8<kF16>(packed, e.activation, e.alpha);
                 }
                 *reinterpret_cast<uint4 *>(out16 + at) = packed;
+            }
+        };
+        if (ok && !*abort_ptr && columns_ok && lean) {
+            using std::bool_constant;
+            if (type == int(Type::F16)) {
+                if (e.chain) finish_rows(bool_constant<true>{}, bool_constant<true>{});
+                else finish_rows(bool_constant<true>{}, bool_constant<false>{});
+            } else {
+                if (e.chain) finish_rows(bool_constant<false>{}, bool_constant<true>{});
+                else finish_rows(bool_constant<false>{}, bool_constant<false>{});
             }
         } else if (ok && !*abort_ptr && columns_ok) {
             for (int local_pass = 0;; ++local_pass) {
@@ -589,16 +682,23 @@ w8a8_tcgen05_gemm(const __grid_constant__ CUtensorMap map_w, const __grid_consta
 #pragma unroll
                     for (int i = 0; i < 8; ++i) value[i] = __fadd_rn(value[i], r8[i]);
                 }
-                if (e.chain) {
+                const auto finish = [&](auto f16_tag) {
+                    constexpr bool kF16 = decltype(f16_tag)::value;
+                    uint4 row = pack8x16<kF16>(value);
+                    if (e.chain) {
+                        uint32_t skip[4] = {0u, 0u, 0u, 0u};
+                        if (e.residual) {
+                            const uint16_t *src = static_cast<const uint16_t *>(e.residual) + size_t(m) * e.residual_ld + n;
 #pragma unroll
-                    for (int i = 0; i < 8; ++i) {
-                        const float skip = e.residual ? load_as(e.residual, size_t(m) * e.residual_ld + n + i, type) : 0.f;
-                        value[i] = finish_chain(e, type, value[i], bias8[i], skip);
+                            for (int i = 0; i < 4; ++i) skip[i] = uint32_t(src[2 * i]) | (uint32_t(src[2 * i + 1]) << 16);
+                        }
+                        row = chain8<kF16>(e, row, bias8, make_uint4(skip[0], skip[1], skip[2], skip[3]));
+                        if (e.activation > 1) row = activate8<kF16>(row, e.activation, e.alpha);
                     }
-                }
+                    return row;
+                };
                 uint16_t *dst = static_cast<uint16_t *>(a.out) + at;
-                const uint4 packed = make_uint4(pack16(value[0], value[1], type), pack16(value[2], value[3], type),
-                                                pack16(value[4], value[5], type), pack16(value[6], value[7], type));
+                const uint4 packed = type == int(Type::F16) ? finish(std::true_type{}) : finish(std::false_type{});
                 if (a.vector_io) {
                     *reinterpret_cast<uint4 *>(dst) = packed;
                 } else {

@@ -23,7 +23,7 @@
 //             shared-memory patches as the per-row prefill kernel (coalesced 8-byte row stores).
 // Every wait is bounded; on expiry the CTA flags the status word and runs to the common exit.
 #pragma once
-#include "kernels/quant_prefill_sm100.cuh"
+#include "kernels/quant_linear_sm100.cuh"
 
 namespace tts::b200 {
 
@@ -32,8 +32,72 @@ constexpr int kGroupedAccumulators = 4;
 constexpr int kScaleSlots = 8;
 constexpr int kGroupedThreads = kGemmThreads + 32; // + the waiter warp
 constexpr int kScaleSlotBytes = 2 * kGroupedTokens * 4; // sx_g slice then sw_g slice of one K block
+constexpr int kPrefillPatchBytes = 2 * 2 * 16 * kBlockChannels * 2; // two chunk groups x two parities x [16][128] 16-bit
 constexpr size_t kGroupedSmem = 1024 + size_t(kGroupedStages) * (kBlockChannels + kGroupedTokens) * kBlockK +
                                 size_t(kScaleSlots) * kScaleSlotBytes + kPrefillPatchBytes;
+
+struct GroupedArgs {
+    int m, n, k;
+    const float *sx, *sw;
+    void *out;
+    int out_type; // Type::BF16 or Type::F16
+    const float *residual_f32;
+    int *status;
+};
+
+// One 16-token chunk of a tile's epilogue, executed by the four warps (one per tensor-memory lane
+// quadrant) that share a chunk. Phase 1, lane = channel: accumulator -> (acc*sx)*sw (+ fp32 residual)
+// -> 16-bit, written to a small shared-memory patch [token][channel]. After a 128-thread barrier,
+// phase 2, lane = four consecutive channels: every warp copies four token rows of the patch to
+// global memory as 8-byte stores, 256 contiguous bytes per row. The patch is double-buffered so one
+// barrier per chunk suffices. `r` holds the chunk's 16 accumulator words of this lane.
+template <bool kInt>
+__device__ __forceinline__ void prefill_store_chunk(const GroupedArgs &a, const uint32_t (&r)[16], const float *sx_chunk,
+                                                    float scale_w, const float *__restrict__ residual, int m_first,
+                                                    int n_tile0, int valid_rows, int quadrant, int lane, int group,
+                                                    uint16_t *patch /* [16][128] of this group and parity */) {
+    const int channel = quadrant * 32 + lane, n = n_tile0 + channel;
+    const bool bf16_out = a.out_type == int(Type::BF16);
+    // All loads (activation scales from shared memory, residuals from global memory) come first: a
+    // load may not be moved above an earlier store it might alias, so interleaving them with the patch
+    // stores would serialise sixteen round trips.
+    float scale_x[16], skip[16];
+    {
+        const float4 *sx4 = reinterpret_cast<const float4 *>(sx_chunk);
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+            const float4 v = sx4[q];
+            scale_x[4 * q] = v.x; scale_x[4 * q + 1] = v.y; scale_x[4 * q + 2] = v.z; scale_x[4 * q + 3] = v.w;
+        }
+    }
+#pragma unroll
+    for (int i = 0; i < 16; ++i)
+        skip[i] = (residual && n < a.n && i < valid_rows) ? __ldg(residual + size_t(m_first + i) * a.n + n) : 0.f;
+    uint16_t bits[16];
+#pragma unroll
+    for (int i = 0; i < 16; ++i) {
+        const float acc = kInt ? float(int(r[i])) : __uint_as_float(r[i]);
+        float value = __fmul_rn(__fmul_rn(acc, scale_x[i]), scale_w);
+        if (residual) value = __fadd_rn(value, skip[i]);
+        if (bf16_out) { __nv_bfloat16 b = __float2bfloat16_rn(value); bits[i] = *reinterpret_cast<uint16_t *>(&b); }
+        else { __half h = __float2half_rn(value); bits[i] = *reinterpret_cast<uint16_t *>(&h); }
+    }
+#pragma unroll
+    for (int i = 0; i < 16; ++i) patch[i * kBlockChannels + channel] = bits[i];
+    if (group == 0) asm volatile("bar.sync 2, 128;" ::: "memory");
+    else asm volatile("bar.sync 3, 128;" ::: "memory");
+    const int n4 = n_tile0 + lane * 4;
+    if (n4 < a.n) {
+#pragma unroll
+        for (int rr = 0; rr < 4; ++rr) {
+            const int i = quadrant * 4 + rr;
+            if (i < valid_rows) {
+                const uint2 four = *reinterpret_cast<const uint2 *>(patch + i * kBlockChannels + lane * 4);
+                *reinterpret_cast<uint2 *>(static_cast<uint16_t *>(a.out) + size_t(m_first + i) * a.n + n4) = four;
+            }
+        }
+    }
+}
 
 namespace ptx {
 // Two fp32 lanes in one 64-bit register, and the packed arithmetic Blackwell has for them.
@@ -66,7 +130,7 @@ template <Type F>
 __global__ void __launch_bounds__(kGroupedThreads, 1)
 w8a8_tcgen05_prefill_grouped(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_x,
                              const __grid_constant__ CUtensorMap map_sw, const __grid_constant__ CUtensorMap map_sx,
-                             const __grid_constant__ PrefillArgs a) {
+                             const __grid_constant__ GroupedArgs a) {
     constexpr bool kInt = F == Type::I8;
     constexpr int BN = kGroupedTokens;
     constexpr int kWeightBytes = kBlockChannels * kBlockK, kTokenBytes = BN * kBlockK;
@@ -86,7 +150,7 @@ w8a8_tcgen05_prefill_grouped(const __grid_constant__ CUtensorMap map_w, const __
     const uint32_t raw_base = ptx::smem_u32(dynamic_smem);
     const uint32_t tiles_base = (raw_base + 1023u) & ~1023u;
     uint8_t *aligned = dynamic_smem + (tiles_base - raw_base);
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int warp = ptx::warp_index(), lane = threadIdx.x & 31;
     const int n_tiles = (a.n + kBlockChannels - 1) / kBlockChannels, m_tiles = (a.m + BN - 1) / BN;
     const int tiles = n_tiles * m_tiles;
     const int kb_count = (a.k + kBlockK - 1) / kBlockK;
@@ -113,39 +177,45 @@ w8a8_tcgen05_prefill_grouped(const __grid_constant__ CUtensorMap map_w, const __
     ptx::tcgen05_fence_before();
     __syncthreads();
     ptx::tcgen05_fence_after();
-    const uint32_t tmem_base = tmem_slot;
+    const uint32_t tmem_base = ptx::warp_uniform(tmem_slot);
     volatile int *abort_ptr = &abort_flag;
     ptx::launch_dependents();
 
     if (warp == 0) {
         // ------------------------------------------------------------ TMA producer
-        if (lane == 0) {
+        // The whole warp runs the loop so that addresses and coordinates stay warp-uniform; one elected lane issues.
+        if (ptx::elect_one()) {
             ptx::prefetch_tensormap(&map_w);
             ptx::prefetch_tensormap(&map_x);
             ptx::prefetch_tensormap(&map_sw);
             ptx::prefetch_tensormap(&map_sx);
-            ptx::wait_for_upstream();
-            int stage = 0, slot = 0;
-            uint32_t phase = 0, slot_phase = 0;
-            bool ok = true;
-            for (int tile = blockIdx.x; tile < tiles && ok; tile += gridDim.x) {
-                const int n0 = (tile % n_tiles) * kBlockChannels, m0 = (tile / n_tiles) * BN;
-                for (int kb = 0; kb < kb_count; ++kb) {
-                    if (!ptx::mbar_wait(ptx::smem_u32(&scale_empty[slot]), slot_phase ^ 1u, abort_ptr)) { ok = false; break; }
-                    const uint32_t scale_bar = ptx::smem_u32(&scale_full[slot]);
-                    const uint32_t scale_dst = tiles_base + kRingBytes + uint32_t(slot) * kScaleSlotBytes;
-                    ptx::mbar_arrive_expect_tx(scale_bar, kScaleSlotBytes);
-                    ptx::tma_load_2d(scale_dst, &map_sx, scale_bar, m0, kb);
-                    ptx::tma_load_2d(scale_dst + BN * 4, &map_sw, scale_bar, n0, kb);
-                    if (++slot == kScaleSlots) { slot = 0; slot_phase ^= 1u; }
-                    if (!ptx::mbar_wait(ptx::smem_u32(&empty_bar[stage]), phase ^ 1u, abort_ptr)) { ok = false; break; }
-                    const uint32_t bar = ptx::smem_u32(&full_bar[stage]);
-                    const uint32_t dst = tiles_base + uint32_t(stage) * kStageBytes;
+        }
+        ptx::wait_for_upstream();
+        int stage = 0, slot = 0;
+        uint32_t phase = 0, slot_phase = 0;
+        bool ok = true;
+        for (int tile = blockIdx.x; tile < tiles && ok; tile += gridDim.x) {
+            const int n0 = (tile % n_tiles) * kBlockChannels, m0 = (tile / n_tiles) * BN;
+            for (int kb = 0; kb < kb_count; ++kb) {
+                ok = ptx::mbar_wait(ptx::smem_u32(&scale_empty[slot]), slot_phase ^ 1u, abort_ptr) &&
+                     ptx::mbar_wait(ptx::smem_u32(&empty_bar[stage]), phase ^ 1u, abort_ptr);
+                ok = __all_sync(0xffffffffu, ok);
+                if (!ok) break;
+                const uint32_t scale_bar = ptx::smem_u32(&scale_full[slot]);
+                const uint32_t scale_dst = tiles_base + kRingBytes + uint32_t(slot) * kScaleSlotBytes;
+                const uint32_t bar = ptx::smem_u32(&full_bar[stage]);
+                const uint32_t dst = tiles_base + uint32_t(stage) * kStageBytes;
+                if (ptx::elect_one()) {
                     ptx::mbar_arrive_expect_tx(bar, kStageBytes);
                     ptx::tma_load_2d(dst, &map_w, bar, kb * kBlockK, n0);
                     ptx::tma_load_2d(dst + kWeightBytes, &map_x, bar, kb * kBlockK, m0);
-                    if (++stage == kGroupedStages) { stage = 0; phase ^= 1u; }
+                    ptx::mbar_arrive_expect_tx(scale_bar, kScaleSlotBytes);
+                    ptx::tma_load_2d(scale_dst, &map_sx, scale_bar, m0, kb);
+                    ptx::tma_load_2d(scale_dst + BN * 4, &map_sw, scale_bar, n0, kb);
                 }
+                __syncwarp();
+                if (++slot == kScaleSlots) { slot = 0; slot_phase ^= 1u; }
+                if (++stage == kGroupedStages) { stage = 0; phase ^= 1u; }
             }
         }
     } else if (warp == 1 || warp == 10) {

@@ -14,11 +14,11 @@ Buffer make_workspace(int device, void *pointer, size_t bytes) {
 
 CudaContext::CudaContext(int ordinal, Quantization requested, cudaStream_t s, void *workspace, size_t bytes)
     : device(ordinal), stream(s), gemm_workspace(make_workspace(ordinal, workspace, bytes)), mode(requested) {
-    cudaDeviceProp p{};
-    if (cudaGetDeviceProperties(&p, device) != cudaSuccess) throw std::runtime_error("cudaGetDeviceProperties failed");
-    multiprocessors = p.multiProcessorCount;
-    sm_major = p.major;
-    sm_minor = p.minor;
+    // Single attributes: cudaGetDeviceProperties takes over a millisecond.
+    if (cudaDeviceGetAttribute(&multiprocessors, cudaDevAttrMultiProcessorCount, device) != cudaSuccess ||
+        cudaDeviceGetAttribute(&sm_major, cudaDevAttrComputeCapabilityMajor, device) != cudaSuccess ||
+        cudaDeviceGetAttribute(&sm_minor, cudaDevAttrComputeCapabilityMinor, device) != cudaSuccess)
+        throw std::runtime_error("cudaDeviceGetAttribute failed");
     int clusters = 0;
     cudaDeviceGetAttribute(&clusters, cudaDevAttrClusterLaunch, device);
     quant_gated_clusters = clusters != 0;

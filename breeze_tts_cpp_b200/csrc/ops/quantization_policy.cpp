@@ -60,6 +60,13 @@ std::vector<LinearPath> quant_linear_candidates(KernelProblem p, KernelLimits li
     while (cover < (group ? kGroupedTokens : kPrefillTokens) && cover < p.rows) cover *= 2;
     std::vector<int> token_tiles{cover};
     if (group && cover == kGroupedTokens) token_tiles.push_back(64); // the split-K kernel's widest K-group tile below 128
+    // Between decode and prefill a batch covers a few narrow tiles: several of them per channel slab (and split K)
+    // occupy the machine where one or two 256-token tiles would leave most of it idle. Beyond 1024 rows the
+    // 256-token tiles fill it by themselves.
+    if (!group && p.rows > kWeightStreamTokens && p.rows <= 1024) {
+        token_tiles.push_back(64);
+        if (cover > 128) token_tiles.push_back(128);
+    }
     for (int tokens : token_tiles)
         for (int splits = 1; splits <= std::min(kb_total, kMaxSplits); ++splits) {
             const LaunchShape shape = launch_shape(tokens, group, blocks(kb_total, splits), splits,
@@ -76,19 +83,35 @@ double linear_cost(KernelProblem p, LinearPath path, Type, const ChipModel &chip
     const int kb_total = blocks(p.reduction, kBlockK);
     const double ops = 2.0 * p.rows * double(p.channels) * p.reduction;
     if (persistent_per_row(p, path)) {
-        // CTA pairs over 256x256 tiles (one CTA per 128x256 tile when N < 256); the tensor pipe
-        // sustains about two thirds of its issue rate, the last wave may be partly empty.
-        const bool pair = p.channels >= 2 * kBlockChannels;
-        const double tiles = double(blocks(p.channels, pair ? 2 * kBlockChannels : kBlockChannels)) * blocks(p.rows, kPrefillTokens);
-        const double workers = pair ? sms / 2 : sms;
-        const double waves = std::ceil(tiles / workers);
-        return chip.kernel_us + ops * (waves * workers / tiles) / (0.65 * chip.tensor_ops_per_us);
+        // CTA pairs: the same estimate the launcher picks the channel tile by, at 1965 MHz, plus launch and fill.
+        const PairTile tile = pair_channel_tile(p.rows, p.channels, kb_total, std::max(1, sms / 2), kPairColumnCycles);
+        return 1.8 + tile.cycles / 1965.;
     }
     if (persistent_grouped(p, path, sms)) {
         // Bound by the fp32 rescale of every K128 partial tile on the CUDA cores.
         const double tiles = double(blocks(p.channels, kBlockChannels)) * blocks(p.rows, kGroupedTokens);
         const double waves = std::ceil(tiles / sms);
         return chip.kernel_us + ops * (waves * sms / tiles) / (0.3 * chip.tensor_ops_per_us);
+    }
+    if (!grouped(p) && p.rows > kWeightStreamTokens) {
+        // Weight-streaming kernel with several token tiles per channel slab. Fitted to launches of 65 to 1024 rows on
+        // K = 512 to 6144, N = 1024 to 12288: a base per token tile, a slope per K block (the operand bytes one SM
+        // pulls), the split-K exchange, and contention for L2 as the grid grows. More than one wave does not pay:
+        // CTAs own their multiprocessor's shared memory, so nothing of the next wave overlaps.
+        const int splits = std::max(1, path.splits), per_split = blocks(kb_total, splits);
+        const LaunchShape shape = launch_shape(path.tokens, false, per_split, splits, 1);
+        if (!shape.fits) return std::numeric_limits<double>::infinity();
+        const int64_t ctas = int64_t(blocks(p.channels, kBlockChannels)) * blocks(p.rows, path.tokens) * splits;
+        const int resident = (path.tokens <= 64 && shape.smem <= 108 * 1024) ? 2 : 1;
+        // Clusters are placed whole inside a GPC (16 to 20 multiprocessors): count what that leaves unusable.
+        const int64_t slots = std::max<int64_t>(splits, int64_t(sms) * resident * 16 / 18 / splits * splits);
+        const double base = path.tokens <= 64 ? 2.5 : path.tokens <= 128 ? 4.0 : 6.2;
+        const double slope = path.tokens <= 128 ? 0.214 : 0.42;
+        const double exchange = splits > 1 ? 0.3 + (path.tokens <= 64 ? 0.15 : 0.25) * splits : 0.0;
+        const double contention = 0.012 * double(std::max<int64_t>(0, std::min(ctas, slots) - 48));
+        const double waves = double((ctas + (splits > 1 ? slots : int64_t(sms) * resident) - 1) / (splits > 1 ? slots : int64_t(sms) * resident));
+        const double one = base + per_split * slope + exchange + contention;
+        return one + (waves - 1.0) * (one - 1.0);
     }
     // Weight-streaming kernel, as it runs inside a decoder chain: the launch starts under programmatic
     // dependent launch while its quantizer still runs, so by the time the activations exist the ring

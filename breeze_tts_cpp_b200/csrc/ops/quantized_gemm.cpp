@@ -63,11 +63,9 @@ QuantizedGemm::QuantizedGemm(cudaStream_t stream, void *, Buffer &workspace, Typ
     : impl(new Impl{stream, format, workspace}) {
     if (format != Type::FP8 && format != Type::I8) throw std::invalid_argument("unsupported quantized storage type");
     quant_linear_initialize(workspace.device());
-    cudaDeviceProp p{};
-    if (cudaGetDeviceProperties(&p, workspace.device()) != cudaSuccess)
-        throw std::runtime_error("cudaGetDeviceProperties failed");
-    impl->multiprocessors = p.multiProcessorCount;
-    impl->chip = ChipModel::b200(p.multiProcessorCount);
+    if (cudaDeviceGetAttribute(&impl->multiprocessors, cudaDevAttrMultiProcessorCount, workspace.device()) != cudaSuccess)
+        throw std::runtime_error("cudaDeviceGetAttribute failed");
+    impl->chip = ChipModel::b200(impl->multiprocessors);
     quant_linear_reset_workspace(workspace.data(), workspace.size(), stream);
 }
 QuantizedGemm::~QuantizedGemm() = default;
