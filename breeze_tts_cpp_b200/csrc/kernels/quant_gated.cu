@@ -8,7 +8,7 @@
 // In K-group mode the 2048-column slabs of one row are independent and are spread over several
 // CTAs for short batches; with one scale per row the CTA holds the whole row (K <= 8192).
 #include "kernels/quant_gated.h"
-#include "kernels/quant_codec.cuh"
+#include "kernels/quant_blocks.cuh"
 #include "kernels/launch.cuh"
 #include <stdexcept>
 #include <string>
@@ -52,6 +52,23 @@ gated_quantize(const T *__restrict__ input, unsigned char *__restrict__ out, flo
                 raw_up[j] = *reinterpret_cast<const uint4 *>(up + column);
             }
         }
+        if (!Rotate && !group) { // parts == 1: the row stays in packed storage precision
+            uint4 product[Items];
+#pragma unroll
+            for (int j = 0; j < Items; ++j) {
+                const uint32_t *g = reinterpret_cast<const uint32_t *>(&raw_gate[j]), *u = reinterpret_cast<const uint32_t *>(&raw_up[j]);
+                uint32_t *p = reinterpret_cast<uint32_t *>(&product[j]);
+#pragma unroll
+                for (int i = 0; i < 4; ++i) {
+                    const float2 f = unpack_f32x2(widen2<T>(g[i]));
+                    // The packed multiply rounds the exact product once, as the fp32 product rounded to storage does.
+                    p[i] = mul16x2<T>(Packed16<T>::pack(gate_activation<Kind>(f.x), gate_activation<Kind>(f.y)), u[i]);
+                }
+            }
+            quantize_row_packed<F, T, kThreads, Items>(product, out + size_t(row) * cols, scales + row, cols,
+                                                       reinterpret_cast<uint32_t *>(slots));
+            return;
+        }
 #pragma unroll
         for (int j = 0; j < Items; ++j) {
             float g[8], u[8];
@@ -82,10 +99,47 @@ gated_quantize(const T *__restrict__ input, unsigned char *__restrict__ out, flo
     quantize_tail<F, kThreads, Items, Rotate>(v, out, scales, row, rows, cols, group, shard, parts, aligned, slots);
 }
 
+// K-group mode with rotation: the blocks of all rows in one list (see row_quantize_blocks), four lanes per block, each
+// gating its 32 columns in packed storage precision before the shared rotate-and-quantize step.
+template <Type F, class T, int Kind>
+__global__ void __launch_bounds__(kThreads, 3)
+gated_quantize_blocks(const T *__restrict__ input, unsigned char *__restrict__ out, float *__restrict__ scales, int rows, int cols,
+                      int blocks) {
+    pdl_launch_dependents();
+    const int first = (int(blockIdx.x) * int(blockDim.x >> 5) + int(threadIdx.x >> 5)) * 8;
+    const int block = first + (int(threadIdx.x & 31) >> 2);
+    const bool active = block < blocks;
+    const int group = active ? block / rows : 0, row = active ? block - group * rows : 0;
+    const int column = group * 128 + int(threadIdx.x & 3) * 32;
+    uint32_t mask[16], raw[16], up[16];
+    load_masks(column, mask); // static: may precede the wait
+    pdl_wait_upstream();
+    if (first >= blocks) return;
+    const T *gate = input + size_t(row) * cols * 2 + column;
+    load_row32(gate, raw);
+    load_row32(gate + cols, up);
+#pragma unroll
+    for (int i = 0; i < 16; ++i) {
+        const float2 g = unpack_f32x2(widen2<T>(raw[i]));
+        // The packed multiply rounds the exact product once, as the fp32 product rounded to storage does.
+        raw[i] = mul16x2<T>(Packed16<T>::pack(gate_activation<Kind>(g.x), gate_activation<Kind>(g.y)), up[i]) ^ mask[i];
+    }
+    rotate_quantize32<F, T>(raw, out + size_t(row) * cols + column, scales + block, active);
+}
+
 template <Type F, class T, int Kind, bool Rotate>
 void launch_items(const T *x, unsigned char *q, float *s, int rows, int cols, int group, int sms, cudaStream_t stream) {
     const bool aligned = cols % 8 == 0 && reinterpret_cast<uintptr_t>(x) % 16 == 0 && reinterpret_cast<uintptr_t>(q) % 8 == 0;
     const int chunks = (cols + kThreads * 8 - 1) / (kThreads * 8);
+    if (Rotate && group == 128 && cols % 128 == 0 && reinterpret_cast<uintptr_t>(x) % 32 == 0 &&
+        reinterpret_cast<uintptr_t>(q) % 32 == 0 && int64_t(rows) * (cols / 128) < INT32_MAX - 4096) {
+        const int blocks = rows * (cols / 128);
+        const int threads = blocks >= 8 * (kThreads / 32) * sms ? kThreads : 64;
+        const int per_cta = 8 * (threads / 32);
+        launch_pdl("quantized gated launch", gated_quantize_blocks<F, T, Kind>, dim3(unsigned((blocks + per_cta - 1) / per_cta)),
+                   dim3(unsigned(threads)), 0, stream, x, q, s, rows, cols, blocks);
+        return;
+    }
     // K-group slabs of a row are independent, so short batches spread them over several CTAs. With
     // one scale per row the CTA keeps the whole row: joining CTAs through a cluster barrier was
     // measured slower than the three 128-bit loads per thread it saves.

@@ -8,7 +8,7 @@
 // thread over its four pairs, then a shuffle-down tree per warp, then serially over the eight
 // warps; the norm uses the hardware reciprocal square root. Compile with --fmad=false.
 #include "kernels/quant_norm.h"
-#include "kernels/quant_codec.cuh"
+#include "kernels/quant_blocks.cuh"
 #include "kernels/launch.cuh"
 #include <stdexcept>
 #include <string>
@@ -97,6 +97,21 @@ rms_quantize(T *__restrict__ x, const T *__restrict__ update, const T *__restric
     float v[1][8];
     {
         const P *vp = reinterpret_cast<const P *>(&value), *wp = reinterpret_cast<const P *>(&w);
+        if (!Rotate && !group && aligned) { // the normalized row stays in packed storage precision
+            uint4 row_words[1];
+            P *np = reinterpret_cast<P *>(&row_words[0]);
+#pragma unroll
+            for (int p = 0; p < 4; ++p) {
+                const float2 f = M::unpack(vp[p]), wf = M::unpack(wp[p]);
+                np[p] = gemma ? M::pack(__fmul_rn(__fmul_rn(f.x, inv_norm), __fadd_rn(wf.x, 1.f)),
+                                        __fmul_rn(__fmul_rn(f.y, inv_norm), __fadd_rn(wf.y, 1.f)))
+                              : __hmul2(M::pack(__fmul_rn(f.x, inv_norm), __fmul_rn(f.y, inv_norm)), wp[p]);
+            }
+            if (column >= cols) row_words[0] = make_uint4(0, 0, 0, 0);
+            quantize_row_packed<F, T, kThreads, 1>(row_words, out + size_t(row) * cols, scales + row, cols,
+                                                   reinterpret_cast<uint32_t *>(slots));
+            return;
+        }
 #pragma unroll
         for (int p = 0; p < 4; ++p) {
             float2 f = M::unpack(vp[p]);
@@ -116,6 +131,82 @@ rms_quantize(T *__restrict__ x, const T *__restrict__ update, const T *__restric
     quantize_tail<F, kThreads, 1, Rotate>(v, out, scales, row, rows, cols, group, 0, 1, aligned, slots);
 }
 
+// K-group mode with rotation: 64 threads per row, 32 consecutive columns each, so that four lanes hold a block for the
+// shared rotate-and-quantize step; one to four rows per CTA. The squares are added up in the order of rms_quantize: a
+// lane's 32 columns are four of that kernel's threads (eight columns each, summed alike), its shuffle distances 16, 8 and
+// 4 are lane distances 4, 2 and 1 here and 2 and 1 fall inside a lane; the eight warp sums are added in order.
+template <Type F, class T, bool Add>
+__global__ void __launch_bounds__(kThreads)
+rms_quantize_blocks(T *__restrict__ x, const T *__restrict__ update, const T *__restrict__ weight, const T *__restrict__ update_scale,
+                    unsigned char *__restrict__ out, float *__restrict__ scales, int rows, int cols, float eps, bool gemma) {
+    __shared__ float slots[kThreads / 64][8];
+    pdl_launch_dependents();
+    const int slot = int(threadIdx.x) / 64, lane = int(threadIdx.x) % 64;
+    const int row = int(blockIdx.x) * int(blockDim.x / 64) + slot, column = lane * 32;
+    const bool active = row < rows && column < cols;
+    uint32_t mask[16], w[16], value[16];
+    if (active) { // static: may precede the wait
+        load_masks(column, mask);
+        load_row32(weight + column, w);
+    } else {
+#pragma unroll
+        for (int i = 0; i < 16; ++i) mask[i] = w[i] = 0u;
+    }
+#pragma unroll
+    for (int i = 0; i < 16; ++i) value[i] = 0u;
+    pdl_wait_upstream();
+    T *mine = x + size_t(row) * cols + column;
+    if (active) {
+        load_row32(mine, value);
+        if (Add) {
+            uint32_t u[16];
+            load_row32(update + size_t(row) * cols + column, u);
+            if (update_scale) {
+                uint32_t s[16];
+                load_row32(update_scale + column, s);
+#pragma unroll
+                for (int i = 0; i < 16; ++i) u[i] = mul16x2<T>(u[i], s[i]);
+            }
+#pragma unroll
+            for (int i = 0; i < 16; ++i) value[i] = add16x2<T>(value[i], u[i]);
+            store_row32(mine, value);
+        }
+    }
+    float sum[4];
+#pragma unroll
+    for (int t = 0; t < 4; ++t) {
+        sum[t] = 0.f;
+#pragma unroll
+        for (int p = 0; p < 4; ++p) {
+            const float2 f = unpack_f32x2(widen2<T>(value[4 * t + p]));
+            sum[t] = __fadd_rn(sum[t], __fadd_rn(__fmul_rn(f.x, f.x), __fmul_rn(f.y, f.y)));
+        }
+    }
+#pragma unroll
+    for (int d = 4; d; d >>= 1)
+#pragma unroll
+        for (int t = 0; t < 4; ++t) sum[t] = __fadd_rn(sum[t], __shfl_down_sync(0xffffffffu, sum[t], d));
+    if (!(lane & 7)) slots[slot][lane >> 3] = __fadd_rn(__fadd_rn(sum[0], sum[2]), __fadd_rn(sum[1], sum[3]));
+    __syncthreads();
+    float total = 0.f;
+#pragma unroll
+    for (int p = 0; p < 8; ++p) total = __fadd_rn(total, slots[slot][p]);
+    const float inv_norm = rsqrtf(__fadd_rn(__fdiv_rn(total, float(cols)), eps));
+#pragma unroll
+    for (int i = 0; i < 16; ++i) {
+        const float2 f = unpack_f32x2(widen2<T>(value[i]));
+        if (gemma) {
+            const float2 wf = unpack_f32x2(widen2<T>(w[i]));
+            value[i] = Packed16<T>::pack(__fmul_rn(__fmul_rn(f.x, inv_norm), __fadd_rn(wf.x, 1.f)),
+                                         __fmul_rn(__fmul_rn(f.y, inv_norm), __fadd_rn(wf.y, 1.f)));
+        } else {
+            value[i] = mul16x2<T>(Packed16<T>::pack(__fmul_rn(f.x, inv_norm), __fmul_rn(f.y, inv_norm)), w[i]);
+        }
+        value[i] ^= mask[i];
+    }
+    rotate_quantize32<F, T>(value, out + size_t(row) * cols + column, scales + size_t(column / 128) * rows + row, active);
+}
+
 template <Type F, class T>
 void launch(T *x, const T *update, const T *weight, const T *update_scale, unsigned char *q, float *s, int rows,
             int cols, float eps, bool gemma, int group, int rotation, cudaStream_t stream) {
@@ -123,6 +214,20 @@ void launch(T *x, const T *update, const T *weight, const T *update_scale, unsig
                          reinterpret_cast<uintptr_t>(weight) % 16 == 0 && reinterpret_cast<uintptr_t>(q) % 8 == 0 &&
                          (!update || reinterpret_cast<uintptr_t>(update) % 16 == 0) &&
                          (!update_scale || reinterpret_cast<uintptr_t>(update_scale) % 16 == 0);
+    const auto aligned32 = [](const void *p) { return reinterpret_cast<uintptr_t>(p) % 32 == 0; };
+    if (rotation && group == 128 && cols % 128 == 0 && aligned32(x) && aligned32(weight) && aligned32(q) && aligned32(update) &&
+        aligned32(update_scale)) {
+        // Four rows per CTA once that still leaves every multiprocessor one.
+        const int per_cta = rows >= 4 * 148 ? 4 : rows >= 2 * 148 ? 2 : 1;
+        const dim3 grid(unsigned((rows + per_cta - 1) / per_cta)), block(unsigned(64 * per_cta));
+        if (update)
+            launch_pdl("quantized norm launch", rms_quantize_blocks<F, T, true>, grid, block, 0, stream, x, update, weight, update_scale, q,
+                       s, rows, cols, eps, gemma);
+        else
+            launch_pdl("quantized norm launch", rms_quantize_blocks<F, T, false>, grid, block, 0, stream, x, update, weight, update_scale,
+                       q, s, rows, cols, eps, gemma);
+        return;
+    }
 #define B200Q_RUN(ADD, ROT)                                                                        \
     launch_pdl("quantized norm launch", rms_quantize<F, T, ADD, ROT>, dim3(rows), dim3(kThreads), 0, stream, x, update,   \
                weight, update_scale, q, s, rows, cols, eps, gemma, group, aligned)

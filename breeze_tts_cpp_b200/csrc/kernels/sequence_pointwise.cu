@@ -111,7 +111,10 @@ pointwise_finish(const T *__restrict__ x, int x_rows, int x_stride, T *y, int y_
     const int packets = (cols + 7) / 8;
     const int64_t index = int64_t(blockIdx.x) * kThreads + threadIdx.x;
     if (index >= int64_t(rows) * packets) return;
-    const int row = int(index / packets), col = int(index % packets) * 8, remaining = cols - col;
+    // A 64-bit division costs more than the rest of a packet's work; only batches past 2^32 packets need one.
+    const bool narrow = int64_t(rows) * packets <= int64_t(0xffffffffu);
+    const int row = narrow ? int(unsigned(index) / unsigned(packets)) : int(index / packets);
+    const int col = int(index - int64_t(row) * packets) * 8, remaining = cols - col;
     float in[8], out[8];
     input8(x, x_rows, x_stride, row / repeat, col, remaining, in);
     const FinishRow r = finish_row(f, row);

@@ -33,6 +33,7 @@ class QuantizationWorkspace {
         values_ = Buffer(size_t(rows) * capacity.columns);
         scales_ = Buffer(size_t(rows) * capacity.scales_per_row * sizeof(float));
     }
+    int rows() const { return rows_; }
     RowScaledView view(int rows, int columns, Type format, QuantizationGroups layout) const {
         auto need = Capacity::matrix(columns, layout.activation);
         if (rows < 1 || rows > rows_ || columns < 1 || columns > capacity_.columns ||
