@@ -58,15 +58,15 @@ CUtensorMap operand_map(const void *base, int rows, int k, int box_rows, bool we
     return map;
 }
 
-// Group-major fp32 scales [K/128, rows]: box = 128 consecutive rows of one K group, no swizzle,
+// Group-major fp32 scales [K/128, rows]: box = `box_rows` consecutive rows of one K group, no swizzle,
 // rows past the end read as zero.
-CUtensorMap scale_map(const float *base, int rows, int groups) {
+CUtensorMap scale_map(const float *base, int rows, int groups, int box_rows) {
     if (reinterpret_cast<uintptr_t>(base) % 16 || rows % 4)
         throw std::invalid_argument("K-group scales must be 16-byte aligned with a row count that is a multiple of 4");
     CUtensorMap map;
     cuuint64_t dims[2] = {cuuint64_t(rows), cuuint64_t(groups)};
     cuuint64_t strides[1] = {cuuint64_t(rows) * 4};
-    cuuint32_t box[2] = {cuuint32_t(kGroupedTokens), 1};
+    cuuint32_t box[2] = {cuuint32_t(box_rows), 1};
     cuuint32_t element_strides[2] = {1, 1};
     CUresult status = encode_tiled()(&map, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 2, const_cast<float *>(base), dims, strides,
                                      box, element_strides, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE,
@@ -98,7 +98,7 @@ void launch_instance(const CUtensorMap &map_w, const CUtensorMap &map_x, const G
                      size_t smem, cudaStream_t stream) {
     cudaLaunchConfig_t config{};
     config.gridDim = grid;
-    config.blockDim = dim3(kGemmThreads);
+    config.blockDim = dim3(kStreamThreads<Grouped>);
     config.dynamicSmemBytes = smem;
     config.stream = stream;
     cudaLaunchAttribute attributes[2];
@@ -173,28 +173,41 @@ void launch_prefill_pair(const CUtensorMap &map_w, const CUtensorMap &map_x, con
     check(cudaLaunchKernelEx(&config, kernel, map_w, map_x, map_out, map_residual, args), "quantized pair GEMM launch");
 }
 
-// Persistent K-group kernel: one CTA per multiprocessor over 128x128 tiles.
+// Persistent K-group kernel: one CTA per multiprocessor over tiles of 128 tokens x `channels` output channels.
+template <Type F, int Channels>
+auto *grouped_kernel(bool chain, bool f16) {
+    return chain ? (f16 ? w8a8_tcgen05_prefill_grouped<F, Channels, true, true> : w8a8_tcgen05_prefill_grouped<F, Channels, true, false>)
+                 : (f16 ? w8a8_tcgen05_prefill_grouped<F, Channels, false, true> : w8a8_tcgen05_prefill_grouped<F, Channels, false, false>);
+}
 template <Type F>
-void launch_prefill_grouped(const CUtensorMap &map_w, const CUtensorMap &map_x, const CUtensorMap &map_sw,
-                            const CUtensorMap &map_sx, const GroupedArgs &args, cudaStream_t stream) {
-    const int tiles = ((args.n + kBlockChannels - 1) / kBlockChannels) * ((args.m + kGroupedTokens - 1) / kGroupedTokens);
+void launch_prefill_grouped(int channels, const CUtensorMap &map_w, const CUtensorMap &map_x, const CUtensorMap &map_sw,
+                            const CUtensorMap &map_out, const CUtensorMap &map_residual, const GroupedArgs &args, Type output_type,
+                            cudaStream_t stream) {
+    const int tiles = ((args.n + channels - 1) / channels) * ((args.m + kGroupedTokens - 1) / kGroupedTokens);
     cudaLaunchConfig_t config{};
     config.gridDim = dim3(unsigned(std::min(tiles, multiprocessor_count())));
     config.blockDim = dim3(kGroupedThreads);
-    config.dynamicSmemBytes = kGroupedSmem;
+    config.dynamicSmemBytes = grouped_smem(channels);
     config.stream = stream;
     cudaLaunchAttribute attribute{};
     attribute.id = cudaLaunchAttributeProgrammaticStreamSerialization;
     attribute.val.programmaticStreamSerializationAllowed = 1;
     config.attrs = &attribute;
     config.numAttrs = 1;
-    check(cudaLaunchKernelEx(&config, w8a8_tcgen05_prefill_grouped<F>, map_w, map_x, map_sw, map_sx, args),
+    const bool chain = args.ep.chain, f16 = output_type == Type::F16;
+    check(cudaLaunchKernelEx(&config, channels == 64 ? grouped_kernel<F, 64>(chain, f16) : grouped_kernel<F, 128>(chain, f16), map_w, map_x,
+                             map_sw, map_out, map_residual, args),
           "quantized K-group prefill GEMM launch");
 }
 
 template <Type F> void raise_limits() {
-    check(cudaFuncSetAttribute(w8a8_tcgen05_prefill_grouped<F>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(kGroupedSmem)),
-          "cudaFuncSetAttribute(shared memory)");
+    for (bool chain : {false, true})
+        for (bool f16 : {false, true}) {
+            check(cudaFuncSetAttribute(grouped_kernel<F, 64>(chain, f16), cudaFuncAttributeMaxDynamicSharedMemorySize, int(grouped_smem(64))),
+                  "cudaFuncSetAttribute(shared memory)");
+            check(cudaFuncSetAttribute(grouped_kernel<F, 128>(chain, f16), cudaFuncAttributeMaxDynamicSharedMemorySize, int(grouped_smem(128))),
+                  "cudaFuncSetAttribute(shared memory)");
+        }
     for (auto *kernel : {w8a8_tcgen05_prefill_pair<F, false, false>, w8a8_tcgen05_prefill_pair<F, false, true>,
                          w8a8_tcgen05_prefill_pair<F, true, false>, w8a8_tcgen05_prefill_pair<F, true, true>})
         check(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(kPairSmem)),
@@ -346,25 +359,28 @@ void launch_quant_linear(LinearPath config, KernelProblem shape, const void *inp
         else launch_prefill_pair<Type::FP8>(map_half, map_x, map_out, map_residual, pair, output_type, stream);
         return;
     }
+    // K-group shapes beyond decode (both operands grouped by 128, no split) take the persistent K-group kernel.
+    if (grouped && shape.input_group == kBlockK && shape.weight_group == kBlockK && bn == kGroupedTokens && splits == 1 &&
+        args.vector_io && aligned16(ws) && (!args.ep.residual || args.ep.residual_vector)) {
+        GroupedArgs group{args.m, args.n, args.k, xs, args.ep.residual_f32, args.status};
+        group.ep = args.ep;
+        const int channels = grouped_channel_tile(shape.rows, shape.channels, multiprocessor_count());
+        const CUtensorMap map_weights = operand_map(weights, shape.channels, shape.reduction, channels, true);
+        const CUtensorMap map_x = operand_map(input, shape.rows, shape.reduction, kGroupedTokens, false);
+        const CUtensorMap map_sw = scale_map(ws, shape.channels, kb_total, channels);
+        const CUtensorMap map_out = slab_map(y, shape.rows, shape.channels, shape.channels, output_type);
+        const CUtensorMap map_residual = args.ep.residual ? slab_map(args.ep.residual, shape.rows, shape.channels, args.ep.residual_ld, output_type)
+                                                          : map_out;
+        if (format == Type::I8) launch_prefill_grouped<Type::I8>(channels, map_weights, map_x, map_sw, map_out, map_residual, group, output_type, stream);
+        else launch_prefill_grouped<Type::FP8>(channels, map_weights, map_x, map_sw, map_out, map_residual, group, output_type, stream);
+        return;
+    }
     // The weight map is the caller's prepared one when it describes these weights, else built here.
     CUtensorMap local_w;
     const bool reuse = prepared && prepared->weights == weights && prepared->channels == shape.channels &&
                        prepared->reduction == shape.reduction;
     if (!reuse) local_w = operand_map(weights, shape.channels, shape.reduction, kBlockChannels, true);
     const CUtensorMap &map_w = reuse ? prepared->values : local_w;
-    // Compute-bound K-group shapes (both operands grouped by 128, enough 128x128 tiles to fill most of
-    // the GPU, plain epilogue, no split) take the persistent K-group kernel.
-    if (grouped && shape.input_group == kBlockK && shape.weight_group == kBlockK && bn == kGroupedTokens && splits == 1 &&
-        !args.ep.chain && args.vector_io && shape.rows % 4 == 0 &&
-        int64_t(n_tiles) * ((shape.rows + kGroupedTokens - 1) / kGroupedTokens) >= int64_t(multiprocessor_count()) * 2 / 3) {
-        GroupedArgs prefill{args.m, args.n, args.k, xs, ws, y, int(output_type), args.ep.residual_f32, args.status};
-        const CUtensorMap map_x = operand_map(input, shape.rows, shape.reduction, kGroupedTokens, false);
-        const CUtensorMap map_sw = scale_map(ws, shape.channels, kb_total);
-        const CUtensorMap map_sx = scale_map(xs, shape.rows, kb_total);
-        if (format == Type::I8) launch_prefill_grouped<Type::I8>(map_w, map_x, map_sw, map_sx, prefill, stream);
-        else launch_prefill_grouped<Type::FP8>(map_w, map_x, map_sw, map_sx, prefill, stream);
-        return;
-    }
     const CUtensorMap map_x = operand_map(input, shape.rows, shape.reduction, bn, false);
     LaunchShape launch = launch_shape(bn, grouped, (kb_total + splits - 1) / splits, splits,
                                       group_units(shape.input_group, shape.weight_group));

@@ -166,8 +166,13 @@ template <bool F16> __device__ __noinline__ uint4 activate8(uint4 row, int kind,
 template <bool F16> __device__ __forceinline__ uint4 pack8x16(const float (&v)[8]) {
     return make_uint4(pack2x16<F16>(v[0], v[1]), pack2x16<F16>(v[2], v[3]), pack2x16<F16>(v[4], v[5]), pack2x16<F16>(v[6], v[7]));
 }
+// The MMA issuer never tests an mbarrier for a refilled stage: the test waits behind the MMAs in flight (200 to 300 cycles per
+// K block). A waiter tests for it and hands the verdict over at a named hardware barrier. K-group mode has a warp of its own
+// for that, because its epilogue warps are busy; per-row mode uses the last epilogue warp, which is idle until the end.
+template <bool Grouped> constexpr int kStreamThreads = kGemmThreads + (Grouped ? 32 : 0);
+
 template <Type F, bool Grouped, int BN>
-__global__ void __launch_bounds__(kGemmThreads, (!Grouped && BN <= 64) ? 2 : 1)
+__global__ void __launch_bounds__(kStreamThreads<Grouped>, (!Grouped && BN <= 64) ? 2 : 1)
 w8a8_tcgen05_gemm(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_x,
                   const __grid_constant__ GemmArgs a) {
     constexpr bool kInt = F == Type::I8;
@@ -182,7 +187,6 @@ w8a8_tcgen05_gemm(const __grid_constant__ CUtensorMap map_w, const __grid_consta
                                       : kAccColumns <= 256 ? 256 : 512;
     constexpr uint32_t kIdesc = kInt ? ptx::idesc_i8(kBlockChannels, BN) : ptx::idesc_e4m3(kBlockChannels, BN);
     constexpr int kChunks = BN / 16;               // 16-token column chunks of the accumulator
-    constexpr int kMyChunks = (kChunks + 1) / 2;   // two epilogue warps share a lane quadrant
     constexpr uint32_t kPassBytes = kRowsPerPass * kBlockChannels * 4;
 
     extern __shared__ uint8_t dynamic_smem[];
@@ -238,6 +242,25 @@ w8a8_tcgen05_gemm(const __grid_constant__ CUtensorMap map_w, const __grid_consta
     ptx::tcgen05_fence_after();
     const uint32_t tmem_base = ptx::warp_uniform(tmem_slot);
     volatile int *abort_ptr = &abort_flag;
+    // K blocks whose MMAs go out in one burst: prefetched, and with an accumulator nobody used before. The others are waited for.
+    const int refill_from = Grouped ? min(min(a.stages, kb_count), kAccBuffers / units) : min(a.stages, kb_count);
+    const auto wait_for_refills = [&](bool ok, long long limit) {
+        int stage = refill_from == a.stages ? 0 : refill_from;
+        uint32_t phase = refill_from == a.stages ? 1u : 0u;
+        const int ahead = min(a.stages, kb_count);
+        // A parity test passes on a barrier whose phase before has not completed either: every phase has to be seen in turn.
+        if (refill_from < kb_count)
+            for (int i = 0; i < ahead && ok; ++i) ok = ptx::mbar_wait(ptx::smem_u32(&full_bar[i]), 0u, abort_ptr, limit);
+        for (int it = refill_from; it < kb_count; ++it) {
+            if (Grouped && it * units >= kAccBuffers) // the epilogue drained these accumulators' previous groups
+                for (int u = 0; u < units && ok; ++u)
+                    ok = ptx::mbar_wait(ptx::smem_u32(&acc_empty[(it * units + u) % kAccBuffers]),
+                                        (uint32_t((it * units + u) / kAccBuffers) & 1u) ^ 1u, abort_ptr, limit);
+            if (it >= ahead) ok = ok && ptx::mbar_wait(ptx::smem_u32(&full_bar[stage]), phase, abort_ptr, limit);
+            ok = ptx::pair_barrier_and(__all_sync(0xffffffffu, ok)); // the vote brings the lanes together for the aligned barrier
+            if (++stage == a.stages) { stage = 0; phase ^= 1u; }
+        }
+    };
     const long long wait_limit = a.wait_limit_cycles > 0 ? a.wait_limit_cycles : ptx::kWaitLimitCycles;
     // The next kernel in the stream may begin its own prologue; peers learn that this CTA is running.
     ptx::launch_dependents();
@@ -307,77 +330,69 @@ w8a8_tcgen05_gemm(const __grid_constant__ CUtensorMap map_w, const __grid_consta
             // (any shared-memory access between MMA issues stalls the issuing warp for a couple of
             // hundred cycles). Stage i holds K block i here; in K-group mode K block i also has
             // accumulator i to itself while fresh accumulators last.
-            // Narrow K groups: the MMAs of one 128-byte K block go to `units` accumulators, `unit_mmas`
-            // each; every accumulator reports on its own barrier.
-            auto issue_units = [&](uint32_t lo_w, uint32_t lo_x, uint32_t d_first, int buffer_first) {
-                for (int u = 0; u < units; ++u) {
-                    for (int s = 0; s < unit_mmas; ++s) {
-                        const uint32_t step = uint32_t(2 * (u * unit_mmas + s)); // 32 bytes of K = 2 descriptor units
-                        if (kInt) ptx::mma_i8_lo(d_first + uint32_t(u * BN), lo_w + step, lo_x + step, kIdesc, uint32_t(s > 0));
-                        else ptx::mma_f8_lo(d_first + uint32_t(u * BN), lo_w + step, lo_x + step, kIdesc, uint32_t(s > 0));
-                    }
-                    ptx::tcgen05_commit(ptx::smem_u32(&acc_full[buffer_first + u]));
-                }
-            };
-            int first = 0;
-            if (ok) {
-                const int burst = Grouped ? min(ahead, kAccBuffers / units) : ahead;
-                ptx::tcgen05_fence_after();
-                for (int it = 0; it < burst; ++it) {
-                    const uint32_t tile = tiles_base + uint32_t(it) * kStageBytes;
+            const int burst = refill_from; // min(ahead, K blocks with a fresh accumulator)
+            int stage = burst == a.stages ? 0 : burst;
+            if (!Grouped || units == 1) {
+                // One K block: four MMAs into its accumulator and its reports. A loop of its own: one that also served the
+                // narrow groups issued K-group blocks at half the rate.
+                const auto issue = [&](int it, int at, uint32_t buffer) {
+                    const uint32_t tile = tiles_base + uint32_t(at) * kStageBytes;
                     const uint32_t lo_w = ptx::smem_desc_lo_k128(tile), lo_x = ptx::smem_desc_lo_k128(tile + kWeightBytes);
-                    const uint32_t d = tmem_base + (Grouped ? uint32_t(it * units * BN) : 0u);
+                    const uint32_t d = tmem_base + buffer * uint32_t(BN), accumulate = Grouped ? 0u : uint32_t(it > 0);
                     if (ptx::elect_one()) {
-                        if (!Grouped || units == 1) {
-                            const uint32_t accumulate = Grouped ? 0u : uint32_t(it > 0);
-                            if (kInt) ptx::mma_i8_k128(d, lo_w, lo_x, kIdesc, accumulate);
-                            else ptx::mma_f8_k128(d, lo_w, lo_x, kIdesc, accumulate);
-                        } else {
-                            issue_units(lo_w, lo_x, d, it * units);
-                        }
-                        // Only a stage that will be refilled needs to report that its MMAs retired.
-                        if (it + a.stages < kb_count) ptx::tcgen05_commit(ptx::smem_u32(&empty_bar[it]));
-                        if (Grouped && units == 1) ptx::tcgen05_commit(ptx::smem_u32(&acc_full[it]));
-                    }
-                    __syncwarp();
-                }
-                first = burst;
-            }
-            int stage = first == a.stages ? 0 : first;
-            uint32_t phase = first == a.stages ? 1u : 0u;
-            // Refilled stages arrive at the rate memory delivers them, one barrier each.
-            for (int it = first; it < kb_count && ok; ++it) {
-                const int buffer = Grouped ? (it * units) % kAccBuffers : 0;
-                if (Grouped && it * units >= kAccBuffers) // the epilogue drained these accumulators' previous groups
-                    for (int u = 0; u < units && ok; ++u)
-                        ok = ptx::mbar_wait(ptx::smem_u32(&acc_empty[buffer + u]),
-                                            (uint32_t((it * units + u) / kAccBuffers) & 1u) ^ 1u, abort_ptr, wait_limit);
-                if (it >= ahead) ok = ok && ptx::mbar_wait(ptx::smem_u32(&full_bar[stage]), phase, abort_ptr, wait_limit);
-                ok = __all_sync(0xffffffffu, ok);
-                if (!ok) break;
-                ptx::tcgen05_fence_after();
-                const uint32_t tile = tiles_base + uint32_t(stage) * kStageBytes;
-                const uint32_t lo_w = ptx::smem_desc_lo_k128(tile), lo_x = ptx::smem_desc_lo_k128(tile + kWeightBytes);
-                const uint32_t d = tmem_base + uint32_t(buffer * BN);
-                if (ptx::elect_one()) {
-                    if (!Grouped || units == 1) {
-                        const uint32_t accumulate = Grouped ? 0u : uint32_t(it > 0);
                         if (kInt) ptx::mma_i8_k128(d, lo_w, lo_x, kIdesc, accumulate);
                         else ptx::mma_f8_k128(d, lo_w, lo_x, kIdesc, accumulate);
-                    } else {
-                        issue_units(lo_w, lo_x, d, buffer);
+                        // Only a stage that will be refilled needs to report that its MMAs retired.
+                        if (it + a.stages < kb_count) ptx::tcgen05_commit(ptx::smem_u32(&empty_bar[at]));
+                        if (Grouped) ptx::tcgen05_commit(ptx::smem_u32(&acc_full[buffer]));
                     }
-                    if (it + a.stages < kb_count) ptx::tcgen05_commit(ptx::smem_u32(&empty_bar[stage]));
-                    if (Grouped && units == 1) ptx::tcgen05_commit(ptx::smem_u32(&acc_full[buffer]));
+                    __syncwarp();
+                };
+                if (ok) {
+                    ptx::tcgen05_fence_after();
+                    for (int it = 0; it < burst; ++it) issue(it, it, Grouped ? uint32_t(it) : 0u);
                 }
-                __syncwarp();
-                if (++stage == a.stages) { stage = 0; phase ^= 1u; }
+                // Refilled stages arrive at the rate memory delivers them.
+                for (int it = burst; it < kb_count; ++it) {
+                    ok = ptx::pair_barrier_and(ok);
+                    ptx::tcgen05_fence_after();
+                    if (ok) issue(it, stage, Grouped ? uint32_t(it) % kAccBuffers : 0u);
+                    if (++stage == a.stages) stage = 0;
+                }
+            } else {
+                // Narrow K groups: the MMAs of one 128-byte K block go to `units` accumulators, `unit_mmas`
+                // each; every accumulator reports on its own barrier.
+                for (int it = 0; it < kb_count; ++it) {
+                    const int at = it < burst ? it : stage, buffer = (it * units) % kAccBuffers;
+                    if (it >= burst) ok = ptx::pair_barrier_and(ok);
+                    ptx::tcgen05_fence_after();
+                    const uint32_t tile = tiles_base + uint32_t(at) * kStageBytes;
+                    const uint32_t lo_w = ptx::smem_desc_lo_k128(tile), lo_x = ptx::smem_desc_lo_k128(tile + kWeightBytes);
+                    if (ok && ptx::elect_one()) {
+                        for (int u = 0; u < units; ++u) {
+                            const uint32_t d = tmem_base + uint32_t((buffer + u) * BN);
+                            for (int m = 0; m < unit_mmas; ++m) {
+                                const uint32_t step = uint32_t(2 * (u * unit_mmas + m)); // 32 bytes of K = 2 descriptor units
+                                if (kInt) ptx::mma_i8_lo(d, lo_w + step, lo_x + step, kIdesc, uint32_t(m > 0));
+                                else ptx::mma_f8_lo(d, lo_w + step, lo_x + step, kIdesc, uint32_t(m > 0));
+                            }
+                            ptx::tcgen05_commit(ptx::smem_u32(&acc_full[buffer + u]));
+                        }
+                        if (it + a.stages < kb_count) ptx::tcgen05_commit(ptx::smem_u32(&empty_bar[at]));
+                    }
+                    __syncwarp();
+                    if (it >= burst && ++stage == a.stages) stage = 0;
+                }
             }
             if (ptx::elect_one()) {
                 if (!Grouped) ptx::tcgen05_commit(ptx::smem_u32(&acc_full[0]));
             }
             __syncwarp();
         }
+        if (splits > 1) ptx::cluster_wait();
+    } else if (Grouped && warp == kGemmThreads / 32) {
+        // ------------------------------------------------------------ waiter (K-group mode)
+        wait_for_refills(true, wait_limit);
         if (splits > 1) ptx::cluster_wait();
     } else {
         // ------------------------------------------------------------ epilogue warps (8 warps)
@@ -408,13 +423,18 @@ w8a8_tcgen05_gemm(const __grid_constant__ CUtensorMap map_w, const __grid_consta
             bias_words[i] = (bias16 && columns_ok) ? uint32_t(bias16[n + 2 * i]) | (uint32_t(bias16[n + 2 * i + 1]) << 16) : 0u;
         const uint4 bias8 = make_uint4(bias_words[0], bias_words[1], bias_words[2], bias_words[3]);
         // K-group mode: the weights' group scales of this CTA's K range are static too, one entry per
-        // accumulation unit (a unit past the end of K, whose accumulator holds zeros, takes scale 1).
+        // accumulation unit (zero for a unit past the end of K, whose accumulator holds zeros). They come by asynchronous
+        // copies, so that nothing waits for them until the activations' have been asked for too.
         const int unit_count = kb_count * units;
         float *sx_smem = scale_smem, *sw_smem = scale_smem + size_t(unit_count) * BN;
         if constexpr (Grouped) {
+            const int shift = __ffs(a.weight_group) - 1; // group widths are powers of two
+            const uint32_t dst = ptx::smem_u32(sw_smem);
             for (int i = e_thread; i < unit_count * kBlockChannels; i += kEpilogueThreads) {
                 const int unit = i / kBlockChannels, channel = n0 + i % kBlockChannels, k0 = kb_begin * kBlockK + unit * unit_k;
-                sw_smem[i] = (a.weight_group && channel < a.n && k0 < a.k) ? a.sw[size_t(k0 / a.weight_group) * a.n + channel] : 1.f;
+                const bool inside = channel < a.n && k0 < a.k;
+                if (a.weight_group) ptx::copy_async4(dst + 4u * i, inside ? a.sw + size_t(k0 >> shift) * a.n + channel : a.sw, inside ? 4u : 0u);
+                else sw_smem[i] = 1.f;
             }
         }
         ptx::wait_for_upstream(); // activation scales, residuals and the output buffer belong to upstream
@@ -460,6 +480,7 @@ w8a8_tcgen05_gemm(const __grid_constant__ CUtensorMap map_w, const __grid_consta
 
         if constexpr (!Grouped) {
             for (int c = e_thread; c < BN; c += kEpilogueThreads) sx_tile[c] = c < valid_tokens ? a.sx[m0 + c] : 0.f;
+            if (warp == kGemmThreads / 32 - 1) wait_for_refills(true, wait_limit);
             ok = ptx::mbar_wait(ptx::smem_u32(&acc_full[0]), 0, abort_ptr, wait_limit);
             ptx::tcgen05_fence_after();
             if (splits > 1) ptx::cluster_wait(); // every peer is running: its shared memory may be written
@@ -480,40 +501,59 @@ w8a8_tcgen05_gemm(const __grid_constant__ CUtensorMap map_w, const __grid_consta
         } else {
             // Stage the activations' group scales of this split (the weights' were staged before the wait):
             // sx_g[unit][token], each operand indexed by its own group width.
+            const int shift = __ffs(a.input_group) - 1;
+            const uint32_t dst = ptx::smem_u32(sx_smem);
             for (int i = e_thread; i < unit_count * BN; i += kEpilogueThreads) {
                 const int unit = i / BN, token = i % BN, k0 = kb_begin * kBlockK + unit * unit_k;
-                sx_smem[i] = (a.input_group && token < valid_tokens && k0 < a.k)
-                                 ? a.sx[size_t(k0 / a.input_group) * a.m + m0 + token] : 1.f;
+                const bool inside = token < valid_tokens && k0 < a.k;
+                if (a.input_group) ptx::copy_async4(dst + 4u * i, inside ? a.sx + size_t(k0 >> shift) * a.m + m0 + token : a.sx, inside ? 4u : 0u);
+                else sx_smem[i] = 1.f;
             }
+            ptx::copy_async_wait_all();
             asm volatile("bar.sync 1, 256;" ::: "memory");
-            float result[kMyChunks * 16];
+            // The two warps of a lane quadrant take half of the tokens each. A round drains kRound units with one wait: a
+            // commit completes after all earlier MMAs, so the last unit's barrier stands for the round. The arithmetic is
+            // packed two-wide (with scalar conversions 64 tokens took 512 cycles of the conversion pipe per K block).
+            constexpr int kHalf = BN / 2, kRound = BN == 16 ? 4 : BN == 32 ? 2 : 1;
+            const ptx::IntBias bias_of_int = ptx::int_bias(raw_base);
+            uint64_t result[kHalf / 2];
 #pragma unroll
-            for (int c = 0; c < kMyChunks * 16; ++c) result[c] = 0.f;
+            for (int c = 0; c < kHalf / 2; ++c) result[c] = 0ull;
 #pragma unroll 1
-            for (int it = 0; it < unit_count && ok; ++it) {
-                const int buffer = it % kAccBuffers;
-                ok = ptx::mbar_wait(ptx::smem_u32(&acc_full[buffer]), uint32_t(it / kAccBuffers) & 1u, abort_ptr, wait_limit);
+            for (int first = 0; first < unit_count && ok; first += kRound) {
+                const int last = min(first + kRound, unit_count) - 1;
+                ok = ptx::mbar_wait(ptx::smem_u32(&acc_full[last % kAccBuffers]), uint32_t(last / kAccBuffers) & 1u, abort_ptr, wait_limit);
                 if (!ok) break;
                 ptx::tcgen05_fence_after();
-                const float scale_w = sw_smem[it * kBlockChannels + channel_in_tile];
-                const float *scale_x = sx_smem + it * BN;
-                uint32_t r[kMyChunks][16];
+                uint32_t r[kRound][kHalf];
 #pragma unroll
-                for (int k = 0; k < kMyChunks; ++k)
-                    if (2 * k + half < kChunks) ptx::tmem_load16(lane_base + uint32_t(buffer * BN + (2 * k + half) * 16), r[k]);
+                for (int u = 0; u < kRound; ++u)
+                    if (first + u <= last) ptx::tmem_load<kHalf>(lane_base + uint32_t(((first + u) % kAccBuffers) * BN + half * kHalf), r[u]);
                 ptx::tmem_load_wait();
-                // Everything this warp needs is in registers: hand the buffer back before the arithmetic.
-                ptx::tcgen05_fence_before();
-                __syncwarp();
-                if (lane == 0) ptx::mbar_arrive(ptx::smem_u32(&acc_empty[buffer]));
+                // Everything this warp needs is in registers: hand the buffers that are used again back before the arithmetic.
+                if (first + kAccBuffers < unit_count) {
+                    ptx::tcgen05_fence_before();
+                    __syncwarp();
+                    if (lane == 0)
+                        for (int u = first; u <= last; ++u) ptx::mbar_arrive(ptx::smem_u32(&acc_empty[u % kAccBuffers]));
+                }
 #pragma unroll
-                for (int k = 0; k < kMyChunks; ++k) {
-                    if (2 * k + half < kChunks) {
+                for (int u = 0; u < kRound; ++u) {
+                    if (first + u <= last) {
+                        const int it = first + u;
+                        const float scale_w = sw_smem[it * kBlockChannels + channel_in_tile];
+                        const uint64_t scale_w2 = ptx::pack2(scale_w, scale_w);
+                        const uint32_t scale_x = ptx::pinned(ptx::smem_u32(sx_smem + it * BN + half * kHalf));
 #pragma unroll
-                        for (int i = 0; i < 16; ++i) {
-                            // |p| <= 128*127^2 < 2^24, so the int -> float conversion is exact.
-                            const float p = kInt ? float(int(r[k][i])) : __uint_as_float(r[k][i]);
-                            result[k * 16 + i] = fmaf(p, scale_x[(2 * k + half) * 16 + i] * scale_w, result[k * 16 + i]);
+                        for (int q = 0; q < kHalf / 4; ++q) {
+                            const ulonglong2 sx4 = ptx::ld_shared_2x64(scale_x + 16u * q); // a broadcast
+#pragma unroll
+                            for (int h = 0; h < 2; ++h) {
+                                const int i = 4 * q + 2 * h;
+                                const uint64_t p = kInt ? ptx::int_to_float2(r[u][i], r[u][i + 1], bias_of_int)
+                                                        : ptx::pack2(__uint_as_float(r[u][i]), __uint_as_float(r[u][i + 1]));
+                                result[i / 2] = ptx::fma2(p, ptx::mul2(h ? sx4.y : sx4.x, scale_w2), result[i / 2]);
+                            }
                         }
                     }
                 }
@@ -523,18 +563,35 @@ w8a8_tcgen05_gemm(const __grid_constant__ CUtensorMap map_w, const __grid_consta
                 // Outer scales exist only when just one operand carries K-group scales.
                 const int channel = n0 + channel_in_tile;
                 const float outer_w = (!a.weight_group && channel < a.n) ? a.sw[channel] : 1.f;
+                constexpr int kRows = kHalf < 16 ? kHalf : 16; // tokens of one 16-row pass this thread holds
 #pragma unroll
-                for (int k = 0; k < kMyChunks; ++k) {
-                    const int chunk = 2 * k + half;
-                    if (chunk < kChunks && chunk * 16 < valid_tokens) {
-                        uint32_t words[16];
+                for (int k = 0; k < kHalf / kRows; ++k) {
+                    const int token0 = half * kHalf + k * kRows, chunk = token0 / 16;
+                    if (token0 < valid_tokens) {
+                        uint32_t words[kRows];
 #pragma unroll
-                        for (int i = 0; i < 16; ++i) {
-                            const int c = chunk * 16 + i;
-                            const float outer = (a.input_group || c >= valid_tokens) ? 1.f : a.sx[m0 + c];
-                            words[i] = __float_as_uint(result[k * 16 + i] * (outer * outer_w));
+                        for (int i = 0; i < kRows; i += 2) {
+                            float v[2];
+                            ptx::unpack2(result[(k * kRows + i) / 2], v[0], v[1]);
+#pragma unroll
+                            for (int h = 0; h < 2; ++h) {
+                                const int c = token0 + i + h;
+                                const float outer = (a.input_group || c >= valid_tokens) ? 1.f : a.sx[m0 + c];
+                                words[i + h] = __float_as_uint(v[h] * (outer * outer_w));
+                            }
                         }
-                        emit_chunk(chunk, words);
+                        if (splits == 1) {
+#pragma unroll
+                            for (int i = 0; i < kRows; ++i)
+                                if (token0 + i < valid_tokens) tile_words[(token0 + i) * kBlockChannels + channel_in_tile] = words[i];
+                        } else {
+                            const uint32_t remote = ptx::map_to_rank(reduce_base + uint32_t(split * a.owned_passes + chunk / splits) * kPassBytes +
+                                                                         uint32_t((token0 & 15) * kBlockChannels + channel_in_tile) * 4u,
+                                                                     uint32_t(chunk % splits));
+#pragma unroll
+                            for (int i = 0; i < kRows; ++i)
+                                if (token0 + i < valid_tokens) ptx::st_cluster_u32(remote + uint32_t(i) * (kBlockChannels * 4u), words[i]);
+                        }
                     }
                 }
             }
@@ -710,7 +767,7 @@ w8a8_tcgen05_gemm(const __grid_constant__ CUtensorMap map_w, const __grid_consta
             }
         }
     }
-    if (warp < 2 && splits > 1) ptx::cluster_sync(); // the producer/MMA warps' share of the phase barrier
+    if ((warp < 2 || warp >= kGemmThreads / 32) && splits > 1) ptx::cluster_sync(); // the other warps' share of the phase barrier
 
     __syncthreads(); // tensor memory is drained and nobody else will touch this CTA's shared memory
     if (warp == 1) {

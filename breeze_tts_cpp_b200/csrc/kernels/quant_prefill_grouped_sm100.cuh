@@ -1,178 +1,109 @@
-// Compute-bound K-group W8A8 GEMM (group_int8 / group_fp8 prefill) for sm_100a: persistent CTAs over
-// 128-channel x 128-token tiles, K-group size 128 on BOTH operands.
+// K-group W8A8 GEMM (group_int8 / group_fp8 beyond decode) for sm_100a: persistent CTAs over tiles of 128 tokens x
+// `Channels` (64 or 128) output channels, K-group size 128 on BOTH operands.
 //
 // Arithmetic (reference grouped_gemm, src/ops/kernels/quant/quant_grouped.cu:16-169): every K block
 // of 128 is its own integer/fp8 dot product p_g, and out[m,n] = D(sum_g float(p_g) * (sx_g[m] *
-// sw_g[n])) (+ fp32 residual). The tensor cores therefore produce one 128x128 partial tile per K
-// block, and CUDA cores rescale and add it; that second part is what bounds this kernel.
+// sw_g[n])) (+ fp32 residual), optionally followed by the finishing chain. The tensor cores therefore produce one
+// partial tile per K block, and CUDA cores rescale and add it; that second part is what bounds this kernel (INT8: issue,
+// 153 instructions per warp and K block of which 88 are the arithmetic; FP8 and many waves: the 32 KB per K block each SM
+// pulls from L2).
 //
-//   warp 0  : TMA producer. Per K block one pipeline stage (weights 128x128 B + tokens 128x128 B,
-//             128-byte swizzle) and one slot of a small scale ring (sx_g row slice and sw_g row slice
-//             of that K block, 2 x 512 B, brought in as plain 2-D TMA boxes of the group-major arrays).
-//   warp 1  : MMA issuer, whole warp in the loop, elected lane issues. Four accumulators of 128
-//             columns rotate through tensor memory, so the tensor cores run up to four K blocks
-//             ahead of the rescale. It never tests an mbarrier itself: a test between MMA issues
-//             costs the issuing warp about 200 cycles, two per K block would double its loop.
-//   warp 10 : waiter. Tests "accumulator free" and "stage full" for the next K block and hands the
-//             result to warp 1 through a named hardware barrier (64 threads), which is free.
-//   warps 2-9: per K block, pull the accumulator into registers (lane = channel, 64 tokens per
-//             thread), hand the buffer back at once, then result += float(p) * (sx * sw) with packed
-//             two-wide fp32 instructions; INT8 partials are converted with the exact
-//             add-a-magic-constant trick (|p| <= 128 * 127^2 < 2^22) instead of the slow conversion
-//             pipe. After the last K block the 64 results per thread go out through the same
-//             shared-memory patches as the per-row prefill kernel (coalesced 8-byte row stores).
+//   warp 0     : producer. Per K block one pipeline stage (128 token rows + `Channels` weight rows of 128 B, 128-byte
+//                swizzle) by TMA and one slot of a small ring for the scales of that K block, on the same barrier: the
+//                channels' by TMA, the tokens' by 4-byte asynchronous copies (a row count need not be a multiple of 4).
+//   warp 1     : MMA issuer, whole warp in the loop, elected lane issues. The tokens are the MMA's M rows. Four (eight)
+//                accumulators rotate through tensor memory, so the tensor cores run that many K blocks
+//                ahead of the rescale. It never tests an mbarrier itself: a test waits behind the MMAs in flight.
+//   warp 18    : waiter. Tests "accumulator free" and "stage full" for the next K block and hands the
+//                result to warp 1 through a named hardware barrier (64 threads), which is free.
+//   warps 2-17 : per K block, pull the accumulator into registers (lane = token, a quarter of the channels per
+//                warp), hand the buffer back at once, then result += float(p) * (sx * sw) with packed
+//                two-wide fp32 instructions. After the last K block the finished rows leave through swizzled
+//                shared-memory slabs and TMA stores, the chain's residual having been prefetched into the same slabs (as in
+//                quant_prefill_pair_sm100.cuh).
+// Sixteen rescale warps: the chain wait - load - hand back - arithmetic of one warp is latency, four warps per scheduler
+// hide one another's (eight warps with twice the channels each took about 1100 cycles per K block whatever the format).
+// Measured, GEMM alone, M=4096: INT8 12288 x 2048 220 -> 164 us, 2048 x 6144 110 -> 88; FP8 192 -> 144 and 92 -> 76; with a row
+// count that is no multiple of four (1021) the weight-streaming kernel used to run: FP8 102 -> 44 us.
 // Every wait is bounded; on expiry the CTA flags the status word and runs to the common exit.
 #pragma once
 #include "kernels/quant_linear_sm100.cuh"
 
 namespace tts::b200 {
 
-constexpr int kGroupedStages = 5;
-constexpr int kGroupedAccumulators = 4;
-constexpr int kScaleSlots = 8;
-constexpr int kGroupedThreads = kGemmThreads + 32; // + the waiter warp
-constexpr int kScaleSlotBytes = 2 * kGroupedTokens * 4; // sx_g slice then sw_g slice of one K block
-constexpr int kPrefillPatchBytes = 2 * 2 * 16 * kBlockChannels * 2; // two chunk groups x two parities x [16][128] 16-bit
-constexpr size_t kGroupedSmem = 1024 + size_t(kGroupedStages) * (kBlockChannels + kGroupedTokens) * kBlockK +
-                                size_t(kScaleSlots) * kScaleSlotBytes + kPrefillPatchBytes;
+constexpr int kGroupedMaxStages = 7;
+__host__ __device__ constexpr int grouped_stages(int channels) { return channels == 64 ? kGroupedMaxStages : 5; } // what shared memory holds
+// Scale slots need no barriers of their own. They are filled with their stage, so an accumulator that is full implies its
+// slot is. And slot c is rewritten for K block c + kScaleSlots only once the MMAs of block c + kScaleSlots - stages
+// have retired, which the rescale warps allowed by emptying the accumulator of a block at most 8 before that, after they were
+// done with the block before that one: c + kScaleSlots - stages - 9 >= c.
+constexpr int kScaleSlots = 16;
+static_assert(kScaleSlots >= kGroupedMaxStages + 9, "a scale slot could be rewritten while it is read");
+constexpr int kGroupedWarps = 16;                          // rescale warps
+constexpr int kGroupedThreads = 32 * (kGroupedWarps + 3);  // + producer, MMA issuer, waiter
+constexpr int kRescaleThreads = 32 * kGroupedWarps;
+constexpr int kScaleSlotBytes = (kBlockChannels + kGroupedTokens) * 4; // channels, then tokens
+constexpr uint32_t kGroupedSlabBytes = kGroupedTokens * 128; // 128 token rows x 64 channels of 16 bits
+constexpr size_t grouped_smem(int channels) {
+    return 1024 + size_t(grouped_stages(channels)) * (kGroupedTokens + channels) * kBlockK + size_t(channels / 64) * kGroupedSlabBytes +
+           size_t(kScaleSlots) * kScaleSlotBytes;
+}
 
 struct GroupedArgs {
     int m, n, k;
-    const float *sx, *sw;
-    void *out;
-    int out_type; // Type::BF16 or Type::F16
-    const float *residual_f32;
+    const float *sx;           // group-major [k / 128, m]
+    const float *residual_f32; // [m, n], added before the first rounding
     int *status;
+    FusedEpilogue ep;          // read by the chain instances only
 };
 
-// One 16-token chunk of a tile's epilogue, executed by the four warps (one per tensor-memory lane
-// quadrant) that share a chunk. Phase 1, lane = channel: accumulator -> (acc*sx)*sw (+ fp32 residual)
-// -> 16-bit, written to a small shared-memory patch [token][channel]. After a 128-thread barrier,
-// phase 2, lane = four consecutive channels: every warp copies four token rows of the patch to
-// global memory as 8-byte stores, 256 contiguous bytes per row. The patch is double-buffered so one
-// barrier per chunk suffices. `r` holds the chunk's 16 accumulator words of this lane.
-template <bool kInt>
-__device__ __forceinline__ void prefill_store_chunk(const GroupedArgs &a, const uint32_t (&r)[16], const float *sx_chunk,
-                                                    float scale_w, const float *__restrict__ residual, int m_first,
-                                                    int n_tile0, int valid_rows, int quadrant, int lane, int group,
-                                                    uint16_t *patch /* [16][128] of this group and parity */) {
-    const int channel = quadrant * 32 + lane, n = n_tile0 + channel;
-    const bool bf16_out = a.out_type == int(Type::BF16);
-    // All loads (activation scales from shared memory, residuals from global memory) come first: a
-    // load may not be moved above an earlier store it might alias, so interleaving them with the patch
-    // stores would serialise sixteen round trips.
-    float scale_x[16], skip[16];
-    {
-        const float4 *sx4 = reinterpret_cast<const float4 *>(sx_chunk);
-#pragma unroll
-        for (int q = 0; q < 4; ++q) {
-            const float4 v = sx4[q];
-            scale_x[4 * q] = v.x; scale_x[4 * q + 1] = v.y; scale_x[4 * q + 2] = v.z; scale_x[4 * q + 3] = v.w;
-        }
-    }
-#pragma unroll
-    for (int i = 0; i < 16; ++i)
-        skip[i] = (residual && n < a.n && i < valid_rows) ? __ldg(residual + size_t(m_first + i) * a.n + n) : 0.f;
-    uint16_t bits[16];
-#pragma unroll
-    for (int i = 0; i < 16; ++i) {
-        const float acc = kInt ? float(int(r[i])) : __uint_as_float(r[i]);
-        float value = __fmul_rn(__fmul_rn(acc, scale_x[i]), scale_w);
-        if (residual) value = __fadd_rn(value, skip[i]);
-        if (bf16_out) { __nv_bfloat16 b = __float2bfloat16_rn(value); bits[i] = *reinterpret_cast<uint16_t *>(&b); }
-        else { __half h = __float2half_rn(value); bits[i] = *reinterpret_cast<uint16_t *>(&h); }
-    }
-#pragma unroll
-    for (int i = 0; i < 16; ++i) patch[i * kBlockChannels + channel] = bits[i];
-    if (group == 0) asm volatile("bar.sync 2, 128;" ::: "memory");
-    else asm volatile("bar.sync 3, 128;" ::: "memory");
-    const int n4 = n_tile0 + lane * 4;
-    if (n4 < a.n) {
-#pragma unroll
-        for (int rr = 0; rr < 4; ++rr) {
-            const int i = quadrant * 4 + rr;
-            if (i < valid_rows) {
-                const uint2 four = *reinterpret_cast<const uint2 *>(patch + i * kBlockChannels + lane * 4);
-                *reinterpret_cast<uint2 *>(static_cast<uint16_t *>(a.out) + size_t(m_first + i) * a.n + n4) = four;
-            }
-        }
-    }
-}
-
-namespace ptx {
-// Two fp32 lanes in one 64-bit register, and the packed arithmetic Blackwell has for them.
-__device__ __forceinline__ uint64_t pack2(float lo, float hi) {
-    uint64_t r;
-    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));
-    return r;
-}
-__device__ __forceinline__ void unpack2(uint64_t v, float &lo, float &hi) {
-    asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(v));
-}
-__device__ __forceinline__ uint64_t mul2(uint64_t a, uint64_t b) {
-    uint64_t r;
-    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
-    return r;
-}
-__device__ __forceinline__ uint64_t add2(uint64_t a, uint64_t b) {
-    uint64_t r;
-    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
-    return r;
-}
-__device__ __forceinline__ uint64_t fma2(uint64_t a, uint64_t b, uint64_t c) {
-    uint64_t r;
-    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
-    return r;
-}
-} // namespace ptx
-
-template <Type F>
+template <Type F, int Channels, bool Chain, bool F16>
 __global__ void __launch_bounds__(kGroupedThreads, 1)
 w8a8_tcgen05_prefill_grouped(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_x,
-                             const __grid_constant__ CUtensorMap map_sw, const __grid_constant__ CUtensorMap map_sx,
-                             const __grid_constant__ GroupedArgs a) {
+                             const __grid_constant__ CUtensorMap map_sw, const __grid_constant__ CUtensorMap map_out,
+                             const __grid_constant__ CUtensorMap map_residual, const __grid_constant__ GroupedArgs a) {
     constexpr bool kInt = F == Type::I8;
-    constexpr int BN = kGroupedTokens;
-    constexpr int kWeightBytes = kBlockChannels * kBlockK, kTokenBytes = BN * kBlockK;
+    constexpr int BM = kGroupedTokens;
+    constexpr int kStages = grouped_stages(Channels);
+    constexpr int kAccumulators = 512 / Channels, kColumns = Channels / 4; // kColumns: channels per rescale thread
+    constexpr int kSlabs = Channels / 64;
+    constexpr int kWeightBytes = Channels * kBlockK, kTokenBytes = BM * kBlockK;
     constexpr int kStageBytes = kWeightBytes + kTokenBytes;
-    constexpr uint32_t kRingBytes = kGroupedStages * kStageBytes;
-    constexpr uint32_t kScaleBytes = kScaleSlots * kScaleSlotBytes;
-    constexpr uint32_t kIdesc = kInt ? ptx::idesc_i8(kBlockChannels, BN) : ptx::idesc_e4m3(kBlockChannels, BN);
+    constexpr uint32_t kRingBytes = kStages * kStageBytes;
+    constexpr uint32_t kIdesc = kInt ? ptx::idesc_i8(BM, Channels) : ptx::idesc_e4m3(BM, Channels);
 
     extern __shared__ uint8_t dynamic_smem[];
-    __shared__ alignas(8) uint64_t full_bar[kGroupedStages], empty_bar[kGroupedStages];
-    __shared__ alignas(8) uint64_t acc_full[kGroupedAccumulators], acc_empty[kGroupedAccumulators];
-    __shared__ alignas(8) uint64_t scale_full[kScaleSlots], scale_empty[kScaleSlots];
+    __shared__ alignas(8) uint64_t full_bar[kStages], empty_bar[kStages];
+    __shared__ alignas(8) uint64_t acc_full[kAccumulators], acc_empty[kAccumulators];
+    __shared__ alignas(8) uint64_t residual_full;
     __shared__ uint32_t tmem_slot;
     __shared__ int abort_flag;
-    __shared__ alignas(16) float ones[16];
 
+    // [pipeline stages | slabs | scale slots], 1024-byte aligned for the swizzled boxes.
     const uint32_t raw_base = ptx::smem_u32(dynamic_smem);
     const uint32_t tiles_base = (raw_base + 1023u) & ~1023u;
     uint8_t *aligned = dynamic_smem + (tiles_base - raw_base);
+    const uint32_t slab_base = tiles_base + kRingBytes, scale_base = slab_base + kSlabs * kGroupedSlabBytes;
     const int warp = ptx::warp_index(), lane = threadIdx.x & 31;
-    const int n_tiles = (a.n + kBlockChannels - 1) / kBlockChannels, m_tiles = (a.m + BN - 1) / BN;
+    const int n_tiles = (a.n + Channels - 1) / Channels, m_tiles = (a.m + BM - 1) / BM;
     const int tiles = n_tiles * m_tiles;
     const int kb_count = (a.k + kBlockK - 1) / kBlockK;
+    const bool skip16 = Chain && a.ep.residual != nullptr;
 
     if (threadIdx.x == 0) {
-        for (int s = 0; s < kGroupedStages; ++s) {
-            ptx::mbar_init(ptx::smem_u32(&full_bar[s]), 1);
+        for (int s = 0; s < kStages; ++s) {
+            ptx::mbar_init(ptx::smem_u32(&full_bar[s]), 1 + 32); // the elected lane with the bytes, every lane with its scales
             ptx::mbar_init(ptx::smem_u32(&empty_bar[s]), 1);
         }
-        for (int b = 0; b < kGroupedAccumulators; ++b) {
+        for (int b = 0; b < kAccumulators; ++b) {
             ptx::mbar_init(ptx::smem_u32(&acc_full[b]), 1);
-            ptx::mbar_init(ptx::smem_u32(&acc_empty[b]), kEpilogueThreads / 32);
+            ptx::mbar_init(ptx::smem_u32(&acc_empty[b]), kGroupedWarps);
         }
-        for (int s = 0; s < kScaleSlots; ++s) {
-            ptx::mbar_init(ptx::smem_u32(&scale_full[s]), 1);
-            ptx::mbar_init(ptx::smem_u32(&scale_empty[s]), kEpilogueThreads / 32);
-        }
+        ptx::mbar_init(ptx::smem_u32(&residual_full), 1);
         abort_flag = 0;
         ptx::fence_barrier_init();
         ptx::fence_proxy_async_smem();
     }
-    if (threadIdx.x < 16) ones[threadIdx.x] = 1.f;
     if (warp == 1) ptx::tmem_alloc(ptx::smem_u32(&tmem_slot), 512);
     ptx::tcgen05_fence_before();
     __syncthreads();
@@ -182,44 +113,57 @@ w8a8_tcgen05_prefill_grouped(const __grid_constant__ CUtensorMap map_w, const __
     ptx::launch_dependents();
 
     if (warp == 0) {
-        // ------------------------------------------------------------ TMA producer
+        // ------------------------------------------------------------ producer
         // The whole warp runs the loop so that addresses and coordinates stay warp-uniform; one elected lane issues.
+        // The first round of the ring fetches the weights and their scales before the wait on upstream.
         if (ptx::elect_one()) {
             ptx::prefetch_tensormap(&map_w);
             ptx::prefetch_tensormap(&map_x);
             ptx::prefetch_tensormap(&map_sw);
-            ptx::prefetch_tensormap(&map_sx);
+        }
+        const int ahead = int(blockIdx.x) < tiles ? min(kStages, kb_count) : 0;
+        const int first_n0 = (int(blockIdx.x) % n_tiles) * Channels;
+        const auto load_weights = [&](int stage, int slot, int kb, int n0) {
+            const uint32_t bar = ptx::smem_u32(&full_bar[stage]);
+            ptx::mbar_arrive_expect_tx(bar, kStageBytes + Channels * 4);
+            ptx::tma_load_2d(tiles_base + uint32_t(stage) * kStageBytes, &map_w, bar, kb * kBlockK, n0);
+            ptx::tma_load_2d(scale_base + uint32_t(slot) * kScaleSlotBytes, &map_sw, bar, n0, kb);
+        };
+        for (int i = 0; i < ahead; ++i) {
+            if (ptx::elect_one()) load_weights(i, i, i, first_n0);
+            __syncwarp();
         }
         ptx::wait_for_upstream();
-        int stage = 0, slot = 0;
-        uint32_t phase = 0, slot_phase = 0;
+        int stage = 0, slot = 0, filled = 0; // filled: K blocks so far, over all tiles
+        uint32_t phase = 0;
         bool ok = true;
         for (int tile = blockIdx.x; tile < tiles && ok; tile += gridDim.x) {
-            const int n0 = (tile % n_tiles) * kBlockChannels, m0 = (tile / n_tiles) * BN;
-            for (int kb = 0; kb < kb_count; ++kb) {
-                ok = ptx::mbar_wait(ptx::smem_u32(&scale_empty[slot]), slot_phase ^ 1u, abort_ptr) &&
-                     ptx::mbar_wait(ptx::smem_u32(&empty_bar[stage]), phase ^ 1u, abort_ptr);
+            const int n0 = (tile % n_tiles) * Channels, m0 = (tile / n_tiles) * BM;
+            for (int kb = 0; kb < kb_count; ++kb, ++filled) {
+                ok = filled < kStages || ptx::mbar_wait(ptx::smem_u32(&empty_bar[stage]), phase ^ 1u, abort_ptr);
                 ok = __all_sync(0xffffffffu, ok);
                 if (!ok) break;
-                const uint32_t scale_bar = ptx::smem_u32(&scale_full[slot]);
-                const uint32_t scale_dst = tiles_base + kRingBytes + uint32_t(slot) * kScaleSlotBytes;
-                const uint32_t bar = ptx::smem_u32(&full_bar[stage]);
-                const uint32_t dst = tiles_base + uint32_t(stage) * kStageBytes;
                 if (ptx::elect_one()) {
-                    ptx::mbar_arrive_expect_tx(bar, kStageBytes);
-                    ptx::tma_load_2d(dst, &map_w, bar, kb * kBlockK, n0);
-                    ptx::tma_load_2d(dst + kWeightBytes, &map_x, bar, kb * kBlockK, m0);
-                    ptx::mbar_arrive_expect_tx(scale_bar, kScaleSlotBytes);
-                    ptx::tma_load_2d(scale_dst, &map_sx, scale_bar, m0, kb);
-                    ptx::tma_load_2d(scale_dst + BN * 4, &map_sw, scale_bar, n0, kb);
+                    if (filled >= ahead) load_weights(stage, slot, kb, n0);
+                    ptx::tma_load_2d(tiles_base + uint32_t(stage) * kStageBytes + kWeightBytes, &map_x,
+                                     ptx::smem_u32(&full_bar[stage]), kb * kBlockK, m0);
                 }
                 __syncwarp();
-                if (++slot == kScaleSlots) { slot = 0; slot_phase ^= 1u; }
-                if (++stage == kGroupedStages) { stage = 0; phase ^= 1u; }
+                const float *sx = a.sx + size_t(kb) * a.m + m0 + lane;
+                const uint32_t sx_slot = scale_base + uint32_t(slot) * kScaleSlotBytes + uint32_t(kBlockChannels + lane) * 4u;
+#pragma unroll
+                for (int i = 0; i < BM / 32; ++i) {
+                    const bool inside = m0 + lane + 32 * i < a.m;
+                    ptx::copy_async4(sx_slot + 128u * i, inside ? sx + 32 * i : a.sx, inside ? 4u : 0u);
+                }
+                ptx::copy_async_arrive(ptx::smem_u32(&full_bar[stage]));
+                slot = (slot + 1) % kScaleSlots;
+                if (++stage == kStages) { stage = 0; phase ^= 1u; }
             }
         }
-    } else if (warp == 1 || warp == 10) {
-        // ------------------------------------------------------------ MMA issuer (1) and its waiter (10)
+        ptx::copy_async_wait_all();
+    } else if (warp == 1 || warp == kGroupedWarps + 2) {
+        // ------------------------------------------------------------ MMA issuer (1) and its waiter
         // Both walk the same K-block sequence and meet once per K block at named barrier 4, which also
         // carries the waiter's verdict. Neither leaves its loop early, so the barrier counts always
         // match; after a failed wait the abort flag makes every later wait return at once and the
@@ -228,111 +172,140 @@ w8a8_tcgen05_prefill_grouped(const __grid_constant__ CUtensorMap map_w, const __
         uint32_t phase = 0, count = 0; // count: K blocks so far, over all tiles
         for (int tile = blockIdx.x; tile < tiles; tile += gridDim.x) {
             for (int kb = 0; kb < kb_count; ++kb, ++count) {
-                const uint32_t buffer = count % kGroupedAccumulators;
-                if (warp == 10) {
-                    const uint32_t use = (count / kGroupedAccumulators) & 1u;
+                const uint32_t buffer = count % kAccumulators;
+                if (warp != 1) {
+                    const uint32_t use = (count / kAccumulators) & 1u;
                     const bool ready = ptx::mbar_wait(ptx::smem_u32(&acc_empty[buffer]), use ^ 1u, abort_ptr) &&
                                        ptx::mbar_wait(ptx::smem_u32(&full_bar[stage]), phase, abort_ptr);
-                    (void)ptx::pair_barrier_and(ready);
+                    (void)ptx::pair_barrier_and(__all_sync(0xffffffffu, ready)); // the vote brings the lanes together
                 } else {
                     const bool ready = ptx::pair_barrier_and(true);
                     ptx::tcgen05_fence_after();
                     const uint32_t tile_smem = tiles_base + uint32_t(stage) * kStageBytes;
                     const uint32_t lo_w = ptx::smem_desc_lo_k128(tile_smem), lo_x = ptx::smem_desc_lo_k128(tile_smem + kWeightBytes);
-                    const uint32_t d = tmem_base + buffer * uint32_t(BN);
+                    const uint32_t d = tmem_base + buffer * uint32_t(Channels);
                     if (ready && ptx::elect_one()) {
-                        if (kInt) ptx::mma_i8_k128(d, lo_w, lo_x, kIdesc, 0u);
-                        else ptx::mma_f8_k128(d, lo_w, lo_x, kIdesc, 0u);
+                        if (kInt) ptx::mma_i8_k128(d, lo_x, lo_w, kIdesc, 0u);
+                        else ptx::mma_f8_k128(d, lo_x, lo_w, kIdesc, 0u);
                         ptx::tcgen05_commit(ptx::smem_u32(&empty_bar[stage]));
                         ptx::tcgen05_commit(ptx::smem_u32(&acc_full[buffer]));
                     }
                     __syncwarp();
                 }
-                if (++stage == kGroupedStages) { stage = 0; phase ^= 1u; }
+                if (++stage == kStages) { stage = 0; phase ^= 1u; }
             }
         }
     } else {
         // ------------------------------------------------------------ rescale + epilogue warps
-        const int quadrant = warp & 3, half = (warp - 2) >> 2;
-        const uint32_t lane_base = tmem_base + (uint32_t(quadrant * 32) << 16);
+        const int quadrant = warp & 3, quarter = (warp - 2) >> 2; // tensor-memory lanes; which kColumns channels
+        const int row = quadrant * 32 + lane, c0 = quarter * kColumns;
+        const uint32_t lane_base = tmem_base + (uint32_t(quadrant * 32) << 16) + uint32_t(c0);
+        const bool storer = threadIdx.x == 64; // issues the tile's TMA traffic
         const float *__restrict__ residual = a.residual_f32;
-        const float *scales = reinterpret_cast<const float *>(aligned + kRingBytes);
-        uint16_t *patches = reinterpret_cast<uint16_t *>(aligned + kRingBytes + kScaleBytes);
-        const uint64_t magic2 = ptx::pack2(-12582912.f, -12582912.f);
+        const float *scales = reinterpret_cast<const float *>(aligned + (scale_base - tiles_base));
+        uint8_t *slab_row = aligned + kRingBytes + uint32_t(c0 / 64) * kGroupedSlabBytes + uint32_t(row) * 128u;
+        const ptx::IntBias bias_of_int = ptx::int_bias(raw_base);
+        if (storer) ptx::prefetch_tensormap(&map_out);
         ptx::wait_for_upstream();
-        uint32_t count = 0;
+        uint32_t count = 0, residual_phase = 0;
         bool ok = true;
         for (int tile = blockIdx.x; tile < tiles && ok; tile += gridDim.x) {
-            const int n0 = (tile % n_tiles) * kBlockChannels, m0 = (tile / n_tiles) * BN;
-            const int valid_tokens = min(BN, a.m - m0);
-            uint64_t result[32]; // [chunk 0..3][pair 0..7]: tokens (2*k + half)*16 + 2*pair, +1
+            const int n0 = (tile % n_tiles) * Channels, m0 = (tile / n_tiles) * BM;
+            const int token = m0 + row;
+            const bool token_ok = token < a.m;
+            const int valid_slabs = min(kSlabs, (a.n - n0 + 63) / 64);
+            if (skip16 && storer) { // into the slabs the results will overwrite: the last tile's stores must have left them
+                ptx::bulk_wait_read<0>();
+                const uint32_t bar = ptx::smem_u32(&residual_full);
+                ptx::mbar_arrive_expect_tx(bar, uint32_t(valid_slabs) * kGroupedSlabBytes);
+                for (int s = 0; s < valid_slabs; ++s)
+                    ptx::tma_load_2d(slab_base + uint32_t(s) * kGroupedSlabBytes, &map_residual, bar, n0 + s * 64, m0);
+            }
+            uint64_t result[kColumns / 2];
 #pragma unroll
-            for (int i = 0; i < 32; ++i) result[i] = 0ull;
+            for (int i = 0; i < kColumns / 2; ++i) result[i] = 0ull;
 #pragma unroll 1
             for (int kb = 0; kb < kb_count; ++kb, ++count) {
-                const uint32_t buffer = count % kGroupedAccumulators, use = (count / kGroupedAccumulators) & 1u;
-                const uint32_t slot = count % kScaleSlots, slot_use = (count / kScaleSlots) & 1u;
-                if (!ptx::mbar_wait(ptx::smem_u32(&acc_full[buffer]), use, abort_ptr)) { ok = false; break; }
+                const uint32_t buffer = count % kAccumulators;
+                ok = ptx::mbar_wait(ptx::smem_u32(&acc_full[buffer]), (count / kAccumulators) & 1u, abort_ptr);
+                if (!ok) break;
                 ptx::tcgen05_fence_after();
-                uint32_t r[4][16];
-#pragma unroll
-                for (int k = 0; k < 4; ++k) ptx::tmem_load16(lane_base + buffer * uint32_t(BN) + uint32_t((2 * k + half) * 16), r[k]);
+                uint32_t r[kColumns];
+                ptx::tmem_load<kColumns>(lane_base + buffer * uint32_t(Channels), r);
                 ptx::tmem_load_wait();
                 // Everything is in registers: the tensor cores may have the buffer back.
                 ptx::tcgen05_fence_before();
                 __syncwarp();
                 if (lane == 0) ptx::mbar_arrive(ptx::smem_u32(&acc_empty[buffer]));
-                if (!ptx::mbar_wait(ptx::smem_u32(&scale_full[slot]), slot_use, abort_ptr)) { ok = false; break; }
-                const float *slot_scales = scales + slot * (kScaleSlotBytes / 4);
-                const float scale_w = slot_scales[BN + quadrant * 32 + lane];
-                const uint64_t scale_w2 = ptx::pack2(scale_w, scale_w);
+                const float scale_x = scales[(count % kScaleSlots) * (kScaleSlotBytes / 4) + kBlockChannels + row];
+                const uint64_t scale_x2 = ptx::pack2(scale_x, scale_x);
+                const uint32_t sw = ptx::pinned(scale_base + (count % kScaleSlots) * kScaleSlotBytes + uint32_t(c0) * 4u);
 #pragma unroll
-                for (int k = 0; k < 4; ++k) {
-                    const float4 *sx4 = reinterpret_cast<const float4 *>(slot_scales + (2 * k + half) * 16);
+                for (int q = 0; q < kColumns / 4; ++q) {
+                    const ulonglong2 sw4 = ptx::ld_shared_2x64(sw + 16u * q); // the same address in every lane: a broadcast
 #pragma unroll
-                    for (int q = 0; q < 4; ++q) {
-                        const float4 sx = sx4[q];
-#pragma unroll
-                        for (int h = 0; h < 2; ++h) {
-                            const int i = 4 * q + 2 * h;
-                            uint64_t p;
-                            if (kInt) {
-                                // float(int) exactly: bits(2^23 + 2^22 + p) read as fp32, minus that constant.
-                                p = ptx::add2(ptx::pack2(__uint_as_float(r[k][i] + 0x4B400000u), __uint_as_float(r[k][i + 1] + 0x4B400000u)), magic2);
-                            } else {
-                                p = ptx::pack2(__uint_as_float(r[k][i]), __uint_as_float(r[k][i + 1]));
-                            }
-                            const uint64_t s = ptx::mul2(h ? ptx::pack2(sx.z, sx.w) : ptx::pack2(sx.x, sx.y), scale_w2);
-                            result[k * 8 + i / 2] = ptx::fma2(p, s, result[k * 8 + i / 2]);
-                        }
+                    for (int h = 0; h < 2; ++h) {
+                        const int i = 4 * q + 2 * h;
+                        const uint64_t p = kInt ? ptx::int_to_float2(r[i], r[i + 1], bias_of_int)
+                                                : ptx::pack2(__uint_as_float(r[i]), __uint_as_float(r[i + 1]));
+                        result[i / 2] = ptx::fma2(p, ptx::mul2(h ? sw4.y : sw4.x, scale_x2), result[i / 2]);
                     }
                 }
-                __syncwarp();
-                if (lane == 0) ptx::mbar_arrive(ptx::smem_u32(&scale_empty[slot]));
             }
-            // All eight warps decide together whether the tile is stored (a warp that left alone would
-            // strand the three that share its staging patch); the same barrier keeps two consecutive
-            // tiles from meeting in one patch.
-            ok = ptx::barrier_and(1, kEpilogueThreads, ok && !*abort_ptr);
+            // ---- tile finished: rows into the slabs, slabs out by TMA.
+            if (skip16) {
+                if (ok) ok = ptx::mbar_wait(ptx::smem_u32(&residual_full), residual_phase, abort_ptr);
+                residual_phase ^= 1u;
+            } else if (storer) {
+                ptx::bulk_wait_read<0>(); // the last tile's stores have left the slabs
+            }
+            // All warps decide together whether the tile is stored; the barrier also publishes that the slabs are free.
+            ok = ptx::barrier_and(1, kRescaleThreads, ok && !*abort_ptr);
             if (!ok) break;
-            // ---- tile finished: 16-token chunks out through the staging patches.
+            const float *skip_row = residual && token_ok ? residual + size_t(token) * a.n + n0 + c0 : nullptr;
 #pragma unroll
-            for (int k = 0; k < 4; ++k) {
-                const int chunk = 2 * k + half;
-                if (chunk * 16 < valid_tokens) { // uniform over the four warps that share the chunk
-                    uint32_t words[16];
+            for (int q = 0; q < kColumns / 8; ++q) { // eight channels = one 16-byte chunk of the slab row
+                uint4 *chunk = reinterpret_cast<uint4 *>(slab_row + ((((c0 & 63) / 8 + q) ^ (row & 7)) * 16));
+                const bool inside = n0 + c0 + 8 * q < a.n; // N is a multiple of 16
+                float value[8];
 #pragma unroll
-                    for (int j = 0; j < 8; ++j) {
-                        float lo, hi;
-                        ptx::unpack2(result[k * 8 + j], lo, hi);
-                        words[2 * j] = __float_as_uint(lo);
-                        words[2 * j + 1] = __float_as_uint(hi);
-                    }
-                    prefill_store_chunk<false>(a, words, ones, 1.f, residual, m0 + chunk * 16, n0, valid_tokens - chunk * 16,
-                                               quadrant, lane, half, patches + ((half * 2 + (k & 1)) * 16 * kBlockChannels));
+                for (int i = 0; i < 4; ++i) ptx::unpack2(result[4 * q + i], value[2 * i], value[2 * i + 1]);
+                if (skip_row && inside) {
+                    const float4 lo = __ldg(reinterpret_cast<const float4 *>(skip_row + 8 * q)), hi = __ldg(reinterpret_cast<const float4 *>(skip_row + 8 * q + 4));
+                    const float s8[8] = {lo.x, lo.y, lo.z, lo.w, hi.x, hi.y, hi.z, hi.w};
+#pragma unroll
+                    for (int i = 0; i < 8; ++i) value[i] = __fadd_rn(value[i], s8[i]);
                 }
+                uint4 packed = pack8x16<F16>(value);
+                if (Chain) {
+                    uint4 bias = make_uint4(0, 0, 0, 0);
+                    if (a.ep.bias && inside) {
+                        const uint16_t *b = static_cast<const uint16_t *>(a.ep.bias) + n0 + c0 + 8 * q;
+                        uint32_t w[4];
+#pragma unroll
+                        for (int i = 0; i < 4; ++i) w[i] = uint32_t(b[2 * i]) | (uint32_t(b[2 * i + 1]) << 16);
+                        bias = make_uint4(w[0], w[1], w[2], w[3]);
+                    }
+                    packed = chain8<F16>(a.ep, packed, bias, skip16 ? *chunk : make_uint4(0, 0, 0, 0));
+                }
+                *chunk = packed;
+            }
+            if (Chain && a.ep.activation > 1) {
+#pragma unroll 1
+                for (int q = 0; q < kColumns / 8; ++q) {
+                    uint4 *chunk = reinterpret_cast<uint4 *>(slab_row + ((((c0 & 63) / 8 + q) ^ (row & 7)) * 16));
+                    *chunk = activate8<F16>(*chunk, a.ep.activation, a.ep.alpha);
+                }
+            }
+            ptx::fence_proxy_async_smem(); // the rows are about to be read by the TMA engine
+            (void)ptx::barrier_and(1, kRescaleThreads, true);
+            if (storer) {
+                for (int s = 0; s < valid_slabs; ++s)
+                    ptx::tma_store_2d(&map_out, slab_base + uint32_t(s) * kGroupedSlabBytes, n0 + s * 64, m0);
+                ptx::bulk_commit();
             }
         }
+        if (storer) ptx::bulk_wait_read<0>(); // the slabs must outlive their stores
         ptx::tcgen05_fence_before();
     }
 

@@ -169,7 +169,8 @@ w8a8_tcgen05_prefill_pair(const __grid_constant__ CUtensorMap map_w, const __gri
                         if (kb == 0) ok = ok && ptx::mbar_wait(ptx::smem_u32(&acc_empty[buffer]), ((uint32_t(local) >> 1) & 1u) ^ 1u, abort_ptr);
                         ok = ok && ptx::mbar_wait(ptx::smem_u32(&full_bar[stage]), phase, abort_ptr);
                     }
-                    ok = use_waiter ? ptx::pair_barrier_and(ok) : __all_sync(0xffffffffu, ok);
+                    if (warp == 10 || !use_waiter) ok = __all_sync(0xffffffffu, ok); // also brings the lanes together
+                    if (use_waiter) ok = ptx::pair_barrier_and(ok);
                     if (warp == 1) {
                         ptx::tcgen05_fence_after();
                         const uint32_t tile_smem = tiles_base + uint32_t(stage * stage_bytes);

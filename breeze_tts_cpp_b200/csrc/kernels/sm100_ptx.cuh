@@ -211,6 +211,27 @@ __device__ __forceinline__ void tmem_load32(uint32_t taddr, uint32_t (&r)[32]) {
                  : "r"(taddr)
                  : "memory");
 }
+// The same with 8 columns.
+__device__ __forceinline__ void tmem_load8(uint32_t taddr, uint32_t (&r)[8]) {
+    asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7])
+                 : "r"(taddr)
+                 : "memory");
+}
+// This warp's 32 lanes x `Columns` consecutive columns.
+template <int Columns> __device__ __forceinline__ void tmem_load(uint32_t taddr, uint32_t (&r)[Columns]) {
+    if constexpr (Columns == 8) {
+        tmem_load8(taddr, r);
+    } else if constexpr (Columns == 16) {
+        tmem_load16(taddr, r);
+    } else if constexpr (Columns == 32) {
+        tmem_load32(taddr, r);
+    } else {
+        static_assert(Columns == 64, "unsupported column count");
+        tmem_load32(taddr, *reinterpret_cast<uint32_t(*)[32]>(&r[0]));
+        tmem_load32(taddr + 32u, *reinterpret_cast<uint32_t(*)[32]>(&r[32]));
+    }
+}
 __device__ __forceinline__ void tmem_load_wait() {
     asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 }
@@ -258,6 +279,74 @@ __device__ __forceinline__ void tcgen05_commit_pair(uint32_t bar, uint16_t cta_m
 // Arrive on a barrier given by a shared::cluster address (own CTA or a peer).
 __device__ __forceinline__ void mbar_arrive_cluster(uint32_t cluster_bar) {
     asm volatile("mbarrier.arrive.shared::cluster.b64 _, [%0];" ::"r"(cluster_bar) : "memory");
+}
+
+// ---------------------------------------------------------------- packed fp32, small asynchronous copies
+// Two fp32 lanes in one 64-bit register, and the packed arithmetic Blackwell has for them.
+__device__ __forceinline__ uint64_t pack2(float lo, float hi) {
+    uint64_t r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));
+    return r;
+}
+__device__ __forceinline__ void unpack2(uint64_t v, float &lo, float &hi) {
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(v));
+}
+__device__ __forceinline__ uint64_t mul2(uint64_t a, uint64_t b) {
+    uint64_t r;
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+__device__ __forceinline__ uint64_t add2(uint64_t a, uint64_t b) {
+    uint64_t r;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+__device__ __forceinline__ uint64_t fma2(uint64_t a, uint64_t b, uint64_t c) {
+    uint64_t r;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+    return r;
+}
+// (a & b) ^ c with all three in registers: one instruction, where two constants would make it two.
+__device__ __forceinline__ uint32_t and_xor(uint32_t a, uint32_t b, uint32_t c) {
+    uint32_t r;
+    asm("lop3.b32 %0, %1, %2, %3, 0x6a;" : "=r"(r) : "r"(a), "r"(b), "r"(c));
+    return r;
+}
+// Exact int -> fp32 of two K-group partials |p| <= 2^21: the bits of 2^23 + 2^22 + p read as fp32, minus that constant. Modulo
+// 2^23 adding 2^22 flips bit 22, so the sum is a logic operation, which runs beside the packed arithmetic (an integer add
+// is issued to the same pipe, and the conversion pipe takes eight cycles per warp instruction). The constants come from
+// int_bias(), which keeps the compiler from fetching them from uniform registers for every use.
+struct IntBias {
+    uint32_t low23, biased;
+    uint64_t minus;
+};
+__device__ __forceinline__ IntBias int_bias(uint32_t smem_base) {
+    const uint32_t zero = (smem_base + (threadIdx.x & 31)) >> 31; // a shared-memory address has no such bit
+    const float m = __uint_as_float(0xCB400000u | zero);          // -(2^23 + 2^22)
+    return {0x7fffffu | zero, 0x4B400000u | zero, pack2(m, m)};
+}
+__device__ __forceinline__ uint64_t int_to_float2(uint32_t a, uint32_t b, const IntBias &k) {
+    return add2(pack2(__uint_as_float(and_xor(a, k.low23, k.biased)), __uint_as_float(and_xor(b, k.low23, k.biased))), k.minus);
+}
+// Four bytes global -> shared (zero when `bytes` is 0), and an arrival on `bar` (counted in its expected arrivals) once this
+// thread's copies so far have landed.
+__device__ __forceinline__ void copy_async4(uint32_t dst, const void *src, uint32_t bytes) {
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"(dst), "l"(src), "r"(bytes) : "memory");
+}
+__device__ __forceinline__ void copy_async_arrive(uint32_t bar) {
+    asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];" ::"r"(bar) : "memory");
+}
+__device__ __forceinline__ void copy_async_wait_all() { asm volatile("cp.async.wait_all;" ::: "memory"); }
+// Four consecutive fp32 in shared memory as two packed pairs. Not ordered against barriers by itself: the address must come
+// from pinned() after the barrier that publishes the data.
+__device__ __forceinline__ ulonglong2 ld_shared_2x64(uint32_t addr) {
+    ulonglong2 v;
+    asm("ld.shared.v2.b64 {%0, %1}, [%2];" : "=l"(v.x), "=l"(v.y) : "r"(addr));
+    return v;
+}
+__device__ __forceinline__ uint32_t pinned(uint32_t v) {
+    asm volatile("" : "+r"(v)::"memory");
+    return v;
 }
 
 // ---------------------------------------------------------------- descriptors
@@ -338,10 +427,12 @@ __device__ __forceinline__ bool pair_barrier_and(bool ok) {
                  : "memory");
     return all != 0;
 }
+// Both forms are aligned: the lanes of a warp have to arrive together (vote after anything that lanes can leave apart).
 // The same over any named barrier: every one of the `threads` participants learns whether all of
 // them passed `ok`. Used where several warps must agree to leave a loop together, because a warp
 // that left alone would strand its siblings at their next named barrier.
 __device__ __forceinline__ bool barrier_and(uint32_t id, uint32_t threads, bool ok) {
+    ok = __all_sync(0xffffffffu, ok);
     uint32_t all;
     asm volatile("{\n\t.reg .pred p, q;\n\tsetp.ne.u32 q, %3, 0;\n\tbar.red.and.pred p, %1, %2, q;\n\t"
                  "selp.u32 %0, 1, 0, p;\n\t}"
