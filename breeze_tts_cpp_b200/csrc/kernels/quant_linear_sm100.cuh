@@ -283,22 +283,22 @@ w8a8_tcgen05_gemm(const __grid_constant__ CUtensorMap map_w, const __grid_consta
         // activations the chain keeps passing from kernel to kernel stay in L2.
         const uint64_t stream_once = ptx::policy_evict_first();
         const int ahead = min(a.stages, kb_count);
-        for (int i = 0; i < ahead; ++i) {
-            const uint32_t bar = ptx::smem_u32(&full_bar[i]);
-            if (ptx::elect_one()) {
+        if (ptx::elect_one()) { // one election around a burst: per copy or per MMA it costs some 20 cycles
+            for (int i = 0; i < ahead; ++i) {
+                const uint32_t bar = ptx::smem_u32(&full_bar[i]);
                 ptx::mbar_arrive_expect_tx(bar, kWeightBytes + (i == 0 ? uint32_t(a.expiry_extra_bytes) : 0u));
                 ptx::tma_load_2d_hint(tiles_base + uint32_t(i) * kStageBytes, &map_w, bar, (kb_begin + i) * kBlockK, n0, stream_once);
             }
-            __syncwarp();
         }
+        __syncwarp();
         ptx::wait_for_upstream();
-        if (ptx::elect_one()) ptx::mbar_arrive_expect_tx(ptx::smem_u32(&x_full), uint32_t(ahead) * kTokenBytes);
-        for (int i = 0; i < ahead; ++i) {
-            if (ptx::elect_one())
+        if (ptx::elect_one()) {
+            ptx::mbar_arrive_expect_tx(ptx::smem_u32(&x_full), uint32_t(ahead) * kTokenBytes);
+            for (int i = 0; i < ahead; ++i)
                 ptx::tma_load_2d(tiles_base + uint32_t(i) * kStageBytes + kWeightBytes, &map_x,
                                  ptx::smem_u32(&x_full), (kb_begin + i) * kBlockK, m0);
-            __syncwarp();
         }
+        __syncwarp();
         int stage = ahead == a.stages ? 0 : ahead;
         uint32_t phase = ahead == a.stages ? 1u : 0u;
         for (int kb = kb_begin + ahead; kb < kb_end; ++kb) {
@@ -339,24 +339,22 @@ w8a8_tcgen05_gemm(const __grid_constant__ CUtensorMap map_w, const __grid_consta
                     const uint32_t tile = tiles_base + uint32_t(at) * kStageBytes;
                     const uint32_t lo_w = ptx::smem_desc_lo_k128(tile), lo_x = ptx::smem_desc_lo_k128(tile + kWeightBytes);
                     const uint32_t d = tmem_base + buffer * uint32_t(BN), accumulate = Grouped ? 0u : uint32_t(it > 0);
-                    if (ptx::elect_one()) {
-                        if (kInt) ptx::mma_i8_k128(d, lo_w, lo_x, kIdesc, accumulate);
-                        else ptx::mma_f8_k128(d, lo_w, lo_x, kIdesc, accumulate);
-                        // Only a stage that will be refilled needs to report that its MMAs retired.
-                        if (it + a.stages < kb_count) ptx::tcgen05_commit(ptx::smem_u32(&empty_bar[at]));
-                        if (Grouped) ptx::tcgen05_commit(ptx::smem_u32(&acc_full[buffer]));
-                    }
-                    __syncwarp();
+                    if (kInt) ptx::mma_i8_k128(d, lo_w, lo_x, kIdesc, accumulate);
+                    else ptx::mma_f8_k128(d, lo_w, lo_x, kIdesc, accumulate);
+                    // Only a stage that will be refilled needs to report that its MMAs retired.
+                    if (it + a.stages < kb_count) ptx::tcgen05_commit(ptx::smem_u32(&empty_bar[at]));
+                    if (Grouped) ptx::tcgen05_commit(ptx::smem_u32(&acc_full[buffer]));
                 };
-                if (ok) {
-                    ptx::tcgen05_fence_after();
+                ptx::tcgen05_fence_after();
+                if (ok && ptx::elect_one())
                     for (int it = 0; it < burst; ++it) issue(it, it, Grouped ? uint32_t(it) : 0u);
-                }
+                __syncwarp();
                 // Refilled stages arrive at the rate memory delivers them.
                 for (int it = burst; it < kb_count; ++it) {
                     ok = ptx::pair_barrier_and(ok);
                     ptx::tcgen05_fence_after();
-                    if (ok) issue(it, stage, Grouped ? uint32_t(it) % kAccBuffers : 0u);
+                    if (ok && ptx::elect_one()) issue(it, stage, Grouped ? uint32_t(it) % kAccBuffers : 0u);
+                    __syncwarp();
                     if (++stage == a.stages) stage = 0;
                 }
             } else {

@@ -43,10 +43,8 @@ int blocks(int size, int tile) { return (size + tile - 1) / tile; }
 bool persistent_per_row(const KernelProblem &p, const LinearPath &path) {
     return !grouped(p) && path.tokens == kPrefillTokens && path.splits == 1;
 }
-bool persistent_grouped(const KernelProblem &p, const LinearPath &path, int sms) {
-    return p.input_group == kBlockK && p.weight_group == kBlockK && path.tokens == kGroupedTokens &&
-           path.splits == 1 && p.rows % 4 == 0 &&
-           int64_t(blocks(p.channels, kBlockChannels)) * blocks(p.rows, kGroupedTokens) >= int64_t(sms) * 2 / 3;
+bool persistent_grouped(const KernelProblem &p, const LinearPath &path) {
+    return p.input_group == kBlockK && p.weight_group == kBlockK && path.tokens == kGroupedTokens && path.splits == 1;
 }
 } // namespace
 
@@ -59,7 +57,11 @@ std::vector<LinearPath> quant_linear_candidates(KernelProblem p, KernelLimits li
     int cover = 16;
     while (cover < (group ? kGroupedTokens : kPrefillTokens) && cover < p.rows) cover *= 2;
     std::vector<int> token_tiles{cover};
-    if (group && cover == kGroupedTokens) token_tiles.push_back(64); // the split-K kernel's widest K-group tile below 128
+    // K groups: narrower tiles of the split-K kernel beside the persistent kernel's 128 tokens (they pay on short batches).
+    if (group && cover == kGroupedTokens) {
+        token_tiles.push_back(64);
+        if (p.rows <= 256) token_tiles.push_back(32);
+    }
     // Between decode and prefill a batch covers a few narrow tiles: several of them per channel slab (and split K)
     // occupy the machine where one or two 256-token tiles would leave most of it idle. Beyond 1024 rows the
     // 256-token tiles fill it by themselves.
@@ -77,7 +79,7 @@ std::vector<LinearPath> quant_linear_candidates(KernelProblem p, KernelLimits li
     return paths;
 }
 
-double linear_cost(KernelProblem p, LinearPath path, Type, const ChipModel &chip) {
+double linear_cost(KernelProblem p, LinearPath path, Type format, const ChipModel &chip) {
     if (path.kind != LinearKind::Tcgen05) return std::numeric_limits<double>::infinity();
     const int sms = std::max(1, chip.sms);
     const int kb_total = blocks(p.reduction, kBlockK);
@@ -87,36 +89,45 @@ double linear_cost(KernelProblem p, LinearPath path, Type, const ChipModel &chip
         const PairTile tile = pair_channel_tile(p.rows, p.channels, kb_total, std::max(1, sms / 2), kPairColumnCycles);
         return 1.8 + tile.cycles / 1965.;
     }
-    if (persistent_grouped(p, path, sms)) {
-        // Bound by the fp32 rescale of every K128 partial tile on the CUDA cores.
-        const double tiles = double(blocks(p.channels, kBlockChannels)) * blocks(p.rows, kGroupedTokens);
-        const double waves = std::ceil(tiles / sms);
-        return chip.kernel_us + ops * (waves * sms / tiles) / (0.3 * chip.tensor_ops_per_us);
+    if (persistent_grouped(p, path)) {
+        // Waves of 128 tokens x 64 or 128 channels, bound by the fp32 rescale of every K128 partial tile (0.34 and 0.44 us per
+        // K block, INT8; FP8 is up to 15 % faster).
+        const int channels = grouped_channel_tile(p.rows, p.channels, sms);
+        const double tiles = double(blocks(p.channels, channels)) * blocks(p.rows, kGroupedTokens);
+        return (channels == 64 ? 2.2 : 2.8) + std::ceil(tiles / sms) * kb_total * (channels == 64 ? 0.34 : 0.44);
     }
-    if (!grouped(p) && p.rows > kWeightStreamTokens) {
+    if (p.rows > kWeightStreamTokens) {
         // Weight-streaming kernel with several token tiles per channel slab. Fitted to launches of 65 to 1024 rows on
         // K = 512 to 6144, N = 1024 to 12288: a base per token tile, a slope per K block (the operand bytes one SM
-        // pulls), the split-K exchange, and contention for L2 as the grid grows. More than one wave does not pay:
-        // CTAs own their multiprocessor's shared memory, so nothing of the next wave overlaps.
+        // pulls; with K groups the rescale), the split-K exchange, and contention for L2 as the grid grows. More than one
+        // wave does not pay: CTAs own their multiprocessor's shared memory, so nothing of the next wave overlaps.
+        const bool group = grouped(p);
         const int splits = std::max(1, path.splits), per_split = blocks(kb_total, splits);
-        const LaunchShape shape = launch_shape(path.tokens, false, per_split, splits, 1);
+        const int units = group_units(p.input_group, p.weight_group);
+        const LaunchShape shape = launch_shape(path.tokens, group, per_split, splits, units);
         if (!shape.fits) return std::numeric_limits<double>::infinity();
         const int64_t ctas = int64_t(blocks(p.channels, kBlockChannels)) * blocks(p.rows, path.tokens) * splits;
-        const int resident = (path.tokens <= 64 && shape.smem <= 108 * 1024) ? 2 : 1;
+        const int resident = (!group && path.tokens <= 64 && shape.smem <= 108 * 1024) ? 2 : 1;
         // Clusters are placed whole inside a GPC (16 to 20 multiprocessors): count what that leaves unusable.
-        const int64_t slots = std::max<int64_t>(splits, int64_t(sms) * resident * 16 / 18 / splits * splits);
-        const double base = path.tokens <= 64 ? 2.5 : path.tokens <= 128 ? 4.0 : 6.2;
-        const double slope = path.tokens <= 128 ? 0.214 : 0.42;
-        const double exchange = splits > 1 ? 0.3 + (path.tokens <= 64 ? 0.15 : 0.25) * splits : 0.0;
+        const int64_t slots = splits > 1 ? std::max<int64_t>(splits, int64_t(sms) * resident * 16 / 18 / splits * splits)
+                                         : int64_t(sms) * resident;
+        const int tile = path.tokens <= 32 ? 0 : path.tokens <= 64 ? 1 : path.tokens <= 128 ? 2 : 3;
+        static constexpr double kBase[2][4] = {{2.3, 2.5, 4.0, 6.2}, {2.7, 3.4, 5.6, 9.0}};
+        static constexpr double kSlope[2][4] = {{0.21, 0.214, 0.214, 0.42}, {0.245, 0.31, 0.44, 0.9}};
+        const double exchange = splits == 1 ? 0.0 : group ? 0.25 + 0.2 * splits : 0.3 + (path.tokens <= 64 ? 0.15 : 0.25) * splits;
         const double contention = 0.012 * double(std::max<int64_t>(0, std::min(ctas, slots) - 48));
-        const double waves = double((ctas + (splits > 1 ? slots : int64_t(sms) * resident) - 1) / (splits > 1 ? slots : int64_t(sms) * resident));
-        const double one = base + per_split * slope + exchange + contention;
+        const double waves = double((ctas + slots - 1) / slots);
+        const double one = kBase[group][tile] + per_split * units * kSlope[group][tile] + exchange + contention;
         return one + (waves - 1.0) * (one - 1.0);
     }
     // Weight-streaming kernel, as it runs inside a decoder chain: the launch starts under programmatic
     // dependent launch while its quantizer still runs, so by the time the activations exist the ring
     // already holds `stages` K blocks of weights. What is left on the critical path is
     //   * the K blocks that did not fit the ring, at what one SM can pull or its share of HBM;
+    //   * the part of the ring the launches before leave no time for: with few rows they are short (about 1 us + 0.06 us a
+    //     row), so more splits, i.e. less weight per SM, pay (down projection, 5 rows: 4 splits 25.4 us a layer, 6 24.1;
+    //     QKV 2 splits 25.3, 4 24.7). Per-row INT8 only: its sums are exact whatever the split, while a split moves the
+    //     rounding of FP8 and K-group sums, which a stack of requantized layers amplifies to the format's own noise;
     //   * the MMAs, which cost a fixed ~0.12 us per K block up to 64 tokens (four instructions of at
     //     least 48 tensor-pipe cycles each, however few tokens), more for wider tiles;
     //   * the split-K exchange, about 0.3 us per CTA of the cluster at 64 tokens (less for narrower tiles); clusters of seven and eight lose
@@ -139,7 +150,9 @@ double linear_cost(KernelProblem p, LinearPath path, Type, const ChipModel &chip
     const double exposed = exposed_blocks * stage_bytes *
                            std::max(1.0 / per_sm, double(std::min(ctas, slots)) / (0.84 * chip.memory_bytes_per_us));
     const double mma_block = path.tokens <= 64 ? 0.12 : path.tokens <= 128 ? 0.16 : 0.29;
-    const double compute = std::max(per_split * mma_block, exposed + mma_block) * (grouped(p) ? 1.5 : 1.0);
+    const bool exact = format == Type::I8 && !grouped(p);
+    const double unhidden = !exact ? 0.0 : std::max(0.0, std::min(per_split, shape.stages) * double(kBlockChannels * kBlockK) / per_sm - 1.0 - 0.06 * p.rows);
+    const double compute = unhidden + std::max(per_split * mma_block, exposed + mma_block) * (grouped(p) ? 1.5 : 1.0);
     const double exchange = splits > 1 ? (0.15 + 0.15 * path.tokens / 64.0) * splits + (kb_total % splits ? 0.15 : 0.0) + (splits > 6 ? 6.0 : 0.0) : 0.0;
     const int passes = blocks(std::min(p.rows, path.tokens), kRowsPerPass);
     const double epilogue = 0.4 * (splits > 1 ? blocks(passes, splits) : passes);
