@@ -117,7 +117,11 @@ void launch_instance(const CUtensorMap &map_w, const CUtensorMap &map_x, const G
     }
     config.attrs = attributes;
     config.numAttrs = count;
-    check(cudaLaunchKernelEx(&config, w8a8_tcgen05_gemm<F, Grouped, BN>, map_w, map_x, args), "quantized GEMM launch");
+    const bool plain = args.vector_io && !args.ep.chain && args.out_type != int(Type::I32) &&
+                       (!Grouped || group_units(args.input_group, args.weight_group) == 1);
+    check(cudaLaunchKernelEx(&config, plain ? w8a8_tcgen05_gemm<F, Grouped, BN, true> : w8a8_tcgen05_gemm<F, Grouped, BN, false>, map_w,
+                             map_x, args),
+          "quantized GEMM launch");
 }
 template <Type F, bool Grouped>
 void launch_tokens(int bn, const CUtensorMap &map_w, const CUtensorMap &map_x, const GemmArgs &args, dim3 grid,
@@ -135,9 +139,8 @@ void launch_tokens(int bn, const CUtensorMap &map_w, const CUtensorMap &map_x, c
 }
 
 template <Type F, bool Grouped, int BN> void raise_limit() {
-    check(cudaFuncSetAttribute(w8a8_tcgen05_gemm<F, Grouped, BN>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                               int(kSmemBudget)),
-          "cudaFuncSetAttribute(shared memory)");
+    for (auto *kernel : {w8a8_tcgen05_gemm<F, Grouped, BN, false>, w8a8_tcgen05_gemm<F, Grouped, BN, true>})
+        check(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(kSmemBudget)), "cudaFuncSetAttribute(shared memory)");
 }
 int multiprocessor_count() {
     static std::atomic<int> cached[64];

@@ -171,7 +171,10 @@ template <bool F16> __device__ __forceinline__ uint4 pack8x16(const float (&v)[8
 // for that, because its epilogue warps are busy; per-row mode uses the last epilogue warp, which is idle until the end.
 template <bool Grouped> constexpr int kStreamThreads = kGemmThreads + (Grouped ? 32 : 0);
 
-template <Type F, bool Grouped, int BN>
+// `Plain` instances serve what a decoder chain asks for: aligned 16-bit rows, nothing behind the product but an fp32 residual,
+// K groups of 128 or none. They carry no other code: in a chain every launch finds the instruction caches cold, and the
+// general kernel's extra paths cost time although they are not taken.
+template <Type F, bool Grouped, int BN, bool Plain>
 __global__ void __launch_bounds__(kStreamThreads<Grouped>, (!Grouped && BN <= 64) ? 2 : 1)
 w8a8_tcgen05_gemm(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_x,
                   const __grid_constant__ GemmArgs a) {
@@ -216,7 +219,7 @@ w8a8_tcgen05_gemm(const __grid_constant__ CUtensorMap map_w, const __grid_consta
     const int kb_end = int(int64_t(kb_total) * (split + 1) / splits);
     const int kb_count = kb_end - kb_begin;
     // K-group mode: accumulation units per 128-byte K block (1, 2 or 4) and MMAs per unit.
-    const int unit_k = Grouped ? min(a.input_group ? a.input_group : kBlockK, a.weight_group ? a.weight_group : kBlockK) : kBlockK;
+    const int unit_k = Grouped && !Plain ? min(a.input_group ? a.input_group : kBlockK, a.weight_group ? a.weight_group : kBlockK) : kBlockK;
     const int units = kBlockK / unit_k, unit_mmas = 4 / units;
     const int tile_linear = blockIdx.y * gridDim.x + blockIdx.x;
     const int valid_tokens = min(BN, a.m - m0);
@@ -332,7 +335,7 @@ w8a8_tcgen05_gemm(const __grid_constant__ CUtensorMap map_w, const __grid_consta
             // accumulator i to itself while fresh accumulators last.
             const int burst = refill_from; // min(ahead, K blocks with a fresh accumulator)
             int stage = burst == a.stages ? 0 : burst;
-            if (!Grouped || units == 1) {
+            if (!Grouped || Plain || units == 1) {
                 // One K block: four MMAs into its accumulator and its reports. A loop of its own: one that also served the
                 // narrow groups issued K-group blocks at half the rate.
                 const auto issue = [&](int it, int at, uint32_t buffer) {
@@ -413,7 +416,7 @@ w8a8_tcgen05_gemm(const __grid_constant__ CUtensorMap map_w, const __grid_consta
         // hides behind the main loop.
         float sw8[8];
         uint32_t bias_words[4]; // packed pairs
-        const uint16_t *bias16 = static_cast<const uint16_t *>(e.bias);
+        const uint16_t *bias16 = Plain ? nullptr : static_cast<const uint16_t *>(e.bias);
 #pragma unroll
         for (int i = 0; i < 8; ++i) sw8[i] = (!Grouped && columns_ok) ? a.sw[n + i] : 1.f;
 #pragma unroll
@@ -442,7 +445,7 @@ w8a8_tcgen05_gemm(const __grid_constant__ CUtensorMap map_w, const __grid_consta
             const int c = split * kRowsPerPass + row_in_pass; // first pass this CTA owns
 #pragma unroll
             for (int i = 0; i < 8; ++i) first_residual[i] = 0.f;
-            if (e.residual && e.residual_vector && columns_ok && c < valid_tokens)
+            if (!Plain && e.residual && e.residual_vector && columns_ok && c < valid_tokens)
                 first_skip = *reinterpret_cast<const uint4 *>(static_cast<const uint16_t *>(e.residual) +
                                                               size_t(m0 + c) * e.residual_ld + n);
             if (e.residual_f32 && columns_ok && c < valid_tokens) {
@@ -603,7 +606,7 @@ w8a8_tcgen05_gemm(const __grid_constant__ CUtensorMap map_w, const __grid_consta
         // ---- phase 2: finish token rows; every global access is a 16-byte vector on a 256-byte row.
         // Aligned 16-bit rows take a loop specialised for the output type and for whether the finishing chain
         // follows; raw accumulators and unaligned rows take the general loop below it.
-        const bool lean = type != int(Type::I32) && a.vector_io && (!e.residual || e.residual_vector);
+        const bool lean = Plain || (type != int(Type::I32) && a.vector_io && (!e.residual || e.residual_vector));
         const auto finish_rows = [&](auto f16_tag, auto chain_tag) {
             constexpr bool kF16 = decltype(f16_tag)::value, kChain = decltype(chain_tag)::value;
             const float *__restrict__ residual = e.residual_f32; // never aliases the output rows
@@ -665,14 +668,9 @@ w8a8_tcgen05_gemm(const __grid_constant__ CUtensorMap map_w, const __grid_consta
         };
         if (ok && !*abort_ptr && columns_ok && lean) {
             using std::bool_constant;
-            if (type == int(Type::F16)) {
-                if (e.chain) finish_rows(bool_constant<true>{}, bool_constant<true>{});
-                else finish_rows(bool_constant<true>{}, bool_constant<false>{});
-            } else {
-                if (e.chain) finish_rows(bool_constant<false>{}, bool_constant<true>{});
-                else finish_rows(bool_constant<false>{}, bool_constant<false>{});
-            }
-        } else if (ok && !*abort_ptr && columns_ok) {
+            if (type == int(Type::F16)) finish_rows(bool_constant<true>{}, bool_constant<!Plain>{});
+            else finish_rows(bool_constant<false>{}, bool_constant<!Plain>{});
+        } else if (!Plain && ok && !*abort_ptr && columns_ok) {
             for (int local_pass = 0;; ++local_pass) {
                 const int pass = local_pass * splits + split;
                 if (pass >= passes) break;
