@@ -29,7 +29,9 @@ template <> __device__ __forceinline__ float round16<__nv_bfloat16>(float v) {
 }
 template <> __device__ __forceinline__ float round16<__half>(float v) { return __half2float(__float2half_rn(v)); }
 
-template <Type F, class T, int Kind, int Items, bool Rotate, int Threads = kThreads>
+// `Packed`: aligned rows, one scale per row, no rotation; an instance of its own without the other paths (in a decoder chain
+// every launch finds the instruction caches cold).
+template <Type F, class T, int Kind, int Items, bool Rotate, bool Packed, int Threads = kThreads>
 __global__ void __launch_bounds__(Threads)
 gated_quantize(const T *__restrict__ input, unsigned char *__restrict__ out, float *__restrict__ scales, int rows,
                int cols, int group, int parts, bool aligned) {
@@ -40,7 +42,7 @@ gated_quantize(const T *__restrict__ input, unsigned char *__restrict__ out, flo
     const int row = blockIdx.x / parts, shard = blockIdx.x % parts;
     const T *gate = input + size_t(row) * cols * 2, *up = gate + cols;
     float v[Items][8];
-    if (aligned) {
+    if (Packed || aligned) {
         // All loads of the row shard are issued before the first value is used.
         uint4 raw_gate[Items], raw_up[Items];
 #pragma unroll
@@ -52,7 +54,7 @@ gated_quantize(const T *__restrict__ input, unsigned char *__restrict__ out, flo
                 raw_up[j] = *reinterpret_cast<const uint4 *>(up + column);
             }
         }
-        if (!Rotate && !group) { // parts == 1: the row stays in packed storage precision
+        if (Packed) { // parts == 1: the row stays in packed storage precision
             uint4 product[Items];
 #pragma unroll
             for (int j = 0; j < Items; ++j) {
@@ -152,7 +154,7 @@ void launch_items(const T *x, unsigned char *q, float *s, int rows, int cols, in
     if (!group && aligned && chunks > 1 && chunks <= 4 && rows <= sms) {
         const int threads = chunks * kThreads;
 #define B200Q_WIDE(N)                                                                                                   \
-    launch_pdl("quantized gated launch", gated_quantize<F, T, Kind, 1, Rotate, N>, dim3(unsigned(rows)), dim3(N), 0, stream, x, \
+    launch_pdl("quantized gated launch", !Rotate ? gated_quantize<F, T, Kind, 1, false, true, N> : gated_quantize<F, T, Kind, 1, Rotate, false, N>, dim3(unsigned(rows)), dim3(N), 0, stream, x, \
                q, s, rows, cols, group, 1, aligned)
         if (threads == 512) B200Q_WIDE(512);
         else if (threads == 768) B200Q_WIDE(768);
@@ -163,7 +165,7 @@ void launch_items(const T *x, unsigned char *q, float *s, int rows, int cols, in
     const int items = (chunks + parts - 1) / parts;
     const unsigned grid = unsigned(rows) * unsigned(parts);
 #define B200Q_RUN(I)                                                                                                  \
-    launch_pdl("quantized gated launch", gated_quantize<F, T, Kind, I, Rotate>, dim3(grid), dim3(kThreads), 0, stream, x, \
+    launch_pdl("quantized gated launch", aligned && !group && !Rotate ? gated_quantize<F, T, Kind, I, false, true> : gated_quantize<F, T, Kind, I, Rotate, false>, dim3(grid), dim3(kThreads), 0, stream, x, \
                q, s, rows, cols, group, parts, aligned)
     switch (items) {
     case 1: B200Q_RUN(1); break;

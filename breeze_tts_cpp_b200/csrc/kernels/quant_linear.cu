@@ -119,9 +119,9 @@ void launch_instance(const CUtensorMap &map_w, const CUtensorMap &map_x, const G
     config.numAttrs = count;
     const bool plain = args.vector_io && !args.ep.chain && args.out_type != int(Type::I32) &&
                        (!Grouped || group_units(args.input_group, args.weight_group) == 1);
-    check(cudaLaunchKernelEx(&config, plain ? w8a8_tcgen05_gemm<F, Grouped, BN, true> : w8a8_tcgen05_gemm<F, Grouped, BN, false>, map_w,
-                             map_x, args),
-          "quantized GEMM launch");
+    auto *kernel = args.splits > 1 ? (plain ? w8a8_tcgen05_gemm<F, Grouped, BN, true, true> : w8a8_tcgen05_gemm<F, Grouped, BN, false, true>)
+                                   : (plain ? w8a8_tcgen05_gemm<F, Grouped, BN, true, false> : w8a8_tcgen05_gemm<F, Grouped, BN, false, false>);
+    check(cudaLaunchKernelEx(&config, kernel, map_w, map_x, args), "quantized GEMM launch");
 }
 template <Type F, bool Grouped>
 void launch_tokens(int bn, const CUtensorMap &map_w, const CUtensorMap &map_x, const GemmArgs &args, dim3 grid,
@@ -139,7 +139,8 @@ void launch_tokens(int bn, const CUtensorMap &map_w, const CUtensorMap &map_x, c
 }
 
 template <Type F, bool Grouped, int BN> void raise_limit() {
-    for (auto *kernel : {w8a8_tcgen05_gemm<F, Grouped, BN, false>, w8a8_tcgen05_gemm<F, Grouped, BN, true>})
+    for (auto *kernel : {w8a8_tcgen05_gemm<F, Grouped, BN, false, false>, w8a8_tcgen05_gemm<F, Grouped, BN, true, false>,
+                         w8a8_tcgen05_gemm<F, Grouped, BN, false, true>, w8a8_tcgen05_gemm<F, Grouped, BN, true, true>})
         check(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(kSmemBudget)), "cudaFuncSetAttribute(shared memory)");
 }
 int multiprocessor_count() {

@@ -47,11 +47,14 @@ template <class T> __device__ __forceinline__ void store_raw8(T *p, uint4 raw, i
         if (i < remaining) p[i] = e[i];
 }
 
-template <Type F, class T, bool Add, bool Rotate>
+// `Packed`: aligned rows, one scale per row, no rotation. An instance of its own without the other paths (in a decoder chain
+// every launch finds the instruction caches cold).
+template <Type F, class T, bool Add, bool Rotate, bool Packed>
 __global__ void __launch_bounds__(kThreads)
 rms_quantize(T *__restrict__ x, const T *__restrict__ update, const T *__restrict__ weight,
              const T *__restrict__ update_scale, unsigned char *__restrict__ out, float *__restrict__ scales,
-             int rows, int cols, float eps, bool gemma, int group, bool aligned) {
+             int rows, int cols, float eps, bool gemma, int group, bool any_aligned) {
+    const bool aligned = Packed || any_aligned;
     using M = Pair16<T>;
     using P = typename M::P;
     __shared__ float slots[kThreads / 32];
@@ -97,7 +100,7 @@ rms_quantize(T *__restrict__ x, const T *__restrict__ update, const T *__restric
     float v[1][8];
     {
         const P *vp = reinterpret_cast<const P *>(&value), *wp = reinterpret_cast<const P *>(&w);
-        if (!Rotate && !group && aligned) { // the normalized row stays in packed storage precision
+        if (Packed) { // the normalized row stays in packed storage precision
             uint4 row_words[1];
             P *np = reinterpret_cast<P *>(&row_words[0]);
 #pragma unroll
@@ -229,7 +232,7 @@ void launch(T *x, const T *update, const T *weight, const T *update_scale, unsig
         return;
     }
 #define B200Q_RUN(ADD, ROT)                                                                        \
-    launch_pdl("quantized norm launch", rms_quantize<F, T, ADD, ROT>, dim3(rows), dim3(kThreads), 0, stream, x, update,   \
+    launch_pdl("quantized norm launch", aligned && !group && !ROT ? rms_quantize<F, T, ADD, false, true> : rms_quantize<F, T, ADD, ROT, false>, dim3(rows), dim3(kThreads), 0, stream, x, update,   \
                weight, update_scale, q, s, rows, cols, eps, gemma, group, aligned)
     if (update) { if (rotation) B200Q_RUN(true, true); else B200Q_RUN(true, false); }
     else { if (rotation) B200Q_RUN(false, true); else B200Q_RUN(false, false); }

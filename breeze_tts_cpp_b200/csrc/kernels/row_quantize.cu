@@ -17,7 +17,9 @@ namespace {
 constexpr int kThreads = 256;
 
 // Register-resident rows: K <= Items * 2048 * parts.
-template <Type F, class T, int Items, bool Rotate>
+// `Packed`: aligned rows, one scale per row, no rotation; an instance of its own without the other paths (in a decoder chain
+// every launch finds the instruction caches cold).
+template <Type F, class T, int Items, bool Rotate, bool Packed>
 __global__ void __launch_bounds__(kThreads)
 row_quantize_cached(const T *__restrict__ x, unsigned char *__restrict__ q, float *__restrict__ scales,
                     int rows, int cols, int stride, int group, int parts, bool aligned) {
@@ -27,7 +29,7 @@ row_quantize_cached(const T *__restrict__ x, unsigned char *__restrict__ q, floa
     const int row = blockIdx.x / parts, shard = blockIdx.x % parts;
     const T *source = x + size_t(row) * stride;
     float v[Items][8];
-    if (aligned) {
+    if (Packed || aligned) {
         // All loads of the row shard are issued before the first value is used.
         uint4 raw[Items];
 #pragma unroll
@@ -35,7 +37,7 @@ row_quantize_cached(const T *__restrict__ x, unsigned char *__restrict__ q, floa
             int column = ((j * parts + shard) * kThreads + int(threadIdx.x)) * 8;
             raw[j] = column < cols ? *reinterpret_cast<const uint4 *>(source + column) : make_uint4(0, 0, 0, 0);
         }
-        if (!Rotate && !group) { // parts == 1
+        if (Packed) { // parts == 1
             quantize_row_packed<F, T, kThreads, Items>(raw, q + size_t(row) * cols, scales + row, cols, reinterpret_cast<uint32_t *>(slots));
             return;
         }
@@ -201,7 +203,8 @@ void launch_typed(const T *x, unsigned char *q, float *scales, int rows, int col
     const int items = (chunks + parts - 1) / parts;
     const unsigned grid = unsigned(rows) * unsigned(parts);
 #define B200Q_LAUNCH(I)                                                                            \
-    launch_pdl("row quantize launch", row_quantize_cached<F, T, I, Rotate>, dim3(grid), dim3(kThreads), 0, stream, x, q, \
+    launch_pdl("row quantize launch", aligned && !group && !Rotate ? row_quantize_cached<F, T, I, false, true>                   \
+                                                                    : row_quantize_cached<F, T, I, Rotate, false>, dim3(grid), dim3(kThreads), 0, stream, x, q, \
                scales, rows, cols, stride, group, parts, aligned)
     switch (items) {
     case 1: B200Q_LAUNCH(1); break;
