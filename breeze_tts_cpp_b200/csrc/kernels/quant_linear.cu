@@ -119,8 +119,10 @@ void launch_instance(const CUtensorMap &map_w, const CUtensorMap &map_x, const G
     config.numAttrs = count;
     const bool plain = args.vector_io && !args.ep.chain && args.out_type != int(Type::I32) &&
                        (!Grouped || group_units(args.input_group, args.weight_group) == 1);
-    auto *kernel = args.splits > 1 ? (plain ? w8a8_tcgen05_gemm<F, Grouped, BN, true, true> : w8a8_tcgen05_gemm<F, Grouped, BN, false, true>)
-                                   : (plain ? w8a8_tcgen05_gemm<F, Grouped, BN, true, false> : w8a8_tcgen05_gemm<F, Grouped, BN, false, false>);
+    constexpr bool kOne = kOneInstance<Grouped, BN>;
+    auto *kernel = kOne || args.splits > 1
+                       ? (plain ? w8a8_tcgen05_gemm<F, Grouped, BN, true, true> : w8a8_tcgen05_gemm<F, Grouped, BN, false, true>)
+                       : (plain ? w8a8_tcgen05_gemm<F, Grouped, BN, true, kOne> : w8a8_tcgen05_gemm<F, Grouped, BN, false, kOne>);
     check(cudaLaunchKernelEx(&config, kernel, map_w, map_x, args), "quantized GEMM launch");
 }
 template <Type F, bool Grouped>
@@ -139,7 +141,8 @@ void launch_tokens(int bn, const CUtensorMap &map_w, const CUtensorMap &map_x, c
 }
 
 template <Type F, bool Grouped, int BN> void raise_limit() {
-    for (auto *kernel : {w8a8_tcgen05_gemm<F, Grouped, BN, false, false>, w8a8_tcgen05_gemm<F, Grouped, BN, true, false>,
+    constexpr bool kOne = kOneInstance<Grouped, BN>;
+    for (auto *kernel : {w8a8_tcgen05_gemm<F, Grouped, BN, false, kOne>, w8a8_tcgen05_gemm<F, Grouped, BN, true, kOne>,
                          w8a8_tcgen05_gemm<F, Grouped, BN, false, true>, w8a8_tcgen05_gemm<F, Grouped, BN, true, true>})
         check(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(kSmemBudget)), "cudaFuncSetAttribute(shared memory)");
 }

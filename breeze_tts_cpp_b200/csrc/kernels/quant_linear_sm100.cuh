@@ -174,7 +174,10 @@ template <bool Grouped> constexpr int kStreamThreads = kGemmThreads + (Grouped ?
 // `Plain` instances serve what a decoder chain asks for: aligned 16-bit rows, nothing behind the product but an fp32 residual,
 // K groups of 128 or none. They carry no other code: in a chain every launch finds the instruction caches cold, and the
 // general kernel's extra paths cost time although they are not taken.
-// `Split` says the same about split K, in both kinds.
+// `Split` says the same about split K. K-group tiles below 64 tokens keep one instance for both: their chain alternates split
+// and unsplit launches, and one resident copy of that larger kernel beats two (28 layers, 3 / 16 / 32 rows: 729 / 796 / 830
+// against 756 / 833 / 855 us; at 57 rows, in the 64-token tile, two are better, 1024 against 1040).
+template <bool Grouped, int BN> constexpr bool kOneInstance = Grouped && BN < 64;
 template <Type F, bool Grouped, int BN, bool Plain, bool Split>
 __global__ void __launch_bounds__(kStreamThreads<Grouped>, (!Grouped && BN <= 64) ? 2 : 1)
 w8a8_tcgen05_gemm(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_x,
@@ -207,13 +210,14 @@ w8a8_tcgen05_gemm(const __grid_constant__ CUtensorMap map_w, const __grid_consta
     const uint32_t tiles_base = (raw_base + 1023u) & ~1023u;
     uint8_t *tiles_ptr = dynamic_smem + (tiles_base - raw_base);
     const int splits = Split ? a.splits : 1;
-    const uint32_t reduce_bytes = Split ? uint32_t(splits * a.owned_passes) * kPassBytes : 0u;
+    const bool split_k = Split && (!kOneInstance<Grouped, BN> || splits > 1);
+    const uint32_t reduce_bytes = split_k ? uint32_t(splits * a.owned_passes) * kPassBytes : 0u;
     const uint32_t reduce_base = tiles_base + uint32_t(a.tile_region);
     uint8_t *reduce_ptr = tiles_ptr + a.tile_region;
     float *scale_smem = reinterpret_cast<float *>(reduce_ptr + reduce_bytes);
 
     const int warp = ptx::warp_index(), lane = threadIdx.x & 31;
-    const int split = Split ? int(ptx::cluster_ctarank()) : 0; // cluster = (1,1,splits): rank == blockIdx.z
+    const int split = split_k ? int(ptx::cluster_ctarank()) : 0; // cluster = (1,1,splits): rank == blockIdx.z
     const int n0 = blockIdx.x * kBlockChannels, m0 = blockIdx.y * BN;
     const int kb_total = (a.k + kBlockK - 1) / kBlockK;
     const int kb_begin = int(int64_t(kb_total) * split / splits);
@@ -268,7 +272,7 @@ w8a8_tcgen05_gemm(const __grid_constant__ CUtensorMap map_w, const __grid_consta
     const long long wait_limit = a.wait_limit_cycles > 0 ? a.wait_limit_cycles : ptx::kWaitLimitCycles;
     // The next kernel in the stream may begin its own prologue; peers learn that this CTA is running.
     ptx::launch_dependents();
-    if (Split) ptx::cluster_arrive();
+    if (split_k) ptx::cluster_arrive();
 
     if (warp == 0) {
         // ------------------------------------------------------------ TMA producer
@@ -317,7 +321,7 @@ w8a8_tcgen05_gemm(const __grid_constant__ CUtensorMap map_w, const __grid_consta
             __syncwarp();
             if (++stage == a.stages) { stage = 0; phase ^= 1u; }
         }
-        if (Split) ptx::cluster_wait();
+        if (split_k) ptx::cluster_wait();
     } else if (warp == 1) {
         // ------------------------------------------------------------ MMA issuer
         // The whole warp runs the loop so that stage indices and descriptors stay warp-uniform (the
@@ -391,11 +395,11 @@ w8a8_tcgen05_gemm(const __grid_constant__ CUtensorMap map_w, const __grid_consta
             }
             __syncwarp();
         }
-        if (Split) ptx::cluster_wait();
+        if (split_k) ptx::cluster_wait();
     } else if (Grouped && warp == kGemmThreads / 32) {
         // ------------------------------------------------------------ waiter (K-group mode)
         wait_for_refills(true, wait_limit);
-        if (Split) ptx::cluster_wait();
+        if (split_k) ptx::cluster_wait();
     } else {
         // ------------------------------------------------------------ epilogue warps (8 warps)
         const int e_thread = threadIdx.x - 64;
@@ -465,7 +469,7 @@ w8a8_tcgen05_gemm(const __grid_constant__ CUtensorMap map_w, const __grid_consta
         // ---- phase 1: accumulators (one lane = one channel) -> [token][channel] rows, either in this
         // CTA's shared memory (unsplit) or pushed into the owning peer's slot for this split.
         auto emit_chunk = [&](int chunk, const uint32_t (&words)[16]) {
-            if (!Split) {
+            if (!split_k) {
 #pragma unroll
                 for (int i = 0; i < 16; ++i)
                     if (chunk * 16 + i < valid_tokens) tile_words[(chunk * 16 + i) * kBlockChannels + channel_in_tile] = words[i];
@@ -485,7 +489,7 @@ w8a8_tcgen05_gemm(const __grid_constant__ CUtensorMap map_w, const __grid_consta
             if (warp == kGemmThreads / 32 - 1) wait_for_refills(true, wait_limit);
             ok = ptx::mbar_wait(ptx::smem_u32(&acc_full[0]), 0, abort_ptr, wait_limit);
             ptx::tcgen05_fence_after();
-            if (Split) ptx::cluster_wait(); // every peer is running: its shared memory may be written
+            if (split_k) ptx::cluster_wait(); // every peer is running: its shared memory may be written
             if (ok) {
                 // Two chunks per round: both loads are in flight before the single wait.
 #pragma unroll 1
@@ -560,7 +564,7 @@ w8a8_tcgen05_gemm(const __grid_constant__ CUtensorMap map_w, const __grid_consta
                     }
                 }
             }
-            if (Split) ptx::cluster_wait();
+            if (split_k) ptx::cluster_wait();
             if (ok) {
                 // Outer scales exist only when just one operand carries K-group scales.
                 const int channel = n0 + channel_in_tile;
@@ -582,7 +586,7 @@ w8a8_tcgen05_gemm(const __grid_constant__ CUtensorMap map_w, const __grid_consta
                                 words[i + h] = __float_as_uint(v[h] * (outer * outer_w));
                             }
                         }
-                        if (!Split) {
+                        if (!split_k) {
 #pragma unroll
                             for (int i = 0; i < kRows; ++i)
                                 if (token0 + i < valid_tokens) tile_words[(token0 + i) * kBlockChannels + channel_in_tile] = words[i];
@@ -601,7 +605,7 @@ w8a8_tcgen05_gemm(const __grid_constant__ CUtensorMap map_w, const __grid_consta
         ptx::tcgen05_fence_before();
 
         // ---- phase boundary: rows are where their finisher will read them.
-        if (Split) ptx::cluster_sync();
+        if (split_k) ptx::cluster_sync();
         else asm volatile("bar.sync 1, 256;" ::: "memory");
 
         // ---- phase 2: finish token rows; every global access is a 16-byte vector on a 256-byte row.
@@ -633,7 +637,7 @@ w8a8_tcgen05_gemm(const __grid_constant__ CUtensorMap map_w, const __grid_consta
                     skip16 = *reinterpret_cast<const uint4 *>(static_cast<const uint16_t *>(e.residual) +
                                                               size_t(m0 + c) * e.residual_ld + n);
                 uint32_t raw[8];
-                if (!Split) {
+                if (!split_k) {
                     const uint8_t *src = tiles_ptr + size_t(c * kBlockChannels + 8 * j) * 4;
                     const uint4 lo = *reinterpret_cast<const uint4 *>(src), hi = *reinterpret_cast<const uint4 *>(src + 16);
                     raw[0] = lo.x; raw[1] = lo.y; raw[2] = lo.z; raw[3] = lo.w; raw[4] = hi.x; raw[5] = hi.y; raw[6] = hi.z; raw[7] = hi.w;
@@ -680,7 +684,7 @@ w8a8_tcgen05_gemm(const __grid_constant__ CUtensorMap map_w, const __grid_consta
                 if (c >= valid_tokens) continue;
                 const int m = m0 + c;
                 uint32_t raw[8];
-                if (!Split) {
+                if (!split_k) {
                     const uint8_t *src = tiles_ptr + size_t(c * kBlockChannels + 8 * j) * 4;
                     const uint4 lo = *reinterpret_cast<const uint4 *>(src), hi = *reinterpret_cast<const uint4 *>(src + 16);
                     raw[0] = lo.x; raw[1] = lo.y; raw[2] = lo.z; raw[3] = lo.w;
@@ -765,7 +769,7 @@ w8a8_tcgen05_gemm(const __grid_constant__ CUtensorMap map_w, const __grid_consta
             }
         }
     }
-    if ((warp < 2 || warp >= kGemmThreads / 32) && Split) ptx::cluster_sync(); // the other warps' share of the phase barrier
+    if ((warp < 2 || warp >= kGemmThreads / 32) && split_k) ptx::cluster_sync(); // the other warps' share of the phase barrier
 
     __syncthreads(); // tensor memory is drained and nobody else will touch this CTA's shared memory
     if (warp == 1) {
