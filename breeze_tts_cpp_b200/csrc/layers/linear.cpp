@@ -180,13 +180,17 @@ bool Linear::normalized_forward(Workspace &workspace, TensorView input, TensorVi
                                 RowScaledView quantized_output) const {
     validate_types(input, output);
     if (writeback) return false;
-    // Two launches, LayerNorm + quantize and the tensor-core projection, wherever the latter takes the shape (K and N
-    // multiples of 16) and the layer was prepared for the rows: 5.1 against 9.4 us at 1 x 256 -> 1024, 8.5 against 169 at
-    // 372 x 512 -> 2048 (the one-launch kernel normalizes a row once per 64 output channels and reads the weights once
-    // per row). What is left for that kernel: narrow projections whose dimensions are not.
-    const bool two_steps = input.rows <= workspace.rows() && input_channels() % 16 == 0 && output_channels() % 16 == 0;
-    if (!two_steps && ops::normalized_linear(input, weight_, bias_, normalized, output, norm_weight, norm_bias, epsilon, fusion, epilogue,
-                               nullptr, quantized_output))
+    // Two launches, LayerNorm + quantize and the tensor-core projection, wherever the latter takes the shape and was prepared
+    // for the rows: 5.1 against 9.4 us at 1 x 256 -> 1024, 8.5 against 169 at 372 x 512 -> 2048 (the one-launch kernel
+    // normalizes a row once per 64 output channels and reads the weights once per row). What is left for that kernel: narrow
+    // projections whose dimensions are no multiples of 16, whose weights TMA cannot address or that nobody prepared, and
+    // callers that want the normalized rows quantized.
+    const auto &quantization = execution_context(input.device).quantization;
+    const bool two_steps = !quantized_output.values.data && input.rows <= workspace.rows() &&
+                           reinterpret_cast<uintptr_t>(weight_.values.data) % 16 == 0 && quantization &&
+                           quantization->prepared(input.rows, output_channels(), input_channels(), output.type, quantization_layout());
+    if (!two_steps && ops::normalized_linear(input, weight_, bias_, normalized, output, norm_weight, norm_bias, epsilon, fusion,
+                                             epilogue, nullptr, quantized_output))
         return true;
     RowScaledView normalized_input = normalize_input(workspace, input, norm_weight, norm_bias, epsilon, fusion, normalized);
     ops::linear(normalized_input, weight_, bias_, output, epilogue, {}, quantized_output);

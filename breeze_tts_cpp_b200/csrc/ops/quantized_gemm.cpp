@@ -178,6 +178,9 @@ bool QuantizedGemm::normalized_linear(TensorView x, TensorView normalized, Tenso
                                        impl->stream);
     return true;
 }
+bool QuantizedGemm::prepared(int rows, int channels, int reduction, Type output_type, QuantizationGroups groups) const {
+    return impl->find(rows, channels, reduction, output_type, groups.activation, groups.weight);
+}
 LinearPath QuantizedGemm::planned_path(int rows, int channels, int reduction, Type output_type,
                                        QuantizationGroups groups) const {
     const Plan *plan = impl->find(rows, channels, reduction, output_type, groups.activation, groups.weight);

@@ -42,7 +42,8 @@ class QuantizedGemm {
                            TensorView norm_bias, float epsilon, const ops::NormFusion &,
                            RowScaledView weight, TensorView output, const ops::Epilogue &,
                            RowScaledView encoded = {}, const QkvProjectionOutput *writeback = nullptr);
-    // Additions: the chosen path of a prepared shape, and the device status word.
+    // Additions: whether a shape has a plan, the chosen path of a prepared shape, and the device status word.
+    bool prepared(int rows, int output_channels, int input_channels, Type output_type, QuantizationGroups groups = {}) const;
     LinearPath planned_path(int rows, int output_channels, int input_channels, Type output_type,
                             QuantizationGroups groups = {}) const;
     int status() const;
