@@ -150,6 +150,7 @@ int b200q_quant_linear(b200q_context *c, const b200q_path *path, const b200q_row
         for (const TensorView *v : {&x.values, &x.scales, &w.values, &w.scales, &y})
             if (v->device != gpu.device) throw std::invalid_argument("operand is not on the context's device");
         ops::Epilogue e = epilogue_of(epilogue);
+        if (e.gate.data) throw std::invalid_argument("unsupported quantized native Finish path");
         launch_quant_linear({static_cast<LinearKind>(path->kind), path->tokens, path->channels, path->splits},
                             {y.rows, y.cols, x.values.cols, x.group_size, w.group_size}, x.values.data,
                             x.scales.ptr<float>(), w.values.data, w.scales.ptr<float>(), y.data,

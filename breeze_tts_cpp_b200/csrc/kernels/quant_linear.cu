@@ -159,6 +159,13 @@ int multiprocessor_count() {
     return count;
 }
 constexpr size_t kPairSmem = 1024 + kPairBytes;
+// What the persistent kernels' instances compile in behind the product: nothing, the finishing chain, the chain with a gate.
+int chain_level(const FusedEpilogue &e) { return e.gate ? 2 : e.chain ? 1 : 0; }
+template <Type F> auto *pair_kernel(int chain, bool f16) {
+    if (chain == 2) return f16 ? w8a8_tcgen05_prefill_pair<F, 2, true> : w8a8_tcgen05_prefill_pair<F, 2, false>;
+    if (chain == 1) return f16 ? w8a8_tcgen05_prefill_pair<F, 1, true> : w8a8_tcgen05_prefill_pair<F, 1, false>;
+    return f16 ? w8a8_tcgen05_prefill_pair<F, 0, true> : w8a8_tcgen05_prefill_pair<F, 0, false>;
+}
 // CTA pairs: one cluster of two per tile, persistent over the tiles.
 template <Type F>
 void launch_prefill_pair(const CUtensorMap &map_w, const CUtensorMap &map_x, const CUtensorMap &map_out,
@@ -175,16 +182,15 @@ void launch_prefill_pair(const CUtensorMap &map_w, const CUtensorMap &map_x, con
     config.attrs = &attribute;
     config.numAttrs = 1;
     const bool f16 = output_type == Type::F16;
-    auto *kernel = args.ep.chain ? (f16 ? w8a8_tcgen05_prefill_pair<F, true, true> : w8a8_tcgen05_prefill_pair<F, true, false>)
-                                 : (f16 ? w8a8_tcgen05_prefill_pair<F, false, true> : w8a8_tcgen05_prefill_pair<F, false, false>);
-    check(cudaLaunchKernelEx(&config, kernel, map_w, map_x, map_out, map_residual, args), "quantized pair GEMM launch");
+    check(cudaLaunchKernelEx(&config, pair_kernel<F>(chain_level(args.ep), f16), map_w, map_x, map_out, map_residual, args), "quantized pair GEMM launch");
 }
 
 // Persistent K-group kernel: one CTA per multiprocessor over tiles of 128 tokens x `channels` output channels.
 template <Type F, int Channels>
-auto *grouped_kernel(bool chain, bool f16) {
-    return chain ? (f16 ? w8a8_tcgen05_prefill_grouped<F, Channels, true, true> : w8a8_tcgen05_prefill_grouped<F, Channels, true, false>)
-                 : (f16 ? w8a8_tcgen05_prefill_grouped<F, Channels, false, true> : w8a8_tcgen05_prefill_grouped<F, Channels, false, false>);
+auto *grouped_kernel(int chain, bool f16) {
+    if (chain == 2) return f16 ? w8a8_tcgen05_prefill_grouped<F, Channels, 2, true> : w8a8_tcgen05_prefill_grouped<F, Channels, 2, false>;
+    if (chain == 1) return f16 ? w8a8_tcgen05_prefill_grouped<F, Channels, 1, true> : w8a8_tcgen05_prefill_grouped<F, Channels, 1, false>;
+    return f16 ? w8a8_tcgen05_prefill_grouped<F, Channels, 0, true> : w8a8_tcgen05_prefill_grouped<F, Channels, 0, false>;
 }
 template <Type F>
 void launch_prefill_grouped(int channels, const CUtensorMap &map_w, const CUtensorMap &map_x, const CUtensorMap &map_sw,
@@ -201,24 +207,23 @@ void launch_prefill_grouped(int channels, const CUtensorMap &map_w, const CUtens
     attribute.val.programmaticStreamSerializationAllowed = 1;
     config.attrs = &attribute;
     config.numAttrs = 1;
-    const bool chain = args.ep.chain, f16 = output_type == Type::F16;
+    const int chain = chain_level(args.ep);
+    const bool f16 = output_type == Type::F16;
     check(cudaLaunchKernelEx(&config, channels == 64 ? grouped_kernel<F, 64>(chain, f16) : grouped_kernel<F, 128>(chain, f16), map_w, map_x,
                              map_sw, map_out, map_residual, args),
           "quantized K-group prefill GEMM launch");
 }
 
 template <Type F> void raise_limits() {
-    for (bool chain : {false, true})
+    for (int chain : {0, 1, 2})
         for (bool f16 : {false, true}) {
             check(cudaFuncSetAttribute(grouped_kernel<F, 64>(chain, f16), cudaFuncAttributeMaxDynamicSharedMemorySize, int(grouped_smem(64))),
                   "cudaFuncSetAttribute(shared memory)");
             check(cudaFuncSetAttribute(grouped_kernel<F, 128>(chain, f16), cudaFuncAttributeMaxDynamicSharedMemorySize, int(grouped_smem(128))),
                   "cudaFuncSetAttribute(shared memory)");
+            check(cudaFuncSetAttribute(pair_kernel<F>(chain, f16), cudaFuncAttributeMaxDynamicSharedMemorySize, int(kPairSmem)),
+                  "cudaFuncSetAttribute(shared memory)");
         }
-    for (auto *kernel : {w8a8_tcgen05_prefill_pair<F, false, false>, w8a8_tcgen05_prefill_pair<F, false, true>,
-                         w8a8_tcgen05_prefill_pair<F, true, false>, w8a8_tcgen05_prefill_pair<F, true, true>})
-        check(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(kPairSmem)),
-              "cudaFuncSetAttribute(shared memory)");
     raise_limit<F, false, 16>(); raise_limit<F, false, 32>(); raise_limit<F, false, 64>();
     raise_limit<F, false, 128>(); raise_limit<F, false, 256>();
     raise_limit<F, true, 16>(); raise_limit<F, true, 32>(); raise_limit<F, true, 64>(); raise_limit<F, true, 128>();
@@ -324,7 +329,7 @@ void launch_quant_linear(LinearPath config, KernelProblem shape, const void *inp
     bool vector_io = aligned16(y) && shape.channels % 8 == 0;
     if (finish) {
         const auto &e = *finish;
-        if (!ops::fusable(e)) throw std::invalid_argument("unsupported quantized native Finish path");
+        if (!ops::fusable(e) && !ops::gate_fusable(e, shape.rows, shape.channels, output_type)) throw std::invalid_argument("unsupported quantized native Finish path");
         auto same_type = [&](const TensorView &v) { return !v.data || v.type == output_type; };
         if (!same_type(e.bias) || !same_type(e.residual) ||
             (e.bias.data && e.bias.numel() != size_t(shape.channels)) ||
@@ -341,7 +346,10 @@ void launch_quant_linear(LinearPath config, KernelProblem shape, const void *inp
         args.ep.output_scale = e.output_scale; args.ep.alpha = e.alpha;
         args.ep.activation = int(e.activation);
         args.ep.plain_residual = e.residual.data && e.value_scale == 1.f && e.residual_scale == 1.f;
-        args.ep.chain = e.bias.data || e.residual.data || e.value_scale != 1.f || e.output_scale != 1.f ||
+        args.ep.gate = e.gate.data;
+        args.ep.gate_ld = e.gate.rows == 1 ? 0 : e.gate.ld();
+        args.ep.rows_per_sequence = e.rows_per_sequence;
+        args.ep.chain = e.bias.data || e.gate.data || e.residual.data || e.value_scale != 1.f || e.output_scale != 1.f ||
                         e.activation != ops::Activation::Identity;
         vector_io = vector_io && aligned16(e.residual_f32.data);
     }

@@ -50,10 +50,12 @@ constexpr size_t kWorkspaceHeader = 32768;
 struct FusedEpilogue {
     const void *bias = nullptr;         // [N], output dtype
     const void *residual = nullptr;     // [M, residual_ld], output dtype
+    const void *gate = nullptr;         // [sequences or 1, gate_ld], output dtype, 16-byte rows
     const float *residual_f32 = nullptr; // [M, N] fp32, added before the first rounding
     float value_scale = 1.f, residual_scale = 1.f, output_scale = 1.f, alpha = .1f;
     int activation = 0;                 // ops::Activation
     int residual_ld = 0;
+    int gate_ld = 0, rows_per_sequence = 1; // gate_ld is 0 for a gate that all sequences share
     int residual_vector = 0;            // residual rows are 16-byte aligned
     int plain_residual = 0;             // a residual with value_scale == residual_scale == 1
     int chain = 0;                      // nonzero when anything beyond residual_f32 is requested
@@ -109,12 +111,22 @@ template <bool F16> __device__ __forceinline__ uint32_t relu2x16(uint32_t v) {
 // including ReLU; rounding points follow the reference's separate pass
 // (src/ops/kernels/sequence/sequence_internal.cuh:52-74), so GEMM + fused chain equals GEMM followed by that pass
 // bit for bit. Every step ends in a storage value, which is why the row can stay packed between them.
-template <bool F16> __device__ __forceinline__ uint4 chain8(const FusedEpilogue &e, uint4 row, uint4 bias, uint4 skip) {
+// The gate is one more rounding step here instead of a pass over the output: the down projection of a modulated block, 372 x
+// 2048 -> 512, 8.9 -> 6.0 us.
+template <bool F16, bool Gate = true> __device__ __forceinline__ uint4 chain8(const FusedEpilogue &e, uint4 row, uint4 bias, uint4 gate, uint4 skip) {
     uint32_t v[4] = {row.x, row.y, row.z, row.w};
     const uint32_t b[4] = {bias.x, bias.y, bias.z, bias.w}, k[4] = {skip.x, skip.y, skip.z, skip.w};
     if (e.bias) {
 #pragma unroll
         for (int i = 0; i < 4; ++i) v[i] = add2x16<F16>(v[i], b[i]);
+    }
+    if (Gate && e.gate) {
+        const uint32_t g[4] = {gate.x, gate.y, gate.z, gate.w};
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            const float2 x = unpack16<F16>(v[i]), y = unpack16<F16>(g[i]);
+            v[i] = pack2x16<F16>(__fmul_rn(x.x, y.x), __fmul_rn(x.y, y.y));
+        }
     }
     if (e.plain_residual) {
 #pragma unroll
@@ -139,6 +151,10 @@ template <bool F16> __device__ __forceinline__ uint4 chain8(const FusedEpilogue 
         for (int i = 0; i < 4; ++i) v[i] = relu2x16<F16>(v[i]);
     }
     return make_uint4(v[0], v[1], v[2], v[3]);
+}
+// The gate of row `m`, from channel `n` on (n a multiple of 8).
+__device__ __forceinline__ const uint4 *gate_at(const FusedEpilogue &e, int m, int n) {
+    return reinterpret_cast<const uint4 *>(static_cast<const uint16_t *>(e.gate) + size_t(m / e.rows_per_sequence) * e.gate_ld + n);
 }
 // The finishing pass's other activations (its own instruction sequences) on eight packed values. Out of line because
 // they are large: one copy per kernel, eight independent evaluations per call, arguments and result in registers.
@@ -446,6 +462,7 @@ w8a8_tcgen05_gemm(const __grid_constant__ CUtensorMap map_w, const __grid_consta
         ptx::wait_for_upstream(); // activation scales, residuals and the output buffer belong to upstream
         float first_residual[8];
         uint4 first_skip = make_uint4(0, 0, 0, 0); // 16-bit residual of that pass
+        uint4 first_gate = make_uint4(0, 0, 0, 0);
         {
             const int c = split * kRowsPerPass + row_in_pass; // first pass this CTA owns
 #pragma unroll
@@ -453,6 +470,7 @@ w8a8_tcgen05_gemm(const __grid_constant__ CUtensorMap map_w, const __grid_consta
             if (!Plain && e.residual && e.residual_vector && columns_ok && c < valid_tokens)
                 first_skip = *reinterpret_cast<const uint4 *>(static_cast<const uint16_t *>(e.residual) +
                                                               size_t(m0 + c) * e.residual_ld + n);
+            if (!Plain && e.gate && columns_ok && c < valid_tokens) first_gate = *gate_at(e, m0 + c, n);
             if (e.residual_f32 && columns_ok && c < valid_tokens) {
                 const float *src = e.residual_f32 + size_t(m0 + c) * a.n + n;
                 if (a.vector_io) {
@@ -636,6 +654,7 @@ w8a8_tcgen05_gemm(const __grid_constant__ CUtensorMap map_w, const __grid_consta
                 if (kChain && e.residual && local_pass > 0)
                     skip16 = *reinterpret_cast<const uint4 *>(static_cast<const uint16_t *>(e.residual) +
                                                               size_t(m0 + c) * e.residual_ld + n);
+                const uint4 gate = kChain && e.gate && local_pass > 0 ? *gate_at(e, m0 + c, n) : first_gate;
                 uint32_t raw[8];
                 if (!split_k) {
                     const uint8_t *src = tiles_ptr + size_t(c * kBlockChannels + 8 * j) * 4;
@@ -665,7 +684,7 @@ w8a8_tcgen05_gemm(const __grid_constant__ CUtensorMap map_w, const __grid_consta
                 }
                 uint4 packed = Plain && type == int(Type::F16) ? pack8x16<true>(value) : pack8x16<kF16>(value);
                 if (kChain) {
-                    packed = chain8<kF16>(e, packed, bias8, skip16);
+                    packed = chain8<kF16>(e, packed, bias8, gate, skip16);
                     if (e.activation > 1) packed = activate8<kF16>(packed, e.activation, e.alpha);
                 }
                 *reinterpret_cast<uint4 *>(out16 + at) = packed;
@@ -751,7 +770,8 @@ w8a8_tcgen05_gemm(const __grid_constant__ CUtensorMap map_w, const __grid_consta
 #pragma unroll
                             for (int i = 0; i < 4; ++i) skip[i] = uint32_t(src[2 * i]) | (uint32_t(src[2 * i + 1]) << 16);
                         }
-                        row = chain8<kF16>(e, row, bias8, make_uint4(skip[0], skip[1], skip[2], skip[3]));
+                        const uint4 gate = e.gate ? *gate_at(e, m, n) : make_uint4(0, 0, 0, 0);
+                        row = chain8<kF16>(e, row, bias8, gate, make_uint4(skip[0], skip[1], skip[2], skip[3]));
                         if (e.activation > 1) row = activate8<kF16>(row, e.activation, e.alpha);
                     }
                     return row;

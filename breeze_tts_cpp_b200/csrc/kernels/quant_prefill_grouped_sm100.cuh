@@ -57,7 +57,7 @@ struct GroupedArgs {
     FusedEpilogue ep;          // read by the chain instances only
 };
 
-template <Type F, int Channels, bool Chain, bool F16>
+template <Type F, int Channels, int Chain, bool F16>
 __global__ void __launch_bounds__(kGroupedThreads, 1)
 w8a8_tcgen05_prefill_grouped(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_x,
                              const __grid_constant__ CUtensorMap map_sw, const __grid_constant__ CUtensorMap map_out,
@@ -262,6 +262,7 @@ w8a8_tcgen05_prefill_grouped(const __grid_constant__ CUtensorMap map_w, const __
             // All warps decide together whether the tile is stored; the barrier also publishes that the slabs are free.
             ok = ptx::barrier_and(1, kRescaleThreads, ok && !*abort_ptr);
             if (!ok) break;
+            const uint4 *gate_row = Chain == 2 && token_ok ? gate_at(a.ep, token, n0 + c0) : nullptr;
             const float *skip_row = residual && token_ok ? residual + size_t(token) * a.n + n0 + c0 : nullptr;
 #pragma unroll
             for (int q = 0; q < kColumns / 8; ++q) { // eight channels = one 16-byte chunk of the slab row
@@ -286,7 +287,7 @@ w8a8_tcgen05_prefill_grouped(const __grid_constant__ CUtensorMap map_w, const __
                         for (int i = 0; i < 4; ++i) w[i] = uint32_t(b[2 * i]) | (uint32_t(b[2 * i + 1]) << 16);
                         bias = make_uint4(w[0], w[1], w[2], w[3]);
                     }
-                    packed = chain8<F16>(a.ep, packed, bias, skip16 ? *chunk : make_uint4(0, 0, 0, 0));
+                    packed = chain8<F16, Chain == 2>(a.ep, packed, bias, gate_row && inside ? __ldg(gate_row + q) : make_uint4(0, 0, 0, 0), skip16 ? *chunk : make_uint4(0, 0, 0, 0));
                 }
                 *chunk = packed;
             }

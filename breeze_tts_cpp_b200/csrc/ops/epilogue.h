@@ -37,6 +37,16 @@ inline bool fusable(const Epilogue &e) {
            e.input_repeat == 1 && !e.residual_rows && e.activation != Activation::Mish && !e.packed &&
            !e.condition_sources && !e.output_rows;
 }
+// True for one more case it can apply: a per-sequence gate over whole sequences that can be read in 16-byte pieces, with a
+// residual row per output row.
+inline bool gate_fusable(const Epilogue &e, int rows, int cols, Type type) {
+    Epilogue rest = e;
+    rest.gate = {};
+    return e.gate.data && fusable(rest) && !e.residual_f32.data && e.gate.type == type && e.gate.cols == cols && cols % 8 == 0 &&
+           e.gate.ld() % 8 == 0 && reinterpret_cast<uintptr_t>(e.gate.data) % 16 == 0 && e.rows_per_sequence >= 1 &&
+           rows % e.rows_per_sequence == 0 && (e.gate.rows == 1 || e.gate.rows == rows / e.rows_per_sequence) &&
+           (!e.residual.data || (e.residual.type == type && e.residual.rows == rows && e.residual.cols == cols));
+}
 // True when nothing at all follows the projection.
 inline bool plain(const Epilogue &e) {
     return !e.bias.data && !e.residual.data && !e.residual_f32.data && !e.gate.data && !e.condition.data &&

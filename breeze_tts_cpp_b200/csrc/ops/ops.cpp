@@ -81,7 +81,8 @@ void linear(const LinearOperand &input, const LinearOperand &weight, TensorView 
         if (quantized_output.values.data) quantize_rows(output, quantized_output);
         return;
     }
-    if (gpu.quantization->linear_finish(activation, *matrix, output, e)) {
+    // A gate followed by the re-quantization leaves `output` as the projection wrote it, so it takes the separate pass.
+    if (!(e.gate.data && quantized_output.values.data) && gpu.quantization->linear_finish(activation, *matrix, output, e)) {
         if (quantized_output.values.data) quantize_rows(output, quantized_output);
         return;
     }

@@ -120,7 +120,7 @@ void QuantizedGemm::linear(RowScaledView input, RowScaledView weight, TensorView
 }
 bool QuantizedGemm::linear_finish(RowScaledView input, RowScaledView weight, TensorView output,
                                   const ops::Epilogue &finish) {
-    if (!ops::fusable(finish)) return false;
+    if (!ops::fusable(finish) && !ops::gate_fusable(finish, output.rows, output.cols, output.type)) return false;
     check_linear(impl->format, input, weight, output, impl->workspace.device());
     const Plan *plan = impl->find(output.rows, output.cols, input.values.cols, output.type, input.group_size,
                                   weight.group_size);
