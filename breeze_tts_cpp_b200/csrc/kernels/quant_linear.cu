@@ -159,12 +159,23 @@ int multiprocessor_count() {
     return count;
 }
 constexpr size_t kPairSmem = 1024 + kPairBytes;
-// What the persistent kernels' instances compile in behind the product: nothing, the finishing chain, the chain with a gate.
-int chain_level(const FusedEpilogue &e) { return e.gate ? 2 : e.chain ? 1 : 0; }
+// What the persistent kernels' instances compile in behind the product: 1 the finishing chain, 2 a gate, 4 an activation beyond
+// ReLU (a gate never comes without the chain, nor does an activation).
+constexpr int kChainLevels[] = {0, 1, 3, 5, 7};
+int chain_level(const FusedEpilogue &e) { return !e.chain ? 0 : 1 + (e.gate ? 2 : 0) + (e.activation > 1 ? 4 : 0); }
+template <class Pick> auto by_chain(int level, Pick pick) {
+    switch (level) {
+    case 0: return pick(std::integral_constant<int, 0>{});
+    case 1: return pick(std::integral_constant<int, 1>{});
+    case 3: return pick(std::integral_constant<int, 3>{});
+    case 5: return pick(std::integral_constant<int, 5>{});
+    default: return pick(std::integral_constant<int, 7>{});
+    }
+}
 template <Type F> auto *pair_kernel(int chain, bool f16) {
-    if (chain == 2) return f16 ? w8a8_tcgen05_prefill_pair<F, 2, true> : w8a8_tcgen05_prefill_pair<F, 2, false>;
-    if (chain == 1) return f16 ? w8a8_tcgen05_prefill_pair<F, 1, true> : w8a8_tcgen05_prefill_pair<F, 1, false>;
-    return f16 ? w8a8_tcgen05_prefill_pair<F, 0, true> : w8a8_tcgen05_prefill_pair<F, 0, false>;
+    return by_chain(chain, [&](auto level) {
+        return f16 ? w8a8_tcgen05_prefill_pair<F, decltype(level)::value, true> : w8a8_tcgen05_prefill_pair<F, decltype(level)::value, false>;
+    });
 }
 // CTA pairs: one cluster of two per tile, persistent over the tiles.
 template <Type F>
@@ -188,9 +199,10 @@ void launch_prefill_pair(const CUtensorMap &map_w, const CUtensorMap &map_x, con
 // Persistent K-group kernel: one CTA per multiprocessor over tiles of 128 tokens x `channels` output channels.
 template <Type F, int Channels>
 auto *grouped_kernel(int chain, bool f16) {
-    if (chain == 2) return f16 ? w8a8_tcgen05_prefill_grouped<F, Channels, 2, true> : w8a8_tcgen05_prefill_grouped<F, Channels, 2, false>;
-    if (chain == 1) return f16 ? w8a8_tcgen05_prefill_grouped<F, Channels, 1, true> : w8a8_tcgen05_prefill_grouped<F, Channels, 1, false>;
-    return f16 ? w8a8_tcgen05_prefill_grouped<F, Channels, 0, true> : w8a8_tcgen05_prefill_grouped<F, Channels, 0, false>;
+    return by_chain(chain, [&](auto level) {
+        return f16 ? w8a8_tcgen05_prefill_grouped<F, Channels, decltype(level)::value, true>
+                   : w8a8_tcgen05_prefill_grouped<F, Channels, decltype(level)::value, false>;
+    });
 }
 template <Type F>
 void launch_prefill_grouped(int channels, const CUtensorMap &map_w, const CUtensorMap &map_x, const CUtensorMap &map_sw,
@@ -215,7 +227,7 @@ void launch_prefill_grouped(int channels, const CUtensorMap &map_w, const CUtens
 }
 
 template <Type F> void raise_limits() {
-    for (int chain : {0, 1, 2})
+    for (int chain : kChainLevels)
         for (bool f16 : {false, true}) {
             check(cudaFuncSetAttribute(grouped_kernel<F, 64>(chain, f16), cudaFuncAttributeMaxDynamicSharedMemorySize, int(grouped_smem(64))),
                   "cudaFuncSetAttribute(shared memory)");
@@ -359,8 +371,8 @@ void launch_quant_linear(LinearPath config, KernelProblem shape, const void *inp
         (!args.ep.residual || args.ep.residual_vector)) {
         PairArgs pair{args.m, args.n, args.k, xs, ws, args.ep.residual_f32, args.status};
         pair.ep = args.ep;
-        // Epilogue cycles per channel of 128 tokens, measured: plain 16, bias and residual 31, an activation 55 (tanh
-        // GELU) to 100 (SiLU).
+        // Epilogue cycles per channel of 128 tokens: plain 16, bias and residual 31, an activation 40 to 55 more (the choice hardly
+        // depends on it).
         const double column_cycles = args.ep.activation > 1 ? 75.0 : args.ep.residual || args.ep.residual_f32 ? 31.0
                                                                   : args.ep.chain ? 20.0 : kPairColumnCycles;
         pair.channels = pair_channel_tile(shape.rows, shape.channels, kb_total, multiprocessor_count() / 2, column_cycles).channels;

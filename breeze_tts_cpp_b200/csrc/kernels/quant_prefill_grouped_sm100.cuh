@@ -262,7 +262,7 @@ w8a8_tcgen05_prefill_grouped(const __grid_constant__ CUtensorMap map_w, const __
             // All warps decide together whether the tile is stored; the barrier also publishes that the slabs are free.
             ok = ptx::barrier_and(1, kRescaleThreads, ok && !*abort_ptr);
             if (!ok) break;
-            const uint4 *gate_row = Chain == 2 && token_ok ? gate_at(a.ep, token, n0 + c0) : nullptr;
+            const uint4 *gate_row = (Chain & 2) && token_ok ? gate_at(a.ep, token, n0 + c0) : nullptr;
             const float *skip_row = residual && token_ok ? residual + size_t(token) * a.n + n0 + c0 : nullptr;
 #pragma unroll
             for (int q = 0; q < kColumns / 8; ++q) { // eight channels = one 16-byte chunk of the slab row
@@ -287,17 +287,13 @@ w8a8_tcgen05_prefill_grouped(const __grid_constant__ CUtensorMap map_w, const __
                         for (int i = 0; i < 4; ++i) w[i] = uint32_t(b[2 * i]) | (uint32_t(b[2 * i + 1]) << 16);
                         bias = make_uint4(w[0], w[1], w[2], w[3]);
                     }
-                    packed = chain8<F16, Chain == 2>(a.ep, packed, bias, gate_row && inside ? __ldg(gate_row + q) : make_uint4(0, 0, 0, 0), skip16 ? *chunk : make_uint4(0, 0, 0, 0));
+                    packed = chain8<F16, (Chain & 2) != 0>(a.ep, packed, bias, gate_row && inside ? __ldg(gate_row + q) : make_uint4(0, 0, 0, 0), skip16 ? *chunk : make_uint4(0, 0, 0, 0));
                 }
                 *chunk = packed;
             }
-            if (Chain && a.ep.activation > 1) {
-#pragma unroll 1
-                for (int q = 0; q < kColumns / 8; ++q) {
-                    uint4 *chunk = reinterpret_cast<uint4 *>(slab_row + ((((c0 & 63) / 8 + q) ^ (row & 7)) * 16));
-                    *chunk = activate8<F16>(*chunk, a.ep.activation, a.ep.alpha);
-                }
-            }
+            if (Chain & 4)
+                activate_chunks<F16, kColumns / 8>(
+                    [&](int q) { return reinterpret_cast<uint4 *>(slab_row + ((((c0 & 63) / 8 + q) ^ (row & 7)) * 16)); }, a.ep.activation, a.ep.alpha);
             ptx::fence_proxy_async_smem(); // the rows are about to be read by the TMA engine
             (void)ptx::barrier_and(1, kRescaleThreads, true);
             if (storer) {

@@ -47,8 +47,8 @@ struct PairArgs {
     FusedEpilogue ep;     // read by the chain instances only
 };
 
-// Instances: `Chain` compiles the finishing chain into the epilogue (2: with a gate, which costs registers that the plain chain
-// would miss: 31.7 against 33.4 us for a 750-row block); `F16` is the output type (else bf16).
+// Instances: `Chain` compiles the finishing chain into the epilogue (bit 0; bit 1: with a gate, bit 2: with an activation beyond
+// ReLU, which cost registers and code that the others would miss: 31.7 against 33.4 us for a 750-row block); `F16` is the output type (else bf16).
 template <Type F, int Chain, bool F16>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kPairThreads, 1)
 w8a8_tcgen05_prefill_pair(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_x,
@@ -242,7 +242,7 @@ w8a8_tcgen05_prefill_pair(const __grid_constant__ CUtensorMap map_w, const __gri
                     ok = ptx::mbar_wait(ptx::smem_u32(&residual_full[slab]), (residual_phase >> slab) & 1u, abort_ptr);
                     residual_phase ^= 1u << slab;
                 }
-                const uint4 *gate_row = Chain == 2 && token_ok ? gate_at(a.ep, token, n0 + c0) : nullptr;
+                const uint4 *gate_row = (Chain & 2) && token_ok ? gate_at(a.ep, token, n0 + c0) : nullptr;
                 const float *skip_row = residual && token_ok && n0 + c0 < a.n ? residual + size_t(token) * a.n + n0 + c0 : nullptr;
 #pragma unroll
                 for (int q = 0; q < 4; ++q) { // eight channels = one 16-byte chunk of the slab row
@@ -265,18 +265,15 @@ w8a8_tcgen05_prefill_pair(const __grid_constant__ CUtensorMap map_w, const __gri
                     }
                     uint4 packed = pack8x16<F16>(value);
                     if (Chain)
-                        packed = chain8<F16, Chain == 2>(a.ep, packed, *reinterpret_cast<const uint4 *>(&bias_tile[c0 + 8 * q]),
+                        packed = chain8<F16, (Chain & 2) != 0>(a.ep, packed, *reinterpret_cast<const uint4 *>(&bias_tile[c0 + 8 * q]),
                                              gate_row && n0 + c0 + 8 * q < a.n ? __ldg(gate_row + q) : make_uint4(0, 0, 0, 0),
                                              skip16 ? *chunk : make_uint4(0, 0, 0, 0));
                     *chunk = packed;
                 }
-                if (Chain && a.ep.activation > 1) {
-                    // A pass of its own over the thread's finished row: nothing but eight values is live in it.
-#pragma unroll 1
-                    for (int q = 0; q < 4; ++q) {
-                        uint4 *chunk = reinterpret_cast<uint4 *>(out_row + (((half * 4 + q) ^ (row & 7)) * 16));
-                        *chunk = activate8<F16>(*chunk, a.ep.activation, a.ep.alpha);
-                    }
+                if (Chain & 4) {
+                    // A pass of its own over the thread's finished row: nothing but its values is live in it.
+                    activate_chunks<F16, 4>([&](int q) { return reinterpret_cast<uint4 *>(out_row + (((half * 4 + q) ^ (row & 7)) * 16)); },
+                                            a.ep.activation, a.ep.alpha);
                 }
                 ptx::fence_proxy_async_smem(); // the rows are about to be read by the TMA engine
                 // With two buffers the next slab's must be free by the time this barrier lets anyone write it.
