@@ -216,21 +216,16 @@ template <bool F16> __device__ __noinline__ uint4 activate8(uint4 row, int kind,
     activate<F16>(v, kind, alpha);
     return make_uint4(v[0], v[1], v[2], v[3]);
 }
-// A thread's finished chunks of eight values in a slab, four at a time: the evaluations are latency (two warps a scheduler). GEMM of 3000 x
-// 2048 -> 8192 with SiLU / tanh GELU, eight values a call against this: 68.5 -> 62.5, 52.9 -> 45.0 us.
+// A thread's finished chunks of eight values in a slab. In line, eight values at a time: four chunks at a time keep more in flight
+// (GEMM 3000 x 2048 -> 8192 with SiLU / tanh GELU: a call per chunk 69 / 53 us, this 66 / 50, four chunks 63 / 45), but their code
+// is met cold when a block has only a few tiles per pair (block of 750 x 1024 with GELU: 32.6, 32.2 and 33.2 us).
 template <bool F16, int Chunks, class At> __device__ __forceinline__ void activate_chunks(At at, int kind, float alpha) {
-    constexpr int kStep = Chunks < 4 ? Chunks : 4;
 #pragma unroll 1
-    for (int q = 0; q < Chunks; q += kStep) {
-        uint32_t v[4 * kStep];
-#pragma unroll
-        for (int i = 0; i < kStep; ++i) {
-            const uint4 row = *at(q + i);
-            v[4 * i] = row.x; v[4 * i + 1] = row.y; v[4 * i + 2] = row.z; v[4 * i + 3] = row.w;
-        }
+    for (int q = 0; q < Chunks; ++q) {
+        const uint4 row = *at(q);
+        uint32_t v[4] = {row.x, row.y, row.z, row.w};
         activate<F16>(v, kind, alpha);
-#pragma unroll
-        for (int i = 0; i < kStep; ++i) *at(q + i) = make_uint4(v[4 * i], v[4 * i + 1], v[4 * i + 2], v[4 * i + 3]);
+        *at(q) = make_uint4(v[0], v[1], v[2], v[3]);
     }
 }
 template <bool F16> __device__ __forceinline__ uint4 pack8x16(const float (&v)[8]) {
