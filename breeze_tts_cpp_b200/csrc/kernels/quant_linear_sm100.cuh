@@ -111,8 +111,8 @@ template <bool F16> __device__ __forceinline__ uint32_t relu2x16(uint32_t v) {
 // including ReLU; rounding points follow the reference's separate pass
 // (src/ops/kernels/sequence/sequence_internal.cuh:52-74), so GEMM + fused chain equals GEMM followed by that pass
 // bit for bit. Every step ends in a storage value, which is why the row can stay packed between them.
-// The gate is one more rounding step here instead of a pass over the output: the down projection of a modulated block, 372 x
-// 2048 -> 512, 8.9 -> 6.0 us.
+// The gate is one more rounding step here instead of a launch and a pass over the output: modulated FP8 block of 4 x 93 x 512,
+// 23.7 -> 18.8 us.
 template <bool F16, bool Gate = true> __device__ __forceinline__ uint4 chain8(const FusedEpilogue &e, uint4 row, uint4 bias, uint4 gate, uint4 skip) {
     uint32_t v[4] = {row.x, row.y, row.z, row.w};
     const uint32_t b[4] = {bias.x, bias.y, bias.z, bias.w}, k[4] = {skip.x, skip.y, skip.z, skip.w};
