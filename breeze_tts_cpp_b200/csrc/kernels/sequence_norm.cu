@@ -231,7 +231,7 @@ layer_norm_quantize_packed(NormArgs a, unsigned char *__restrict__ q, float *__r
             for (int i = 0; i < 4; ++i) {
                 w[i] = add16x2<T>(w[i], pw[i]);
                 if (fusion.gate) w[i] = mul16x2<T>(w[i], gw[i]);
-                if (fusion.gate || fusion.residual) w[i] = add16x2<T>(w[i], rw[i]);
+                w[i] = add16x2<T>(w[i], rw[i]); // also without a residual: -0 + 0 is +0
             }
             mine[col / 8] = v[j];
             if (raw) *reinterpret_cast<uint4 *>(raw + col) = v[j];
