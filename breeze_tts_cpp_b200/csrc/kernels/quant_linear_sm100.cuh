@@ -77,6 +77,7 @@ struct GemmArgs {
     // `wait_limit_cycles` (0 = the regular limit). Both zero in normal operation.
     int expiry_extra_bytes;
     long long wait_limit_cycles;
+    long long refill_delay_cycles; // the refill waiter's start held back (quant_linear_inject_refill_delay); 0 in normal operation
     FusedEpilogue ep;
 };
 
@@ -321,9 +322,15 @@ w8a8_tcgen05_gemm(const __grid_constant__ CUtensorMap map_w, const __grid_consta
         int stage = refill_from == a.stages ? 0 : refill_from;
         uint32_t phase = refill_from == a.stages ? 1u : 0u;
         const int ahead = min(a.stages, kb_count);
-        // A parity test passes on a barrier whose phase before has not completed either: every phase has to be seen in turn.
-        if (refill_from < kb_count)
-            for (int i = 0; i < ahead && ok; ++i) ok = ptx::mbar_wait(ptx::smem_u32(&full_bar[i]), 0u, abort_ptr, limit);
+        // A parity test tells a phase from the one before and the one after only, so a waiter has to see every phase in turn. The
+        // stages' first phases are the issuer's: it has seen all of them when it arrives here. The second ones cannot complete
+        // unseen, because the third needs MMAs that wait for this warp's verdict on the second. (A waiter that tested the first
+        // phases itself could come so late that a stage had been filled twice, and then wait for a phase that never comes.)
+        if (refill_from < kb_count) {
+            __syncwarp();
+            ptx::pair_wait();
+            for (const long long start = clock64(); clock64() - start < a.refill_delay_cycles;) {}
+        }
         for (int it = refill_from; it < kb_count; ++it) {
             if (Grouped && it * units >= kAccBuffers) // the epilogue drained these accumulators' previous groups
                 for (int u = 0; u < units && ok; ++u)
@@ -399,6 +406,7 @@ w8a8_tcgen05_gemm(const __grid_constant__ CUtensorMap map_w, const __grid_consta
             for (int i = 0; i < ahead && ok; ++i) ok = ptx::mbar_wait(ptx::smem_u32(&full_bar[i]), 0u, abort_ptr, wait_limit);
             ok = ok && ptx::mbar_wait(ptx::smem_u32(&x_full), 0u, abort_ptr, wait_limit);
             ok = __all_sync(0xffffffffu, ok);
+            if (refill_from < kb_count) ptx::pair_arrive(); // before the burst, whose commits let the producer refill
             // The prefetched stages need no barrier at all any more, so their MMAs go out back to back
             // (any shared-memory access between MMA issues stalls the issuing warp for a couple of
             // hundred cycles). Stage i holds K block i here; in K-group mode K block i also has

@@ -42,10 +42,11 @@ def test_persistent_group_kernel_matches_weight_streaming_kernel(ctx_factory, mo
         assert float((out.double() - other.double()).norm() / other.double().norm()) < 2e-3
 
 
+@pytest.mark.parametrize("late", [0, 200_000])  # cycles the refill waiter starts late: by then stages may have been filled twice
 @pytest.mark.parametrize("group,m,tokens,splits,k", [(128, 3, 16, 1, 6144), (128, 20, 32, 1, 4096), (128, 64, 64, 1, 2560), (128, 100, 128, 2, 2304),
                                                      (32, 9, 16, 1, 3072), (64, 33, 64, 1, 2048), (0, 16, 16, 1, 6144), (0, 64, 64, 1, 3072)])
-def test_weight_streaming_kernel_refills_ring_and_accumulators(oracle, ctx_factory, group, m, tokens, splits, k):
-    from breeze_tts_cpp_b200 import ops
+def test_weight_streaming_kernel_refills_ring_and_accumulators(oracle, ctx_factory, group, m, tokens, splits, k, late):
+    from breeze_tts_cpp_b200 import _lib, ops
     ctx = ctx_factory("group_int8" if group else "int8")
     n = 144
     xq, sx = oracle.row_quantize(oracle.to_bf16(synth.activations(m, k, m + k, student_t=3.0)), I8, group, 0)
@@ -54,6 +55,7 @@ def test_weight_streaming_kernel_refills_ring_and_accumulators(oracle, ctx_facto
     xv = ops.RowScaledView(torch.from_numpy(xq).cuda(), scales(sx, m), I8, group, 0)
     wv = ops.RowScaledView(torch.from_numpy(wq).cuda(), scales(sw, n), I8, group, 0)
     out = torch.empty(m, n, dtype=torch.bfloat16, device="cuda")
+    _lib.call("b200q_inject_refill_delay", late)
     ctx.quant_linear((TCGEN05, tokens, 128, splits), xv, wv, out)
     want, exact = oracle.quant_linear(xq, sx, wq, sw, I8, group, group)
     assert ctx.status() == 0
