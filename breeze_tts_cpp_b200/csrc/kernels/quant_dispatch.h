@@ -47,8 +47,8 @@ void quant_linear_reset_workspace(void *workspace, size_t workspace_bytes, cudaS
 // teardown, stores nothing and raises the status word. One-shot; nothing is left in flight.
 void quant_linear_inject_wait_expiry(int extra_bytes, long long limit_cycles);
 // The same for scheduling: in the NEXT weight-streaming GEMM of this thread the warp that waits for refilled stages starts
-// `cycles` SM cycles late (at most 10^7), as it may when its multiprocessor is busy. Results do not depend on it.
-void quant_linear_inject_refill_delay(long long cycles);
+// about that many nanoseconds late (at most 10^6), as it may when its multiprocessor is busy. Results do not depend on it.
+void quant_linear_inject_refill_delay(int nanoseconds);
 // Blocking read of the status word: 0 = clean, otherwise 1 + index of the tile whose bounded wait gave up.
 int quant_linear_status(const void *workspace, cudaStream_t stream);
 } // namespace tts

@@ -285,15 +285,15 @@ struct WaitExpiry {
     long long limit_cycles = 0;
 };
 thread_local WaitExpiry pending_expiry;
-thread_local long long pending_refill_delay = 0;
+thread_local unsigned pending_refill_delay = 0;
 } // namespace
 void quant_linear_inject_wait_expiry(int extra_bytes, long long limit_cycles) {
     if (extra_bytes < 0 || extra_bytes > 1024 || limit_cycles < 0) throw std::invalid_argument("invalid wait-expiry injection");
     pending_expiry = {extra_bytes, limit_cycles};
 }
-void quant_linear_inject_refill_delay(long long cycles) {
-    if (cycles < 0 || cycles > 10000000) throw std::invalid_argument("invalid refill delay");
-    pending_refill_delay = cycles;
+void quant_linear_inject_refill_delay(int nanoseconds) {
+    if (nanoseconds < 0 || nanoseconds > 1000000) throw std::invalid_argument("invalid refill delay");
+    pending_refill_delay = unsigned(nanoseconds);
 }
 
 LinearPath select_tcgen05_path(KernelProblem p, Type format, int sms, size_t workspace_bytes) {
@@ -425,7 +425,7 @@ void launch_quant_linear(LinearPath config, KernelProblem shape, const void *inp
     args.expiry_extra_bytes = pending_expiry.extra_bytes; // one-shot, only the weight-streaming kernel honours it
     args.wait_limit_cycles = pending_expiry.limit_cycles;
     pending_expiry = {};
-    args.refill_delay_cycles = pending_refill_delay;
+    args.refill_delay_ns = pending_refill_delay;
     pending_refill_delay = 0;
     args.stages = launch.stages;
     args.tile_region = int(launch.tile_region);

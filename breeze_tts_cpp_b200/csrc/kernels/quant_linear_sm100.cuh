@@ -77,7 +77,7 @@ struct GemmArgs {
     // `wait_limit_cycles` (0 = the regular limit). Both zero in normal operation.
     int expiry_extra_bytes;
     long long wait_limit_cycles;
-    long long refill_delay_cycles; // the refill waiter's start held back (quant_linear_inject_refill_delay); 0 in normal operation
+    unsigned refill_delay_ns; // the refill waiter's start held back (quant_linear_inject_refill_delay); 0 in normal operation
     FusedEpilogue ep;
 };
 
@@ -263,7 +263,8 @@ w8a8_tcgen05_gemm(const __grid_constant__ CUtensorMap map_w, const __grid_consta
     constexpr uint32_t kPassBytes = kRowsPerPass * kBlockChannels * 4;
 
     extern __shared__ uint8_t dynamic_smem[];
-    __shared__ alignas(8) uint64_t full_bar[kMaxStages], empty_bar[kMaxStages], acc_full[kAccBuffers], acc_empty[kAccBuffers], x_full;
+    __shared__ alignas(8) uint64_t full_bar[kMaxStages], empty_bar[kMaxStages], acc_full[kAccBuffers], acc_empty[kAccBuffers];
+    __shared__ alignas(8) uint64_t w_full, x_full; // the first fill of all stages: weights, activations
     __shared__ uint32_t tmem_slot;
     __shared__ int abort_flag;
     __shared__ float sx_tile[BN]; // per-row activation scales of this token tile
@@ -305,6 +306,7 @@ w8a8_tcgen05_gemm(const __grid_constant__ CUtensorMap map_w, const __grid_consta
             ptx::mbar_init(ptx::smem_u32(&acc_full[b]), 1);
             ptx::mbar_init(ptx::smem_u32(&acc_empty[b]), kEpilogueThreads / 32);
         }
+        ptx::mbar_init(ptx::smem_u32(&w_full), 1);
         ptx::mbar_init(ptx::smem_u32(&x_full), 1);
         abort_flag = 0;
         ptx::fence_barrier_init();
@@ -320,17 +322,12 @@ w8a8_tcgen05_gemm(const __grid_constant__ CUtensorMap map_w, const __grid_consta
     const int refill_from = Grouped ? min(min(a.stages, kb_count), kAccBuffers / units) : min(a.stages, kb_count);
     const auto wait_for_refills = [&](bool ok, long long limit) {
         int stage = refill_from == a.stages ? 0 : refill_from;
-        uint32_t phase = refill_from == a.stages ? 1u : 0u;
+        uint32_t phase = refill_from == a.stages ? 0u : 1u;
         const int ahead = min(a.stages, kb_count);
-        // A parity test tells a phase from the one before and the one after only, so a waiter has to see every phase in turn. The
-        // stages' first phases are the issuer's: it has seen all of them when it arrives here. The second ones cannot complete
-        // unseen, because the third needs MMAs that wait for this warp's verdict on the second. (A waiter that tested the first
-        // phases itself could come so late that a stage had been filled twice, and then wait for a phase that never comes.)
-        if (refill_from < kb_count) {
-            __syncwarp();
-            ptx::pair_wait();
-            for (const long long start = clock64(); clock64() - start < a.refill_delay_cycles;) {}
-        }
+        // A parity test cannot tell a phase from the second one after it, so this warp, however late it comes, must find no barrier
+        // two phases on. It does not: full_bar counts refills only (the first fill has barriers of its own), and the next refill of
+        // a stage needs MMAs that wait for the verdict on this one; likewise the accumulators.
+        if (a.refill_delay_ns) __nanosleep(a.refill_delay_ns);
         for (int it = refill_from; it < kb_count; ++it) {
             if (Grouped && it * units >= kAccBuffers) // the epilogue drained these accumulators' previous groups
                 for (int u = 0; u < units && ok; ++u)
@@ -355,20 +352,18 @@ w8a8_tcgen05_gemm(const __grid_constant__ CUtensorMap map_w, const __grid_consta
             ptx::prefetch_tensormap(&map_w);
             ptx::prefetch_tensormap(&map_x);
         }
-        // Weights do not depend on the upstream kernel: fill the ring with weight tiles first
-        // (one barrier per stage), then wait for upstream and add the activation tiles of all
-        // those stages under ONE barrier. A barrier test between MMA issues costs the issuing
-        // thread about 200 cycles, so the burst over the prefetched stages must not need any.
+        // Weights do not depend on the upstream kernel: fill the ring with weight tiles first, then wait for upstream
+        // and add the activation tiles of all those stages, each under ONE barrier. A barrier test between MMA issues
+        // costs the issuing thread about 200 cycles, so the burst over the prefetched stages must not need any.
         // Weights are streamed once: they are marked first-to-evict so that the few megabytes of
         // activations the chain keeps passing from kernel to kernel stay in L2.
         const uint64_t stream_once = ptx::policy_evict_first();
         const int ahead = min(a.stages, kb_count);
         if (ptx::elect_one()) { // one election around a burst: per copy or per MMA it costs some 20 cycles
-            for (int i = 0; i < ahead; ++i) {
-                const uint32_t bar = ptx::smem_u32(&full_bar[i]);
-                ptx::mbar_arrive_expect_tx(bar, kWeightBytes + (i == 0 ? uint32_t(a.expiry_extra_bytes) : 0u));
+            const uint32_t bar = ptx::smem_u32(&w_full);
+            ptx::mbar_arrive_expect_tx(bar, uint32_t(ahead) * kWeightBytes + uint32_t(a.expiry_extra_bytes));
+            for (int i = 0; i < ahead; ++i)
                 ptx::tma_load_2d_hint(tiles_base + uint32_t(i) * kStageBytes, &map_w, bar, (kb_begin + i) * kBlockK, n0, stream_once);
-            }
         }
         __syncwarp();
         ptx::wait_for_upstream();
@@ -399,14 +394,11 @@ w8a8_tcgen05_gemm(const __grid_constant__ CUtensorMap map_w, const __grid_consta
         // The whole warp runs the loop so that stage indices and descriptors stay warp-uniform (the
         // tensor-core instructions take them from uniform registers); one elected lane issues.
         {
-            // The weight tiles of the prefetched stages land while the upstream kernel still runs:
-            // collect those barriers now, off the critical path, then wait once for the activations.
-            const int ahead = min(a.stages, kb_count);
-            bool ok = true;
-            for (int i = 0; i < ahead && ok; ++i) ok = ptx::mbar_wait(ptx::smem_u32(&full_bar[i]), 0u, abort_ptr, wait_limit);
+            // The weight tiles of the prefetched stages land while the upstream kernel still runs: they are waited
+            // for first, off the critical path, then the activations.
+            bool ok = ptx::mbar_wait(ptx::smem_u32(&w_full), 0u, abort_ptr, wait_limit);
             ok = ok && ptx::mbar_wait(ptx::smem_u32(&x_full), 0u, abort_ptr, wait_limit);
             ok = __all_sync(0xffffffffu, ok);
-            if (refill_from < kb_count) ptx::pair_arrive(); // before the burst, whose commits let the producer refill
             // The prefetched stages need no barrier at all any more, so their MMAs go out back to back
             // (any shared-memory access between MMA issues stalls the issuing warp for a couple of
             // hundred cycles). Stage i holds K block i here; in K-group mode K block i also has

@@ -427,11 +427,7 @@ __device__ __forceinline__ bool pair_barrier_and(bool ok) {
                  : "memory");
     return all != 0;
 }
-// Named hardware barrier 5 between the same two warps, one-sided: the issuer's arrival does not wait, the waiter goes on once
-// the issuer has come this far.
-__device__ __forceinline__ void pair_arrive() { asm volatile("bar.arrive 5, 64;" ::: "memory"); }
-__device__ __forceinline__ void pair_wait() { asm volatile("bar.sync 5, 64;" ::: "memory"); }
-// All of these are aligned: the lanes of a warp have to arrive together (vote after anything that lanes can leave apart).
+// Both forms are aligned: the lanes of a warp have to arrive together (vote after anything that lanes can leave apart).
 // The same over any named barrier: every one of the `threads` participants learns whether all of
 // them passed `ok`. Used where several warps must agree to leave a loop together, because a warp
 // that left alone would strand its siblings at their next named barrier.

@@ -228,9 +228,9 @@ int b200q_static_status(int32_t device, void *stream, int32_t *status, char *err
 int b200q_inject_wait_expiry(int32_t extra_bytes, int64_t limit_cycles, char *error, size_t error_capacity);
 
 /* No counterpart in the reference. In the next weight-streaming GEMM this thread launches, the warp that
- * waits for refilled pipeline stages starts `cycles` (at most 10^7) SM cycles late; nothing else changes and
- * the results must not. One-shot. */
-int b200q_inject_refill_delay(int64_t cycles, char *error, size_t error_capacity);
+ * waits for refilled pipeline stages starts that many nanoseconds late (at most 10^6, about); nothing else
+ * changes and the results must not. One-shot. */
+int b200q_inject_refill_delay(int32_t nanoseconds, char *error, size_t error_capacity);
 
 /* Blocks until the context's stream is idle and returns the device status word through `status`:
  * 0 = clean; nonzero = a bounded device-side wait gave up (results are invalid). */
