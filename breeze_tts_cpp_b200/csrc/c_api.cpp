@@ -155,7 +155,7 @@ int b200q_quant_linear(b200q_context *c, const b200q_path *path, const b200q_row
                             {y.rows, y.cols, x.values.cols, x.group_size, w.group_size}, x.values.data,
                             x.scales.ptr<float>(), w.values.data, w.scales.ptr<float>(), y.data,
                             gpu.gemm_workspace.data(), gpu.gemm_workspace.size(), gpu.stream, x.values.type, y.type,
-                            epilogue ? &e : nullptr);
+                            epilogue ? &e : nullptr, gpu.quantization->announced(w.values));
     });
 }
 int b200q_select_path(b200q_context *c, int32_t rows, int32_t channels, int32_t reduction, int32_t activation_group,

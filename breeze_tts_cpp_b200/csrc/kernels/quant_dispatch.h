@@ -22,11 +22,12 @@ void launch_quant_linear(LinearPath config, KernelProblem shape, const void *inp
 KernelResources quant_linear_finish_resources(LinearPath, Type format, Type output_type);
 
 // --- additions of this build -------------------------------------------------------------------
-// The TMA descriptor of a weight matrix, built once while plans are prepared and handed to
-// `launch_quant_linear` through its last, optional argument; a launch whose weights it does not
-// describe (or that passes none) builds the descriptor itself.
+// An announced weight matrix, handed to `launch_quant_linear` through its last, optional argument. It says two things: here
+// is the matrix's TMA descriptor (the weight-streaming kernel's), and the matrix and its scales were complete when it was made,
+// so that a launch may fetch them before the kernels upstream of it are done. A launch whose weights it does not describe (or
+// that passes none) builds the descriptor itself and reads nothing before its wait.
 struct WeightMaps {
-    CUtensorMap values;
+    CUtensorMap values; // 128 bytes of K x 128 rows
     const void *weights = nullptr;
     int channels = 0, reduction = 0;
 };
@@ -49,6 +50,10 @@ void quant_linear_inject_wait_expiry(int extra_bytes, long long limit_cycles);
 // The same for scheduling: in the NEXT weight-streaming GEMM of this thread the warp that waits for refilled stages starts
 // about that many nanoseconds late (at most 10^6), as it may when its multiprocessor is busy. Results do not depend on it.
 void quant_linear_inject_refill_delay(int nanoseconds);
+// Orders everything enqueued on `stream` so far before the start of everything after. The kernels of this library let their
+// successors start while they still run, and pass that on: two launches after a kernel its results may not be there yet. A
+// memory operation between them is an ordinary dependency on either side.
+void quant_linear_settle(void *workspace, cudaStream_t stream);
 // Blocking read of the status word: 0 = clean, otherwise 1 + index of the tile whose bounded wait gave up.
 int quant_linear_status(const void *workspace, cudaStream_t stream);
 } // namespace tts

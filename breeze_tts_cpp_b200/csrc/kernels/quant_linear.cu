@@ -267,6 +267,10 @@ void quant_linear_reset_workspace(void *workspace, size_t bytes, cudaStream_t st
     check(cudaMemsetAsync(workspace, 0, kWorkspaceHeader, stream), "cudaMemsetAsync(workspace header)");
 }
 
+void quant_linear_settle(void *workspace, cudaStream_t stream) {
+    check(cudaMemsetAsync(static_cast<char *>(workspace) + kSettleOffset, 0, sizeof(int), stream), "cudaMemsetAsync(settle)");
+}
+
 int quant_linear_status(const void *workspace, cudaStream_t stream) {
     int status = 0;
     check(cudaMemcpyAsync(&status, static_cast<const char *>(workspace) + kStatusOffset, sizeof(int),
@@ -371,11 +375,15 @@ void launch_quant_linear(LinearPath config, KernelProblem shape, const void *inp
         vector_io = vector_io && aligned16(e.residual_f32.data);
     }
     args.vector_io = vector_io;
+    const bool announced = prepared && prepared->weights == weights && prepared->channels == shape.channels &&
+                           prepared->reduction == shape.reduction;
+    args.early = announced;
     // Compute-bound shapes take the persistent, double-buffered CTA-pair kernel (its epilogue moves whole aligned rows).
     if (!grouped && bn == kPrefillTokens && splits == 1 && output_type != Type::I32 && args.vector_io &&
         (!args.ep.residual || args.ep.residual_vector)) {
         PairArgs pair{args.m, args.n, args.k, xs, ws, args.ep.residual_f32, args.status};
         pair.ep = args.ep;
+        pair.early = announced;
         // Epilogue cycles per channel of 128 tokens: plain 16, bias and residual 31, an activation 40 to 55 more (the choice hardly
         // depends on it).
         const double column_cycles = args.ep.activation > 1 ? 75.0 : args.ep.residual || args.ep.residual_f32 ? 31.0
@@ -396,6 +404,7 @@ void launch_quant_linear(LinearPath config, KernelProblem shape, const void *inp
         args.vector_io && aligned16(ws) && (!args.ep.residual || args.ep.residual_vector)) {
         GroupedArgs group{args.m, args.n, args.k, xs, args.ep.residual_f32, args.status};
         group.ep = args.ep;
+        group.early = announced;
         const int channels = grouped_channel_tile(shape.rows, shape.channels, multiprocessor_count());
         const CUtensorMap map_weights = operand_map(weights, shape.channels, shape.reduction, channels, true);
         const CUtensorMap map_x = operand_map(input, shape.rows, shape.reduction, kGroupedTokens, false);
@@ -409,10 +418,8 @@ void launch_quant_linear(LinearPath config, KernelProblem shape, const void *inp
     }
     // The weight map is the caller's prepared one when it describes these weights, else built here.
     CUtensorMap local_w;
-    const bool reuse = prepared && prepared->weights == weights && prepared->channels == shape.channels &&
-                       prepared->reduction == shape.reduction;
-    if (!reuse) local_w = operand_map(weights, shape.channels, shape.reduction, kBlockChannels, true);
-    const CUtensorMap &map_w = reuse ? prepared->values : local_w;
+    if (!announced) local_w = operand_map(weights, shape.channels, shape.reduction, kBlockChannels, true);
+    const CUtensorMap &map_w = announced ? prepared->values : local_w;
     const CUtensorMap map_x = operand_map(input, shape.rows, shape.reduction, bn, false);
     LaunchShape launch = launch_shape(bn, grouped, (kb_total + splits - 1) / splits, splits,
                                       group_units(shape.input_group, shape.weight_group));

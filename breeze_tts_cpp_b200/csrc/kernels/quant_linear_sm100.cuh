@@ -24,7 +24,9 @@
 //   launch overlap : the kernel starts under programmatic dependent launch: barriers, tensor
 //                    memory and the first pipeline stages of WEIGHT tiles are set up while the
 //                    producer of the activations is still running; only the activation tiles, the
-//                    scales and the residual wait for it.
+//                    scales and the residual wait for it. Weights nobody has announced as complete
+//                    (WeightMaps) wait too: every kernel lets its successor start at once, so an
+//                    upstream kernel, or the one before it, may still be writing them.
 //   epilogue       : accumulators leave tensor memory lane-per-channel, are transposed through
 //                    shared memory, and are finished token-row-wise so that every global access
 //                    (fp32 residual, bias, bf16 store) is a coalesced 16-byte vector.
@@ -45,6 +47,7 @@ constexpr int kEpilogueThreads = 256;
 // Workspace carve-up (owner zeroes the first kWorkspaceHeader bytes once). The GEMM itself needs
 // no scratch; only the status word lives here.
 constexpr size_t kStatusOffset = 16384;    // int status[4]: nonzero after a bounded wait gave up
+constexpr size_t kSettleOffset = 16640;    // int: written by quant_linear_settle, read by nobody
 constexpr size_t kWorkspaceHeader = 32768;
 
 struct FusedEpilogue {
@@ -72,6 +75,7 @@ struct GemmArgs {
     int owned_passes; // split-K: 16-row passes each CTA of the cluster may own (slots per split)
     int vector_io;   // every global row touched by the epilogue is 16-byte aligned
     int *status;
+    int early; // the weights and their scales are complete: fetch them before the upstream kernel is
     // Failure-path exercise (host-side injection, see quant_linear_inject_wait_expiry): the first weight
     // barrier expects `expiry_extra_bytes` more than its copy delivers, and every wait gives up after
     // `wait_limit_cycles` (0 = the regular limit). Both zero in normal operation.
@@ -359,6 +363,7 @@ w8a8_tcgen05_gemm(const __grid_constant__ CUtensorMap map_w, const __grid_consta
         // activations the chain keeps passing from kernel to kernel stay in L2.
         const uint64_t stream_once = ptx::policy_evict_first();
         const int ahead = min(a.stages, kb_count);
+        if (!a.early) ptx::wait_for_upstream();
         if (ptx::elect_one()) { // one election around a burst: per copy or per MMA it costs some 20 cycles
             const uint32_t bar = ptx::smem_u32(&w_full);
             ptx::mbar_arrive_expect_tx(bar, uint32_t(ahead) * kWeightBytes + uint32_t(a.expiry_extra_bytes));
@@ -482,17 +487,11 @@ w8a8_tcgen05_gemm(const __grid_constant__ CUtensorMap map_w, const __grid_consta
         const FusedEpilogue &e = a.ep;
         const int type = a.out_type;
         const int passes = (valid_tokens + kRowsPerPass - 1) / kRowsPerPass;
-        // Static operands (weights' scales, bias) are fetched before anything else so their latency
-        // hides behind the main loop.
+        if (!a.early) ptx::wait_for_upstream();
+        // Weights' scales are fetched before anything else so their latency hides behind the main loop.
         float sw8[8];
-        uint32_t bias_words[4]; // packed pairs
-        const uint16_t *bias16 = Plain ? nullptr : static_cast<const uint16_t *>(e.bias);
 #pragma unroll
         for (int i = 0; i < 8; ++i) sw8[i] = (!Grouped && columns_ok) ? a.sw[n + i] : 1.f;
-#pragma unroll
-        for (int i = 0; i < 4; ++i)
-            bias_words[i] = (bias16 && columns_ok) ? uint32_t(bias16[n + 2 * i]) | (uint32_t(bias16[n + 2 * i + 1]) << 16) : 0u;
-        const uint4 bias8 = make_uint4(bias_words[0], bias_words[1], bias_words[2], bias_words[3]);
         // K-group mode: the weights' group scales of this CTA's K range are static too, one entry per
         // accumulation unit (zero for a unit past the end of K, whose accumulator holds zeros). They come by asynchronous
         // copies, so that nothing waits for them until the activations' have been asked for too.
@@ -508,7 +507,13 @@ w8a8_tcgen05_gemm(const __grid_constant__ CUtensorMap map_w, const __grid_consta
                 else sw_smem[i] = 1.f;
             }
         }
-        ptx::wait_for_upstream(); // activation scales, residuals and the output buffer belong to upstream
+        ptx::wait_for_upstream(); // activation scales, residuals, bias and the output buffer belong to upstream
+        uint32_t bias_words[4]; // packed pairs
+        const uint16_t *bias16 = Plain ? nullptr : static_cast<const uint16_t *>(e.bias);
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+            bias_words[i] = (bias16 && columns_ok) ? uint32_t(bias16[n + 2 * i]) | (uint32_t(bias16[n + 2 * i + 1]) << 16) : 0u;
+        const uint4 bias8 = make_uint4(bias_words[0], bias_words[1], bias_words[2], bias_words[3]);
         float first_residual[8];
         uint4 first_skip = make_uint4(0, 0, 0, 0); // 16-bit residual of that pass
         uint4 first_gate = make_uint4(0, 0, 0, 0);

@@ -54,6 +54,7 @@ struct GroupedArgs {
     const float *sx;           // group-major [k / 128, m]
     const float *residual_f32; // [m, n], added before the first rounding
     int *status;
+    int early;                 // the weights and their scales are complete (GemmArgs)
     FusedEpilogue ep;          // read by the chain instances only
 };
 
@@ -115,7 +116,8 @@ w8a8_tcgen05_prefill_grouped(const __grid_constant__ CUtensorMap map_w, const __
     if (warp == 0) {
         // ------------------------------------------------------------ producer
         // The whole warp runs the loop so that addresses and coordinates stay warp-uniform; one elected lane issues.
-        // The first round of the ring fetches the weights and their scales before the wait on upstream.
+        // The first round of the ring fetches announced weights and their scales before the wait on upstream.
+        if (!a.early) ptx::wait_for_upstream();
         if (ptx::elect_one()) {
             ptx::prefetch_tensormap(&map_w);
             ptx::prefetch_tensormap(&map_x);

@@ -44,6 +44,7 @@ struct PairArgs {
     const float *residual_f32; // [m, n], added before the first rounding (instances without the chain: optional)
     int *status;
     int channels, stages; // channel tile and ring stages
+    int early;            // the weights are complete (GemmArgs)
     FusedEpilogue ep;     // read by the chain instances only
 };
 
@@ -113,8 +114,9 @@ w8a8_tcgen05_prefill_pair(const __grid_constant__ CUtensorMap map_w, const __gri
             ptx::prefetch_tensormap(&map_w);
             ptx::prefetch_tensormap(&map_x);
         }
-        // Weights do not depend on the upstream kernel: the first round of the ring starts with them and adds
+        // Announced weights do not depend on the upstream kernel: the first round of the ring starts with them and adds
         // the activation tiles once upstream is done (each stage's barrier expects both from the start).
+        if (!a.early) ptx::wait_for_upstream();
         const uint32_t full_leader = ptx::map_to_rank(ptx::smem_u32(&full_bar[0]), 0);
         const int first_n0 = (cluster_id % n_tiles) * channels + int(rank) * (channels / 2);
         const int ahead = cluster_id < tiles ? min(stages, kb_count) : 0;

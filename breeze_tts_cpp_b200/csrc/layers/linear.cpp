@@ -53,8 +53,7 @@ Linear Linear::quantize(const std::vector<TensorView> &parts, Quantization mode,
         }
         ops::quantize_rows(gathered.view(rows, columns, source_type), whole);
     }
-    // The GEMM prefetches weight tiles and weight scales ahead of its wait on the preceding kernel,
-    // so a weight must be complete on the device before the first GEMM that uses it is enqueued.
+    // The gathered copy above must outlive its readers, and a layer may be used from another stream than this one.
     if (cudaStreamSynchronize(execution_context(device).stream) != cudaSuccess)
         throw std::runtime_error("weight quantization failed");
     Linear layer(whole, source_type, bias);
@@ -68,11 +67,12 @@ void Linear::prepare_range(int max_rows, ops::Activation activation) const {
     ops::Epilogue finish;
     finish.activation = activation;
     const auto layout = quantization_layout();
-    // One plan per capacity class: walk the classes upward until max_rows is covered.
+    // One plan per capacity class: walk the classes upward until max_rows is covered. The weight is announced once.
+    TensorView weight = weight_.values;
     for (int rows = 1;;) {
         const int capacity = row_capacity(rows);
-        ops::prepare_quantized(weight_.values, capacity, output_channels(), input_channels(), activation_type_, finish,
-                               layout);
+        ops::prepare_quantized(weight, capacity, output_channels(), input_channels(), activation_type_, finish, layout);
+        weight.data = nullptr;
         if (capacity >= max_rows) break;
         rows = capacity + 1;
     }

@@ -24,6 +24,10 @@ struct CudaContext {
     CudaContext(int device, Quantization mode, cudaStream_t stream = nullptr, void *workspace = nullptr,
                 size_t workspace_bytes = 0);
     CudaContext(const CudaContext &) = delete;
+    // Every operator that wrote a quantized view calls this, in case the view is (part of) an announced weight.
+    void written(const RowScaledView &view) {
+        if (quantization) quantization->written(view.values);
+    }
 };
 class ExecutionScope {
     CudaContext *previous_;

@@ -14,6 +14,7 @@ void quantize_rows(TensorView input, RowScaledView output) {
         throw std::invalid_argument("quantization source/destination shape/type mismatch");
     auto &gpu = execution_context(input, {output.values, output.scales});
     launch_row_quantize(input, output, gpu.stream, gpu.multiprocessors);
+    gpu.written(output);
 }
 // reference: src/ops/basic.cpp:64-67
 void matmul(RowScaledView input, RowScaledView weight, TensorView output) {
@@ -35,11 +36,13 @@ void quantized_norm(TensorView input, TensorView update, TensorView weight, RowS
                     bool gemma, TensorView scale) {
     auto &gpu = execution_context(input, {update, weight, output.values, output.scales, scale});
     launch_quantized_norm(input, update, weight, output, epsilon, gemma, scale, gpu.stream);
+    gpu.written(output);
 }
 // reference: src/ops/basic.cpp:59-63
 void quantized_gated(TensorView input, RowScaledView output, int kind) {
     auto &gpu = execution_context(input, {output.values, output.scales});
     launch_quantized_gated(input, output, kind, gpu.stream, gpu.multiprocessors, gpu.quant_gated_clusters);
+    gpu.written(output);
 }
 void seal(int device) {
     auto &gpu = execution_context(device);

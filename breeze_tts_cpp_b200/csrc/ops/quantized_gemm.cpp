@@ -4,6 +4,7 @@
 #include "ops/epilogue.h"
 #include "ops/quantization_policy.h"
 #include "ops/sequence.h"
+#include <algorithm>
 #include <map>
 #include <tuple>
 
@@ -38,9 +39,9 @@ struct QuantizedGemm::Impl {
     int multiprocessors = 0;
     bool sealed = false;
     std::map<PlanKey, Plan> plans;
-    // TMA descriptors of the weight matrices announced before seal(), looked up by pointer at run time
-    // (a few tree steps; weights that were never announced get their descriptor built per launch).
+    // Weight matrices announced before seal(), looked up by pointer at run time (a few tree steps).
     std::map<const void *, WeightMaps> weight_maps;
+    size_t largest_weight = 0; // bytes
     ChipModel chip;
     SelectionStats stats;
 
@@ -101,9 +102,32 @@ void QuantizedGemm::prepare(int rows, int channels, int reduction, Type output_t
 }
 void QuantizedGemm::prepare_weight(TensorView values) {
     if (!values.data || (values.type != Type::I8 && values.type != Type::FP8) || !values.dense()) return;
-    if (impl->weight_maps.count(values.data)) return;
-    if (impl->sealed) throw std::logic_error("prepared resource missing after initialization");
-    impl->weight_maps.emplace(values.data, quant_linear_weight_maps(values.data, values.rows, values.cols));
+    const auto known = impl->weight_maps.find(values.data);
+    const bool described = known != impl->weight_maps.end() && known->second.channels == values.rows && known->second.reduction == values.cols;
+    if (!described) {
+        if (impl->sealed) {
+            if (known == impl->weight_maps.end()) throw std::logic_error("prepared resource missing after initialization");
+            return; // other dimensions at a known address: launches describe it themselves
+        }
+        impl->weight_maps.insert_or_assign(values.data, quant_linear_weight_maps(values.data, values.rows, values.cols));
+        impl->largest_weight = std::max(impl->largest_weight, values.size());
+    }
+    quant_linear_settle(impl->workspace.data(), impl->stream);
+}
+void QuantizedGemm::written(TensorView values) {
+    if (impl->weight_maps.empty() || !values.data) return;
+    // From the last matrix that begins before the end of `values` back to where the largest one would still reach it.
+    const auto begin = reinterpret_cast<uintptr_t>(values.data);
+    for (auto it = impl->weight_maps.lower_bound(reinterpret_cast<const void *>(begin + values.span_bytes())); it != impl->weight_maps.begin();) {
+        --it;
+        const auto matrix = reinterpret_cast<uintptr_t>(it->first);
+        if (matrix + impl->largest_weight <= begin) return;
+        if (matrix + size_t(it->second.channels) * it->second.reduction > begin) return quant_linear_settle(impl->workspace.data(), impl->stream);
+    }
+}
+const WeightMaps *QuantizedGemm::announced(TensorView values) const {
+    const auto known = impl->weight_maps.find(values.data);
+    return known == impl->weight_maps.end() ? nullptr : &known->second;
 }
 void QuantizedGemm::prepare_finish(int rows, int channels, int reduction, Type output_type,
                                    const ops::Epilogue &finish, QuantizationGroups groups) {
@@ -176,6 +200,7 @@ bool QuantizedGemm::normalized_linear(TensorView x, TensorView normalized, Tenso
     }
     launch_normalized_quantized_linear(x, normalized, norm_weight, norm_bias, epsilon, f, weight, output, e, encoded,
                                        impl->stream);
+    written(encoded.values);
     return true;
 }
 bool QuantizedGemm::prepared(int rows, int channels, int reduction, Type output_type, QuantizationGroups groups) const {

@@ -28,9 +28,14 @@ class QuantizedGemm {
     QuantCacheStats cache_stats() const;
     void prepare(int rows, int output_channels, int input_channels, Type output_type = Type::BF16,
                  QuantizationGroups groups = {});
-    // Addition: builds the TMA descriptor of a quantized weight matrix ahead of time (before seal()),
-    // so that no launch has to encode it. Views that are not one-byte dense matrices are ignored.
+    // Addition: announces a quantized weight matrix and its scales as complete in stream order (before seal(); repeated
+    // for contents that were replaced). Launches may then fetch them ahead of the kernels upstream, and the streaming
+    // kernel need not encode the matrix's TMA descriptor. Views that are not one-byte dense matrices are ignored.
     void prepare_weight(TensorView quantized_values);
+    // Addition: to be called after a kernel that wrote `quantized_values` was enqueued; keeps the announcement true when it
+    // overwrote an announced matrix.
+    void written(TensorView quantized_values);
+    const struct WeightMaps *announced(TensorView quantized_values) const;
     void prepare_finish(int rows, int output_channels, int input_channels, Type output_type,
                         const ops::Epilogue &, QuantizationGroups groups = {});
     void linear(RowScaledView input, RowScaledView weight, TensorView output);

@@ -125,6 +125,7 @@ void pointwise_quantize(TensorView x, RowScaledView q, const Epilogue &e, Tensor
     auto &gpu = execution_context(x, {q.values, q.scales, retained, e.bias, e.residual, e.gate, e.condition, e.raw});
     validate_pointwise_quantize(x, q, e, retained);
     launch_pointwise_quantize(x, q, e, retained, multiprocessors > 0 ? multiprocessors : gpu.multiprocessors, gpu.stream);
+    gpu.written(q);
 }
 
 void layer_norm_quantize(TensorView x, RowScaledView q, TensorView w, TensorView bias, float eps, const NormFusion &f,
@@ -140,5 +141,6 @@ void layer_norm_quantize(TensorView x, RowScaledView q, TensorView w, TensorView
         check_row_alias(output, f.residual, !f.source_rows);
     }
     launch_layer_norm_quantize(x, q, w, bias, eps, f, retained, gpu.stream);
+    gpu.written(q);
 }
 } // namespace tts::ops

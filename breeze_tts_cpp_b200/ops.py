@@ -144,6 +144,9 @@ class Context:
     # ---- GEMM
     def prepare_quantized(self, rows: int, channels: int, reduction: int, out_dtype=torch.bfloat16,
                           groups: tuple[int, int] | None = None, weight: RowScaledView | None = None) -> tuple[int, int, int, int]:
+        """Plans the shape. `weight` announces a weight of it: its producers are enqueued on this context's stream, so GEMMs may
+        fetch its values and scales ahead of the kernels before them. Replaced by one of this context's calls it stays announced;
+        replaced in any other way it has to be announced again (or the stream synchronized) before it is used."""
         ga, gw = groups if groups is not None else groups_of(self.mode)[:2]
         path = Path_()
         _lib.call("b200q_prepare", self._handle, rows, channels, reduction, _TORCH_TYPES[out_dtype], ga, gw, C.byref(path))
@@ -161,6 +164,7 @@ class Context:
         _lib.call("b200q_seal", self._handle)
 
     def matmul(self, x: RowScaledView, w: RowScaledView, out: torch.Tensor, **epilogue) -> torch.Tensor:
+        """out = dequantized x @ w^T, for a shape that prepare_quantized has planned; a little faster on an announced weight."""
         if _native.linear(self._address, x, w, out, epilogue) is NotImplemented:
             ep = C.byref(_epilogue(**epilogue)) if epilogue else None
             _lib.call("b200q_linear", self._handle, C.byref(x.c()), C.byref(w.c()), C.byref(_tensor(out)), ep)

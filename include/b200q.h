@@ -8,9 +8,11 @@
  * Conventions (same as the reference's bindings/c_api.cpp:25-40): every call returns 0 on success
  * and -1 on failure, copying a message into `error` (capacity `error_capacity`, may be NULL).
  * All device pointers are borrowed; nothing here allocates at call time except the *_create calls.
- * Weights and weight scales must be complete on the device (stream-synchronized, or ordered by an
- * ordinary stream dependency) before the first GEMM that reads them is enqueued: the GEMM kernels
- * prefetch weight tiles and weight scales ahead of their wait on the preceding kernel.
+ * Calls on one stream see one another's results, with one exception to keep in mind: a weight announced
+ * through b200q_prepare_weight (layers announce theirs when they are prepared) is fetched, values and scales,
+ * ahead of the kernels before the GEMM. Announce it once its producers are enqueued on the context's stream or
+ * are complete. Replacing it later by a call of this library on the same context needs nothing; after replacing
+ * it in any other way (a copy, a kernel of one's own), announce it again or synchronize the stream.
  * Type codes are the integer values of the reference's tts::Type (src/core/tensor.h:8):
  * BF16=0 F32=1 I32=2 FP8=3 I8=4 F16=5.
  */
@@ -107,7 +109,8 @@ int b200q_prepare(b200q_context *, int32_t rows, int32_t output_channels, int32_
                   char *error, size_t error_capacity);
 /* reference: the weight argument of ops::prepare_quantized (src/ops/basic.h:25-26). Builds the TMA
  * descriptor of a quantized weight matrix once, before b200q_seal, so that launches on that weight
- * need not encode it. Optional: weights that were never announced still work. */
+ * need not encode it, and allows them to fetch the weight ahead of the kernels before them (see the
+ * conventions above). Optional: weights that were never announced still work, a little slower. */
 int b200q_prepare_weight(b200q_context *, const b200q_row_scaled *weight, char *error, size_t error_capacity);
 /* reference: QuantizedGemm::seal / ops::seal (src/ops/cuda/quantization.h:24). */
 int b200q_seal(b200q_context *, char *error, size_t error_capacity);
