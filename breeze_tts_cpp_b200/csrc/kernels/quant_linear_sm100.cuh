@@ -346,6 +346,7 @@ w8a8_tcgen05_gemm(const __grid_constant__ CUtensorMap map_w, const __grid_consta
     // The next kernel in the stream may begin its own prologue; peers learn that this CTA is running.
     ptx::launch_dependents();
     if (split_k) ptx::cluster_arrive();
+    if (!a.early) ptx::wait_for_upstream();
 
     if (warp == 0) {
         // ------------------------------------------------------------ TMA producer
@@ -363,7 +364,6 @@ w8a8_tcgen05_gemm(const __grid_constant__ CUtensorMap map_w, const __grid_consta
         // activations the chain keeps passing from kernel to kernel stay in L2.
         const uint64_t stream_once = ptx::policy_evict_first();
         const int ahead = min(a.stages, kb_count);
-        if (!a.early) ptx::wait_for_upstream();
         if (ptx::elect_one()) { // one election around a burst: per copy or per MMA it costs some 20 cycles
             const uint32_t bar = ptx::smem_u32(&w_full);
             ptx::mbar_arrive_expect_tx(bar, uint32_t(ahead) * kWeightBytes + uint32_t(a.expiry_extra_bytes));
@@ -487,7 +487,6 @@ w8a8_tcgen05_gemm(const __grid_constant__ CUtensorMap map_w, const __grid_consta
         const FusedEpilogue &e = a.ep;
         const int type = a.out_type;
         const int passes = (valid_tokens + kRowsPerPass - 1) / kRowsPerPass;
-        if (!a.early) ptx::wait_for_upstream();
         // Weights' scales are fetched before anything else so their latency hides behind the main loop.
         float sw8[8];
 #pragma unroll
@@ -508,12 +507,7 @@ w8a8_tcgen05_gemm(const __grid_constant__ CUtensorMap map_w, const __grid_consta
             }
         }
         ptx::wait_for_upstream(); // activation scales, residuals, bias and the output buffer belong to upstream
-        uint32_t bias_words[4]; // packed pairs
-        const uint16_t *bias16 = Plain ? nullptr : static_cast<const uint16_t *>(e.bias);
-#pragma unroll
-        for (int i = 0; i < 4; ++i)
-            bias_words[i] = (bias16 && columns_ok) ? uint32_t(bias16[n + 2 * i]) | (uint32_t(bias16[n + 2 * i + 1]) << 16) : 0u;
-        const uint4 bias8 = make_uint4(bias_words[0], bias_words[1], bias_words[2], bias_words[3]);
+        uint4 bias8 = make_uint4(0, 0, 0, 0);
         float first_residual[8];
         uint4 first_skip = make_uint4(0, 0, 0, 0); // 16-bit residual of that pass
         uint4 first_gate = make_uint4(0, 0, 0, 0);
@@ -525,6 +519,13 @@ w8a8_tcgen05_gemm(const __grid_constant__ CUtensorMap map_w, const __grid_consta
                 first_skip = *reinterpret_cast<const uint4 *>(static_cast<const uint16_t *>(e.residual) +
                                                               size_t(m0 + c) * e.residual_ld + n);
             if (!Plain && e.gate && columns_ok && c < valid_tokens) first_gate = *gate_at(e, m0 + c, n);
+            if (!Plain && e.bias && columns_ok) {
+                const uint16_t *bias16 = static_cast<const uint16_t *>(e.bias) + n;
+                uint32_t w[4]; // packed pairs
+#pragma unroll
+                for (int i = 0; i < 4; ++i) w[i] = uint32_t(bias16[2 * i]) | (uint32_t(bias16[2 * i + 1]) << 16);
+                bias8 = make_uint4(w[0], w[1], w[2], w[3]);
+            }
             if (e.residual_f32 && columns_ok && c < valid_tokens) {
                 const float *src = e.residual_f32 + size_t(m0 + c) * a.n + n;
                 if (a.vector_io) {

@@ -112,12 +112,12 @@ w8a8_tcgen05_prefill_grouped(const __grid_constant__ CUtensorMap map_w, const __
     const uint32_t tmem_base = ptx::warp_uniform(tmem_slot);
     volatile int *abort_ptr = &abort_flag;
     ptx::launch_dependents();
+    if (!a.early) ptx::wait_for_upstream();
 
     if (warp == 0) {
         // ------------------------------------------------------------ producer
         // The whole warp runs the loop so that addresses and coordinates stay warp-uniform; one elected lane issues.
         // The first round of the ring fetches announced weights and their scales before the wait on upstream.
-        if (!a.early) ptx::wait_for_upstream();
         if (ptx::elect_one()) {
             ptx::prefetch_tensormap(&map_w);
             ptx::prefetch_tensormap(&map_x);

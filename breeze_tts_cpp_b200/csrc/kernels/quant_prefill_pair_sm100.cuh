@@ -105,6 +105,7 @@ w8a8_tcgen05_prefill_pair(const __grid_constant__ CUtensorMap map_w, const __gri
     const uint32_t tmem_base = ptx::warp_uniform(tmem_slot);
     volatile int *abort_ptr = &abort_flag;
     ptx::launch_dependents();
+    if (!a.early) ptx::wait_for_upstream();
 
     if (warp == 0) {
         // ------------------------------------------------------------ TMA producer (both CTAs)
@@ -116,7 +117,6 @@ w8a8_tcgen05_prefill_pair(const __grid_constant__ CUtensorMap map_w, const __gri
         }
         // Announced weights do not depend on the upstream kernel: the first round of the ring starts with them and adds
         // the activation tiles once upstream is done (each stage's barrier expects both from the start).
-        if (!a.early) ptx::wait_for_upstream();
         const uint32_t full_leader = ptx::map_to_rank(ptx::smem_u32(&full_bar[0]), 0);
         const int first_n0 = (cluster_id % n_tiles) * channels + int(rank) * (channels / 2);
         const int ahead = cluster_id < tiles ? min(stages, kb_count) : 0;
