@@ -337,11 +337,11 @@ __device__ __forceinline__ void copy_async_arrive(uint32_t bar) {
     asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];" ::"r"(bar) : "memory");
 }
 __device__ __forceinline__ void copy_async_wait_all() { asm volatile("cp.async.wait_all;" ::: "memory"); }
-// Four consecutive fp32 in shared memory as two packed pairs. Not ordered against barriers by itself: the address must come
-// from pinned() after the barrier that publishes the data.
+// Four consecutive fp32 in shared memory as two packed pairs. Volatile keeps it behind the barrier that publishes the data and in
+// front of the arrival that gives it up; the address still comes from pinned(), so that it is computed once.
 __device__ __forceinline__ ulonglong2 ld_shared_2x64(uint32_t addr) {
     ulonglong2 v;
-    asm("ld.shared.v2.b64 {%0, %1}, [%2];" : "=l"(v.x), "=l"(v.y) : "r"(addr));
+    asm volatile("ld.shared.v2.b64 {%0, %1}, [%2];" : "=l"(v.x), "=l"(v.y) : "r"(addr));
     return v;
 }
 __device__ __forceinline__ uint32_t pinned(uint32_t v) {
