@@ -117,7 +117,7 @@ template <class T> __device__ __forceinline__ uint32_t mul16x2(uint32_t a, uint3
 
 // Sign flips of the rotation as XOR masks for packed pairs of 16-bit values (column 2i in the low half).
 constexpr int kMaskedColumns = 8192;
-struct RotationMasks {
+struct alignas(16) RotationMasks { // load_masks reads 16 bytes at a time
     uint32_t pair[kMaskedColumns / 2];
 };
 __host__ __device__ constexpr uint32_t rotation_flip(uint32_t column) { // 1 = the column's sign is flipped (rotation_sign == -1)
