@@ -183,10 +183,11 @@ bool Linear::normalized_forward(Workspace &workspace, TensorView input, TensorVi
     // Two launches, LayerNorm + quantize and the tensor-core projection, wherever the latter takes the shape and was prepared
     // for the rows: 5.1 against 9.4 us at 1 x 256 -> 1024, 8.5 against 169 at 372 x 512 -> 2048 (the one-launch kernel
     // normalizes a row once per 64 output channels and reads the weights once per row). What is left for that kernel: narrow
-    // projections whose dimensions are no multiples of 16, whose weights TMA cannot address or that nobody prepared, and
-    // callers that want the normalized rows quantized.
+    // projections whose dimensions are no multiples of 16, whose weights TMA cannot address or that nobody prepared, strided
+    // output rows, callers that want the normalized rows quantized, and epilogues that it refuses.
     const auto &quantization = execution_context(input.device).quantization;
-    const bool two_steps = !quantized_output.values.data && input.rows <= workspace.rows() &&
+    const bool two_steps = !quantized_output.values.data && input.rows <= workspace.rows() && output.dense() &&
+                           epilogue.rows_per_sequence >= 1 && input.rows % epilogue.rows_per_sequence == 0 &&
                            reinterpret_cast<uintptr_t>(weight_.values.data) % 16 == 0 && quantization &&
                            quantization->prepared(input.rows, output_channels(), input_channels(), output.type, quantization_layout());
     if (!two_steps && ops::normalized_linear(input, weight_, bias_, normalized, output, norm_weight, norm_bias, epsilon, fusion,

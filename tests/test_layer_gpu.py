@@ -110,9 +110,8 @@ def test_phase_switch_plan_prepare_execute(ctx_factory, oracle):
 
 @pytest.mark.parametrize("k,fused", [(512, True), (1024, False)])
 def test_normalized_forward_fused_and_two_step_agree(ctx_factory, oracle, k, fused):
-    """reference: Linear::normalized_forward (src/layers/linear.cpp:195-214). For K <= 512 one launch does
-    LayerNorm + quantize + projection; beyond that LayerNorm + quantize is followed by the GEMM. Both give
-    the result of running the two steps by hand."""
+    """reference: Linear::normalized_forward (src/layers/linear.cpp:195-214): the result is that of running LayerNorm +
+    quantize and the GEMM by hand, at a width the one-launch kernel also takes and beyond it."""
     from breeze_tts_cpp_b200 import ops
     ctx = ctx_factory("int8")
     n, rows = 256, 12
@@ -139,4 +138,29 @@ def test_normalized_forward_fused_and_two_step_agree(ctx_factory, oracle, k, fus
     else:
         assert torch.equal(out.view(torch.int16), by_hand.view(torch.int16))
     assert float(normalized.float().abs().max()) > 0
+    layer.close()
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("rows,k,n", [(1, 256, 1024), (37, 512, 2048)])
+def test_normalized_forward_into_strided_rows(ctx_factory, dtype, rows, k, n):
+    """The one-launch kernel writes rows of any stride, as columns of a wider buffer; nothing beside them is touched. It multiplies
+    (acc * sw) * sx and the two launches for dense rows (acc * sx) * sw, two fp32 roundings apart, so at most one storage step. And
+    a sequence length that does not divide the rows is refused, as by that kernel."""
+    from breeze_tts_cpp_b200 import B200QError, ops
+    ctx = ctx_factory("int8")
+    g = torch.Generator(device="cuda").manual_seed(rows)
+    draw = lambda *shape: torch.randn(*shape, generator=g, device="cuda").to(dtype)
+    layer = ops.Linear(ctx, [draw(n, k) * 0.05], max_rows=rows)
+    x, gamma, beta = draw(rows, k), draw(1, k), draw(1, k)
+    dense = torch.empty(rows, n, dtype=dtype, device="cuda")
+    wide = torch.full((rows, n + 64), 7.0, dtype=dtype, device="cuda")
+    layer.normalized_forward(x, dense, gamma, beta, 1e-5, activation=1)
+    layer.normalized_forward(x, wide[:, 32:32 + n], gamma, beta, 1e-5, activation=1)
+    assert ctx.status() == 0
+    a, b = wide[:, 32:32 + n].double(), dense.double()
+    assert bool(((a - b).abs() <= torch.finfo(dtype).eps * torch.maximum(a, b)).all()) and float(a.max()) > 0
+    assert bool((wide[:, :32] == 7).all()) and bool((wide[:, 32 + n:] == 7).all())
+    with pytest.raises(B200QError, match="invalid epilogue sequence length"):
+        layer.normalized_forward(x, dense, gamma, beta, 1e-5, rows_per_sequence=rows + 1)
     layer.close()
