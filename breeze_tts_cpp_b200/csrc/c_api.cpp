@@ -129,7 +129,8 @@ int b200q_linear(b200q_context *c, const b200q_row_scaled *input, const b200q_ro
             return;
         }
         auto e = epilogue_of(epilogue);
-        if (!gpu.quantization->linear_finish(scaled_of(input), scaled_of(weight), view_of(output), e))
+        // A gate checks its sequences in ops::linear only (b200q_linear_forward).
+        if (e.gate.data || !gpu.quantization->linear_finish(scaled_of(input), scaled_of(weight), view_of(output), e))
             throw std::invalid_argument("epilogue cannot be fused, or the shape was not prepared");
     });
 }

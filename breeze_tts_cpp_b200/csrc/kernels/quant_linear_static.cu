@@ -106,6 +106,7 @@ extern "C" int b200q_quant_linear_static(int32_t device, void *stream, const b20
             throw std::invalid_argument("this problem needs " + std::to_string(need) + " bytes of scratch; the built-in scratch holds " +
                                         std::to_string(kStaticScratchBytes) + " and this entry point never allocates");
         const ops::Epilogue finish = capi::epilogue_of(epilogue);
+        if (finish.gate.data) throw std::invalid_argument("unsupported quantized native Finish path");
         auto s = static_cast<cudaStream_t>(stream);
         // The shared array still holds whatever the previous call left; the GEMM expects its header
         // (status word included) to start at zero, so clear it on the stream ahead of the launch.

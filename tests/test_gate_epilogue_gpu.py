@@ -29,3 +29,24 @@ def test_gate_equals_finishing_pass(ctx_factory, mode, sequences, length, k, n, 
     ctx.pointwise(raw, two, bias=bias, **finish)
     assert ctx.status() == 0
     assert torch.equal(fused.view(torch.int16), two.view(torch.int16))
+
+
+def test_gate_is_refused_where_only_a_fused_finish_is_taken(ctx_factory):
+    """matmul and the path-level entry points take what the GEMM alone has always taken; a gate goes through linear()."""
+    import ctypes as C
+
+    from breeze_tts_cpp_b200 import B200QError, _lib, ops
+    ctx, m, n, k = ctx_factory("int8"), 4, 128, 256
+    make = lambda *shape: torch.ones(*shape, dtype=torch.bfloat16, device="cuda")
+    x, w = (ctx.quantize_rows(make(r, k), ops.RowScaledView.empty(r, k, ops.I8)) for r in (m, n))
+    out, gate = torch.zeros(m, n, dtype=torch.bfloat16, device="cuda"), make(1, n)
+    ctx.prepare_quantized(m, n, k)
+    with pytest.raises(B200QError, match="epilogue cannot be fused"):
+        ctx.matmul(x, w, out, gate=gate)
+    with pytest.raises(B200QError, match="unsupported quantized native Finish path"):
+        ctx.quant_linear((5, 16, 128, 1), x, w, out, gate=gate)
+    with pytest.raises(B200QError, match="unsupported quantized native Finish path"):
+        _lib.call("b200q_quant_linear_static", 0, None, None, C.byref(x.c()), C.byref(w.c()), C.byref(ops._tensor(out)),
+                  C.byref(ops._epilogue(gate=gate)))
+    torch.cuda.synchronize()
+    assert bool((out == 0).all())
