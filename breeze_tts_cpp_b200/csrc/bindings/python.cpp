@@ -6,8 +6,9 @@
 //
 // Every function returns None when the call ran, raises the package's error type with the library's message
 // when it failed, and returns NotImplemented for an argument it does not take itself (not a CUDA tensor, not
-// 2-D, an unknown keyword, a view whose `c` was replaced): the caller then goes the ctypes way, which either
-// handles the argument or raises the error that belongs to it. The GIL is released around each call.
+// 2-D, an unknown keyword, a view whose `c` was replaced; a tensor without storage or with symbolic sizes, as
+// under vmap, functional transforms and tracing, whose accessors throw): the caller then goes the ctypes way,
+// which either handles the argument or raises the error that belongs to it. The GIL is released around each call.
 #include "b200q.h"
 #include <torch/csrc/autograd/python_variable.h>
 #include <cstring>
@@ -185,13 +186,13 @@ PyObject *quantized_norm(PyObject *, Args a, Py_ssize_t n) { // context, residua
     b200q_tensor x, u, w, scale;
     b200q_row_scaled out;
     float epsilon;
+    int32_t gemma;
     if (n != 8 || !tensor_of(a[1], x) || !tensor_of(a[2], u) || !tensor_of(a[3], w) || !view_of(a[4], out) ||
-        !float_of(a[5], epsilon) || !tensor_of(a[7], scale))
+        !float_of(a[5], epsilon) || !int_of(a[6], gemma) || !tensor_of(a[7], scale))
         return declined();
-    const int gemma = PyObject_IsTrue(a[6]);
     auto *c = handle_of<b200q_context>(a[0]);
     return finish("b200q_quantized_norm", [&](char *m, size_t s) {
-        return b200q_quantized_norm(c, &x, &u, &w, &out, epsilon, gemma > 0, &scale, m, s);
+        return b200q_quantized_norm(c, &x, &u, &w, &out, epsilon, gemma, &scale, m, s);
     });
 }
 PyObject *quantized_gated(PyObject *, Args a, Py_ssize_t n) { // context, x, out, kind
@@ -297,7 +298,16 @@ PyObject *bind(PyObject *, Args a, Py_ssize_t n) { // error type, RowScaledView.
     Py_RETURN_NONE;
 }
 
-#define B200Q_METHOD(name) {#name, reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(name)), METH_FASTCALL, nullptr}
+// No C++ exception may reach the interpreter: what torch throws at an argument is left to the caller's slow path.
+template <PyObject *(*Method)(PyObject *, Args, Py_ssize_t)> PyObject *guarded(PyObject *self, Args a, Py_ssize_t n) {
+    try {
+        return Method(self, a, n);
+    } catch (...) {
+        PyErr_Clear();
+        return declined();
+    }
+}
+#define B200Q_METHOD(name) {#name, reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(guarded<name>)), METH_FASTCALL, nullptr}
 PyMethodDef methods[] = {B200Q_METHOD(row_quantize),   B200Q_METHOD(quantized_norm),      B200Q_METHOD(quantized_gated),
                          B200Q_METHOD(linear),         B200Q_METHOD(linear_forward),      B200Q_METHOD(layer_forward),
                          B200Q_METHOD(pointwise),      B200Q_METHOD(pointwise_quantize),  B200Q_METHOD(layer_norm_quantize),
