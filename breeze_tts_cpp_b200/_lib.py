@@ -112,6 +112,17 @@ class B200QError(RuntimeError):
     pass
 
 
+class MissingBinding:
+    """Stands for the compiled binding where it cannot be imported; every use raises with the build command."""
+
+    def __init__(self, reason: ImportError):
+        self._reason = reason
+
+    def __getattr__(self, name):
+        raise RuntimeError(f"the compiled binding is missing or does not fit this Python and torch ({self._reason}): build it with "
+                           "`python -m breeze_tts_cpp_b200.build`")
+
+
 def call(name: str, *args):
     """Calls an int-returning entry point, appending the error buffer; raises B200QError on -1."""
     lib = load()

@@ -87,15 +87,13 @@ def build(verbose: bool = False, force: bool = False) -> Path:
         done = subprocess.run(cmd, capture_output=True, text=True)
         if done.returncode:
             raise RuntimeError(f"link failed:\n{done.stdout}\n{done.stderr}")
-    _build_binding(verbose)
+    _build_binding(verbose, force)
     return LIB
 
 
-def _build_binding(verbose: bool) -> None:
-    """The binding calls the C ABI only, so it is rebuilt for its own source and the ABI's header alone."""
-    stamp = max(p.stat().st_mtime for p in (BINDING_SOURCE, INCLUDE / "b200q.h"))
-    if BINDING.exists() and BINDING.stat().st_mtime >= stamp:
-        return
+def _build_binding(verbose: bool, force: bool = False) -> None:
+    """The binding calls the C ABI only, so of this library's files its own source and the ABI's header matter. It is compiled
+    against one Python and one torch: the command and both versions are kept beside the objects, and others rebuild it."""
     import torch
     from torch.utils import cpp_extension
     torch_lib = Path(torch.__file__).parent / "lib"
@@ -103,11 +101,17 @@ def _build_binding(verbose: bool) -> None:
            f"-I{INCLUDE}", f"-I{sysconfig.get_paths()['include']}", *(f"-isystem{p}" for p in cpp_extension.include_paths()),
            str(BINDING_SOURCE), "-o", str(BINDING), f"-L{HERE}", "-l:libb200q.so", "-Wl,-rpath,$ORIGIN",
            f"-L{torch_lib}", "-ltorch_python", "-ltorch_cpu", "-lc10"]
+    key = "\n".join([torch.__version__, sysconfig.get_config_var("SOABI") or "", *cmd])
+    made_with = OBJ / "binding.key"
+    stamp = max(p.stat().st_mtime for p in (BINDING_SOURCE, INCLUDE / "b200q.h"))
+    if not force and BINDING.exists() and BINDING.stat().st_mtime >= stamp and made_with.exists() and made_with.read_text() == key:
+        return
     if verbose:
         print(" ".join(cmd), flush=True)
     done = subprocess.run(cmd, capture_output=True, text=True)
     if done.returncode:
         raise RuntimeError(f"building the Python binding failed:\n{done.stdout}\n{done.stderr}")
+    made_with.write_text(key)
 
 
 if __name__ == "__main__":

@@ -15,8 +15,13 @@ from dataclasses import dataclass
 
 import torch
 
-from . import _lib, _native
+from . import _lib
 from ._lib import BF16, F16, F32, FP8, I8, I32, Epilogue, NormFusion, Path_, RowScaled, Tensor
+
+try:
+    from . import _native
+except ImportError as error:  # not built (or for another torch): importing this module still works, calling does not
+    _native = _lib.MissingBinding(error)
 
 MODES = ("int8", "fp8", "group_int8", "group_fp8")
 _TORCH_TYPES = {torch.bfloat16: BF16, torch.float16: F16, torch.float32: F32, torch.int32: I32,
@@ -92,7 +97,8 @@ def _fusion(residual=None, projection_bias=None, raw=None, gate=None, shift=None
                       _tensor(scale), rows_per_sequence, rows_ptr)
 
 
-_native.bind(_lib.B200QError, RowScaledView.c)
+if not isinstance(_native, _lib.MissingBinding):
+    _native.bind(_lib.B200QError, RowScaledView.c)
 
 
 class Context:
