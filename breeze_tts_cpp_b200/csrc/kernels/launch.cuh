@@ -3,7 +3,8 @@
 // kernel before it in the stream. The contract each kernel keeps in return:
 //   * it executes `pdl_launch_dependents()` early, and
 //   * it executes `pdl_wait_upstream()` before its first read of data a previous kernel may have
-//     written and before its first global write.
+//     written and before its first global write. Only parameters that are complete by contract are read
+//     earlier: announced weights with their scales (GEMMs) and RMSNorm weights.
 // Because every kernel waits for its predecessor to finish before it finishes itself, ordering
 // stays transitive along the whole chain. Outside such a launch both instructions do nothing.
 #pragma once

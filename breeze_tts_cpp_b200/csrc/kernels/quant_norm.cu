@@ -61,7 +61,7 @@ rms_quantize(T *__restrict__ x, const T *__restrict__ update, const T *__restric
     pdl_launch_dependents();
     const int row = blockIdx.x, column = threadIdx.x * 8;
     uint4 value = make_uint4(0, 0, 0, 0), w = make_uint4(0, 0, 0, 0);
-    if (column < cols) w = load_raw8(weight + column, cols - column, aligned); // static: may precede the wait
+    if (column < cols) w = load_raw8(weight + column, cols - column, aligned); // a parameter: may precede the wait
     pdl_wait_upstream();
     if (column < cols) {
         const int remaining = cols - column;
@@ -148,7 +148,7 @@ rms_quantize_blocks(T *__restrict__ x, const T *__restrict__ update, const T *__
     const int row = int(blockIdx.x) * int(blockDim.x / 64) + slot, column = lane * 32;
     const bool active = row < rows && column < cols;
     uint32_t mask[16], w[16], value[16];
-    if (active) { // static: may precede the wait
+    if (active) { // a table and a parameter: may precede the wait (behind it the weight costs 2 % of a K-group decode step)
         load_masks(column, mask);
         load_row32(weight + column, w);
     } else {

@@ -137,6 +137,8 @@ class Context:
         return out
 
     def quantized_norm(self, residual, update, weight, out: RowScaledView, epsilon: float, gemma=False, update_scale=None):
+        """residual += update (times update_scale); out = quantized RMSNorm of it. `weight` is a parameter: it is read ahead of the
+        kernels before this call, so the stream has to have been synchronized since it was written."""
         if _native.quantized_norm(self._address, residual, update, weight, out, epsilon, gemma, update_scale) is NotImplemented:
             _lib.call("b200q_quantized_norm", self._handle, C.byref(_tensor(residual)), C.byref(_tensor(update)),
                       C.byref(_tensor(weight)), C.byref(out.c()), epsilon, int(gemma), C.byref(_tensor(update_scale)))

@@ -8,11 +8,13 @@
  * Conventions (same as the reference's bindings/c_api.cpp:25-40): every call returns 0 on success
  * and -1 on failure, copying a message into `error` (capacity `error_capacity`, may be NULL).
  * All device pointers are borrowed; nothing here allocates at call time except the *_create calls.
- * Calls on one stream see one another's results, with one exception to keep in mind: a weight announced
+ * Calls on one stream see one another's results, with two exceptions to keep in mind. A weight announced
  * through b200q_prepare_weight (layers announce theirs when they are prepared) is fetched, values and scales,
  * ahead of the kernels before the GEMM. Announce it once its producers are enqueued on the context's stream or
  * are complete. Replacing it later by a call of this library on the same context needs nothing; after replacing
- * it in any other way (a copy, a kernel of one's own), announce it again or synchronize the stream.
+ * it in any other way (a copy, a kernel of one's own), announce it again or synchronize the stream. And the
+ * norm weight of b200q_quantized_norm is read ahead of the kernels before that call: it is a parameter, to be
+ * complete on the device (the stream synchronized since it was written) when the call is made.
  * Type codes are the integer values of the reference's tts::Type (src/core/tensor.h:8):
  * BF16=0 F32=1 I32=2 FP8=3 I8=4 F16=5.
  */
