@@ -212,7 +212,7 @@ rms_quantize_blocks(T *__restrict__ x, const T *__restrict__ update, const T *__
 
 template <Type F, class T>
 void launch(T *x, const T *update, const T *weight, const T *update_scale, unsigned char *q, float *s, int rows,
-            int cols, float eps, bool gemma, int group, int rotation, cudaStream_t stream) {
+            int cols, float eps, bool gemma, int group, int rotation, int sms, cudaStream_t stream) {
     const bool aligned = cols % 8 == 0 && reinterpret_cast<uintptr_t>(x) % 16 == 0 &&
                          reinterpret_cast<uintptr_t>(weight) % 16 == 0 && reinterpret_cast<uintptr_t>(q) % 8 == 0 &&
                          (!update || reinterpret_cast<uintptr_t>(update) % 16 == 0) &&
@@ -221,7 +221,7 @@ void launch(T *x, const T *update, const T *weight, const T *update_scale, unsig
     if (rotation && group == 128 && cols % 128 == 0 && aligned32(x) && aligned32(weight) && aligned32(q) && aligned32(update) &&
         aligned32(update_scale)) {
         // Four rows per CTA once that still leaves every multiprocessor one.
-        const int per_cta = rows >= 4 * 148 ? 4 : rows >= 2 * 148 ? 2 : 1;
+        const int per_cta = rows >= 4 * sms ? 4 : rows >= 2 * sms ? 2 : 1;
         const dim3 grid(unsigned((rows + per_cta - 1) / per_cta)), block(unsigned(64 * per_cta));
         if (update)
             launch_pdl("quantized norm launch", rms_quantize_blocks<F, T, true>, grid, block, 0, stream, x, update, weight, update_scale, q,
@@ -242,8 +242,9 @@ void launch(T *x, const T *update, const T *weight, const T *update_scale, unsig
 } // namespace b200
 
 void launch_quantized_norm(TensorView residual, TensorView update, TensorView weight, RowScaledView output,
-                           float epsilon, bool gemma, TensorView update_scale, cudaStream_t stream) {
+                           float epsilon, bool gemma, TensorView update_scale, cudaStream_t stream, int multiprocessors) {
     output.validate();
+    if (multiprocessors <= 0) multiprocessors = 148;
     // reference: quant_norm.cu:170-180
     if ((residual.type != Type::BF16 && residual.type != Type::F16) || !residual.data || !weight.data ||
         !output.values.data || !output.scales.data || !residual.dense() || residual.cols < 1 ||
@@ -263,11 +264,11 @@ void launch_quantized_norm(TensorView residual, TensorView update, TensorView we
         if (fp8)
             b200::launch<Type::FP8, T>(residual.ptr<T>(), update.ptr<const T>(), weight.ptr<const T>(),
                                        update_scale.ptr<const T>(), q, s, residual.rows, residual.cols, epsilon, gemma,
-                                       output.group_size, output.rotation_size, stream);
+                                       output.group_size, output.rotation_size, multiprocessors, stream);
         else
             b200::launch<Type::I8, T>(residual.ptr<T>(), update.ptr<const T>(), weight.ptr<const T>(),
                                       update_scale.ptr<const T>(), q, s, residual.rows, residual.cols, epsilon, gemma,
-                                      output.group_size, output.rotation_size, stream);
+                                      output.group_size, output.rotation_size, multiprocessors, stream);
     };
     if (residual.type == Type::F16) run(__half{});
     else run(__nv_bfloat16{});

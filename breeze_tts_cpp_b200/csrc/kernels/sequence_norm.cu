@@ -406,15 +406,16 @@ bool rows_aligned(const NormArgs &a, int cols, const void *q) {
 }
 
 template <Type F, class T, bool Rotate>
-void launch_norm(const NormArgs &a, RowScaledView out, cudaStream_t stream) {
+void launch_norm(const NormArgs &a, RowScaledView out, int sms, cudaStream_t stream) {
     const int rows = out.values.rows, cols = out.values.cols;
     auto *q = out.values.ptr<unsigned char>();
     auto *s = out.scales.ptr<float>();
     // Aligned rows of up to 2048 columns: one warp per row up to 512 columns, 128 threads per row beyond (a single warp
-    // takes too long over a wide row, 9.4 us at 2048 columns however few the rows).
+    // takes too long over a wide row, 9.4 us at 2048 columns however few the rows). Four warp rows per CTA once that still
+    // leaves every multiprocessor one.
     if (cols <= 2048 && rows_aligned(a, cols, q)) {
         const int chunks = (cols + 255) / 256;
-        const int per_cta = rows >= 4 * 148 ? 4 : 1;
+        const int per_cta = rows >= 4 * sms ? 4 : 1;
         const auto run = [&](auto lanes, auto count, int rows_per_cta) {
             constexpr int kLanes = decltype(lanes)::value, kCount = decltype(count)::value;
             launch_pdl("layer norm + quantize launch", layer_norm_quantize_packed<F, T, kLanes, kCount, Rotate>,
@@ -575,17 +576,17 @@ NormArgs norm_args(TensorView x, TensorView weight, TensorView bias, float eps, 
 } // namespace b200
 
 void launch_layer_norm_quantize(TensorView x, RowScaledView q, TensorView weight, TensorView bias, float eps,
-                                const ops::NormFusion &f, TensorView retained, cudaStream_t stream) {
+                                const ops::NormFusion &f, TensorView retained, int multiprocessors, cudaStream_t stream) {
     const b200::NormArgs a = b200::norm_args(x, weight, bias, eps, f, retained);
     const bool fp8 = q.values.type == Type::FP8, rotate = q.rotation_size != 0;
     auto run = [&](auto tag) {
         using T = decltype(tag);
         if (fp8) {
-            if (rotate) b200::launch_norm<Type::FP8, T, true>(a, q, stream);
-            else b200::launch_norm<Type::FP8, T, false>(a, q, stream);
+            if (rotate) b200::launch_norm<Type::FP8, T, true>(a, q, multiprocessors, stream);
+            else b200::launch_norm<Type::FP8, T, false>(a, q, multiprocessors, stream);
         } else {
-            if (rotate) b200::launch_norm<Type::I8, T, true>(a, q, stream);
-            else b200::launch_norm<Type::I8, T, false>(a, q, stream);
+            if (rotate) b200::launch_norm<Type::I8, T, true>(a, q, multiprocessors, stream);
+            else b200::launch_norm<Type::I8, T, false>(a, q, multiprocessors, stream);
         }
     };
     if (x.type == Type::F16) run(__half{});

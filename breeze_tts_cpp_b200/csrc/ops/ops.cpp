@@ -35,7 +35,7 @@ void prepare_quantized(TensorView weight, int rows, int output_channels, int inp
 void quantized_norm(TensorView input, TensorView update, TensorView weight, RowScaledView output, float epsilon,
                     bool gemma, TensorView scale) {
     auto &gpu = execution_context(input, {update, weight, output.values, output.scales, scale});
-    launch_quantized_norm(input, update, weight, output, epsilon, gemma, scale, gpu.stream);
+    launch_quantized_norm(input, update, weight, output, epsilon, gemma, scale, gpu.stream, gpu.multiprocessors);
     gpu.written(output);
 }
 // reference: src/ops/basic.cpp:59-63

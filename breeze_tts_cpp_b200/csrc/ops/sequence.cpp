@@ -140,7 +140,7 @@ void layer_norm_quantize(TensorView x, RowScaledView q, TensorView w, TensorView
         check_row_alias(output, x, !f.source_rows);
         check_row_alias(output, f.residual, !f.source_rows);
     }
-    launch_layer_norm_quantize(x, q, w, bias, eps, f, retained, gpu.stream);
+    launch_layer_norm_quantize(x, q, w, bias, eps, f, retained, gpu.multiprocessors, gpu.stream);
     gpu.written(q);
 }
 } // namespace tts::ops
