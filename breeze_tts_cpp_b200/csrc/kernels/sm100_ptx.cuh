@@ -104,14 +104,6 @@ __device__ __forceinline__ uint32_t map_to_rank(uint32_t smem_addr, uint32_t ran
     asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(remote) : "r"(smem_addr), "r"(rank));
     return remote;
 }
-__device__ __forceinline__ uint4 ld_cluster_v4(uint32_t addr) {
-    uint4 v;
-    asm volatile("ld.shared::cluster.v4.u32 {%0, %1, %2, %3}, [%4];"
-                 : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w)
-                 : "r"(addr)
-                 : "memory");
-    return v;
-}
 
 // ---------------------------------------------------------------- TMA (2-D tiled load, no multicast)
 __device__ __forceinline__ void prefetch_tensormap(const CUtensorMap *map) {
@@ -134,11 +126,6 @@ __device__ __forceinline__ void tma_load_2d_hint(uint32_t dst, const CUtensorMap
 __device__ __forceinline__ uint64_t policy_evict_first() {
     uint64_t p;
     asm volatile("createpolicy.fractional.L2::evict_first.b64 %0, 1.0;" : "=l"(p));
-    return p;
-}
-__device__ __forceinline__ uint64_t policy_evict_last() {
-    uint64_t p;
-    asm volatile("createpolicy.fractional.L2::evict_last.b64 %0, 1.0;" : "=l"(p));
     return p;
 }
 
@@ -174,20 +161,6 @@ __device__ __forceinline__ void tcgen05_fence_after() {
 // Arrives on `bar` once every MMA issued so far by this thread has finished.
 __device__ __forceinline__ void tcgen05_commit(uint32_t bar) {
     asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar) : "memory");
-}
-__device__ __forceinline__ void mma_i8(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t idesc,
-                                       uint32_t accumulate) {
-    asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
-                 "tcgen05.mma.cta_group::1.kind::i8 [%0], %1, %2, %3, p;\n\t}" ::"r"(d_tmem),
-                 "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate)
-                 : "memory");
-}
-__device__ __forceinline__ void mma_f8(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t idesc,
-                                       uint32_t accumulate) {
-    asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
-                 "tcgen05.mma.cta_group::1.kind::f8f6f4 [%0], %1, %2, %3, p;\n\t}" ::"r"(d_tmem),
-                 "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate)
-                 : "memory");
 }
 // This warp's 32 lanes x 16 consecutive 32-bit columns starting at `taddr`.
 __device__ __forceinline__ void tmem_load16(uint32_t taddr, uint32_t (&r)[16]) {
@@ -253,20 +226,6 @@ __device__ __forceinline__ void tma_load_2d_pair(uint32_t dst, const CUtensorMap
     asm volatile("cp.async.bulk.tensor.2d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes "
                  "[%0], [%1, {%3, %4}], [%2];" ::"r"(dst),
                  "l"(reinterpret_cast<uint64_t>(map)), "r"(bar), "r"(x), "r"(y)
-                 : "memory");
-}
-__device__ __forceinline__ void mma_i8_pair(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t idesc,
-                                            uint32_t accumulate) {
-    asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
-                 "tcgen05.mma.cta_group::2.kind::i8 [%0], %1, %2, %3, p;\n\t}" ::"r"(d_tmem),
-                 "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate)
-                 : "memory");
-}
-__device__ __forceinline__ void mma_f8_pair(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t idesc,
-                                            uint32_t accumulate) {
-    asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
-                 "tcgen05.mma.cta_group::2.kind::f8f6f4 [%0], %1, %2, %3, p;\n\t}" ::"r"(d_tmem),
-                 "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate)
                  : "memory");
 }
 // Arrives on the barrier at the same shared-memory offset in every CTA named by `cta_mask` once
@@ -354,16 +313,7 @@ __device__ __forceinline__ uint32_t pinned(uint32_t v) {
 // with the 128-byte swizzle: 8-row groups are 1024 bytes apart (stride byte offset), the leading
 // offset is unused for this layout, descriptor version 1, layout code 2 (128B swizzle).
 // Stepping along K inside the swizzled row is a plain byte offset on the start address.
-__device__ __forceinline__ uint64_t smem_desc_k128(uint32_t smem_addr) {
-    uint64_t d = 0;
-    d |= uint64_t((smem_addr & 0x3ffffu) >> 4);
-    d |= uint64_t(1) << 16;
-    d |= uint64_t(1024 >> 4) << 32;
-    d |= uint64_t(1) << 46;
-    d |= uint64_t(2) << 61;
-    return d;
-}
-// The same descriptor as two 32-bit halves. Only the low half (start address) changes from tile to
+// It is kept as two 32-bit halves: only the low half (start address) changes from tile to
 // tile and from K step to K step, so an issue loop that carries the halves separately keeps the high
 // half loop-invariant and steps the low half with 32-bit adds.
 constexpr uint32_t kDescHiK128 = (1024u >> 4) | (1u << 14) | (2u << 29);

@@ -83,7 +83,6 @@ double linear_cost(KernelProblem p, LinearPath path, Type format, const ChipMode
     if (path.kind != LinearKind::Tcgen05) return std::numeric_limits<double>::infinity();
     const int sms = std::max(1, chip.sms);
     const int kb_total = blocks(p.reduction, kBlockK);
-    const double ops = 2.0 * p.rows * double(p.channels) * p.reduction;
     if (persistent_per_row(p, path)) {
         // CTA pairs: the same estimate the launcher picks the channel tile by, at 1965 MHz, plus launch and fill.
         const PairTile tile = pair_channel_tile(p.rows, p.channels, kb_total, std::max(1, sms / 2), kPairColumnCycles);
