@@ -456,8 +456,8 @@ def sustained_tensor_rates(torch, device, stream, seconds=1.5):
             xq = ctx.quantize_rows(synth_activations(torch, m, k, SEED, device).to(torch.bfloat16),
                                    ops.RowScaledView.empty(m, k, fmt, device=device))
             y = torch.empty(m, n, dtype=torch.bfloat16, device=device)
-            ctx.prepare_quantized(m, n, k)
             for w in ws:
+                ctx.prepare_quantized(m, n, k, weight=w)
                 ctx.matmul(xq, w, y)
             stream.synchronize()
             graph = torch.cuda.CUDAGraph()
@@ -547,7 +547,7 @@ def config_rows(torch, device, stream, peaks, tensor_peaks):
             xq = ops.RowScaledView.empty(m, k, fmt, group, group, device=device)
             out = torch.empty(m, n, dtype=torch.bfloat16, device=device)
             res = torch.randn(m, n, device=device) if residual else None
-            path = ctx.prepare_quantized(m, n, k)
+            path = [ctx.prepare_quantized(m, n, k, weight=w) for w in ws][0]
             kw = {"residual_f32": res} if residual else {}
             ctx.quantize_rows(x, xq)
             ctx.matmul(xq, ws[-1], out, **kw)
@@ -672,7 +672,7 @@ def run_case(spec):
         x = synth_activations(torch, rows, k, SEED, device, student_t=bool(group)).to(torch.bfloat16)
         xq = ops.RowScaledView.empty(rows, k, fmt, group, rotation, device=device)
         out = torch.empty(rows, n, dtype=torch.bfloat16, device=device)
-        path = ctx.prepare_quantized(rows, n, k)
+        path = [ctx.prepare_quantized(rows, n, k, weight=w) for w in weights][0]
         ctx.quantize_rows(x, xq)
         ctx.matmul(xq, weights[0], out)
         stream.synchronize()

@@ -458,7 +458,8 @@ struct ProjectionArgs {
 // Grid (ceil(N / 64), rows). Every CTA of a row normalizes and quantizes the row into shared memory
 // (the first one also stores the row-level results), then each warp produces eight output channels:
 // lanes stride the K axis four bytes at a time exactly as the reference's warp does, so FP8 sums are
-// added in the same order; INT8 sums are exact integers.
+// added in the same order; INT8 sums are exact integers. (A layer that was prepared for its rows runs LayerNorm +
+// quantize and the GEMM instead, Linear::normalized_forward; its FP8 sums are the tensor cores'.)
 template <Type F, class T>
 __global__ void __launch_bounds__(kThreads)
 norm_quantize_project(NormArgs a, ProjectionArgs p, FinishArgs finish) {

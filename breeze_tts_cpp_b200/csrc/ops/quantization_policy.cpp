@@ -84,7 +84,8 @@ double linear_cost(KernelProblem p, LinearPath path, Type format, const ChipMode
     const int sms = std::max(1, chip.sms);
     const int kb_total = blocks(p.reduction, kBlockK);
     if (persistent_per_row(p, path)) {
-        // CTA pairs: the same estimate the launcher picks the channel tile by, at 1965 MHz, plus launch and fill.
+        // CTA pairs: the estimate the launcher picks the channel tile by, at 1965 MHz, plus launch and fill. Plans know no
+        // epilogue, so this is the plain one; the launcher puts 20 to 75 cycles per column in the place of 16 when a chain follows.
         const PairTile tile = pair_channel_tile(p.rows, p.channels, kb_total, std::max(1, sms / 2), kPairColumnCycles);
         return 1.8 + tile.cycles / 1965.;
     }

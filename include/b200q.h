@@ -49,7 +49,8 @@ typedef struct b200q_row_scaled {
  * residual_rows (device int32 per output row, negative = no residual) indexes the residual rows;
  * input_repeat > 1 reads input row r / input_repeat (finishing passes only). Zero-initialise the
  * struct and set value_scale = output_scale = residual_scale = 1, rows_per_sequence = input_repeat = 1.
- * bias, residual, residual_f32, the scales and activations 0-5,7,8 ride inside the GEMM; everything
+ * bias, residual, residual_f32, the scales and activations 0-5,7,8 ride inside the GEMM, and so does, in
+ * b200q_linear_forward and the layer calls, a gate with 16-byte aligned rows; everything
  * else runs as a separate finishing pass, as in the reference (src/ops/linear.cpp:76-82). */
 typedef struct b200q_epilogue {
     b200q_tensor bias, residual, residual_f32;
