@@ -5,7 +5,7 @@
 // of 128 is its own integer/fp8 dot product p_g, and out[m,n] = D(sum_g float(p_g) * (sx_g[m] *
 // sw_g[n])) (+ fp32 residual), optionally followed by the finishing chain. The tensor cores therefore produce one
 // partial tile per K block, and CUDA cores rescale and add it; that second part is what bounds this kernel (INT8: issue,
-// 153 instructions per warp and K block of which 88 are the arithmetic; FP8 and many waves: the 32 KB per K block each SM
+// 147 instructions per rescale warp and K block, 88 of them the arithmetic and its scale reads, 69 % of the slots; FP8 and many waves: the 32 KB per K block each SM
 // pulls from L2).
 //
 //   warp 0     : producer. Per K block one pipeline stage (128 token rows + `Channels` weight rows of 128 B, 128-byte

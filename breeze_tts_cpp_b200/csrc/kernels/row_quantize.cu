@@ -139,7 +139,7 @@ row_quantize_warp_rows(const T *__restrict__ x, unsigned char *__restrict__ q, f
 // rows, four lanes per block, eight blocks per warp. A block's scale then belongs at scales[i], a warp's eight scales
 // share one 32-byte sector, and neither rows nor columns leave lanes idle. 12288 x 2048: 43.9 -> 19.6 us (3.9 TB/s), 1021 x
 // 2048 5.1 -> 3.1, 16 x 2048 1.7 -> 1.4. One set of eight per warp: looping over four with the next one's loads in flight
-// took 24.9 us, resident warps hide more. What is left is issue (475 instructions per 32 columns, 57 % busy).
+// took 24.9 us, resident warps hide more. What is left is issue (491 instructions per 32 columns, 57 % busy).
 template <Type F, class T>
 __global__ void __launch_bounds__(kThreads, 3)
 row_quantize_blocks(const T *__restrict__ x, unsigned char *__restrict__ q, float *__restrict__ scales, int rows, int cols,
