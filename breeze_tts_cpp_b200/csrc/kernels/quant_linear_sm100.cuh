@@ -592,9 +592,8 @@ w8a8_tcgen05_gemm(const __grid_constant__ CUtensorMap map_w, const __grid_consta
             asm volatile("bar.sync 1, 256;" ::: "memory");
             // The two warps of a lane quadrant take half of the tokens each. A round drains kRound units with one wait: a
             // commit completes after all earlier MMAs, so the last unit's barrier stands for the round. The arithmetic is
-            // packed two-wide (with scalar conversions 64 tokens took 512 cycles of the conversion pipe per K block).
+            // packed two-wide.
             constexpr int kHalf = BN / 2, kRound = BN == 16 ? 4 : BN == 32 ? 2 : 1;
-            const ptx::IntBias bias_of_int = ptx::int_bias(raw_base);
             uint64_t result[kHalf / 2];
 #pragma unroll
             for (int c = 0; c < kHalf / 2; ++c) result[c] = 0ull;
@@ -629,7 +628,7 @@ w8a8_tcgen05_gemm(const __grid_constant__ CUtensorMap map_w, const __grid_consta
 #pragma unroll
                             for (int h = 0; h < 2; ++h) {
                                 const int i = 4 * q + 2 * h;
-                                const uint64_t p = kInt ? ptx::int_to_float2(r[u][i], r[u][i + 1], bias_of_int)
+                                const uint64_t p = kInt ? ptx::int_to_float2(r[u][i], r[u][i + 1])
                                                         : ptx::pack2(__uint_as_float(r[u][i]), __uint_as_float(r[u][i + 1]));
                                 result[i / 2] = ptx::fma2(p, ptx::mul2(h ? sx4.y : sx4.x, scale_w2), result[i / 2]);
                             }

@@ -4,27 +4,30 @@
 // Arithmetic (reference grouped_gemm, src/ops/kernels/quant/quant_grouped.cu:16-169): every K block
 // of 128 is its own integer/fp8 dot product p_g, and out[m,n] = D(sum_g float(p_g) * (sx_g[m] *
 // sw_g[n])) (+ fp32 residual), optionally followed by the finishing chain. The tensor cores therefore produce one
-// partial tile per K block, and CUDA cores rescale and add it; that second part is what bounds this kernel (INT8: issue,
-// 147 instructions per rescale warp and K block, 88 of them the arithmetic and its scale reads, 69 % of the slots; FP8 and many waves: the 32 KB per K block each SM
-// pulls from L2).
+// partial tile per K block, and CUDA cores rescale and add it. What bounds the kernel is both halves together: the rescale alone takes
+// 49 (FP8) or 57 us (INT8) of a 4096 x 6144 -> 2048 GEMM's 71 or 80, the operands and MMAs alone 50 (32 KB per K block and SM, 18 TB/s
+// from L2), and each waits for the other at times; the clock falls from 1.96 to 1.82-1.9 GHz besides.
 //
-//   warp 0     : producer. Per K block one pipeline stage (128 token rows + `Channels` weight rows of 128 B, 128-byte
-//                swizzle) by TMA and one slot of a small ring for the scales of that K block, on the same barrier: the
-//                channels' by TMA, the tokens' by 4-byte asynchronous copies (a row count need not be a multiple of 4).
-//   warp 1     : MMA issuer, whole warp in the loop, elected lane issues. The tokens are the MMA's M rows. Four (eight)
-//                accumulators rotate through tensor memory, so the tensor cores run that many K blocks
-//                ahead of the rescale. It never tests an mbarrier itself: a test waits behind the MMAs in flight.
-//   warp 18    : waiter. Tests "accumulator free" and "stage full" for the next K block and hands the
+//   warps 0, 19: producers of the weights and their scales (0) and of the tokens and theirs (19). Per K block one pipeline stage (128
+//                token rows + `Channels` weight rows of 128 B, 128-byte swizzle) by TMA and one slot of a small ring for the scales of
+//                that K block, on the same barrier: the channels' by TMA, the tokens' by 4-byte asynchronous copies (a row count
+//                need not be a multiple of 4). One warp for both was late: 84.7 against 81.3 us (INT8, as above).
+//   warp 1     : MMA issuer, whole warp in the loop, elected lane issues. The tokens are the MMA's M rows. The accumulators of a
+//                round (two K blocks, four at 64 channels) fill half of tensor memory and change hands together: a barrier test
+//                and a hand-over per round instead of per K block take a fifth of the rescale warps' instructions out. It
+//                never tests an mbarrier itself: a test waits behind the MMAs in flight.
+//   warp 18    : waiter. Tests "accumulators free" and "stage full" for the next K block and hands the
 //                result to warp 1 through a named hardware barrier (64 threads), which is free.
-//   warps 2-17 : per K block, pull the accumulator into registers (lane = token, a quarter of the channels per
-//                warp), hand the buffer back at once, then result += float(p) * (sx * sw) with packed
-//                two-wide fp32 instructions. After the last K block the finished rows leave through swizzled
+//   warps 2-17 : per K block, pull 32 token rows x a quarter of the channels into registers, then result += float(p) * (sx * sw)
+//                with packed two-wide fp32 instructions. After the last K block the finished rows leave through swizzled
 //                shared-memory slabs and TMA stores, the chain's residual having been prefetched into the same slabs (as in
 //                quant_prefill_pair_sm100.cuh).
-// Sixteen rescale warps: the chain wait - load - hand back - arithmetic of one warp is latency, four warps per scheduler
+// Sixteen rescale warps: the chain wait - load - arithmetic of one warp is latency, four warps per scheduler
 // hide one another's (eight warps with twice the channels each took about 1100 cycles per K block whatever the format).
-// Measured, GEMM alone, M=4096: INT8 12288 x 2048 220 -> 164 us, 2048 x 6144 110 -> 88; FP8 192 -> 144 and 92 -> 76; with a row
-// count that is no multiple of four (1021) the weight-streaming kernel used to run: FP8 102 -> 44 us.
+// Measured, GEMM alone, one K block per hand-over, one token row per thread and one producer against this: M=4096, 2048 x 6144: INT8 90 ->
+// 80 us, FP8 77 -> 71; 12288 x 2048 at M=1021: 50 -> 46, 45 -> 41; at 64 channels 114 -> 91, 107 -> 88.
+// CTA pairs with tiles of 256 x 256 (half the operand bytes) were slower, 90 and 94 us with four accumulators of 128 channels and 82
+// and 72 with two of 256: the way from a free accumulator to the next full one crosses the two CTAs.
 // Every wait is bounded; on expiry the CTA flags the status word and runs to the common exit.
 #pragma once
 #include "kernels/quant_linear_sm100.cuh"
@@ -33,14 +36,17 @@ namespace tts::b200 {
 
 constexpr int kGroupedMaxStages = 7;
 __host__ __device__ constexpr int grouped_stages(int channels) { return channels == 64 ? kGroupedMaxStages : 5; } // what shared memory holds
+// K blocks per round: the accumulators change hands once per round, two rounds of 256 tensor-memory columns alternate.
+__host__ __device__ constexpr int grouped_round(int channels) { return 256 / channels; }
 // Scale slots need no barriers of their own. They are filled with their stage, so an accumulator that is full implies its
-// slot is. And slot c is rewritten for K block c + kScaleSlots only once the MMAs of block c + kScaleSlots - stages
-// have retired, which the rescale warps allowed by emptying the accumulator of a block at most 8 before that, after they were
-// done with the block before that one: c + kScaleSlots - stages - 9 >= c.
+// slot is. And slot c is rewritten for K block c + kScaleSlots only once the MMAs of block b = c + kScaleSlots - stages have
+// retired. Those of b's round were issued when the rescale warps had taken the round two before it out of tensor memory: at least
+// block b - 2 * round, and so they had done with the scales of block b - 2 * round - 1 >= c.
 constexpr int kScaleSlots = 16;
-static_assert(kScaleSlots >= kGroupedMaxStages + 9, "a scale slot could be rewritten while it is read");
+static_assert(kScaleSlots - grouped_stages(64) - 2 * grouped_round(64) - 1 >= 0 && kScaleSlots - grouped_stages(128) - 2 * grouped_round(128) - 1 >= 0,
+              "a scale slot could be rewritten while it is read");
 constexpr int kGroupedWarps = 16;                          // rescale warps
-constexpr int kGroupedThreads = 32 * (kGroupedWarps + 3);  // + producer, MMA issuer, waiter
+constexpr int kGroupedThreads = 32 * (kGroupedWarps + 4);  // + two producers, MMA issuer, waiter
 constexpr int kRescaleThreads = 32 * kGroupedWarps;
 constexpr int kScaleSlotBytes = (kBlockChannels + kGroupedTokens) * 4; // channels, then tokens
 constexpr uint32_t kGroupedSlabBytes = kGroupedTokens * 128; // 128 token rows x 64 channels of 16 bits
@@ -58,6 +64,100 @@ struct GroupedArgs {
     FusedEpilogue ep;          // read by the chain instances only
 };
 
+// What a rescale thread holds of a 32-row x Columns partial tile: rows t, t + 8, t + 16 and t + 24 (t = lane / 4) and of every eight
+// channels the pair 2 * (lane % 4), as packed pairs [row k][pair j]. In this shape (16x256b) a thread needs a quarter of the
+// channels' scales and four tokens'; one token row per thread (32x32b) needs them all, and those shared-memory reads were a fourth of
+// the loop (rescale alone, cycles per 128 x 128 K block: FP8 420 -> 335, INT8 504 -> 460).
+template <int Columns> using GroupedSums = uint64_t[4][Columns / 8];
+// result += float(p) * (sx * sw) for one K block. `hand_back` runs once the partials are in registers.
+template <bool Int, int Columns, class HandBack>
+__device__ __forceinline__ void grouped_rescale(GroupedSums<Columns> &result, uint32_t partials, uint32_t sx_at, uint32_t sw_at, HandBack hand_back) {
+    uint32_t r[2][Columns / 2]; // 16 token rows each
+    ptx::tmem_load_rows16<Columns>(partials, r[0]);
+    ptx::tmem_load_rows16<Columns>(partials + (16u << 16), r[1]);
+    const float4 sx = ptx::ld_shared_4x32(sx_at);
+    uint64_t sw[Columns / 8];
+#pragma unroll
+    for (int j = 0; j < Columns / 8; ++j) sw[j] = ptx::ld_shared_64(sw_at + 32u * j);
+    ptx::tmem_load_wait();
+    hand_back();
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+        const float scale_x = k == 0 ? sx.x : k == 1 ? sx.y : k == 2 ? sx.z : sx.w;
+        const uint64_t scale_x2 = ptx::pack2(scale_x, scale_x);
+#pragma unroll
+        for (int j = 0; j < Columns / 8; ++j) {
+            const uint32_t lo = r[k >> 1][4 * j + 2 * (k & 1)], hi = r[k >> 1][4 * j + 2 * (k & 1) + 1];
+            const uint64_t p = Int ? ptx::int_to_float2(lo, hi) : ptx::pack2(__uint_as_float(lo), __uint_as_float(hi));
+            result[k][j] = ptx::fma2(p, ptx::mul2(sw[j], scale_x2), result[k][j]);
+        }
+    }
+}
+// The tokens' scales of a K block, four bytes per lane and 32 tokens, laid down as a rescale thread reads them: tokens t, t + 8, t + 16
+// and t + 24 of a quadrant side by side. Arrives on `bar` once they have landed; zeros past the last token.
+__device__ __forceinline__ void grouped_copy_token_scales(const GroupedArgs &a, int kb, int m0, int lane, uint32_t slot, uint32_t bar) {
+    const float *sx = a.sx + size_t(kb) * a.m + m0 + lane;
+    const uint32_t dst = slot + uint32_t((lane & 7) * 4 + (lane >> 3)) * 4u;
+#pragma unroll
+    for (int i = 0; i < kGroupedTokens / 32; ++i) {
+        const bool inside = m0 + lane + 32 * i < a.m;
+        ptx::copy_async4(dst + 128u * i, inside ? sx + 32 * i : a.sx, inside ? 4u : 0u);
+    }
+    ptx::copy_async_arrive(bar);
+}
+// A warp's finished sums into the slab of its channels (128 token rows x 64 channels, swizzled), through the chain. `row`: the thread's
+// first row (all four are the same modulo 8), `token` its token, `channel` its first channel, `chunk` the slab's 16-byte chunk of it.
+template <bool F16, int Chain, int Columns>
+__device__ __forceinline__ void grouped_rows_to_slab(const GroupedArgs &a, const GroupedSums<Columns> &result, uint8_t *slab, int row, int token,
+                                                     int channel, int chunk, bool skip16) {
+    constexpr int kWords = Columns / 8;
+    const int lane = threadIdx.x & 31;
+    const float *__restrict__ residual = a.residual_f32;
+    const auto slab_word = [&](int k, int j) {
+        return reinterpret_cast<uint32_t *>(slab + uint32_t(row + 8 * k) * 128u + (((chunk + j) ^ (row & 7)) * 16) + 4 * (lane & 3));
+    };
+    // The chain works value by value, so four of a thread's channel pairs at a time stand for its eight consecutive channels.
+#pragma unroll
+    for (int q = 0; q < kWords; ++q) {
+        float value[8];
+        uint32_t bias[4] = {0u, 0u, 0u, 0u}, gate[4] = {0u, 0u, 0u, 0u}, skip[4] = {0u, 0u, 0u, 0u};
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            const int k = (4 * q + i) / kWords, j = (4 * q + i) % kWords, m = token + 8 * k, n = channel + 8 * j;
+            const bool inside = n < a.n; // N is a multiple of 16
+            ptx::unpack2(result[k][j], value[2 * i], value[2 * i + 1]);
+            if (residual && inside && m < a.m) {
+                const float2 s = __ldg(reinterpret_cast<const float2 *>(residual + size_t(m) * a.n + n));
+                value[2 * i] = __fadd_rn(value[2 * i], s.x);
+                value[2 * i + 1] = __fadd_rn(value[2 * i + 1], s.y);
+            }
+            if (Chain) {
+                if (a.ep.bias && inside) {
+                    const uint16_t *b = static_cast<const uint16_t *>(a.ep.bias) + n;
+                    bias[i] = uint32_t(b[0]) | (uint32_t(b[1]) << 16);
+                }
+                if ((Chain & 2) && inside && m < a.m)
+                    gate[i] = __ldg(reinterpret_cast<const uint32_t *>(static_cast<const uint16_t *>(a.ep.gate) +
+                                                                       size_t(m / a.ep.rows_per_sequence) * a.ep.gate_ld + n));
+                if (skip16) skip[i] = *slab_word(k, j);
+            }
+        }
+        uint4 packed = pack8x16<F16>(value);
+        if (Chain)
+            packed = chain8<F16, (Chain & 2) != 0>(a.ep, packed, make_uint4(bias[0], bias[1], bias[2], bias[3]),
+                                                   make_uint4(gate[0], gate[1], gate[2], gate[3]), make_uint4(skip[0], skip[1], skip[2], skip[3]));
+        const uint32_t words[4] = {packed.x, packed.y, packed.z, packed.w};
+#pragma unroll
+        for (int i = 0; i < 4; ++i) *slab_word((4 * q + i) / kWords, (4 * q + i) % kWords) = words[i];
+    }
+    if (Chain & 4) { // a pass over the warp's rows, one per thread
+        __syncwarp();
+        const int mine = (row & ~31) + lane;
+        activate_chunks<F16, kWords>([&](int q) { return reinterpret_cast<uint4 *>(slab + uint32_t(mine) * 128u + (((chunk + q) ^ (mine & 7)) * 16)); },
+                                     a.ep.activation, a.ep.alpha);
+    }
+}
+
 template <Type F, int Channels, int Chain, bool F16>
 __global__ void __launch_bounds__(kGroupedThreads, 1)
 w8a8_tcgen05_prefill_grouped(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_x,
@@ -66,7 +166,8 @@ w8a8_tcgen05_prefill_grouped(const __grid_constant__ CUtensorMap map_w, const __
     constexpr bool kInt = F == Type::I8;
     constexpr int BM = kGroupedTokens;
     constexpr int kStages = grouped_stages(Channels);
-    constexpr int kAccumulators = 512 / Channels, kColumns = Channels / 4; // kColumns: channels per rescale thread
+    constexpr int kRound = grouped_round(Channels), kColumns = Channels / 4; // kColumns: channels per rescale warp
+    constexpr int kWords = kColumns / 8; // packed channel pairs of one token per rescale thread
     constexpr int kSlabs = Channels / 64;
     constexpr int kWeightBytes = Channels * kBlockK, kTokenBytes = BM * kBlockK;
     constexpr int kStageBytes = kWeightBytes + kTokenBytes;
@@ -75,7 +176,7 @@ w8a8_tcgen05_prefill_grouped(const __grid_constant__ CUtensorMap map_w, const __
 
     extern __shared__ uint8_t dynamic_smem[];
     __shared__ alignas(8) uint64_t full_bar[kStages], empty_bar[kStages];
-    __shared__ alignas(8) uint64_t acc_full[kAccumulators], acc_empty[kAccumulators];
+    __shared__ alignas(8) uint64_t acc_full[2], acc_empty[2]; // one pair per round in flight
     __shared__ alignas(8) uint64_t residual_full;
     __shared__ uint32_t tmem_slot;
     __shared__ int abort_flag;
@@ -93,10 +194,10 @@ w8a8_tcgen05_prefill_grouped(const __grid_constant__ CUtensorMap map_w, const __
 
     if (threadIdx.x == 0) {
         for (int s = 0; s < kStages; ++s) {
-            ptx::mbar_init(ptx::smem_u32(&full_bar[s]), 1 + 32); // the elected lane with the bytes, every lane with its scales
+            ptx::mbar_init(ptx::smem_u32(&full_bar[s]), 2 + 32); // both producers with their bytes, every lane of one with its scales
             ptx::mbar_init(ptx::smem_u32(&empty_bar[s]), 1);
         }
-        for (int b = 0; b < kAccumulators; ++b) {
+        for (int b = 0; b < 2; ++b) {
             ptx::mbar_init(ptx::smem_u32(&acc_full[b]), 1);
             ptx::mbar_init(ptx::smem_u32(&acc_empty[b]), kGroupedWarps);
         }
@@ -114,28 +215,16 @@ w8a8_tcgen05_prefill_grouped(const __grid_constant__ CUtensorMap map_w, const __
     ptx::launch_dependents();
     if (!a.early) ptx::wait_for_upstream();
 
-    if (warp == 0) {
-        // ------------------------------------------------------------ producer
-        // The whole warp runs the loop so that addresses and coordinates stay warp-uniform; one elected lane issues.
-        // The first round of the ring fetches announced weights and their scales before the wait on upstream.
+    if (warp == 0 || warp == kGroupedWarps + 3) {
+        // ------------------------------------------------------------ producers: weights and their scales (0), tokens (19)
+        // Whole warps run the loop so that addresses and coordinates stay warp-uniform; one elected lane issues. Announced
+        // weights need no upstream kernel, so their producer fills the ring ahead of it.
+        const bool weights = warp == 0;
         if (ptx::elect_one()) {
-            ptx::prefetch_tensormap(&map_w);
-            ptx::prefetch_tensormap(&map_x);
-            ptx::prefetch_tensormap(&map_sw);
+            ptx::prefetch_tensormap(weights ? &map_w : &map_x);
+            if (weights) ptx::prefetch_tensormap(&map_sw);
         }
-        const int ahead = int(blockIdx.x) < tiles ? min(kStages, kb_count) : 0;
-        const int first_n0 = (int(blockIdx.x) % n_tiles) * Channels;
-        const auto load_weights = [&](int stage, int slot, int kb, int n0) {
-            const uint32_t bar = ptx::smem_u32(&full_bar[stage]);
-            ptx::mbar_arrive_expect_tx(bar, kStageBytes + Channels * 4);
-            ptx::tma_load_2d(tiles_base + uint32_t(stage) * kStageBytes, &map_w, bar, kb * kBlockK, n0);
-            ptx::tma_load_2d(scale_base + uint32_t(slot) * kScaleSlotBytes, &map_sw, bar, n0, kb);
-        };
-        for (int i = 0; i < ahead; ++i) {
-            if (ptx::elect_one()) load_weights(i, i, i, first_n0);
-            __syncwarp();
-        }
-        ptx::wait_for_upstream();
+        if (!weights) ptx::wait_for_upstream();
         int stage = 0, slot = 0, filled = 0; // filled: K blocks so far, over all tiles
         uint32_t phase = 0;
         bool ok = true;
@@ -145,20 +234,23 @@ w8a8_tcgen05_prefill_grouped(const __grid_constant__ CUtensorMap map_w, const __
                 ok = filled < kStages || ptx::mbar_wait(ptx::smem_u32(&empty_bar[stage]), phase ^ 1u, abort_ptr);
                 ok = __all_sync(0xffffffffu, ok);
                 if (!ok) break;
-                if (ptx::elect_one()) {
-                    if (filled >= ahead) load_weights(stage, slot, kb, n0);
-                    ptx::tma_load_2d(tiles_base + uint32_t(stage) * kStageBytes + kWeightBytes, &map_x,
-                                     ptx::smem_u32(&full_bar[stage]), kb * kBlockK, m0);
+                const uint32_t bar = ptx::smem_u32(&full_bar[stage]), tile_smem = tiles_base + uint32_t(stage) * kStageBytes;
+                const uint32_t scale_slot = scale_base + uint32_t(slot) * kScaleSlotBytes;
+                if (weights) {
+                    if (ptx::elect_one()) {
+                        ptx::mbar_arrive_expect_tx(bar, kWeightBytes + Channels * 4);
+                        ptx::tma_load_2d(tile_smem, &map_w, bar, kb * kBlockK, n0);
+                        ptx::tma_load_2d(scale_slot, &map_sw, bar, n0, kb);
+                    }
+                    __syncwarp();
+                } else {
+                    if (ptx::elect_one()) {
+                        ptx::mbar_arrive_expect_tx(bar, kTokenBytes);
+                        ptx::tma_load_2d(tile_smem + kWeightBytes, &map_x, bar, kb * kBlockK, m0);
+                    }
+                    __syncwarp();
+                    grouped_copy_token_scales(a, kb, m0, lane, scale_slot + kBlockChannels * 4u, bar);
                 }
-                __syncwarp();
-                const float *sx = a.sx + size_t(kb) * a.m + m0 + lane;
-                const uint32_t sx_slot = scale_base + uint32_t(slot) * kScaleSlotBytes + uint32_t(kBlockChannels + lane) * 4u;
-#pragma unroll
-                for (int i = 0; i < BM / 32; ++i) {
-                    const bool inside = m0 + lane + 32 * i < a.m;
-                    ptx::copy_async4(sx_slot + 128u * i, inside ? sx + 32 * i : a.sx, inside ? 4u : 0u);
-                }
-                ptx::copy_async_arrive(ptx::smem_u32(&full_bar[stage]));
                 slot = (slot + 1) % kScaleSlots;
                 if (++stage == kStages) { stage = 0; phase ^= 1u; }
             }
@@ -171,13 +263,13 @@ w8a8_tcgen05_prefill_grouped(const __grid_constant__ CUtensorMap map_w, const __
         // match; after a failed wait the abort flag makes every later wait return at once and the
         // issuer stops issuing.
         int stage = 0;
-        uint32_t phase = 0, count = 0; // count: K blocks so far, over all tiles
+        uint32_t phase = 0, round = 0; // rounds so far, over all tiles
         for (int tile = blockIdx.x; tile < tiles; tile += gridDim.x) {
-            for (int kb = 0; kb < kb_count; ++kb, ++count) {
-                const uint32_t buffer = count % kAccumulators;
+            for (int kb = 0; kb < kb_count; ++kb) {
+                const int in_round = kb % kRound;
+                const bool last = in_round == kRound - 1 || kb + 1 == kb_count;
                 if (warp != 1) {
-                    const uint32_t use = (count / kAccumulators) & 1u;
-                    const bool ready = ptx::mbar_wait(ptx::smem_u32(&acc_empty[buffer]), use ^ 1u, abort_ptr) &&
+                    const bool ready = (in_round || ptx::mbar_wait(ptx::smem_u32(&acc_empty[round & 1u]), ((round >> 1) & 1u) ^ 1u, abort_ptr)) &&
                                        ptx::mbar_wait(ptx::smem_u32(&full_bar[stage]), phase, abort_ptr);
                     (void)ptx::pair_barrier_and(__all_sync(0xffffffffu, ready)); // the vote brings the lanes together
                 } else {
@@ -185,36 +277,33 @@ w8a8_tcgen05_prefill_grouped(const __grid_constant__ CUtensorMap map_w, const __
                     ptx::tcgen05_fence_after();
                     const uint32_t tile_smem = tiles_base + uint32_t(stage) * kStageBytes;
                     const uint32_t lo_w = ptx::smem_desc_lo_k128(tile_smem), lo_x = ptx::smem_desc_lo_k128(tile_smem + kWeightBytes);
-                    const uint32_t d = tmem_base + buffer * uint32_t(Channels);
+                    const uint32_t d = tmem_base + (round & 1u) * 256u + uint32_t(in_round * Channels);
                     if (ready && ptx::elect_one()) {
                         if (kInt) ptx::mma_i8_k128(d, lo_x, lo_w, kIdesc, 0u);
                         else ptx::mma_f8_k128(d, lo_x, lo_w, kIdesc, 0u);
                         ptx::tcgen05_commit(ptx::smem_u32(&empty_bar[stage]));
-                        ptx::tcgen05_commit(ptx::smem_u32(&acc_full[buffer]));
+                        if (last) ptx::tcgen05_commit(ptx::smem_u32(&acc_full[round & 1u]));
                     }
                     __syncwarp();
                 }
+                if (last) ++round;
                 if (++stage == kStages) { stage = 0; phase ^= 1u; }
             }
         }
     } else {
         // ------------------------------------------------------------ rescale + epilogue warps
         const int quadrant = warp & 3, quarter = (warp - 2) >> 2; // tensor-memory lanes; which kColumns channels
-        const int row = quadrant * 32 + lane, c0 = quarter * kColumns;
+        const int row = quadrant * 32 + (lane >> 2), c0 = quarter * kColumns, pair = 2 * (lane & 3);
         const uint32_t lane_base = tmem_base + (uint32_t(quadrant * 32) << 16) + uint32_t(c0);
         const bool storer = threadIdx.x == 64; // issues the tile's TMA traffic
-        const float *__restrict__ residual = a.residual_f32;
-        const float *scales = reinterpret_cast<const float *>(aligned + (scale_base - tiles_base));
-        uint8_t *slab_row = aligned + kRingBytes + uint32_t(c0 / 64) * kGroupedSlabBytes + uint32_t(row) * 128u;
-        const ptx::IntBias bias_of_int = ptx::int_bias(raw_base);
+        uint8_t *slab = aligned + kRingBytes + uint32_t(c0 / 64) * kGroupedSlabBytes;
+        const uint32_t sx_at = uint32_t(kBlockChannels + quadrant * 32 + (lane >> 2) * 4) * 4u, sw_at = uint32_t(c0 + pair) * 4u;
         if (storer) ptx::prefetch_tensormap(&map_out);
         ptx::wait_for_upstream();
-        uint32_t count = 0, residual_phase = 0;
+        uint32_t round = 0, slot_at = 0, residual_phase = 0;
         bool ok = true;
         for (int tile = blockIdx.x; tile < tiles && ok; tile += gridDim.x) {
             const int n0 = (tile % n_tiles) * Channels, m0 = (tile / n_tiles) * BM;
-            const int token = m0 + row;
-            const bool token_ok = token < a.m;
             const int valid_slabs = min(kSlabs, (a.n - n0 + 63) / 64);
             if (skip16 && storer) { // into the slabs the results will overwrite: the last tile's stores must have left them
                 ptx::bulk_wait_read<0>();
@@ -223,35 +312,27 @@ w8a8_tcgen05_prefill_grouped(const __grid_constant__ CUtensorMap map_w, const __
                 for (int s = 0; s < valid_slabs; ++s)
                     ptx::tma_load_2d(slab_base + uint32_t(s) * kGroupedSlabBytes, &map_residual, bar, n0 + s * 64, m0);
             }
-            uint64_t result[kColumns / 2];
+            GroupedSums<kColumns> result;
 #pragma unroll
-            for (int i = 0; i < kColumns / 2; ++i) result[i] = 0ull;
+            for (int i = 0; i < 4 * kWords; ++i) result[i / kWords][i % kWords] = 0ull;
 #pragma unroll 1
-            for (int kb = 0; kb < kb_count; ++kb, ++count) {
-                const uint32_t buffer = count % kAccumulators;
-                ok = ptx::mbar_wait(ptx::smem_u32(&acc_full[buffer]), (count / kAccumulators) & 1u, abort_ptr);
+            for (int first = 0; first < kb_count; first += kRound, ++round) {
+                const int blocks = min(kRound, kb_count - first);
+                ok = ptx::mbar_wait(ptx::smem_u32(&acc_full[round & 1u]), (round >> 1) & 1u, abort_ptr);
                 if (!ok) break;
                 ptx::tcgen05_fence_after();
-                uint32_t r[kColumns];
-                ptx::tmem_load<kColumns>(lane_base + buffer * uint32_t(Channels), r);
-                ptx::tmem_load_wait();
-                // Everything is in registers: the tensor cores may have the buffer back.
-                ptx::tcgen05_fence_before();
-                __syncwarp();
-                if (lane == 0) ptx::mbar_arrive(ptx::smem_u32(&acc_empty[buffer]));
-                const float scale_x = scales[(count % kScaleSlots) * (kScaleSlotBytes / 4) + kBlockChannels + row];
-                const uint64_t scale_x2 = ptx::pack2(scale_x, scale_x);
-                const uint32_t sw = ptx::pinned(scale_base + (count % kScaleSlots) * kScaleSlotBytes + uint32_t(c0) * 4u);
+                const uint32_t from = lane_base + (round & 1u) * 256u;
 #pragma unroll
-                for (int q = 0; q < kColumns / 4; ++q) {
-                    const ulonglong2 sw4 = ptx::ld_shared_2x64(sw + 16u * q); // the same address in every lane: a broadcast
-#pragma unroll
-                    for (int h = 0; h < 2; ++h) {
-                        const int i = 4 * q + 2 * h;
-                        const uint64_t p = kInt ? ptx::int_to_float2(r[i], r[i + 1], bias_of_int)
-                                                : ptx::pack2(__uint_as_float(r[i]), __uint_as_float(r[i + 1]));
-                        result[i / 2] = ptx::fma2(p, ptx::mul2(h ? sw4.y : sw4.x, scale_x2), result[i / 2]);
-                    }
+                for (int u = 0; u < kRound; ++u) {
+                    if (u > 0 && u >= blocks) break;
+                    const uint32_t scales = ptx::pinned(scale_base + slot_at);
+                    slot_at = (slot_at + kScaleSlotBytes) % (kScaleSlots * kScaleSlotBytes);
+                    grouped_rescale<kInt, kColumns>(result, from + uint32_t(u * Channels), scales + sx_at, scales + sw_at, [&] {
+                        if (u + 1 < blocks) return;
+                        ptx::tcgen05_fence_before(); // the tensor cores may have the round's buffers back
+                        __syncwarp();
+                        if (lane == 0) ptx::mbar_arrive(ptx::smem_u32(&acc_empty[round & 1u]));
+                    });
                 }
             }
             // ---- tile finished: rows into the slabs, slabs out by TMA.
@@ -264,38 +345,7 @@ w8a8_tcgen05_prefill_grouped(const __grid_constant__ CUtensorMap map_w, const __
             // All warps decide together whether the tile is stored; the barrier also publishes that the slabs are free.
             ok = ptx::barrier_and(1, kRescaleThreads, ok && !*abort_ptr);
             if (!ok) break;
-            const uint4 *gate_row = (Chain & 2) && token_ok ? gate_at(a.ep, token, n0 + c0) : nullptr;
-            const float *skip_row = residual && token_ok ? residual + size_t(token) * a.n + n0 + c0 : nullptr;
-#pragma unroll
-            for (int q = 0; q < kColumns / 8; ++q) { // eight channels = one 16-byte chunk of the slab row
-                uint4 *chunk = reinterpret_cast<uint4 *>(slab_row + ((((c0 & 63) / 8 + q) ^ (row & 7)) * 16));
-                const bool inside = n0 + c0 + 8 * q < a.n; // N is a multiple of 16
-                float value[8];
-#pragma unroll
-                for (int i = 0; i < 4; ++i) ptx::unpack2(result[4 * q + i], value[2 * i], value[2 * i + 1]);
-                if (skip_row && inside) {
-                    const float4 lo = __ldg(reinterpret_cast<const float4 *>(skip_row + 8 * q)), hi = __ldg(reinterpret_cast<const float4 *>(skip_row + 8 * q + 4));
-                    const float s8[8] = {lo.x, lo.y, lo.z, lo.w, hi.x, hi.y, hi.z, hi.w};
-#pragma unroll
-                    for (int i = 0; i < 8; ++i) value[i] = __fadd_rn(value[i], s8[i]);
-                }
-                uint4 packed = pack8x16<F16>(value);
-                if (Chain) {
-                    uint4 bias = make_uint4(0, 0, 0, 0);
-                    if (a.ep.bias && inside) {
-                        const uint16_t *b = static_cast<const uint16_t *>(a.ep.bias) + n0 + c0 + 8 * q;
-                        uint32_t w[4];
-#pragma unroll
-                        for (int i = 0; i < 4; ++i) w[i] = uint32_t(b[2 * i]) | (uint32_t(b[2 * i + 1]) << 16);
-                        bias = make_uint4(w[0], w[1], w[2], w[3]);
-                    }
-                    packed = chain8<F16, (Chain & 2) != 0>(a.ep, packed, bias, gate_row && inside ? __ldg(gate_row + q) : make_uint4(0, 0, 0, 0), skip16 ? *chunk : make_uint4(0, 0, 0, 0));
-                }
-                *chunk = packed;
-            }
-            if (Chain & 4)
-                activate_chunks<F16, kColumns / 8>(
-                    [&](int q) { return reinterpret_cast<uint4 *>(slab_row + ((((c0 & 63) / 8 + q) ^ (row & 7)) * 16)); }, a.ep.activation, a.ep.alpha);
+            grouped_rows_to_slab<F16, Chain, kColumns>(a, result, slab, row, m0 + row, n0 + c0 + pair, (c0 & 63) / 8, skip16);
             ptx::fence_proxy_async_smem(); // the rows are about to be read by the TMA engine
             (void)ptx::barrier_and(1, kRescaleThreads, true);
             if (storer) {

@@ -205,6 +205,24 @@ template <int Columns> __device__ __forceinline__ void tmem_load(uint32_t taddr,
         tmem_load32(taddr + 32u, *reinterpret_cast<uint32_t(*)[32]>(&r[32]));
     }
 }
+// 16 lanes x `Columns` consecutive columns starting at `taddr`, dealt to the warp as a matrix fragment: lane l holds rows l / 4 (r[4j],
+// r[4j + 1]) and l / 4 + 8 (r[4j + 2], r[4j + 3]), columns 8j + 2 * (l % 4) and the next.
+template <int Columns> __device__ __forceinline__ void tmem_load_rows16(uint32_t taddr, uint32_t (&r)[Columns / 2]) {
+    static_assert(Columns == 16 || Columns == 32, "unsupported column count");
+    if constexpr (Columns == 16)
+        asm volatile("tcgen05.ld.sync.aligned.16x256b.x2.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+                     : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7])
+                     : "r"(taddr)
+                     : "memory");
+    else
+        asm volatile("tcgen05.ld.sync.aligned.16x256b.x4.b32 "
+                     "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];"
+                     : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]),
+                       "=r"(r[7]), "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]),
+                       "=r"(r[14]), "=r"(r[15])
+                     : "r"(taddr)
+                     : "memory");
+}
 __device__ __forceinline__ void tmem_load_wait() {
     asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 }
@@ -265,28 +283,10 @@ __device__ __forceinline__ uint64_t fma2(uint64_t a, uint64_t b, uint64_t c) {
     asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
     return r;
 }
-// (a & b) ^ c with all three in registers: one instruction, where two constants would make it two.
-__device__ __forceinline__ uint32_t and_xor(uint32_t a, uint32_t b, uint32_t c) {
-    uint32_t r;
-    asm("lop3.b32 %0, %1, %2, %3, 0x6a;" : "=r"(r) : "r"(a), "r"(b), "r"(c));
-    return r;
-}
-// Exact int -> fp32 of two K-group partials |p| <= 2^21: the bits of 2^23 + 2^22 + p read as fp32, minus that constant. Modulo
-// 2^23 adding 2^22 flips bit 22, so the sum is a logic operation, which runs beside the packed arithmetic (an integer add
-// is issued to the same pipe, and the conversion pipe takes eight cycles per warp instruction). The constants come from
-// int_bias(), which keeps the compiler from fetching them from uniform registers for every use.
-struct IntBias {
-    uint32_t low23, biased;
-    uint64_t minus;
-};
-__device__ __forceinline__ IntBias int_bias(uint32_t smem_base) {
-    const uint32_t zero = (smem_base + (threadIdx.x & 31)) >> 31; // a shared-memory address has no such bit
-    const float m = __uint_as_float(0xCB400000u | zero);          // -(2^23 + 2^22)
-    return {0x7fffffu | zero, 0x4B400000u | zero, pack2(m, m)};
-}
-__device__ __forceinline__ uint64_t int_to_float2(uint32_t a, uint32_t b, const IntBias &k) {
-    return add2(pack2(__uint_as_float(and_xor(a, k.low23, k.biased)), __uint_as_float(and_xor(b, k.low23, k.biased))), k.minus);
-}
+// int -> fp32 of two K-group partials (|p| <= 2^21, so exact). The conversion takes two cycles per warp instruction and multiprocessor
+// quarter, like any integer instruction; building the float's bits by logic and subtracting a constant (a packed add) takes longer
+// (rescale alone, cycles per 128 x 128 K block: 630 -> 504).
+__device__ __forceinline__ uint64_t int_to_float2(uint32_t a, uint32_t b) { return pack2(float(int(a)), float(int(b))); }
 // Four bytes global -> shared (zero when `bytes` is 0), and an arrival on `bar` (counted in its expected arrivals) once this
 // thread's copies so far have landed.
 __device__ __forceinline__ void copy_async4(uint32_t dst, const void *src, uint32_t bytes) {
@@ -301,6 +301,16 @@ __device__ __forceinline__ void copy_async_wait_all() { asm volatile("cp.async.w
 __device__ __forceinline__ ulonglong2 ld_shared_2x64(uint32_t addr) {
     ulonglong2 v;
     asm volatile("ld.shared.v2.b64 {%0, %1}, [%2];" : "=l"(v.x), "=l"(v.y) : "r"(addr));
+    return v;
+}
+__device__ __forceinline__ uint64_t ld_shared_64(uint32_t addr) {
+    uint64_t v;
+    asm volatile("ld.shared.b64 %0, [%1];" : "=l"(v) : "r"(addr));
+    return v;
+}
+__device__ __forceinline__ float4 ld_shared_4x32(uint32_t addr) {
+    float4 v;
+    asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(addr));
     return v;
 }
 __device__ __forceinline__ uint32_t pinned(uint32_t v) {

@@ -90,11 +90,11 @@ double linear_cost(KernelProblem p, LinearPath path, Type format, const ChipMode
         return 1.8 + tile.cycles / 1965.;
     }
     if (persistent_grouped(p, path)) {
-        // Waves of 128 tokens x 64 or 128 channels, bound by the fp32 rescale of every K128 partial tile (0.34 and 0.44 us per
+        // Waves of 128 tokens x 64 or 128 channels, bound by the fp32 rescale of every K128 partial tile (0.28 and 0.42 us per
         // K block, INT8; FP8 is up to 15 % faster).
         const int channels = grouped_channel_tile(p.rows, p.channels, sms);
         const double tiles = double(blocks(p.channels, channels)) * blocks(p.rows, kGroupedTokens);
-        return (channels == 64 ? 2.2 : 2.8) + std::ceil(tiles / sms) * kb_total * (channels == 64 ? 0.34 : 0.44);
+        return (channels == 64 ? 2.9 : 3.2) + std::ceil(tiles / sms) * kb_total * (channels == 64 ? 0.28 : 0.42);
     }
     if (p.rows > kWeightStreamTokens) {
         // Weight-streaming kernel with several token tiles per channel slab. Fitted to launches of 65 to 1024 rows on

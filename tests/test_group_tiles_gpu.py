@@ -42,6 +42,22 @@ def test_persistent_group_kernel_matches_weight_streaming_kernel(ctx_factory, mo
         assert float((out.double() - other.double()).norm() / other.double().norm()) < 2e-3
 
 
+# Rounds of K blocks that are not full, over several tiles per CTA and over one; an fp32 residual, rows and channels past the end.
+@pytest.mark.parametrize("m,n,k", [(1302, 4096, 384), (1150, 2064, 640), (301, 4096, 128), (300, 144, 640), (97, 1024, 896)])
+def test_persistent_group_kernel_with_fp32_residual(ctx_factory, m, n, k):
+    from breeze_tts_cpp_b200 import ops
+    ctx = ctx_factory("group_int8")
+    g = torch.Generator(device="cuda").manual_seed(m * n + k)
+    xv = ctx.quantize_rows(torch.randn(m, k, generator=g, device="cuda").to(torch.bfloat16), ops.RowScaledView.empty(m, k, I8, 128, 128))
+    wv = ctx.quantize_rows(torch.randn(n, k, generator=g, device="cuda").to(torch.bfloat16), ops.RowScaledView.empty(n, k, I8, 128, 128))
+    residual = torch.randn(m, n, generator=g, device="cuda")
+    out, other = (torch.full((m, n), float("nan"), dtype=torch.bfloat16, device="cuda") for _ in range(2))
+    ctx.quant_linear((TCGEN05, 128, 128, 1), xv, wv, out, residual_f32=residual)
+    ctx.quant_linear((TCGEN05, 64, 128, 1), xv, wv, other, residual_f32=residual)
+    assert ctx.status() == 0
+    assert torch.equal(out.view(torch.int16), other.view(torch.int16))  # the same products added in the same order
+
+
 @pytest.mark.parametrize("late", [0, 100_000])  # nanoseconds the refill waiter starts late: by then stages may have been filled twice
 @pytest.mark.parametrize("group,m,tokens,splits,k", [(128, 3, 16, 1, 6144), (128, 20, 32, 1, 4096), (128, 64, 64, 1, 2560), (128, 100, 128, 2, 2304),
                                                      (32, 9, 16, 1, 3072), (64, 33, 64, 1, 2048), (0, 16, 16, 1, 6144), (0, 64, 64, 1, 3072)])
