@@ -5,7 +5,7 @@
 // of 128 is its own integer/fp8 dot product p_g, and out[m,n] = D(sum_g float(p_g) * (sx_g[m] *
 // sw_g[n])) (+ fp32 residual), optionally followed by the finishing chain. The tensor cores therefore produce one
 // partial tile per K block, and CUDA cores rescale and add it. What bounds the kernel is both halves together: the rescale alone takes
-// 49 (FP8) or 57 us (INT8) of a 4096 x 6144 -> 2048 GEMM's 71 or 80, the operands and MMAs alone 50 (32 KB per K block and SM, 18 TB/s
+// 49 (FP8) or 57 us (INT8) of a 4096 x 6144 -> 2048 GEMM's 68 or 80, the operands and MMAs alone 50 (32 KB per K block and SM, 18 TB/s
 // from L2), and each waits for the other at times; the clock falls from 1.96 to 1.82-1.9 GHz besides.
 //
 //   warps 0, 19: producers of the weights and their scales (0) and of the tokens and theirs (19). Per K block one pipeline stage (128
@@ -13,7 +13,7 @@
 //                that K block, on the same barrier: the channels' by TMA, the tokens' by 4-byte asynchronous copies (a row count
 //                need not be a multiple of 4). One warp for both was late: 84.7 against 81.3 us (INT8, as above).
 //   warp 1     : MMA issuer, whole warp in the loop, elected lane issues. The tokens are the MMA's M rows. The accumulators of a
-//                round (two K blocks, four at 64 channels) fill half of tensor memory and change hands together: a barrier test
+//                round (two K blocks) change hands together: a barrier test
 //                and a hand-over per round instead of per K block take a fifth of the rescale warps' instructions out. It
 //                never tests an mbarrier itself: a test waits behind the MMAs in flight.
 //   warp 18    : waiter. Tests "accumulators free" and "stage full" for the next K block and hands the
@@ -25,7 +25,8 @@
 // Sixteen rescale warps: the chain wait - load - arithmetic of one warp is latency, four warps per scheduler
 // hide one another's (eight warps with twice the channels each took about 1100 cycles per K block whatever the format).
 // Measured, GEMM alone, one K block per hand-over, one token row per thread and one producer against this: M=4096, 2048 x 6144: INT8 90 ->
-// 80 us, FP8 77 -> 71; 12288 x 2048 at M=1021: 50 -> 46, 45 -> 41; at 64 channels 114 -> 91, 107 -> 88.
+// 80 us, FP8 77 -> 68; 12288 x 2048 at M=1021: 50 -> 44, 45 -> 38; at 64 channels 114 -> 95, 107 -> 84. Short sums gain nothing (three
+// K blocks, 1305 x 384 -> 1536: 5.4 -> 5.5 us): there the prologue, the epilogue and the code itself are what takes the time.
 // CTA pairs with tiles of 256 x 256 (half the operand bytes) were slower, 90 and 94 us with four accumulators of 128 channels and 82
 // and 72 with two of 256: the way from a free accumulator to the next full one crosses the two CTAs.
 // Every wait is bounded; on expiry the CTA flags the status word and runs to the common exit.
@@ -36,15 +37,17 @@ namespace tts::b200 {
 
 constexpr int kGroupedMaxStages = 7;
 __host__ __device__ constexpr int grouped_stages(int channels) { return channels == 64 ? kGroupedMaxStages : 5; } // what shared memory holds
-// K blocks per round: the accumulators change hands once per round, two rounds of 256 tensor-memory columns alternate.
-__host__ __device__ constexpr int grouped_round(int channels) { return 256 / channels; }
+// K blocks per round: the accumulators change hands once per round. Two rounds of 256 tensor-memory columns alternate at 128 channels,
+// four of 128 columns at 64 (one of four K blocks each is as fast, but twice the code, which a chain of launches finds cold).
+constexpr int kGroupedRound = 2;
+__host__ __device__ constexpr int grouped_buffers(int channels) { return 512 / (kGroupedRound * channels); }
 // Scale slots need no barriers of their own. They are filled with their stage, so an accumulator that is full implies its
 // slot is. And slot c is rewritten for K block c + kScaleSlots only once the MMAs of block b = c + kScaleSlots - stages have
-// retired. Those of b's round were issued when the rescale warps had taken the round two before it out of tensor memory: at least
-// block b - 2 * round, and so they had done with the scales of block b - 2 * round - 1 >= c.
+// retired. Those of b's round were issued when the rescale warps had taken the round `buffers` before it out of tensor memory: at
+// least block b - buffers * round, and so they had done with the scales of the block before that, which is c or later.
 constexpr int kScaleSlots = 16;
-static_assert(kScaleSlots - grouped_stages(64) - 2 * grouped_round(64) - 1 >= 0 && kScaleSlots - grouped_stages(128) - 2 * grouped_round(128) - 1 >= 0,
-              "a scale slot could be rewritten while it is read");
+constexpr bool grouped_slots_suffice(int channels) { return kScaleSlots - grouped_stages(channels) - grouped_buffers(channels) * kGroupedRound - 1 >= 0; }
+static_assert(grouped_slots_suffice(64) && grouped_slots_suffice(128), "a scale slot could be rewritten while it is read");
 constexpr int kGroupedWarps = 16;                          // rescale warps
 constexpr int kGroupedThreads = 32 * (kGroupedWarps + 4);  // + two producers, MMA issuer, waiter
 constexpr int kRescaleThreads = 32 * kGroupedWarps;
@@ -108,14 +111,30 @@ __device__ __forceinline__ void grouped_copy_token_scales(const GroupedArgs &a, 
 // A warp's finished sums into the slab of its channels (128 token rows x 64 channels, swizzled), through the chain. `row`: the thread's
 // first row (all four are the same modulo 8), `token` its token, `channel` its first channel, `chunk` the slab's 16-byte chunk of it.
 template <bool F16, int Chain, int Columns>
-__device__ __forceinline__ void grouped_rows_to_slab(const GroupedArgs &a, const GroupedSums<Columns> &result, uint8_t *slab, int row, int token,
+__device__ __forceinline__ void grouped_rows_to_slab(const GroupedArgs &a, GroupedSums<Columns> &result, uint8_t *slab, int row, int token,
                                                      int channel, int chunk, bool skip16) {
     constexpr int kWords = Columns / 8;
     const int lane = threadIdx.x & 31;
-    const float *__restrict__ residual = a.residual_f32;
+    if (a.residual_f32) {
+#pragma unroll
+        for (int i = 0; i < 4 * kWords; ++i) {
+            const int k = i / kWords, j = i % kWords, m = token + 8 * k, n = channel + 8 * j;
+            if (n >= a.n || m >= a.m) continue; // N is a multiple of 16
+            const float2 s = __ldg(reinterpret_cast<const float2 *>(a.residual_f32 + size_t(m) * a.n + n));
+            result[k][j] = ptx::add2(result[k][j], ptx::pack2(s.x, s.y));
+        }
+    }
     const auto slab_word = [&](int k, int j) {
         return reinterpret_cast<uint32_t *>(slab + uint32_t(row + 8 * k) * 128u + (((chunk + j) ^ (row & 7)) * 16) + 4 * (lane & 3));
     };
+    uint32_t bias_words[kWords]; // the same for all four rows
+    if (Chain) {
+#pragma unroll
+        for (int j = 0; j < kWords; ++j) {
+            const uint16_t *b = static_cast<const uint16_t *>(a.ep.bias) + channel + 8 * j;
+            bias_words[j] = a.ep.bias && channel + 8 * j < a.n ? uint32_t(__ldg(b)) | (uint32_t(__ldg(b + 1)) << 16) : 0u;
+        }
+    }
     // The chain works value by value, so four of a thread's channel pairs at a time stand for its eight consecutive channels.
 #pragma unroll
     for (int q = 0; q < kWords; ++q) {
@@ -124,19 +143,10 @@ __device__ __forceinline__ void grouped_rows_to_slab(const GroupedArgs &a, const
 #pragma unroll
         for (int i = 0; i < 4; ++i) {
             const int k = (4 * q + i) / kWords, j = (4 * q + i) % kWords, m = token + 8 * k, n = channel + 8 * j;
-            const bool inside = n < a.n; // N is a multiple of 16
             ptx::unpack2(result[k][j], value[2 * i], value[2 * i + 1]);
-            if (residual && inside && m < a.m) {
-                const float2 s = __ldg(reinterpret_cast<const float2 *>(residual + size_t(m) * a.n + n));
-                value[2 * i] = __fadd_rn(value[2 * i], s.x);
-                value[2 * i + 1] = __fadd_rn(value[2 * i + 1], s.y);
-            }
             if (Chain) {
-                if (a.ep.bias && inside) {
-                    const uint16_t *b = static_cast<const uint16_t *>(a.ep.bias) + n;
-                    bias[i] = uint32_t(b[0]) | (uint32_t(b[1]) << 16);
-                }
-                if ((Chain & 2) && inside && m < a.m)
+                bias[i] = bias_words[j];
+                if ((Chain & 2) && n < a.n && m < a.m)
                     gate[i] = __ldg(reinterpret_cast<const uint32_t *>(static_cast<const uint16_t *>(a.ep.gate) +
                                                                        size_t(m / a.ep.rows_per_sequence) * a.ep.gate_ld + n));
                 if (skip16) skip[i] = *slab_word(k, j);
@@ -166,7 +176,8 @@ w8a8_tcgen05_prefill_grouped(const __grid_constant__ CUtensorMap map_w, const __
     constexpr bool kInt = F == Type::I8;
     constexpr int BM = kGroupedTokens;
     constexpr int kStages = grouped_stages(Channels);
-    constexpr int kRound = grouped_round(Channels), kColumns = Channels / 4; // kColumns: channels per rescale warp
+    constexpr int kRound = kGroupedRound, kBuffers = grouped_buffers(Channels), kBufferColumns = kRound * Channels;
+    constexpr int kColumns = Channels / 4; // kColumns: channels per rescale warp
     constexpr int kWords = kColumns / 8; // packed channel pairs of one token per rescale thread
     constexpr int kSlabs = Channels / 64;
     constexpr int kWeightBytes = Channels * kBlockK, kTokenBytes = BM * kBlockK;
@@ -176,7 +187,7 @@ w8a8_tcgen05_prefill_grouped(const __grid_constant__ CUtensorMap map_w, const __
 
     extern __shared__ uint8_t dynamic_smem[];
     __shared__ alignas(8) uint64_t full_bar[kStages], empty_bar[kStages];
-    __shared__ alignas(8) uint64_t acc_full[2], acc_empty[2]; // one pair per round in flight
+    __shared__ alignas(8) uint64_t acc_full[kBuffers], acc_empty[kBuffers]; // one pair per round in flight
     __shared__ alignas(8) uint64_t residual_full;
     __shared__ uint32_t tmem_slot;
     __shared__ int abort_flag;
@@ -197,7 +208,7 @@ w8a8_tcgen05_prefill_grouped(const __grid_constant__ CUtensorMap map_w, const __
             ptx::mbar_init(ptx::smem_u32(&full_bar[s]), 2 + 32); // both producers with their bytes, every lane of one with its scales
             ptx::mbar_init(ptx::smem_u32(&empty_bar[s]), 1);
         }
-        for (int b = 0; b < 2; ++b) {
+        for (int b = 0; b < kBuffers; ++b) {
             ptx::mbar_init(ptx::smem_u32(&acc_full[b]), 1);
             ptx::mbar_init(ptx::smem_u32(&acc_empty[b]), kGroupedWarps);
         }
@@ -268,8 +279,9 @@ w8a8_tcgen05_prefill_grouped(const __grid_constant__ CUtensorMap map_w, const __
             for (int kb = 0; kb < kb_count; ++kb) {
                 const int in_round = kb % kRound;
                 const bool last = in_round == kRound - 1 || kb + 1 == kb_count;
+                const uint32_t buffer = round % kBuffers;
                 if (warp != 1) {
-                    const bool ready = (in_round || ptx::mbar_wait(ptx::smem_u32(&acc_empty[round & 1u]), ((round >> 1) & 1u) ^ 1u, abort_ptr)) &&
+                    const bool ready = (in_round || ptx::mbar_wait(ptx::smem_u32(&acc_empty[buffer]), ((round / kBuffers) & 1u) ^ 1u, abort_ptr)) &&
                                        ptx::mbar_wait(ptx::smem_u32(&full_bar[stage]), phase, abort_ptr);
                     (void)ptx::pair_barrier_and(__all_sync(0xffffffffu, ready)); // the vote brings the lanes together
                 } else {
@@ -277,12 +289,12 @@ w8a8_tcgen05_prefill_grouped(const __grid_constant__ CUtensorMap map_w, const __
                     ptx::tcgen05_fence_after();
                     const uint32_t tile_smem = tiles_base + uint32_t(stage) * kStageBytes;
                     const uint32_t lo_w = ptx::smem_desc_lo_k128(tile_smem), lo_x = ptx::smem_desc_lo_k128(tile_smem + kWeightBytes);
-                    const uint32_t d = tmem_base + (round & 1u) * 256u + uint32_t(in_round * Channels);
+                    const uint32_t d = tmem_base + buffer * kBufferColumns + uint32_t(in_round * Channels);
                     if (ready && ptx::elect_one()) {
                         if (kInt) ptx::mma_i8_k128(d, lo_x, lo_w, kIdesc, 0u);
                         else ptx::mma_f8_k128(d, lo_x, lo_w, kIdesc, 0u);
                         ptx::tcgen05_commit(ptx::smem_u32(&empty_bar[stage]));
-                        if (last) ptx::tcgen05_commit(ptx::smem_u32(&acc_full[round & 1u]));
+                        if (last) ptx::tcgen05_commit(ptx::smem_u32(&acc_full[buffer]));
                     }
                     __syncwarp();
                 }
@@ -318,10 +330,11 @@ w8a8_tcgen05_prefill_grouped(const __grid_constant__ CUtensorMap map_w, const __
 #pragma unroll 1
             for (int first = 0; first < kb_count; first += kRound, ++round) {
                 const int blocks = min(kRound, kb_count - first);
-                ok = ptx::mbar_wait(ptx::smem_u32(&acc_full[round & 1u]), (round >> 1) & 1u, abort_ptr);
+                const uint32_t buffer = round % kBuffers;
+                ok = ptx::mbar_wait(ptx::smem_u32(&acc_full[buffer]), (round / kBuffers) & 1u, abort_ptr);
                 if (!ok) break;
                 ptx::tcgen05_fence_after();
-                const uint32_t from = lane_base + (round & 1u) * 256u;
+                const uint32_t from = lane_base + buffer * kBufferColumns;
 #pragma unroll
                 for (int u = 0; u < kRound; ++u) {
                     if (u > 0 && u >= blocks) break;
@@ -331,7 +344,7 @@ w8a8_tcgen05_prefill_grouped(const __grid_constant__ CUtensorMap map_w, const __
                         if (u + 1 < blocks) return;
                         ptx::tcgen05_fence_before(); // the tensor cores may have the round's buffers back
                         __syncwarp();
-                        if (lane == 0) ptx::mbar_arrive(ptx::smem_u32(&acc_empty[round & 1u]));
+                        if (lane == 0) ptx::mbar_arrive(ptx::smem_u32(&acc_empty[buffer]));
                     });
                 }
             }
