@@ -30,6 +30,7 @@ SOURCES = [
     ("kernels/quant_norm.cu", ["--fmad=false"]),
     ("kernels/quant_gated.cu", ["--fmad=false"]),
     ("kernels/quant_linear.cu", []),
+    ("kernels/quant_linear_dense.cu", []),
     ("kernels/quant_linear_static.cu", []),
     ("ops/quantized_gemm.cpp", []),
     ("ops/quantization_policy.cpp", []),

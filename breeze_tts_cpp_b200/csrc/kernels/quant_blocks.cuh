@@ -173,13 +173,10 @@ template <Type F, bool Finite> __device__ __forceinline__ uint64_t encode8(const
     }
 }
 
-// Rotates and quantizes the 128-column block this lane's group of four holds (lane & 3 = which 32 columns; `column` =
-// the first of this lane's). `raw` = its 32 storage values with the signs already flipped (XOR with load_masks: the
-// product with +-1). Writes 32 bytes at `q` (32-byte aligned) and, from the
-// first lane of the four, the block's scale. Every lane of the warp must call this; lanes with `active` false store
-// nothing.
-template <Type F, class T>
-__device__ __forceinline__ void rotate_quantize32(const uint32_t (&raw)[16], unsigned char *q, float *scale, bool active) {
+// Rotates and quantizes the 128-column block this lane's group of four holds (lane & 3 = which 32 columns). `raw` = its 32 storage
+// values with the signs already flipped (XOR with load_masks: the product with +-1). Hands every lane's 32 bytes and the block's
+// scale to `store`. Every lane of the warp must call this.
+template <Type F, class T, class Store> __device__ __forceinline__ void rotate_quantize32(const uint32_t (&raw)[16], Store store) {
     uint64_t v[16];
 #pragma unroll
     for (int i = 0; i < 16; ++i) v[i] = widen2<T>(raw[i]);
@@ -229,10 +226,7 @@ __device__ __forceinline__ void rotate_quantize32(const uint32_t (&raw)[16], uns
         Words8 bytes;
 #pragma unroll
         for (int i = 0; i < 4; ++i) bytes.w[i] = encode8<F, true>(v + 4 * i, inverse2);
-        if (active) {
-            store_words8(q, bytes);
-            if (!(threadIdx.x & 3)) *scale = step;
-        }
+        store(bytes, step);
         return;
     }
     // Infinities or NaN somewhere in the warp: the maximum that skips NaN, and the clamping encoder.
@@ -250,10 +244,17 @@ __device__ __forceinline__ void rotate_quantize32(const uint32_t (&raw)[16], uns
     Words8 bytes;
 #pragma unroll
     for (int i = 0; i < 4; ++i) bytes.w[i] = encode8<F, false>(v + 4 * i, inverse2);
-    if (active) {
+    store(bytes, step);
+}
+// The same into global memory: 32 bytes at `q` (32-byte aligned) and, from the first lane of the four, the scale; lanes with `active`
+// false store nothing.
+template <Type F, class T>
+__device__ __forceinline__ void rotate_quantize32(const uint32_t (&raw)[16], unsigned char *q, float *scale, bool active) {
+    rotate_quantize32<F, T>(raw, [&](const Words8 &bytes, float step) {
+        if (!active) return;
         store_words8(q, bytes);
         if (!(threadIdx.x & 3)) *scale = step;
-    }
+    });
 }
 
 // ---------------------------------------------------------------- unrotated rows, kept in packed storage precision

@@ -3,6 +3,7 @@
 // switch without edits; `LinearKind::Tcgen05` is the only kind this build executes.
 #pragma once
 #include "core/quantization.h"
+#include "core/tensor.h"
 #include <cuda.h>
 #include <cuda_runtime.h>
 
@@ -31,6 +32,11 @@ struct WeightMaps {
     const void *weights = nullptr;
     int channels = 0, reduction = 0;
 };
+// The GEMM on 16-bit activations, quantized inside the launch (a few rows): the bytes, scales and sums of launch_row_quantize and
+// launch_quant_linear with this path. False when the launch does not take the operands or two launches are faster.
+bool launch_dense_linear(LinearPath config, KernelProblem shape, int rotation, TensorView x, const void *weights, const float *weight_scales,
+                         void *output, void *workspace, size_t workspace_bytes, cudaStream_t stream, Type format, Type output_type,
+                         const ops::Epilogue *finish, const WeightMaps *prepared);
 WeightMaps quant_linear_weight_maps(const void *weights, int channels, int reduction);
 // Tile/split choice for a problem with the B200 chip model: tokens = token tile (16..256),
 // channels = 128, splits = split-K. Shorthand for `select_linear` (ops/quantization_policy.h).

@@ -2,6 +2,7 @@
 // launch. Drop-in for the reference launchers `launch_quant_linear` and `grouped_quant_gemm`
 // (src/ops/kernels/quant/quant_dispatch.cu:194-234, quant_grouped.cu:221-239).
 #include "kernels/quant_dispatch.h"
+#include "kernels/quant_linear_dense.h"
 #include "kernels/quant_linear_sm100.cuh"
 #include "kernels/quant_prefill_pair_sm100.cuh"
 #include "kernels/quant_prefill_grouped_sm100.cuh"
@@ -257,6 +258,7 @@ void quant_linear_initialize(int device) {
                                  std::to_string(p.major) + std::to_string(p.minor));
     raise_limits<Type::I8>();
     raise_limits<Type::FP8>();
+    raise_dense_limits();
     encode_tiled();
     check(cudaSetDevice(current), "cudaSetDevice");
     done[device] = true;
@@ -313,10 +315,10 @@ WeightMaps quant_linear_weight_maps(const void *weights, int channels, int reduc
     return maps;
 }
 
-void launch_quant_linear(LinearPath config, KernelProblem shape, const void *input, const float *xs,
-                         const void *weights, const float *ws, void *y, void *workspace, size_t bytes,
-                         cudaStream_t stream, Type format, Type output_type, const ops::Epilogue *finish,
-                         const WeightMaps *prepared) {
+namespace {
+// What every launch checks and hands to its kernel, whichever that is.
+GemmArgs checked_args(LinearPath config, KernelProblem shape, const void *input, const float *xs, const void *weights, const float *ws, void *y,
+                      void *workspace, size_t bytes, Type format, Type output_type, const ops::Epilogue *finish, const WeightMaps *prepared) {
     const bool grouped = shape.input_group || shape.weight_group;
     if (output_type != Type::BF16 && output_type != Type::F16 &&
         !(output_type == Type::I32 && format == Type::I8 && !grouped && !finish))
@@ -331,12 +333,12 @@ void launch_quant_linear(LinearPath config, KernelProblem shape, const void *inp
     for (int group : {shape.input_group, shape.weight_group})
         if (group && group != 32 && group != 64 && group != 128)
             throw std::invalid_argument("unsupported GEMM quantization group size");
-    if (!input || !xs || !weights || !ws || !y) throw std::invalid_argument("quantized GEMM null operand");
+    if (!input || !weights || !ws || !y) throw std::invalid_argument("quantized GEMM null operand");
     const int kb_total = (shape.reduction + kBlockK - 1) / kBlockK;
     const int bn = config.tokens, splits = config.splits;
     if (config.channels != kBlockChannels || splits < 1 || splits > kb_total || splits > kMaxSplits)
         throw std::invalid_argument("invalid tcgen05 tile or split (splits form a cluster of at most 8 CTAs)");
-    const int n_tiles = (shape.channels + kBlockChannels - 1) / kBlockChannels, m_tiles = (shape.rows + bn - 1) / bn;
+    const int m_tiles = (shape.rows + bn - 1) / bn;
     if (m_tiles > 65535 || splits > 65535) throw std::invalid_argument("quantized GEMM grid exceeds capacity");
     if (!workspace || bytes < kWorkspaceHeader) throw std::invalid_argument("quantized GEMM workspace missing");
 
@@ -375,9 +377,28 @@ void launch_quant_linear(LinearPath config, KernelProblem shape, const void *inp
         vector_io = vector_io && aligned16(e.residual_f32.data);
     }
     args.vector_io = vector_io;
-    const bool announced = prepared && prepared->weights == weights && prepared->channels == shape.channels &&
-                           prepared->reduction == shape.reduction;
-    args.early = announced;
+    args.early = prepared && prepared->weights == weights && prepared->channels == shape.channels && prepared->reduction == shape.reduction;
+    return args;
+}
+// Failure-path injections, one-shot; only the weight-streaming kernel honours them.
+void take_injections(GemmArgs &args) {
+    args.expiry_extra_bytes = pending_expiry.extra_bytes;
+    args.wait_limit_cycles = pending_expiry.limit_cycles;
+    pending_expiry = {};
+    args.refill_delay_ns = pending_refill_delay;
+    pending_refill_delay = 0;
+}
+} // namespace
+
+void launch_quant_linear(LinearPath config, KernelProblem shape, const void *input, const float *xs,
+                         const void *weights, const float *ws, void *y, void *workspace, size_t bytes,
+                         cudaStream_t stream, Type format, Type output_type, const ops::Epilogue *finish,
+                         const WeightMaps *prepared) {
+    GemmArgs args = checked_args(config, shape, input, xs, weights, ws, y, workspace, bytes, format, output_type, finish, prepared);
+    if (!xs) throw std::invalid_argument("quantized GEMM null operand");
+    const bool grouped = shape.input_group || shape.weight_group, announced = args.early;
+    const int kb_total = (shape.reduction + kBlockK - 1) / kBlockK, bn = config.tokens, splits = config.splits;
+    const int n_tiles = (shape.channels + kBlockChannels - 1) / kBlockChannels, m_tiles = (shape.rows + bn - 1) / bn;
     // Compute-bound shapes take the persistent, double-buffered CTA-pair kernel (its epilogue moves whole aligned rows).
     if (!grouped && bn == kPrefillTokens && splits == 1 && output_type != Type::I32 && args.vector_io &&
         (!args.ep.residual || args.ep.residual_vector)) {
@@ -401,7 +422,7 @@ void launch_quant_linear(LinearPath config, KernelProblem shape, const void *inp
     }
     // K-group shapes beyond decode (both operands grouped by 128, no split) take the persistent K-group kernel.
     if (grouped && shape.input_group == kBlockK && shape.weight_group == kBlockK && bn == kGroupedTokens && splits == 1 &&
-        args.vector_io && aligned16(ws) && (!args.ep.residual || args.ep.residual_vector)) {
+        args.vector_io && reinterpret_cast<uintptr_t>(ws) % 16 == 0 && (!args.ep.residual || args.ep.residual_vector)) {
         GroupedArgs group{args.m, args.n, args.k, xs, args.ep.residual_f32, args.status};
         group.ep = args.ep;
         group.early = announced;
@@ -429,11 +450,7 @@ void launch_quant_linear(LinearPath config, KernelProblem shape, const void *inp
     // multiprocessor (the second allocation would wait for the first CTA, and with split-K clusters
     // two such waits can form a cycle): ask for more than half of the shared memory.
     if (grouped) launch.smem = std::max(launch.smem, size_t(120) * 1024);
-    args.expiry_extra_bytes = pending_expiry.extra_bytes; // one-shot, only the weight-streaming kernel honours it
-    args.wait_limit_cycles = pending_expiry.limit_cycles;
-    pending_expiry = {};
-    args.refill_delay_ns = pending_refill_delay;
-    pending_refill_delay = 0;
+    take_injections(args);
     args.stages = launch.stages;
     args.tile_region = int(launch.tile_region);
     args.owned_passes = launch.owned_passes;
@@ -445,6 +462,38 @@ void launch_quant_linear(LinearPath config, KernelProblem shape, const void *inp
         if (grouped) launch_tokens<Type::FP8, true>(bn, map_w, map_x, args, grid, launch.smem, stream);
         else launch_tokens<Type::FP8, false>(bn, map_w, map_x, args, grid, launch.smem, stream);
     }
+}
+
+bool launch_dense_linear(LinearPath config, KernelProblem shape, int rotation, TensorView x, const void *weights, const float *ws, void *y,
+                         void *workspace, size_t bytes, cudaStream_t stream, Type format, Type output_type, const ops::Epilogue *finish,
+                         const WeightMaps *prepared) {
+    const bool grouped = shape.input_group || shape.weight_group;
+    const int kb_total = shape.reduction / kBlockK;
+    // Whole K blocks, K groups of 128 with their rotation or neither, rows that can be read in 16 (groups: 32) byte pieces.
+    if (config.kind != LinearKind::Tcgen05 || config.tokens > kDenseTokens || shape.rows > config.tokens || shape.reduction % kBlockK ||
+        (x.type != Type::BF16 && x.type != Type::F16) || x.ld() % (grouped ? 16 : 8) || reinterpret_cast<uintptr_t>(x.data) % (grouped ? 32 : 16) ||
+        (grouped ? shape.input_group != kBlockK || shape.weight_group != kBlockK || rotation != kBlockK : rotation != 0))
+        return false;
+    const int per_split = (kb_total + config.splits - 1) / config.splits;
+    if (!dense_pays(shape.rows, shape.reduction, per_split, grouped)) return false;
+    const DenseShape launch = dense_launch_shape(config.tokens, grouped, per_split, config.splits);
+    if (!launch.fits) return false;
+    DenseArgs args{};
+    static_cast<GemmArgs &>(args) = checked_args(config, shape, x.data, nullptr, weights, ws, y, workspace, bytes, format, output_type, finish, prepared);
+    take_injections(args);
+    args.stages = launch.stages;
+    args.tile_region = int(launch.tile_region);
+    args.owned_passes = launch.owned_passes;
+    args.x = x.data;
+    args.x_ld = x.ld();
+    args.token_offset = launch.token_offset;
+    args.largest_offset = launch.largest_offset;
+    // As below: a K-group CTA takes all of tensor memory and must have its multiprocessor to itself.
+    const size_t smem = grouped ? std::max(launch.smem, size_t(120) * 1024) : launch.smem;
+    const CUtensorMap map_w = args.early ? prepared->values : operand_map(weights, shape.channels, shape.reduction, kBlockChannels, true);
+    launch_dense_instance(format, grouped, config.tokens, x.type, map_w, args,
+                          dim3((shape.channels + kBlockChannels - 1) / kBlockChannels, 1, config.splits), smem, stream);
+    return true;
 }
 
 void grouped_quant_gemm(KernelProblem problem, const void *input, const float *input_scales,

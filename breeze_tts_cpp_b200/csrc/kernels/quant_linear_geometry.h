@@ -91,4 +91,37 @@ inline LaunchShape launch_shape(int bn, bool grouped, int kb_per_split, int spli
     shape.smem = fixed + shape.tile_region;
     return shape;
 }
+// The same kernel when it quantizes 16-bit activations itself: the ring holds weights only, every K block's token tile stays.
+constexpr int kDenseTokens = 32;
+struct DenseShape : LaunchShape {
+    int token_offset = 0, largest_offset = 0;
+};
+inline DenseShape dense_launch_shape(int bn, bool grouped, int kb_per_split, int splits) {
+    const LaunchShape usual = launch_shape(bn, grouped, kb_per_split, splits);
+    const size_t stage = size_t(kBlockChannels) * kBlockK, tokens = size_t(kb_per_split) * bn * kBlockK;
+    DenseShape shape;
+    if (!usual.fits) return shape;
+    const size_t largest = grouped ? 0 : size_t(2) * bn * sizeof(uint32_t);
+    const size_t fixed = usual.smem - usual.tile_region + tokens + largest;
+    if (fixed + 2 * stage > kSmemBudget) return shape;
+    shape.fits = true;
+    shape.stages = std::max(2, std::min({int((kSmemBudget - fixed) / stage), kMaxStages, std::max(2, kb_per_split)}));
+    shape.owned_passes = usual.owned_passes;
+    shape.token_offset = int(shape.stages * stage); // at least the transposed tile of an unsplit launch (32 tokens x 128 channels x 4 bytes)
+    shape.tile_region = size_t(shape.token_offset) + tokens;
+    shape.smem = fixed - tokens + shape.tile_region;
+    shape.largest_offset = int(shape.smem - largest - 1024); // from the 1024-byte aligned start
+    return shape;
+}
+// Whether quantizing inside the GEMM is possible (per-row scales: a thread's registers hold its part of a row) and pays. It takes
+// the launch of the quantizer out, 3.1 of 6.2 us on the host; on the device it is no shorter, since every CTA encodes its K range of
+// all rows. One call after another, two launches against one: K=2048 -> 2048 in four splits 6.1 -> 5.1 us at one row, 5.4 at eight;
+// -> 4096 in two 6.2 -> 5.4, 5.8; -> 12288 unsplit 6.5 -> 6.4 at three rows, but 6.3 -> 6.6 at four and 6.9 at eight; K groups,
+// 6144 -> 2048 in six 6.3 -> 6.0 at one, 6.7 -> 6.5 at eight, 7.3 -> 8.2 at sixteen. So the line lies by a CTA's share of blocks.
+inline bool dense_pays(int rows, int reduction, int kb_per_split, bool grouped) {
+    if (grouped) return rows * kb_per_split <= 64;
+    int spread = 1; // rows the eight warps share, one to eight
+    while (spread < rows) spread *= 2;
+    return spread <= 8 && int64_t(spread) * reduction <= 16384 && rows * kb_per_split <= 48;
+}
 } // namespace tts::b200

@@ -32,6 +32,7 @@
 //                    (fp32 residual, bias, bf16 store) is a coalesced 16-byte vector.
 #pragma once
 #include "kernels/sm100_ptx.cuh"
+#include "kernels/quant_blocks.cuh"
 #include "kernels/quant_linear_geometry.h"
 #include "kernels/sequence_finish.cuh"
 #include "core/tensor.h"
@@ -83,6 +84,12 @@ struct GemmArgs {
     long long wait_limit_cycles;
     unsigned refill_delay_ns; // the refill waiter's start held back (quant_linear_inject_refill_delay); 0 in normal operation
     FusedEpilogue ep;
+};
+// Of the instances that quantize 16-bit activations: those, their row stride in elements, and where in the dynamic shared memory
+// their quantized tiles lie (behind the weight ring) and the rows' largest magnitudes (behind everything).
+struct DenseArgs : GemmArgs {
+    const void *x;
+    int x_ld, token_offset, largest_offset;
 };
 
 // Two 16-bit values in one word -> fp32.
@@ -248,14 +255,19 @@ template <bool Grouped> constexpr int kStreamThreads = kGemmThreads + (Grouped ?
 // and unsplit launches, and one resident copy of that larger kernel beats two (28 layers, 3 / 16 / 32 rows: 729 / 796 / 830
 // against 756 / 833 / 855 us; at 57 rows, in the 64-token tile, two are better, 1024 against 1040).
 template <bool Grouped, int BN> constexpr bool kOneInstance = Grouped && BN < 64;
-template <Type F, bool Grouped, int BN, bool Plain, bool Split>
-__global__ void __launch_bounds__(kStreamThreads<Grouped>, (!Grouped && BN <= 64) ? 2 : 1)
+constexpr int kDenseLoads = 8; // 16-byte pieces of a row that a thread holds: 16384 values per CTA
+// `X`, when not void, is the type of 16-bit activations that this launch quantizes itself (GemmArgs::x): the epilogue warps, idle until
+// the accumulators are full, encode the CTA's K range into resident token tiles while the weights arrive. A few rows only: every
+// CTA of a channel slab encodes the same rows again, and with one scale per row reads them whole.
+template <Type F, bool Grouped, int BN, bool Plain, bool Split, class X = void>
+__global__ void __launch_bounds__(kStreamThreads<Grouped>, (!Grouped && BN <= 64 && std::is_void_v<X>) ? 2 : 1)
 w8a8_tcgen05_gemm(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_x,
-                  const __grid_constant__ GemmArgs a) {
+                  const __grid_constant__ std::conditional_t<std::is_void_v<X>, GemmArgs, DenseArgs> a) {
     constexpr bool kInt = F == Type::I8;
     constexpr bool kIntAcc = kInt && !Grouped; // partial tiles / raw outputs carry int32 bit patterns
     constexpr int kWeightBytes = kBlockChannels * kBlockK, kTokenBytes = BN * kBlockK;
-    constexpr int kStageBytes = kWeightBytes + kTokenBytes;
+    constexpr bool kDense = !std::is_void_v<X>, kOne = kOneInstance<Grouped, BN> || kDense;
+    constexpr int kStageBytes = kWeightBytes + (kDense ? 0 : kTokenBytes);
     // K-group mode gives every K block its own accumulator for as long as tensor memory lasts (512
     // columns: 32 buffers at BN=16 ... 4 at BN=128) and reuses them round-robin after that.
     constexpr int kAccBuffers = Grouped ? (512 / BN > 32 ? 32 : 512 / BN) : 1;
@@ -274,14 +286,14 @@ w8a8_tcgen05_gemm(const __grid_constant__ CUtensorMap map_w, const __grid_consta
     __shared__ float sx_tile[BN]; // per-row activation scales of this token tile
 
     // Dynamic shared memory, 1024-byte aligned for the swizzled TMA boxes:
-    //   [pipeline stages | split-K slots pushed by the cluster peers | K-group scales]
+    //   [pipeline stages | dense: token tiles | split-K slots pushed by the cluster peers | K-group scales]
     // Unsplit launches reuse the stage memory for the transposed tile once the last MMA retired;
     // split launches must not, because peers push while this CTA may still be in its main loop.
     const uint32_t raw_base = ptx::smem_u32(dynamic_smem);
     const uint32_t tiles_base = (raw_base + 1023u) & ~1023u;
     uint8_t *tiles_ptr = dynamic_smem + (tiles_base - raw_base);
     const int splits = Split ? a.splits : 1;
-    const bool split_k = Split && (!kOneInstance<Grouped, BN> || splits > 1);
+    const bool split_k = Split && (!kOne || splits > 1);
     const uint32_t reduce_bytes = split_k ? uint32_t(splits * a.owned_passes) * kPassBytes : 0u;
     const uint32_t reduce_base = tiles_base + uint32_t(a.tile_region);
     uint8_t *reduce_ptr = tiles_ptr + a.tile_region;
@@ -295,7 +307,7 @@ w8a8_tcgen05_gemm(const __grid_constant__ CUtensorMap map_w, const __grid_consta
     const int kb_end = int(int64_t(kb_total) * (split + 1) / splits);
     const int kb_count = kb_end - kb_begin;
     // K-group mode: accumulation units per 128-byte K block (1, 2 or 4) and MMAs per unit.
-    const int unit_k = Grouped && !Plain ? min(a.input_group ? a.input_group : kBlockK, a.weight_group ? a.weight_group : kBlockK) : kBlockK;
+    const int unit_k = Grouped && !Plain && !kDense ? min(a.input_group ? a.input_group : kBlockK, a.weight_group ? a.weight_group : kBlockK) : kBlockK;
     const int units = kBlockK / unit_k, unit_mmas = 4 / units;
     const int tile_linear = blockIdx.y * gridDim.x + blockIdx.x;
     const int valid_tokens = min(BN, a.m - m0);
@@ -311,16 +323,24 @@ w8a8_tcgen05_gemm(const __grid_constant__ CUtensorMap map_w, const __grid_consta
             ptx::mbar_init(ptx::smem_u32(&acc_empty[b]), kEpilogueThreads / 32);
         }
         ptx::mbar_init(ptx::smem_u32(&w_full), 1);
-        ptx::mbar_init(ptx::smem_u32(&x_full), 1);
+        ptx::mbar_init(ptx::smem_u32(&x_full), kDense ? kEpilogueThreads / 32 : 1);
         abort_flag = 0;
         ptx::fence_barrier_init();
         ptx::fence_proxy_async_smem();
+    }
+    // Per-row dense instances: the rows' largest magnitudes as bits, without NaN from BN on.
+    [[maybe_unused]] uint32_t *row_largest = nullptr;
+    if constexpr (kDense && !Grouped) {
+        row_largest = reinterpret_cast<uint32_t *>(tiles_ptr + a.largest_offset);
+        if (threadIdx.x >= 64 && threadIdx.x < 64 + 2 * BN) row_largest[threadIdx.x - 64] = 0u;
     }
     if (warp == 1) ptx::tmem_alloc(ptx::smem_u32(&tmem_slot), kTmemColumns);
     ptx::tcgen05_fence_before();
     __syncthreads();
     ptx::tcgen05_fence_after();
     const uint32_t tmem_base = ptx::warp_uniform(tmem_slot);
+    [[maybe_unused]] uint32_t token_base = 0; // dense: the token tiles, one per K block
+    if constexpr (kDense) token_base = tiles_base + uint32_t(a.token_offset);
     volatile int *abort_ptr = &abort_flag;
     // K blocks whose MMAs go out in one burst: prefetched, and with an accumulator nobody used before. The others are waited for.
     const int refill_from = Grouped ? min(min(a.stages, kb_count), kAccBuffers / units) : min(a.stages, kb_count);
@@ -355,7 +375,7 @@ w8a8_tcgen05_gemm(const __grid_constant__ CUtensorMap map_w, const __grid_consta
         // there); one elected lane issues.
         if (ptx::elect_one()) {
             ptx::prefetch_tensormap(&map_w);
-            ptx::prefetch_tensormap(&map_x);
+            if (!kDense) ptx::prefetch_tensormap(&map_x);
         }
         // Weights do not depend on the upstream kernel: fill the ring with weight tiles first, then wait for upstream
         // and add the activation tiles of all those stages, each under ONE barrier. A barrier test between MMA issues
@@ -371,14 +391,16 @@ w8a8_tcgen05_gemm(const __grid_constant__ CUtensorMap map_w, const __grid_consta
                 ptx::tma_load_2d_hint(tiles_base + uint32_t(i) * kStageBytes, &map_w, bar, (kb_begin + i) * kBlockK, n0, stream_once);
         }
         __syncwarp();
-        ptx::wait_for_upstream();
-        if (ptx::elect_one()) {
-            ptx::mbar_arrive_expect_tx(ptx::smem_u32(&x_full), uint32_t(ahead) * kTokenBytes);
-            for (int i = 0; i < ahead; ++i)
-                ptx::tma_load_2d(tiles_base + uint32_t(i) * kStageBytes + kWeightBytes, &map_x,
-                                 ptx::smem_u32(&x_full), (kb_begin + i) * kBlockK, m0);
+        if constexpr (!kDense) {
+            ptx::wait_for_upstream();
+            if (ptx::elect_one()) {
+                ptx::mbar_arrive_expect_tx(ptx::smem_u32(&x_full), uint32_t(ahead) * kTokenBytes);
+                for (int i = 0; i < ahead; ++i)
+                    ptx::tma_load_2d(tiles_base + uint32_t(i) * kStageBytes + kWeightBytes, &map_x,
+                                     ptx::smem_u32(&x_full), (kb_begin + i) * kBlockK, m0);
+            }
+            __syncwarp();
         }
-        __syncwarp();
         int stage = ahead == a.stages ? 0 : ahead;
         uint32_t phase = ahead == a.stages ? 1u : 0u;
         for (int kb = kb_begin + ahead; kb < kb_end; ++kb) {
@@ -388,7 +410,7 @@ w8a8_tcgen05_gemm(const __grid_constant__ CUtensorMap map_w, const __grid_consta
             if (ptx::elect_one()) {
                 ptx::mbar_arrive_expect_tx(bar, kStageBytes);
                 ptx::tma_load_2d_hint(dst, &map_w, bar, kb * kBlockK, n0, stream_once);
-                ptx::tma_load_2d(dst + kWeightBytes, &map_x, bar, kb * kBlockK, m0);
+                if (!kDense) ptx::tma_load_2d(dst + kWeightBytes, &map_x, bar, kb * kBlockK, m0);
             }
             __syncwarp();
             if (++stage == a.stages) { stage = 0; phase ^= 1u; }
@@ -410,12 +432,12 @@ w8a8_tcgen05_gemm(const __grid_constant__ CUtensorMap map_w, const __grid_consta
             // accumulator i to itself while fresh accumulators last.
             const int burst = refill_from; // min(ahead, K blocks with a fresh accumulator)
             int stage = burst == a.stages ? 0 : burst;
-            if (!Grouped || Plain || units == 1) {
+            if (!Grouped || Plain || kDense || units == 1) {
                 // One K block: four MMAs into its accumulator and its reports. A loop of its own: one that also served the
                 // narrow groups issued K-group blocks at half the rate.
                 const auto issue = [&](int it, int at, uint32_t buffer) {
                     const uint32_t tile = tiles_base + uint32_t(at) * kStageBytes;
-                    const uint32_t lo_w = ptx::smem_desc_lo_k128(tile), lo_x = ptx::smem_desc_lo_k128(tile + kWeightBytes);
+                    const uint32_t lo_w = ptx::smem_desc_lo_k128(tile), lo_x = ptx::smem_desc_lo_k128(kDense ? token_base + uint32_t(it) * kTokenBytes : tile + kWeightBytes);
                     const uint32_t d = tmem_base + buffer * uint32_t(BN), accumulate = Grouped ? 0u : uint32_t(it > 0);
                     if (kInt) ptx::mma_i8_k128(d, lo_w, lo_x, kIdesc, accumulate);
                     else ptx::mma_f8_k128(d, lo_w, lo_x, kIdesc, accumulate);
@@ -539,6 +561,78 @@ w8a8_tcgen05_gemm(const __grid_constant__ CUtensorMap map_w, const __grid_consta
             }
         }
 
+        // ---- dense activations: this CTA's K range of the rows into the token tiles, bytes and scales as the row quantizers write them.
+        if constexpr (kDense) {
+            const X *x = static_cast<const X *>(a.x) + size_t(m0) * a.x_ld;
+            const auto chunk_at = [&](int kb, int row, int chunk) { // 16 columns of a 128-byte swizzled row
+                return token_base + uint32_t(kb) * kTokenBytes + uint32_t(row) * 128u + uint32_t((chunk ^ (row & 7)) * 16);
+            };
+            if constexpr (Grouped) {
+                float *scales = scale_smem; // [K block][token]
+                const int blocks = kb_count * valid_tokens;
+#pragma unroll 1
+                for (int first = (warp - 2) * 8; first < blocks; first += kEpilogueThreads / 4) { // four lanes per block of 128
+                    const int block = first + (lane >> 2), part = lane & 3;
+                    const bool active = block < blocks;
+                    const int kb = active ? block / valid_tokens : 0, row = active ? block - kb * valid_tokens : 0;
+                    const int column = (kb_begin + kb) * kBlockK + part * 32;
+                    uint32_t mask[16], raw[16];
+                    load_masks(column, mask);
+                    load_row32(x + size_t(row) * a.x_ld + column, raw);
+#pragma unroll
+                    for (int i = 0; i < 16; ++i) raw[i] ^= mask[i];
+                    rotate_quantize32<F, X>(raw, [&](const Words8 &bytes, float step) {
+                        if (!active) return;
+                        ptx::st_shared_2x64(chunk_at(kb, row, 2 * part), bytes.w[0], bytes.w[1]);
+                        ptx::st_shared_2x64(chunk_at(kb, row, 2 * part + 1), bytes.w[2], bytes.w[3]);
+                        if (!part) scales[kb * BN + row] = step;
+                    });
+                }
+            } else {
+                // A row per warp, or up to eight warps: each thread keeps its columns in registers between the maximum and the bytes.
+                const int log = valid_tokens > 4 ? 5 : valid_tokens > 2 ? 6 : valid_tokens > 1 ? 7 : 8; // threads per row
+                const int row = e_thread >> log, mine = (e_thread & ((1 << log) - 1)) * 8;
+                const X *source = x + size_t(row) * a.x_ld;
+                uint4 v[kDenseLoads];
+                uint32_t largest = 0u;
+#pragma unroll
+                for (int j = 0; j < kDenseLoads; ++j) {
+                    const int column = (j << (log + 3)) + mine;
+                    v[j] = row < valid_tokens && column < a.k ? *reinterpret_cast<const uint4 *>(source + column) : make_uint4(0, 0, 0, 0);
+                }
+#pragma unroll
+                for (int j = 0; j < kDenseLoads; ++j)
+                    largest = max_magnitude16x2(max_magnitude16x2(max_magnitude16x2(max_magnitude16x2(largest, v[j].x), v[j].y), v[j].z), v[j].w);
+                uint32_t bits = __reduce_max_sync(0xffffffffu, fold_magnitude(largest));
+                if (!lane) atomicMax(&row_largest[row], bits);
+                const bool finite = ptx::barrier_and(1, kEpilogueThreads, magnitude_finite<X>(bits));
+                bits = row_largest[row];
+                float amax = magnitude_value<X>(bits);
+                if (!finite) { // infinities or NaN somewhere: also the maximum that skips NaN
+                    float known = 0.f;
+#pragma unroll
+                    for (int j = 0; j < kDenseLoads; ++j)
+                        for (uint32_t word : {v[j].x, v[j].y, v[j].z, v[j].w}) known = max_skipping_nan<X>(known, word);
+                    const uint32_t known_bits = __reduce_max_sync(0xffffffffu, __float_as_uint(known)); // non-negative floats order like their bits
+                    if (!lane) atomicMax(&row_largest[BN + row], known_bits);
+                    asm volatile("bar.sync 1, 256;" ::: "memory");
+                    if (!magnitude_finite<X>(bits)) amax = __uint_as_float(row_largest[BN + row]);
+                }
+                const float step = quant_scale<F>(amax), inverse = __fdiv_rn(1.f, step);
+                const uint64_t inverse2 = f32x2(inverse, inverse);
+                if (!mine && row < valid_tokens) sx_tile[row] = step;
+#pragma unroll
+                for (int j = 0; j < kDenseLoads; ++j) {
+                    const int column = (j << (log + 3)) + mine - kb_begin * kBlockK, chunk = column >> 4;
+                    if (row < valid_tokens && column >= 0 && column < kb_count * kBlockK)
+                        ptx::st_shared_64(chunk_at(chunk >> 3, row, chunk & 7) + uint32_t(column & 8), encode_words<F, X>(v[j], inverse2, magnitude_finite<X>(bits)));
+                }
+            }
+            ptx::fence_proxy_async_smem(); // the tiles are about to be read by the tensor cores
+            __syncwarp();
+            if (lane == 0) ptx::mbar_arrive(ptx::smem_u32(&x_full));
+        }
+
         // ---- phase 1: accumulators (one lane = one channel) -> [token][channel] rows, either in this
         // CTA's shared memory (unsplit) or pushed into the owning peer's slot for this split.
         auto emit_chunk = [&](int chunk, const uint32_t (&words)[16]) {
@@ -558,7 +652,8 @@ w8a8_tcgen05_gemm(const __grid_constant__ CUtensorMap map_w, const __grid_consta
         };
 
         if constexpr (!Grouped) {
-            for (int c = e_thread; c < BN; c += kEpilogueThreads) sx_tile[c] = c < valid_tokens ? a.sx[m0 + c] : 0.f;
+            if constexpr (!kDense)
+                for (int c = e_thread; c < BN; c += kEpilogueThreads) sx_tile[c] = c < valid_tokens ? a.sx[m0 + c] : 0.f;
             if (warp == kGemmThreads / 32 - 1) wait_for_refills(true, wait_limit);
             ok = ptx::mbar_wait(ptx::smem_u32(&acc_full[0]), 0, abort_ptr, wait_limit);
             ptx::tcgen05_fence_after();
@@ -582,7 +677,7 @@ w8a8_tcgen05_gemm(const __grid_constant__ CUtensorMap map_w, const __grid_consta
             // sx_g[unit][token], each operand indexed by its own group width.
             const int shift = __ffs(a.input_group) - 1;
             const uint32_t dst = ptx::smem_u32(sx_smem);
-            for (int i = e_thread; i < unit_count * BN; i += kEpilogueThreads) {
+            for (int i = e_thread; !kDense && i < unit_count * BN; i += kEpilogueThreads) {
                 const int unit = i / BN, token = i % BN, k0 = kb_begin * kBlockK + unit * unit_k;
                 const bool inside = token < valid_tokens && k0 < a.k;
                 if (a.input_group) ptx::copy_async4(dst + 4u * i, inside ? a.sx + size_t(k0 >> shift) * a.m + m0 + token : a.sx, inside ? 4u : 0u);

@@ -313,6 +313,10 @@ __device__ __forceinline__ float4 ld_shared_4x32(uint32_t addr) {
     asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(addr));
     return v;
 }
+__device__ __forceinline__ void st_shared_64(uint32_t addr, uint64_t a) { asm volatile("st.shared.b64 [%0], %1;" ::"r"(addr), "l"(a) : "memory"); }
+__device__ __forceinline__ void st_shared_2x64(uint32_t addr, uint64_t a, uint64_t b) {
+    asm volatile("st.shared.v2.b64 [%0], {%1, %2};" ::"r"(addr), "l"(a), "l"(b) : "memory");
+}
 __device__ __forceinline__ uint32_t pinned(uint32_t v) {
     asm volatile("" : "+r"(v)::"memory");
     return v;

@@ -94,12 +94,12 @@ void Linear::forward(Workspace &workspace, TensorView input, TensorView output, 
     if (input.type != activation_type_ || output.type != activation_type_ || input.cols != input_channels() ||
         output.cols != output_channels() || input.rows != output.rows)
         throw std::invalid_argument("Linear activation shape/type mismatch");
-    ops::linear(input, weight_, bias_, output, epilogue, quantized_view(workspace, input.rows), quantized_output);
+    ops::linear(input, weight_, bias_, output, epilogue, quantized_view(workspace, input.rows), quantized_output, true);
 }
 
 void Linear::project(Workspace &workspace, TensorView input, TensorView output) const {
     validate_types(input, output);
-    ops::linear(input, weight_, {}, output, {}, quantized_view(workspace, input.rows));
+    ops::linear(input, weight_, {}, output, {}, quantized_view(workspace, input.rows), {}, true);
 }
 
 Linear::Workspace &Linear::context_workspace(const ForwardContext &context) const {
@@ -122,7 +122,7 @@ TensorView Linear::apply_context(TensorView input, TensorView output, ForwardCon
         context_workspace(context);
         if (input.data && output.data) prepare_range(context.max_rows, finish.activation);
     } else if (context.mode == ForwardContext::Execute) {
-        ops::linear(input, weight_, bias, output, finish, quantized_view(context_workspace(context), input.rows));
+        ops::linear(input, weight_, bias, output, finish, quantized_view(context_workspace(context), input.rows), {}, true);
     }
     return output;
 }

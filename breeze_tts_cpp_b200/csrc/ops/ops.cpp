@@ -55,7 +55,7 @@ void seal(int device) {
 // in its own epilogue; any other legal epilogue runs as the separate finishing pass the reference
 // uses (src/ops/linear.cpp:76-82), fused with the re-quantization when `quantized_output` is asked for.
 void linear(const LinearOperand &input, const LinearOperand &weight, TensorView bias, TensorView output, Epilogue e,
-            RowScaledView scratch, RowScaledView quantized_output) {
+            RowScaledView scratch, RowScaledView quantized_output, bool private_scratch) {
     auto &gpu = execution_context(output, {bias, e.residual, e.gate, e.condition, e.raw, e.residual_f32,
                                            scratch.values, scratch.scales, quantized_output.values,
                                            quantized_output.scales});
@@ -71,6 +71,11 @@ void linear(const LinearOperand &input, const LinearOperand &weight, TensorView 
     matrix->validate();
     RowScaledView activation;
     if (const auto *dense = std::get_if<TensorView>(&input)) {
+        if (private_scratch && !(e.gate.data && quantized_output.values.data) &&
+            gpu.quantization->linear_dense(*dense, {scratch.group_size, matrix->group_size, scratch.rotation_size}, *matrix, output, plain(e) ? nullptr : &e)) {
+            if (quantized_output.values.data) quantize_rows(output, quantized_output);
+            return;
+        }
         quantize_rows(*dense, scratch);
         activation = scratch;
     } else {

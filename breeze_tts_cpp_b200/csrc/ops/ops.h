@@ -25,9 +25,10 @@ void quantized_norm(TensorView input, TensorView update, TensorView weight, RowS
 void quantized_gated(TensorView input, RowScaledView output, int kind);
 // Quantized Linear: quantizes a dense activation into `scratch` when needed, runs the GEMM and
 // applies bias + epilogue inside it. With `quantized_output`, the finished rows are re-quantized
-// for the next layer and `output` is scratch.
+// for the next layer and `output` is scratch. `private_scratch`: nobody reads `scratch` after the call, so a few rows may
+// be quantized inside the GEMM, which leaves it unwritten.
 void linear(const LinearOperand &input, const LinearOperand &weight, TensorView bias, TensorView output,
-            Epilogue = {}, RowScaledView scratch = {}, RowScaledView quantized_output = {});
+            Epilogue = {}, RowScaledView scratch = {}, RowScaledView quantized_output = {}, bool private_scratch = false);
 // LayerNorm + quantize + projection + finish in one launch for narrow rows (K <= 512, per-row scales).
 // False means "not taken": the caller runs layer_norm_quantize + linear instead, exactly as with the
 // reference (src/ops/linear.h:15-18). The attention write-back argument is accepted and declined.

@@ -152,6 +152,22 @@ bool QuantizedGemm::linear_finish(RowScaledView input, RowScaledView weight, Ten
     impl->run(*plan, input, weight, output, &finish);
     return true;
 }
+bool QuantizedGemm::linear_dense(TensorView x, QuantizationGroups layout, RowScaledView weight, TensorView output, const ops::Epilogue *finish) {
+    weight.validate();
+    const int device = impl->workspace.device();
+    // Every CTA reads the rows for itself: none of them may be written by another one's results.
+    if ((x.type != Type::BF16 && x.type != Type::F16) || !x.data || x.rows < 1 || x.overlaps(output) || layout.weight != weight.group_size ||
+        layout.rotation != weight.rotation_size || weight.values.type != impl->format || x.cols != weight.values.cols || x.rows != output.rows ||
+        weight.values.rows != output.cols || (output.type != Type::BF16 && output.type != Type::F16) || !output.dense() ||
+        (finish && !ops::fusable(*finish) && !ops::gate_fusable(*finish, output.rows, output.cols, output.type)))
+        return false;
+    for (const TensorView *v : {&x, &weight.values, &weight.scales, &output})
+        if (v->device != device) return false;
+    const Plan *plan = impl->find(output.rows, output.cols, x.cols, output.type, layout.activation, layout.weight);
+    return plan && launch_dense_linear(plan->path, {output.rows, plan->channels, plan->reduction, layout.activation, layout.weight}, layout.rotation, x,
+                                       weight.values.data, weight.scales.ptr<float>(), output.data, impl->workspace.data(), impl->workspace.size(),
+                                       impl->stream, impl->format, plan->output_type, finish, announced(weight.values));
+}
 // reference: QuantizedGemm::normalized_linear (src/ops/cuda/quantization.cpp:479-494) in front of
 // normalized_quantized_linear (src/ops/kernels/sequence/sequence_norm.cu:518-575): every condition
 // under which that kernel declines returns false here too.

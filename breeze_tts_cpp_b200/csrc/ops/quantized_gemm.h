@@ -41,6 +41,9 @@ class QuantizedGemm {
     void linear(RowScaledView input, RowScaledView weight, TensorView output);
     // True when the epilogue ran inside the GEMM; false leaves it to the caller's separate pass.
     bool linear_finish(RowScaledView input, RowScaledView weight, TensorView output, const ops::Epilogue &);
+    // Addition: the same two on 16-bit activations, quantized inside the GEMM's launch with the bytes and scales of quantize_rows;
+    // `layout` as of the quantized rows, `finish` null for none. False where that is not possible or not faster.
+    bool linear_dense(TensorView input, QuantizationGroups layout, RowScaledView weight, TensorView output, const ops::Epilogue *finish);
     // Fused LayerNorm + quantize + projection for K <= 512 with per-row scales; false = not taken, which
     // by contract leaves the caller's two-step path responsible.
     bool normalized_linear(TensorView input, TensorView normalized, TensorView norm_weight,
