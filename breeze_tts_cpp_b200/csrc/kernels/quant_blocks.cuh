@@ -66,6 +66,13 @@ __device__ __forceinline__ Words8 load_words8(const void *p) {
 __device__ __forceinline__ void store_words8(void *p, const Words8 &v) {
     asm volatile("st.global.v4.b64 [%0], {%1, %2, %3, %4};" ::"l"(p), "l"(v.w[0]), "l"(v.w[1]), "l"(v.w[2]), "l"(v.w[3]) : "memory");
 }
+// 16 bytes of what an upstream kernel wrote. The compiler may take a plain load through a pointer to const __restrict__ out of a loop,
+// wait on upstream or not; this one stays behind the wait.
+__device__ __forceinline__ uint4 load_upstream16(const void *p) {
+    uint4 r;
+    asm volatile("ld.global.v4.b32 {%0, %1, %2, %3}, [%4];" : "=r"(r.x), "=r"(r.y), "=r"(r.z), "=r"(r.w) : "l"(p) : "memory");
+    return r;
+}
 // 32 consecutive 16-bit elements (64 bytes, 32-byte aligned) as 16 packed words.
 __device__ __forceinline__ void load_row32(const void *p, uint32_t (&raw)[16]) {
 #pragma unroll
@@ -286,7 +293,8 @@ template <Type F, class T> __device__ __forceinline__ uint64_t encode_words(uint
 // (j*Threads + t)*8 .. +7 (zeros past the end); one scale. `slots` holds one word per warp. Equals quantize_tail
 // (quant_codec.cuh) bit for bit with about a third of its instructions.
 template <Type F, class T, int Threads, int Items>
-__device__ __forceinline__ void quantize_row_packed(const uint4 (&v)[Items], unsigned char *out, float *scale, int cols, uint32_t *slots) {
+__device__ __forceinline__ void quantize_row_packed(const uint4 (&v)[Items], unsigned char *out, float *scale, int cols, uint32_t *slots,
+                                                    bool store = true) {
     const auto cta_largest = [&](uint32_t bits) {
         bits = __reduce_max_sync(0xffffffffu, bits);
         if (!(threadIdx.x & 31)) slots[threadIdx.x >> 5] = bits;
@@ -313,11 +321,11 @@ __device__ __forceinline__ void quantize_row_packed(const uint4 (&v)[Items], uns
     }
     const float step = quant_scale<F>(amax), inverse = __fdiv_rn(1.f, step);
     const uint64_t inverse2 = f32x2(inverse, inverse);
-    if (!threadIdx.x) *scale = step;
+    if (!threadIdx.x && store) *scale = step;
 #pragma unroll
     for (int j = 0; j < Items; ++j) {
         const int column = (j * Threads + int(threadIdx.x)) * 8;
-        if (column < cols) *reinterpret_cast<uint64_t *>(out + column) = encode_words<F, T>(v[j], inverse2, finite);
+        if (column < cols && store) *reinterpret_cast<uint64_t *>(out + column) = encode_words<F, T>(v[j], inverse2, finite);
     }
 }
 } // namespace tts::b200

@@ -31,7 +31,7 @@ template <> struct Pair16<__half> {
 
 template <class T> __device__ __forceinline__ uint4 load_raw8(const T *p, int remaining, bool aligned) {
     uint4 raw = make_uint4(0, 0, 0, 0);
-    if (aligned && remaining >= 8) return *reinterpret_cast<const uint4 *>(p);
+    if (aligned && remaining >= 8) return load_upstream16(p);
     T *e = reinterpret_cast<T *>(&raw);
     for (int i = 0; i < 8; ++i)
         if (i < remaining) e[i] = p[i];
@@ -53,85 +53,93 @@ template <Type F, class T, bool Add, bool Rotate, bool Packed>
 __global__ void __launch_bounds__(kThreads)
 rms_quantize(T *__restrict__ x, const T *__restrict__ update, const T *__restrict__ weight,
              const T *__restrict__ update_scale, unsigned char *__restrict__ out, float *__restrict__ scales,
-             int rows, int cols, float eps, bool gemma, int group, bool any_aligned) {
+             int rows, int cols, float eps, bool gemma, int group, bool any_aligned, bool rehearse) {
     const bool aligned = Packed || any_aligned;
     using M = Pair16<T>;
     using P = typename M::P;
     __shared__ float slots[kThreads / 32];
     pdl_launch_dependents();
     const int row = blockIdx.x, column = threadIdx.x * 8;
-    uint4 value = make_uint4(0, 0, 0, 0), w = make_uint4(0, 0, 0, 0);
+    uint4 w = make_uint4(0, 0, 0, 0);
     if (column < cols) w = load_raw8(weight + column, cols - column, aligned); // a parameter: may precede the wait
-    pdl_wait_upstream();
-    if (column < cols) {
-        const int remaining = cols - column;
-        value = load_raw8(x + size_t(row) * cols + column, remaining, aligned);
-        if (Add) {
-            uint4 u = load_raw8(update + size_t(row) * cols + column, remaining, aligned);
-            uint4 s = update_scale ? load_raw8(update_scale + column, remaining, aligned) : make_uint4(0, 0, 0, 0);
-            P *vp = reinterpret_cast<P *>(&value), *up = reinterpret_cast<P *>(&u), *sp = reinterpret_cast<P *>(&s);
+    // `rehearse` (short batches): once through on zeros before the wait, without a global access. A launch finds the instruction caches cold,
+    // and fetching the code while there is nothing else to do takes that off the chain's critical path (with the other two
+    // quantizers, 28 layers: 64 rows INT8 813 -> 809 us, 5 rows FP8 671 -> 661).
+#pragma unroll 1
+    for (int pass = Packed && rehearse ? 0 : 1; pass < 2; ++pass) {
+        const bool real = !Packed || pass;
+        if (real) pdl_wait_upstream();
+        uint4 value = make_uint4(0, 0, 0, 0);
+        if (real && column < cols) {
+            const int remaining = cols - column;
+            value = load_raw8(x + size_t(row) * cols + column, remaining, aligned);
+            if (Add) {
+                uint4 u = load_raw8(update + size_t(row) * cols + column, remaining, aligned);
+                uint4 s = update_scale ? load_raw8(update_scale + column, remaining, aligned) : make_uint4(0, 0, 0, 0);
+                P *vp = reinterpret_cast<P *>(&value), *up = reinterpret_cast<P *>(&u), *sp = reinterpret_cast<P *>(&s);
+#pragma unroll
+                for (int p = 0; p < 4; ++p) {
+                    P b = up[p];
+                    if (update_scale) b = __hmul2(b, sp[p]);
+                    vp[p] = __hadd2(vp[p], b);
+                }
+                store_raw8(x + size_t(row) * cols + column, value, remaining, aligned);
+            }
+        }
+        float sum = 0.f;
+        {
+            const P *vp = reinterpret_cast<const P *>(&value);
 #pragma unroll
             for (int p = 0; p < 4; ++p) {
-                P b = up[p];
-                if (update_scale) b = __hmul2(b, sp[p]);
-                vp[p] = __hadd2(vp[p], b);
+                float2 f = M::unpack(vp[p]);
+                sum = __fadd_rn(sum, __fadd_rn(__fmul_rn(f.x, f.x), __fmul_rn(f.y, f.y)));
             }
-            store_raw8(x + size_t(row) * cols + column, value, remaining, aligned);
         }
-    }
-    float sum = 0.f;
-    {
-        const P *vp = reinterpret_cast<const P *>(&value);
 #pragma unroll
-        for (int p = 0; p < 4; ++p) {
-            float2 f = M::unpack(vp[p]);
-            sum = __fadd_rn(sum, __fadd_rn(__fmul_rn(f.x, f.x), __fmul_rn(f.y, f.y)));
-        }
-    }
+        for (int d = 16; d; d >>= 1) sum = __fadd_rn(sum, __shfl_down_sync(0xffffffffu, sum, d));
+        if (!(threadIdx.x & 31)) slots[threadIdx.x >> 5] = sum;
+        __syncthreads();
+        float total = 0.f;
 #pragma unroll
-    for (int d = 16; d; d >>= 1) sum = __fadd_rn(sum, __shfl_down_sync(0xffffffffu, sum, d));
-    if (!(threadIdx.x & 31)) slots[threadIdx.x >> 5] = sum;
-    __syncthreads();
-    float total = 0.f;
+        for (int p = 0; p < kThreads / 32; ++p) total = __fadd_rn(total, slots[p]);
+        __syncthreads();
+        const float inv_norm = rsqrtf(__fadd_rn(__fdiv_rn(total, float(cols)), eps));
+        float v[1][8];
+        {
+            const P *vp = reinterpret_cast<const P *>(&value), *wp = reinterpret_cast<const P *>(&w);
+            if (Packed) { // the normalized row stays in packed storage precision
+                uint4 row_words[1];
+                P *np = reinterpret_cast<P *>(&row_words[0]);
 #pragma unroll
-    for (int p = 0; p < kThreads / 32; ++p) total = __fadd_rn(total, slots[p]);
-    __syncthreads();
-    const float inv_norm = rsqrtf(__fadd_rn(__fdiv_rn(total, float(cols)), eps));
-    float v[1][8];
-    {
-        const P *vp = reinterpret_cast<const P *>(&value), *wp = reinterpret_cast<const P *>(&w);
-        if (Packed) { // the normalized row stays in packed storage precision
-            uint4 row_words[1];
-            P *np = reinterpret_cast<P *>(&row_words[0]);
+                for (int p = 0; p < 4; ++p) {
+                    const float2 f = M::unpack(vp[p]), wf = M::unpack(wp[p]);
+                    np[p] = gemma ? M::pack(__fmul_rn(__fmul_rn(f.x, inv_norm), __fadd_rn(wf.x, 1.f)),
+                                            __fmul_rn(__fmul_rn(f.y, inv_norm), __fadd_rn(wf.y, 1.f)))
+                                  : __hmul2(M::pack(__fmul_rn(f.x, inv_norm), __fmul_rn(f.y, inv_norm)), wp[p]);
+                }
+                if (column >= cols) row_words[0] = make_uint4(0, 0, 0, 0);
+                quantize_row_packed<F, T, kThreads, 1>(row_words, out + size_t(row) * cols, scales + row, cols,
+                                                       reinterpret_cast<uint32_t *>(slots), real);
+                continue;
+            }
 #pragma unroll
             for (int p = 0; p < 4; ++p) {
-                const float2 f = M::unpack(vp[p]), wf = M::unpack(wp[p]);
-                np[p] = gemma ? M::pack(__fmul_rn(__fmul_rn(f.x, inv_norm), __fadd_rn(wf.x, 1.f)),
-                                        __fmul_rn(__fmul_rn(f.y, inv_norm), __fadd_rn(wf.y, 1.f)))
-                              : __hmul2(M::pack(__fmul_rn(f.x, inv_norm), __fmul_rn(f.y, inv_norm)), wp[p]);
+                float2 f = M::unpack(vp[p]);
+                P normalized;
+                if (gemma) {
+                    float2 wf = M::unpack(wp[p]);
+                    normalized = M::pack(__fmul_rn(__fmul_rn(f.x, inv_norm), __fadd_rn(wf.x, 1.f)),
+                                         __fmul_rn(__fmul_rn(f.y, inv_norm), __fadd_rn(wf.y, 1.f)));
+                } else {
+                    normalized = __hmul2(M::pack(__fmul_rn(f.x, inv_norm), __fmul_rn(f.y, inv_norm)), wp[p]);
+                }
+                float2 r = M::unpack(normalized);
+                v[0][2 * p] = column < cols ? r.x : 0.f;
+                v[0][2 * p + 1] = column < cols ? r.y : 0.f;
             }
-            if (column >= cols) row_words[0] = make_uint4(0, 0, 0, 0);
-            quantize_row_packed<F, T, kThreads, 1>(row_words, out + size_t(row) * cols, scales + row, cols,
-                                                   reinterpret_cast<uint32_t *>(slots));
-            return;
         }
-#pragma unroll
-        for (int p = 0; p < 4; ++p) {
-            float2 f = M::unpack(vp[p]);
-            P normalized;
-            if (gemma) {
-                float2 wf = M::unpack(wp[p]);
-                normalized = M::pack(__fmul_rn(__fmul_rn(f.x, inv_norm), __fadd_rn(wf.x, 1.f)),
-                                     __fmul_rn(__fmul_rn(f.y, inv_norm), __fadd_rn(wf.y, 1.f)));
-            } else {
-                normalized = __hmul2(M::pack(__fmul_rn(f.x, inv_norm), __fmul_rn(f.y, inv_norm)), wp[p]);
-            }
-            float2 r = M::unpack(normalized);
-            v[0][2 * p] = column < cols ? r.x : 0.f;
-            v[0][2 * p + 1] = column < cols ? r.y : 0.f;
-        }
+        quantize_tail<F, kThreads, 1, Rotate>(v, out, scales, row, rows, cols, group, 0, 1, aligned, slots);
     }
-    quantize_tail<F, kThreads, 1, Rotate>(v, out, scales, row, rows, cols, group, 0, 1, aligned, slots);
 }
 
 // K-group mode with rotation: 64 threads per row, 32 consecutive columns each, so that four lanes hold a block for the
@@ -233,7 +241,7 @@ void launch(T *x, const T *update, const T *weight, const T *update_scale, unsig
     }
 #define B200Q_RUN(ADD, ROT)                                                                        \
     launch_pdl("quantized norm launch", aligned && !group && !ROT ? rms_quantize<F, T, ADD, false, true> : rms_quantize<F, T, ADD, ROT, false>, dim3(rows), dim3(kThreads), 0, stream, x, update,   \
-               weight, update_scale, q, s, rows, cols, eps, gemma, group, aligned)
+               weight, update_scale, q, s, rows, cols, eps, gemma, group, aligned, rows <= sms)
     if (update) { if (rotation) B200Q_RUN(true, true); else B200Q_RUN(true, false); }
     else { if (rotation) B200Q_RUN(false, true); else B200Q_RUN(false, false); }
 #undef B200Q_RUN

@@ -22,9 +22,26 @@ constexpr int kThreads = 256;
 template <Type F, class T, int Items, bool Rotate, bool Packed>
 __global__ void __launch_bounds__(kThreads)
 row_quantize_cached(const T *__restrict__ x, unsigned char *__restrict__ q, float *__restrict__ scales,
-                    int rows, int cols, int stride, int group, int parts, bool aligned) {
+                    int rows, int cols, int stride, int group, int parts, bool aligned, bool rehearse) {
     __shared__ float slots[kThreads / 32];
     pdl_launch_dependents();
+    if (Packed) {
+        const T *source = x + size_t(blockIdx.x) * stride;
+#pragma unroll 1
+        for (int pass = rehearse ? 0 : 1; pass < 2; ++pass) {
+            if (pass) pdl_wait_upstream();
+            uint4 raw[Items];
+#pragma unroll
+            for (int j = 0; j < Items; ++j) {
+                const int column = (j * kThreads + int(threadIdx.x)) * 8;
+                raw[j] = make_uint4(0, 0, 0, 0);
+                if (pass && column < cols) raw[j] = load_upstream16(source + column);
+            }
+            quantize_row_packed<F, T, kThreads, Items>(raw, q + size_t(blockIdx.x) * cols, scales + blockIdx.x, cols, reinterpret_cast<uint32_t *>(slots), pass);
+            __syncthreads();
+        }
+        return;
+    }
     pdl_wait_upstream();
     const int row = blockIdx.x / parts, shard = blockIdx.x % parts;
     const T *source = x + size_t(row) * stride;
@@ -36,10 +53,6 @@ row_quantize_cached(const T *__restrict__ x, unsigned char *__restrict__ q, floa
         for (int j = 0; j < Items; ++j) {
             int column = ((j * parts + shard) * kThreads + int(threadIdx.x)) * 8;
             raw[j] = column < cols ? *reinterpret_cast<const uint4 *>(source + column) : make_uint4(0, 0, 0, 0);
-        }
-        if (Packed) { // parts == 1
-            quantize_row_packed<F, T, kThreads, Items>(raw, q + size_t(row) * cols, scales + row, cols, reinterpret_cast<uint32_t *>(slots));
-            return;
         }
 #pragma unroll
         for (int j = 0; j < Items; ++j) unpack8<T>(raw[j], v[j]);
@@ -205,7 +218,7 @@ void launch_typed(const T *x, unsigned char *q, float *scales, int rows, int col
 #define B200Q_LAUNCH(I)                                                                            \
     launch_pdl("row quantize launch", aligned && !group && !Rotate ? row_quantize_cached<F, T, I, false, true>                   \
                                                                     : row_quantize_cached<F, T, I, Rotate, false>, dim3(grid), dim3(kThreads), 0, stream, x, q, \
-               scales, rows, cols, stride, group, parts, aligned)
+               scales, rows, cols, stride, group, parts, aligned, rows <= multiprocessors)
     switch (items) {
     case 1: B200Q_LAUNCH(1); break;
     case 2: B200Q_LAUNCH(2); break;
