@@ -14,19 +14,23 @@
 // Channel tile: chosen per problem by pair_channel_tile (quant_linear_geometry.h). A batch whose 256-wide tiles leave
 // many pairs idle takes narrower ones.
 //
-// Epilogue: one thread = one token row. Per 64-channel slab the eight warps (two per 32-lane quadrant, 32 channels
-// each) pull 32 accumulators per thread, finish them and lay the 16-bit rows down in a swizzled shared-memory slab
+// Epilogue: one thread = one token row. Per 64-channel slab the eight or sixteen warps (two or four per 32-lane quadrant,
+// 32 or 16 channels each) pull their accumulators, finish them and lay the 16-bit rows down in a swizzled shared-memory slab
 // that one thread hands to a TMA store, which clips ragged M and N. The 16-bit residual of the chain comes in the
 // same way, prefetched by TMA into the slabs the results will overwrite while the MMAs run. What it replaces: direct
 // row-wise stores (32 rows per warp instruction: 24 cycles per column of 128 tokens, 84 with a residual) and, for
 // wide outputs, a transposition through shared-memory patches with a barrier per 16 tokens (37 and 95 cycles).
+// Sixteen warps where the chain follows, because the last tile's epilogue, and that of every tile with an activation, is not hidden:
+// eight / sixteen, 750 x 1024 -> 4096 (INT8) with bias 8.1 / 7.6 us, with GELU 9.6 / 8.9; 2048 x 2048 -> 2048 11.7 / 11.2, 13.3 / 12.6;
+// a block of 750 x 1024 with GELU 31.4 / 29.5. Plain rows keep eight: a decoder layer of 1025 rows 87.6 / 89.2, of 2048 FP8 137 / 138.
+// The producers' split (weights, tokens) is that of quant_prefill_grouped_sm100.cuh.
 //
 // Barrier protocol (L = leader, even rank; P = peer):
-//   full[s]      in L : L's producer arrives with expect_tx for BOTH CTAs' bytes; both producers'
+//   full[s]      in L : L's producers arrive with expect_tx for BOTH CTAs' bytes; all four producers'
 //                       TMA loads complete their bytes on it.
 //   empty[s]     in L and P : one multicast tcgen05.commit after the MMAs that read stage s.
 //   acc_full[b]  in L and P : multicast commit after the last MMA of a tile.
-//   acc_empty[b] in L : 16 arrivals (8 epilogue warps of each CTA, the peer's arrive remotely).
+//   acc_empty[b] in L : one arrival per epilogue warp of each CTA (the peer's arrive remotely).
 //   residual_full[i] in each CTA : the residual slab i of the current tile has landed.
 // Every wait is bounded; on expiry the CTA flags the status word and runs to the common exit.
 #pragma once
@@ -34,7 +38,8 @@
 
 namespace tts::b200 {
 
-constexpr int kPairThreads = kGemmThreads + 32; // + the waiter warp
+__host__ __device__ constexpr int pair_epilogue_warps(int chain) { return chain ? 16 : 8; }
+__host__ __device__ constexpr int pair_threads(int chain) { return 32 * (pair_epilogue_warps(chain) + 4); } // + two producers, MMA issuer, waiter
 constexpr int kSlabChannels = 64;
 constexpr uint32_t kSlabBytes = kBlockChannels * kSlabChannels * 2; // 128 token rows of 128 bytes
 
@@ -51,12 +56,13 @@ struct PairArgs {
 // Instances: `Chain` compiles the finishing chain into the epilogue (bit 0; bit 1: with a gate, bit 2: with an activation beyond
 // ReLU, which cost registers and code that the others would miss: 31.7 against 33.4 us for a 750-row block); `F16` is the output type (else bf16).
 template <Type F, int Chain, bool F16>
-__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kPairThreads, 1)
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(pair_threads(Chain), 1)
 w8a8_tcgen05_prefill_pair(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_x,
                           const __grid_constant__ CUtensorMap map_out, const __grid_constant__ CUtensorMap map_residual,
                           const __grid_constant__ PairArgs a) {
     constexpr bool kInt = F == Type::I8;
     constexpr int kTokens = kPrefillTokens, kMyTokens = kTokens / 2; // per tile, per CTA
+    constexpr int kWarps = pair_epilogue_warps(Chain), kColumns = 256 / kWarps; // epilogue warps; channels of a slab that each takes
     constexpr int kAccumulatorColumns = 256;                         // spacing of the two accumulators
     const int channels = a.channels, stages = a.stages;
     const int weight_bytes = channels / 2 * kBlockK, stage_bytes = weight_bytes + kMyTokens * kBlockK; // per CTA
@@ -85,12 +91,12 @@ w8a8_tcgen05_prefill_pair(const __grid_constant__ CUtensorMap map_w, const __gri
 
     if (threadIdx.x == 0) {
         for (int s = 0; s < stages; ++s) {
-            ptx::mbar_init(ptx::smem_u32(&full_bar[s]), 1);
+            ptx::mbar_init(ptx::smem_u32(&full_bar[s]), 2); // the leader's producers with both CTAs' bytes
             ptx::mbar_init(ptx::smem_u32(&empty_bar[s]), 1);
         }
         for (int b = 0; b < 2; ++b) {
             ptx::mbar_init(ptx::smem_u32(&acc_full[b]), 1);
-            ptx::mbar_init(ptx::smem_u32(&acc_empty[b]), 2 * (kEpilogueThreads / 32));
+            ptx::mbar_init(ptx::smem_u32(&acc_empty[b]), 2 * kWarps);
         }
         for (int i = 0; i < kPairResidualSlabs; ++i) ptx::mbar_init(ptx::smem_u32(&residual_full[i]), 1);
         abort_flag = 0;
@@ -107,52 +113,37 @@ w8a8_tcgen05_prefill_pair(const __grid_constant__ CUtensorMap map_w, const __gri
     ptx::launch_dependents();
     if (!a.early) ptx::wait_for_upstream();
 
-    if (warp == 0) {
-        // ------------------------------------------------------------ TMA producer (both CTAs)
-        // The whole warp runs the loop so that addresses and coordinates stay warp-uniform (a copy takes them from
-        // uniform registers); one elected lane issues.
-        if (ptx::elect_one()) {
-            ptx::prefetch_tensormap(&map_w);
-            ptx::prefetch_tensormap(&map_x);
-        }
-        // Announced weights do not depend on the upstream kernel: the first round of the ring starts with them and adds
-        // the activation tiles once upstream is done (each stage's barrier expects both from the start).
+    if (warp == 0 || warp == kWarps + 3) {
+        // ------------------------------------------------------------ producers: weights (0) and tokens (the last warp); both CTAs
+        // Whole warps run the loop so that addresses and coordinates stay warp-uniform (a copy takes them from
+        // uniform registers); one elected lane issues. Announced weights need no upstream kernel, so their producer fills the
+        // ring ahead of it.
+        const bool weights = warp == 0;
+        if (ptx::elect_one()) ptx::prefetch_tensormap(weights ? &map_w : &map_x);
+        if (!weights) ptx::wait_for_upstream();
         const uint32_t full_leader = ptx::map_to_rank(ptx::smem_u32(&full_bar[0]), 0);
-        const int first_n0 = (cluster_id % n_tiles) * channels + int(rank) * (channels / 2);
-        const int ahead = cluster_id < tiles ? min(stages, kb_count) : 0;
-        for (int i = 0; i < ahead; ++i) {
-            if (ptx::elect_one()) {
-                if (leader) ptx::mbar_arrive_expect_tx(ptx::smem_u32(&full_bar[i]), uint32_t(2 * stage_bytes));
-                ptx::tma_load_2d_pair(tiles_base + uint32_t(i * stage_bytes), &map_w, full_leader + uint32_t(i) * 8u, i * kBlockK, first_n0);
-            }
-            __syncwarp();
-        }
-        ptx::wait_for_upstream();
+        const uint32_t bytes = uint32_t(weights ? weight_bytes : kMyTokens * kBlockK), place = weights ? 0u : uint32_t(weight_bytes);
+        const CUtensorMap *map = weights ? &map_w : &map_x;
         int stage = 0, filled = 0; // filled: K blocks so far, over all tiles
         uint32_t phase = 0;
         bool ok = true;
         for (int tile = cluster_id; tile < tiles && ok; tile += clusters) {
-            const int n0 = (tile % n_tiles) * channels + int(rank) * (channels / 2);
-            const int m0 = (tile / n_tiles) * kTokens + int(rank) * kMyTokens;
+            const int y = weights ? (tile % n_tiles) * channels + int(rank) * (channels / 2) : (tile / n_tiles) * kTokens + int(rank) * kMyTokens;
             for (int kb = 0; kb < kb_count; ++kb, ++filled) {
                 if (filled >= stages) {
                     ok = __all_sync(0xffffffffu, ptx::mbar_wait(ptx::smem_u32(&empty_bar[stage]), phase ^ 1u, abort_ptr));
                     if (!ok) break;
                 }
-                const uint32_t bar = full_leader + uint32_t(stage) * 8u, dst = tiles_base + uint32_t(stage * stage_bytes);
                 if (ptx::elect_one()) {
-                    if (filled >= ahead) {
-                        if (leader) ptx::mbar_arrive_expect_tx(ptx::smem_u32(&full_bar[stage]), uint32_t(2 * stage_bytes));
-                        ptx::tma_load_2d_pair(dst, &map_w, bar, kb * kBlockK, n0);
-                    }
-                    ptx::tma_load_2d_pair(dst + uint32_t(weight_bytes), &map_x, bar, kb * kBlockK, m0);
+                    if (leader) ptx::mbar_arrive_expect_tx(ptx::smem_u32(&full_bar[stage]), 2 * bytes);
+                    ptx::tma_load_2d_pair(tiles_base + uint32_t(stage * stage_bytes) + place, map, full_leader + uint32_t(stage) * 8u, kb * kBlockK, y);
                 }
                 __syncwarp();
                 if (++stage == stages) { stage = 0; phase ^= 1u; }
             }
         }
-    } else if (warp == 1 || warp == 10) {
-        // ------------------------------------------------------------ MMA issuer (1) and its waiter (10), leader CTA only
+    } else if (warp == 1 || warp == kWarps + 2) {
+        // ------------------------------------------------------------ MMA issuer (1) and its waiter, leader CTA only
         // The whole warp runs the loop (warp-uniform stage arithmetic); one elected lane issues the
         // four MMAs of a K block from a single instruction block and commits.
         // A barrier test between MMA issues waits behind them: about 550 cycles per K block, which the 512 MMA cycles of
@@ -168,11 +159,11 @@ w8a8_tcgen05_prefill_pair(const __grid_constant__ CUtensorMap map_w, const __gri
                 const int buffer = local & 1;
                 const uint32_t d = tmem_base + uint32_t(buffer * kAccumulatorColumns);
                 for (int kb = 0; kb < kb_count; ++kb) {
-                    if (warp == 10 || !use_waiter) {
+                    if (warp != 1 || !use_waiter) {
                         if (kb == 0) ok = ok && ptx::mbar_wait(ptx::smem_u32(&acc_empty[buffer]), ((uint32_t(local) >> 1) & 1u) ^ 1u, abort_ptr);
                         ok = ok && ptx::mbar_wait(ptx::smem_u32(&full_bar[stage]), phase, abort_ptr);
                     }
-                    if (warp == 10 || !use_waiter) ok = __all_sync(0xffffffffu, ok); // also brings the lanes together
+                    if (warp != 1 || !use_waiter) ok = __all_sync(0xffffffffu, ok); // also brings the lanes together
                     if (use_waiter) ok = ptx::pair_barrier_and(ok);
                     if (warp == 1) {
                         ptx::tcgen05_fence_after();
@@ -193,7 +184,7 @@ w8a8_tcgen05_prefill_pair(const __grid_constant__ CUtensorMap map_w, const __gri
     } else {
         // ------------------------------------------------------------ epilogue warps (both CTAs)
         const int e_thread = threadIdx.x - 64;
-        const int quadrant = warp & 3, half = (warp - 2) >> 2;
+        const int quadrant = warp & 3, quarter = (warp - 2) >> 2; // tensor-memory lanes; which kColumns channels of a slab
         const int row = quadrant * 32 + lane; // token row of this CTA's half = tensor-memory lane
         const uint32_t lane_base = tmem_base + (uint32_t(quadrant * 32) << 16);
         const bool storer = e_thread == 0; // issues every slab's TMA traffic
@@ -222,21 +213,21 @@ w8a8_tcgen05_prefill_pair(const __grid_constant__ CUtensorMap map_w, const __gri
                 }
             }
             const float scale_x = token_ok ? a.sx[token] : 0.f;
-            sw_tile[e_thread] = n0 + e_thread < a.n && e_thread < channels ? a.sw[n0 + e_thread] : 0.f;
-            if (Chain)
+            if (e_thread < kAccumulatorColumns) sw_tile[e_thread] = n0 + e_thread < a.n && e_thread < channels ? a.sw[n0 + e_thread] : 0.f;
+            if (Chain && e_thread < kAccumulatorColumns)
                 bias_tile[e_thread] = a.ep.bias && n0 + e_thread < a.n && e_thread < channels
                                           ? static_cast<const uint16_t *>(a.ep.bias)[n0 + e_thread] : uint16_t(0);
-            // One barrier publishes the scales and makes the verdict of the wait common to all eight
+            // One barrier publishes the scales and makes the verdict of the wait common to all epilogue
             // warps: they leave the loop together or not at all.
-            if (!ptx::barrier_and(1, kEpilogueThreads, ptx::mbar_wait(ptx::smem_u32(&acc_full[buffer]), (uint32_t(local) >> 1) & 1u, abort_ptr)))
+            if (!ptx::barrier_and(1, 32 * kWarps, ptx::mbar_wait(ptx::smem_u32(&acc_full[buffer]), (uint32_t(local) >> 1) & 1u, abort_ptr)))
                 break;
             ptx::tcgen05_fence_after();
             bool ok = true;
 #pragma unroll 1
             for (int slab = 0; slab < valid_slabs; ++slab, ++slab_count) {
-                const int c0 = slab * kSlabChannels + half * 32; // this thread's 32 columns of the tile
-                uint32_t r[32];
-                ptx::tmem_load32(lane_base + uint32_t(buffer * kAccumulatorColumns + c0), r);
+                const int c0 = slab * kSlabChannels + quarter * kColumns; // this thread's columns of the tile
+                uint32_t r[kColumns];
+                ptx::tmem_load<kColumns>(lane_base + uint32_t(buffer * kAccumulatorColumns + c0), r);
                 const uint32_t place = skip16 ? uint32_t(slab) : slab_count % kPairSlabs;
                 uint8_t *out_row = slab_ptr + place * kSlabBytes + uint32_t(row) * 128u;
                 ptx::tmem_load_wait();
@@ -247,8 +238,8 @@ w8a8_tcgen05_prefill_pair(const __grid_constant__ CUtensorMap map_w, const __gri
                 const uint4 *gate_row = (Chain & 2) && token_ok ? gate_at(a.ep, token, n0 + c0) : nullptr;
                 const float *skip_row = residual && token_ok && n0 + c0 < a.n ? residual + size_t(token) * a.n + n0 + c0 : nullptr;
 #pragma unroll
-                for (int q = 0; q < 4; ++q) { // eight channels = one 16-byte chunk of the slab row
-                    uint4 *chunk = reinterpret_cast<uint4 *>(out_row + (((half * 4 + q) ^ (row & 7)) * 16));
+                for (int q = 0; q < kColumns / 8; ++q) { // eight channels = one 16-byte chunk of the slab row
+                    uint4 *chunk = reinterpret_cast<uint4 *>(out_row + (((quarter * (kColumns / 8) + q) ^ (row & 7)) * 16));
                     const float4 w_lo = *reinterpret_cast<const float4 *>(&sw_tile[c0 + 8 * q]);
                     const float4 w_hi = *reinterpret_cast<const float4 *>(&sw_tile[c0 + 8 * q + 4]);
                     const float w8[8] = {w_lo.x, w_lo.y, w_lo.z, w_lo.w, w_hi.x, w_hi.y, w_hi.z, w_hi.w};
@@ -274,13 +265,13 @@ w8a8_tcgen05_prefill_pair(const __grid_constant__ CUtensorMap map_w, const __gri
                 }
                 if (Chain & 4) {
                     // A pass of its own over the thread's finished row: nothing but its values is live in it.
-                    activate_chunks<F16, 4>([&](int q) { return reinterpret_cast<uint4 *>(out_row + (((half * 4 + q) ^ (row & 7)) * 16)); },
+                    activate_chunks<F16, kColumns / 8>([&](int q) { return reinterpret_cast<uint4 *>(out_row + (((quarter * (kColumns / 8) + q) ^ (row & 7)) * 16)); },
                                             a.ep.activation, a.ep.alpha);
                 }
                 ptx::fence_proxy_async_smem(); // the rows are about to be read by the TMA engine
                 // With two buffers the next slab's must be free by the time this barrier lets anyone write it.
                 if (!skip16 && storer) ptx::bulk_wait_read<0>();
-                ok = ptx::barrier_and(1, kEpilogueThreads, ok);
+                ok = ptx::barrier_and(1, 32 * kWarps, ok);
                 if (!ok) break;
                 if (storer) {
                     ptx::tma_store_2d(&map_out, slab_base + place * kSlabBytes, n0 + slab * kSlabChannels, m0);
