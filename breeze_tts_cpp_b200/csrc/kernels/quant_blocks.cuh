@@ -10,6 +10,7 @@
 // are bit-identical to it.
 #pragma once
 #include "kernels/quant_codec.cuh"
+#include <algorithm>
 
 namespace tts::b200 {
 
@@ -36,6 +37,17 @@ __device__ __forceinline__ uint64_t mul_f32x2(uint64_t a, uint64_t b) {
 __device__ __forceinline__ uint64_t fma_f32x2(uint64_t a, uint64_t b, uint64_t c) {
     uint64_t r;
     asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+    return r;
+}
+__device__ __forceinline__ uint64_t sub_f32x2(uint64_t a, uint64_t b) {
+    uint64_t r;
+    asm("sub.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+// Largest magnitude of three, NaN if any is.
+__device__ __forceinline__ float max_magnitude3(float a, float b, float c) {
+    float r;
+    asm("max.NaN.abs.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(a), "f"(b), "f"(c));
     return r;
 }
 // Larger magnitude of the two, NaN if either is; the sign of the result means nothing.
@@ -262,6 +274,105 @@ __device__ __forceinline__ void rotate_quantize32(const uint32_t (&raw)[16], uns
         store_words8(q, bytes);
         if (!(threadIdx.x & 3)) *scale = step;
     });
+}
+
+// ---------------------------------------------------------------- long lists of blocks: one lane per block
+// A warp takes 32 rows of one K group, a lane one row's whole 128 columns: no shuffle stage, signs that are the same for the warp, and
+// one scale, division and address per 128 columns instead of per 32. About 1280 instructions per 32 blocks against 1960 with four lanes
+// each. What that costs is warps (160 registers, three per scheduler), so the rows come by asynchronous copies, the next task's while
+// this one is computed.
+constexpr int kLaneBlockThreads = 64, kLaneBlockResident = 6; // CTAs per multiprocessor
+constexpr int kLaneBlockBytes = 32 * 256;                      // 32 rows of 128 16-bit columns, per warp and operand
+inline int lane_blocks_grid(int tasks, int sms) { return std::min((tasks + kLaneBlockThreads / 32 - 1) / (kLaneBlockThreads / 32), kLaneBlockResident * sms); }
+// From three tasks per warp on: 12288 x 2048 20.2 -> 18.4 us and 4096 x 6144 17.2 -> 15.6, but 8192 x 2048 11.5 -> 12.2.
+inline bool lane_blocks_pay(int tasks, int cols, int sms) { return cols <= kMaskedColumns && tasks >= 3 * kLaneBlockResident * (kLaneBlockThreads / 32) * sms; }
+
+// 32 rows x 256 bytes from `source` (the first row's block, rows `stride` elements apart, `rows` of them left) into `buffer`; 16-byte
+// pieces, XOR-swizzled by the row so that lanes read their rows without bank conflicts. Rows past the last one repeat it.
+template <class T> __device__ __forceinline__ void lane_blocks_fetch(uint32_t buffer, const T *source, int stride, int rows) {
+    const int lane = threadIdx.x & 31, piece = lane & 15;
+#pragma unroll
+    for (int i = 0; i < 16; ++i) {
+        const int r = 2 * i + (lane >> 4), row = min(r, rows - 1);
+        asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(buffer + uint32_t((r * 16 + (piece ^ (r & 7))) * 16)),
+                     "l"(source + size_t(row) * stride + piece * 8)
+                     : "memory");
+    }
+}
+__device__ __forceinline__ void lane_blocks_landed() {
+    asm volatile("cp.async.wait_all;" ::: "memory");
+    __syncwarp();
+}
+// Piece `p` (eight columns) of this lane's row.
+__device__ __forceinline__ uint4 lane_blocks_read(uint32_t buffer, int p) {
+    const int lane = threadIdx.x & 31;
+    uint4 v;
+    asm volatile("ld.shared.v4.b32 {%0, %1, %2, %3}, [%4];"
+                 : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w)
+                 : "r"(buffer + uint32_t((lane * 16 + (p ^ (lane & 7))) * 16))
+                 : "memory");
+    return v;
+}
+// Rotates and quantizes a lane's block (K group `group`; the arithmetic of rotate_quantize32, butterfly by butterfly). Writes 128 bytes
+// at `q` (32-byte aligned) and the scale; lanes with `active` false store nothing. All lanes of the warp call this.
+template <Type F, class T>
+__device__ __forceinline__ void rotate_quantize128(const uint32_t (&raw)[64], int group, unsigned char *q, float *scale, bool active) {
+    uint64_t v[64];
+    const uint4 *masks = reinterpret_cast<const uint4 *>(&rotation_masks.pair[group * 64]); // one address for the warp
+#pragma unroll
+    for (int p = 0; p < 16; ++p) { // span 1: inside a pair
+        const uint4 m = __ldg(masks + p);
+        const uint32_t flip[4] = {m.x, m.y, m.z, m.w};
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            const float2 f = unpack_f32x2(widen2<T>(raw[4 * p + i] ^ flip[i]));
+            v[4 * p + i] = f32x2(__fadd_rn(f.x, f.y), __fsub_rn(f.x, f.y));
+        }
+    }
+#pragma unroll
+    for (int span = 1; span < 64; span <<= 1) { // spans 2 to 64
+#pragma unroll
+        for (int i = 0; i < 64; ++i) {
+            if (!(i & span)) {
+                const uint64_t a = v[i], b = v[i | span];
+                v[i] = add_f32x2(a, b);
+                v[i | span] = sub_f32x2(a, b);
+            }
+        }
+    }
+    const uint64_t norm = f32x2(0.08838834764831845f, 0.08838834764831845f);
+    float m[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+    for (int i = 0; i < 64; ++i) {
+        v[i] = mul_f32x2(v[i], norm);
+        const float2 f = unpack_f32x2(v[i]);
+        m[i & 3] = max_magnitude3(m[i & 3], f.x, f.y);
+    }
+    float amax = max_magnitude3(max_magnitude3(m[0], m[1], m[2]), m[3], 0.f);
+    const bool finite = __all_sync(0xffffffffu, amax <= FLT_MAX); // false for infinities and NaN anywhere in the warp
+    if (!finite) {                                                // the maximum that skips NaN, and the clamping encoder
+        amax = 0.f;
+#pragma unroll
+        for (int i = 0; i < 64; ++i) {
+            const float2 f = unpack_f32x2(v[i]);
+            amax = fmaxf(amax, fmaxf(fabsf(f.x), fabsf(f.y)));
+        }
+    }
+    const float step = quant_scale<F>(amax), inverse = __fdiv_rn(1.f, step);
+    const uint64_t inverse2 = f32x2(inverse, inverse);
+    if (active) *scale = step;
+#pragma unroll
+    for (int p = 0; p < 4; ++p) {
+        Words8 bytes;
+        if (finite) {
+#pragma unroll
+            for (int i = 0; i < 4; ++i) bytes.w[i] = encode8<F, true>(v + 16 * p + 4 * i, inverse2);
+        } else {
+#pragma unroll
+            for (int i = 0; i < 4; ++i) bytes.w[i] = encode8<F, false>(v + 16 * p + 4 * i, inverse2);
+        }
+        if (active) store_words8(q + 32 * p, bytes);
+    }
 }
 
 // ---------------------------------------------------------------- unrotated rows, kept in packed storage precision
