@@ -99,8 +99,8 @@ double linear_cost(KernelProblem p, LinearPath path, Type format, const ChipMode
     if (p.rows > kWeightStreamTokens) {
         // Weight-streaming kernel with several token tiles per channel slab. Fitted to launches of 65 to 1024 rows on
         // K = 512 to 6144, N = 1024 to 12288: a base per token tile, a slope per K block (the operand bytes one SM
-        // pulls; with K groups the rescale), the split-K exchange, and contention for L2 as the grid grows. More than one
-        // wave does not pay: CTAs own their multiprocessor's shared memory, so nothing of the next wave overlaps.
+        // pulls; with K groups the rescale), the split-K exchange (per-row scales: 1.0 to 1.6 us at 64 tokens, 2.1 to 2.4 at
+        // 128), and contention for L2 as the grid grows. More than one wave does not pay: CTAs own their multiprocessor's shared memory, so nothing of the next wave overlaps.
         const bool group = grouped(p);
         const int splits = std::max(1, path.splits), per_split = blocks(kb_total, splits);
         const int units = group_units(p.input_group, p.weight_group);
@@ -112,9 +112,9 @@ double linear_cost(KernelProblem p, LinearPath path, Type format, const ChipMode
         const int64_t slots = splits > 1 ? std::max<int64_t>(splits, int64_t(sms) * resident * 16 / 18 / splits * splits)
                                          : int64_t(sms) * resident;
         const int tile = path.tokens <= 32 ? 0 : path.tokens <= 64 ? 1 : path.tokens <= 128 ? 2 : 3;
-        static constexpr double kBase[2][4] = {{2.3, 2.5, 4.0, 6.2}, {2.7, 3.4, 5.6, 9.0}};
-        static constexpr double kSlope[2][4] = {{0.21, 0.214, 0.214, 0.42}, {0.245, 0.31, 0.44, 0.9}};
-        const double exchange = splits == 1 ? 0.0 : group ? 0.25 + 0.2 * splits : 0.3 + (path.tokens <= 64 ? 0.15 : 0.25) * splits;
+        static constexpr double kBase[2][4] = {{2.3, 2.5, 3.4, 6.2}, {2.7, 3.4, 5.6, 9.0}};
+        static constexpr double kSlope[2][4] = {{0.17, 0.17, 0.17, 0.42}, {0.245, 0.31, 0.44, 0.9}};
+        const double exchange = splits == 1 ? 0.0 : group ? 0.25 + 0.2 * splits : path.tokens <= 64 ? 1.0 + 0.08 * splits : 2.2;
         const double contention = 0.012 * double(std::max<int64_t>(0, std::min(ctas, slots) - 48));
         const double waves = double((ctas + slots - 1) / slots);
         const double one = kBase[group][tile] + per_split * units * kSlope[group][tile] + exchange + contention;
