@@ -112,7 +112,7 @@ gated_quantize(const T *__restrict__ input, unsigned char *__restrict__ out, flo
 template <Type F, class T, int Kind>
 __global__ void __launch_bounds__(kThreads, 3)
 gated_quantize_blocks(const T *__restrict__ input, unsigned char *__restrict__ out, float *__restrict__ scales, int rows, int cols,
-                      int blocks) {
+                      int blocks, bool rehearse) {
     pdl_launch_dependents();
     const int first = (int(blockIdx.x) * int(blockDim.x >> 5) + int(threadIdx.x >> 5)) * 8;
     const int block = first + (int(threadIdx.x & 31) >> 2);
@@ -121,18 +121,28 @@ gated_quantize_blocks(const T *__restrict__ input, unsigned char *__restrict__ o
     const int column = group * 128 + int(threadIdx.x & 3) * 32;
     uint32_t mask[16], raw[16], up[16];
     load_masks(column, mask); // static: may precede the wait
-    pdl_wait_upstream();
-    if (first >= blocks) return;
-    const T *gate = input + size_t(row) * cols * 2 + column;
-    load_row32(gate, raw);
-    load_row32(gate + cols, up);
-#pragma unroll
-    for (int i = 0; i < 16; ++i) {
-        const float2 g = unpack_f32x2(widen2<T>(raw[i]));
-        // The packed multiply rounds the exact product once, as the fp32 product rounded to storage does.
-        raw[i] = mul16x2<T>(Packed16<T>::pack(gate_activation<Kind>(g.x), gate_activation<Kind>(g.y)), up[i]) ^ mask[i];
+    if (first >= blocks) {
+        pdl_wait_upstream();
+        return;
     }
-    rotate_quantize32<F, T>(raw, out + size_t(row) * cols + column, scales + block, active);
+    const T *gate = input + size_t(row) * cols * 2 + column;
+#pragma unroll 1
+    for (int pass = rehearse ? 0 : 1; pass < 2; ++pass) { // as in row_quantize_blocks
+#pragma unroll
+        for (int i = 0; i < 16; ++i) raw[i] = up[i] = 0u;
+        if (pass) {
+            pdl_wait_upstream();
+            load_row32(gate, raw);
+            load_row32(gate + cols, up);
+        }
+#pragma unroll
+        for (int i = 0; i < 16; ++i) {
+            const float2 g = unpack_f32x2(widen2<T>(raw[i]));
+            // The packed multiply rounds the exact product once, as the fp32 product rounded to storage does.
+            raw[i] = mul16x2<T>(Packed16<T>::pack(gate_activation<Kind>(g.x), gate_activation<Kind>(g.y)), up[i]) ^ mask[i];
+        }
+        rotate_quantize32<F, T>(raw, out + size_t(row) * cols + column, scales + block, active && pass);
+    }
 }
 
 template <Type F, class T, int Kind, bool Rotate>
@@ -145,7 +155,7 @@ void launch_items(const T *x, unsigned char *q, float *s, int rows, int cols, in
         const int threads = blocks >= 8 * (kThreads / 32) * sms ? kThreads : 64;
         const int per_cta = 8 * (threads / 32);
         launch_pdl("quantized gated launch", gated_quantize_blocks<F, T, Kind>, dim3(unsigned((blocks + per_cta - 1) / per_cta)),
-                   dim3(unsigned(threads)), 0, stream, x, q, s, rows, cols, blocks);
+                   dim3(unsigned(threads)), 0, stream, x, q, s, rows, cols, blocks, blocks <= 8 * kThreads / 32 * sms);
         return;
     }
     // K-group slabs of a row are independent, so short batches spread them over several CTAs. With

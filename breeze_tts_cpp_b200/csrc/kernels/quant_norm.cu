@@ -149,7 +149,7 @@ rms_quantize(T *__restrict__ x, const T *__restrict__ update, const T *__restric
 template <Type F, class T, bool Add>
 __global__ void __launch_bounds__(kThreads)
 rms_quantize_blocks(T *__restrict__ x, const T *__restrict__ update, const T *__restrict__ weight, const T *__restrict__ update_scale,
-                    unsigned char *__restrict__ out, float *__restrict__ scales, int rows, int cols, float eps, bool gemma) {
+                    unsigned char *__restrict__ out, float *__restrict__ scales, int rows, int cols, float eps, bool gemma, bool rehearse) {
     __shared__ float slots[kThreads / 64][8];
     pdl_launch_dependents();
     const int slot = int(threadIdx.x) / 64, lane = int(threadIdx.x) % 64;
@@ -163,59 +163,65 @@ rms_quantize_blocks(T *__restrict__ x, const T *__restrict__ update, const T *__
 #pragma unroll
         for (int i = 0; i < 16; ++i) mask[i] = w[i] = 0u;
     }
-#pragma unroll
-    for (int i = 0; i < 16; ++i) value[i] = 0u;
-    pdl_wait_upstream();
     T *mine = x + size_t(row) * cols + column;
-    if (active) {
-        load_row32(mine, value);
-        if (Add) {
-            uint32_t u[16];
-            load_row32(update + size_t(row) * cols + column, u);
-            if (update_scale) {
-                uint32_t s[16];
-                load_row32(update_scale + column, s);
+#pragma unroll 1
+    for (int pass = rehearse ? 0 : 1; pass < 2; ++pass) { // as in rms_quantize
+        if (pass) {
+            __syncthreads(); // the rehearsal's sums have been read
+            pdl_wait_upstream();
+        }
 #pragma unroll
-                for (int i = 0; i < 16; ++i) u[i] = mul16x2<T>(u[i], s[i]);
+        for (int i = 0; i < 16; ++i) value[i] = 0u;
+        if (active && pass) {
+            load_row32(mine, value);
+            if (Add) {
+                uint32_t u[16];
+                load_row32(update + size_t(row) * cols + column, u);
+                if (update_scale) {
+                    uint32_t s[16];
+                    load_row32(update_scale + column, s);
+#pragma unroll
+                    for (int i = 0; i < 16; ++i) u[i] = mul16x2<T>(u[i], s[i]);
+                }
+#pragma unroll
+                for (int i = 0; i < 16; ++i) value[i] = add16x2<T>(value[i], u[i]);
+                store_row32(mine, value);
             }
-#pragma unroll
-            for (int i = 0; i < 16; ++i) value[i] = add16x2<T>(value[i], u[i]);
-            store_row32(mine, value);
         }
-    }
-    float sum[4];
+        float sum[4];
 #pragma unroll
-    for (int t = 0; t < 4; ++t) {
-        sum[t] = 0.f;
+        for (int t = 0; t < 4; ++t) {
+            sum[t] = 0.f;
 #pragma unroll
-        for (int p = 0; p < 4; ++p) {
-            const float2 f = unpack_f32x2(widen2<T>(value[4 * t + p]));
-            sum[t] = __fadd_rn(sum[t], __fadd_rn(__fmul_rn(f.x, f.x), __fmul_rn(f.y, f.y)));
+            for (int p = 0; p < 4; ++p) {
+                const float2 f = unpack_f32x2(widen2<T>(value[4 * t + p]));
+                sum[t] = __fadd_rn(sum[t], __fadd_rn(__fmul_rn(f.x, f.x), __fmul_rn(f.y, f.y)));
+            }
         }
-    }
 #pragma unroll
-    for (int d = 4; d; d >>= 1)
+        for (int d = 4; d; d >>= 1)
 #pragma unroll
-        for (int t = 0; t < 4; ++t) sum[t] = __fadd_rn(sum[t], __shfl_down_sync(0xffffffffu, sum[t], d));
-    if (!(lane & 7)) slots[slot][lane >> 3] = __fadd_rn(__fadd_rn(sum[0], sum[2]), __fadd_rn(sum[1], sum[3]));
-    __syncthreads();
-    float total = 0.f;
+            for (int t = 0; t < 4; ++t) sum[t] = __fadd_rn(sum[t], __shfl_down_sync(0xffffffffu, sum[t], d));
+        if (!(lane & 7)) slots[slot][lane >> 3] = __fadd_rn(__fadd_rn(sum[0], sum[2]), __fadd_rn(sum[1], sum[3]));
+        __syncthreads();
+        float total = 0.f;
 #pragma unroll
-    for (int p = 0; p < 8; ++p) total = __fadd_rn(total, slots[slot][p]);
-    const float inv_norm = rsqrtf(__fadd_rn(__fdiv_rn(total, float(cols)), eps));
+        for (int p = 0; p < 8; ++p) total = __fadd_rn(total, slots[slot][p]);
+        const float inv_norm = rsqrtf(__fadd_rn(__fdiv_rn(total, float(cols)), eps));
 #pragma unroll
-    for (int i = 0; i < 16; ++i) {
-        const float2 f = unpack_f32x2(widen2<T>(value[i]));
-        if (gemma) {
-            const float2 wf = unpack_f32x2(widen2<T>(w[i]));
-            value[i] = Packed16<T>::pack(__fmul_rn(__fmul_rn(f.x, inv_norm), __fadd_rn(wf.x, 1.f)),
-                                         __fmul_rn(__fmul_rn(f.y, inv_norm), __fadd_rn(wf.y, 1.f)));
-        } else {
-            value[i] = mul16x2<T>(Packed16<T>::pack(__fmul_rn(f.x, inv_norm), __fmul_rn(f.y, inv_norm)), w[i]);
+        for (int i = 0; i < 16; ++i) {
+            const float2 f = unpack_f32x2(widen2<T>(value[i]));
+            if (gemma) {
+                const float2 wf = unpack_f32x2(widen2<T>(w[i]));
+                value[i] = Packed16<T>::pack(__fmul_rn(__fmul_rn(f.x, inv_norm), __fadd_rn(wf.x, 1.f)),
+                                             __fmul_rn(__fmul_rn(f.y, inv_norm), __fadd_rn(wf.y, 1.f)));
+            } else {
+                value[i] = mul16x2<T>(Packed16<T>::pack(__fmul_rn(f.x, inv_norm), __fmul_rn(f.y, inv_norm)), w[i]);
+            }
+            value[i] ^= mask[i];
         }
-        value[i] ^= mask[i];
+        rotate_quantize32<F, T>(value, out + size_t(row) * cols + column, scales + size_t(column / 128) * rows + row, active && pass);
     }
-    rotate_quantize32<F, T>(value, out + size_t(row) * cols + column, scales + size_t(column / 128) * rows + row, active);
 }
 
 template <Type F, class T>
@@ -233,10 +239,10 @@ void launch(T *x, const T *update, const T *weight, const T *update_scale, unsig
         const dim3 grid(unsigned((rows + per_cta - 1) / per_cta)), block(unsigned(64 * per_cta));
         if (update)
             launch_pdl("quantized norm launch", rms_quantize_blocks<F, T, true>, grid, block, 0, stream, x, update, weight, update_scale, q,
-                       s, rows, cols, eps, gemma);
+                       s, rows, cols, eps, gemma, rows <= sms);
         else
             launch_pdl("quantized norm launch", rms_quantize_blocks<F, T, false>, grid, block, 0, stream, x, update, weight, update_scale,
-                       q, s, rows, cols, eps, gemma);
+                       q, s, rows, cols, eps, gemma, rows <= sms);
         return;
     }
 #define B200Q_RUN(ADD, ROT)                                                                        \

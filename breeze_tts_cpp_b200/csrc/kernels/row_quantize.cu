@@ -156,7 +156,7 @@ row_quantize_warp_rows(const T *__restrict__ x, unsigned char *__restrict__ q, f
 template <Type F, class T>
 __global__ void __launch_bounds__(kThreads, 3)
 row_quantize_blocks(const T *__restrict__ x, unsigned char *__restrict__ q, float *__restrict__ scales, int rows, int cols,
-                    int stride, int blocks) {
+                    int stride, int blocks, bool rehearse) {
     pdl_launch_dependents();
     const int first = (int(blockIdx.x) * int(blockDim.x >> 5) + int(threadIdx.x >> 5)) * 8;
     const int block = first + (int(threadIdx.x & 31) >> 2);
@@ -165,12 +165,23 @@ row_quantize_blocks(const T *__restrict__ x, unsigned char *__restrict__ q, floa
     const int column = group * 128 + int(threadIdx.x & 3) * 32;
     uint32_t mask[16], raw[16];
     load_masks(column, mask); // static: may precede the wait
-    pdl_wait_upstream();
-    if (first >= blocks) return;
-    load_row32(x + size_t(row) * stride + column, raw);
+    if (first >= blocks) {
+        pdl_wait_upstream();
+        return;
+    }
+    // `rehearse` (short lists): once through on the masks before the wait, so that the code is in the instruction caches.
+#pragma unroll 1
+    for (int pass = rehearse ? 0 : 1; pass < 2; ++pass) {
 #pragma unroll
-    for (int i = 0; i < 16; ++i) raw[i] ^= mask[i];
-    rotate_quantize32<F, T>(raw, q + size_t(row) * cols + column, scales + block, active);
+        for (int i = 0; i < 16; ++i) raw[i] = 0u;
+        if (pass) {
+            pdl_wait_upstream();
+            load_row32(x + size_t(row) * stride + column, raw);
+        }
+#pragma unroll
+        for (int i = 0; i < 16; ++i) raw[i] ^= mask[i];
+        rotate_quantize32<F, T>(raw, q + size_t(row) * cols + column, scales + block, active && pass);
+    }
 }
 
 // The same with one lane per block for long lists (lane_blocks_pay): persistent warps over tasks of 32 rows x one K group, neighbouring
@@ -237,7 +248,7 @@ void launch_typed(const T *x, unsigned char *q, float *scales, int rows, int col
         const int threads = blocks >= 8 * (kThreads / 32) * multiprocessors ? kThreads : 64;
         const int per_cta = 8 * (threads / 32);
         launch_pdl("row quantize launch", row_quantize_blocks<F, T>, dim3(unsigned((blocks + per_cta - 1) / per_cta)),
-                   dim3(unsigned(threads)), 0, stream, x, q, scales, rows, cols, stride, blocks);
+                   dim3(unsigned(threads)), 0, stream, x, q, scales, rows, cols, stride, blocks, blocks <= 8 * kThreads / 32 * multiprocessors);
         return;
     }
     int parts = 1;
