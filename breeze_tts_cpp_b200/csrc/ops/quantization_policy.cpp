@@ -39,7 +39,7 @@ std::string path_name(const LinearPath &p) {
 namespace {
 bool grouped(const KernelProblem &p) { return p.input_group || p.weight_group; }
 int blocks(int size, int tile) { return (size + tile - 1) / tile; }
-// Which kernel the launcher picks for a path (mirrors launch_quant_linear's dispatch).
+// Which kernel the launcher picks for a path and plain rows (mirrors launch_quant_linear's dispatch).
 bool persistent_per_row(const KernelProblem &p, const LinearPath &path) {
     return !grouped(p) && path.tokens == kPrefillTokens && path.splits == 1;
 }
