@@ -114,7 +114,9 @@ double linear_cost(KernelProblem p, LinearPath path, Type format, const ChipMode
         const int tile = path.tokens <= 32 ? 0 : path.tokens <= 64 ? 1 : path.tokens <= 128 ? 2 : 3;
         static constexpr double kBase[2][4] = {{2.3, 2.5, 3.4, 6.2}, {2.7, 3.4, 5.6, 9.0}};
         static constexpr double kSlope[2][4] = {{0.17, 0.17, 0.17, 0.42}, {0.245, 0.31, 0.44, 0.9}};
-        const double exchange = splits == 1 ? 0.0 : group ? 0.25 + 0.2 * splits : path.tokens <= 64 ? 1.0 + 0.08 * splits : 2.2;
+        // A second 64-token tile with up to eight rows exchanges next to nothing (67 rows: a decoder layer with QKV split in two 36.4 us, unsplit 37.3).
+        const double exchange64 = p.rows <= kWeightStreamTokens + 8 ? 0.25 + 0.15 * splits : 1.0 + 0.08 * splits;
+        const double exchange = splits == 1 ? 0.0 : group ? 0.25 + 0.2 * splits : path.tokens <= 64 ? exchange64 : 2.2;
         const double contention = 0.012 * double(std::max<int64_t>(0, std::min(ctas, slots) - 48));
         const double waves = double((ctas + slots - 1) / slots);
         const double one = kBase[group][tile] + per_split * units * kSlope[group][tile] + exchange + contention;
