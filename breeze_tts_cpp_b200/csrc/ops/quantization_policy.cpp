@@ -91,10 +91,13 @@ double linear_cost(KernelProblem p, LinearPath path, Type format, const ChipMode
     }
     if (persistent_grouped(p, path)) {
         // Waves of 128 tokens x 64 or 128 channels, bound by the fp32 rescale of every K128 partial tile (0.28 and 0.42 us per
-        // K block, INT8; FP8 is up to 15 % faster).
+        // K block, INT8; FP8 is up to 15 % faster). With a single token tile all CTAs pull the same rows: QKV of 103, 111, 119 and 127 rows on
+        // this kernel 50.1, 50.3, 50.6 and 51.3 us a decoder layer, in two splits of 64 tokens 47.4, 48.3, 48.6 and 49.1 (FP8 48.2,
+        // 48.3, 48.5 and 48.6 against 46.2, 46.4, 47.4 and 48.4); O of 255 rows, as many CTAs on two tiles, FP8 60.6 against 62.1.
         const int channels = grouped_channel_tile(p.rows, p.channels, sms);
         const double tiles = double(blocks(p.channels, channels)) * blocks(p.rows, kGroupedTokens);
-        return (channels == 64 ? 2.9 : 3.2) + std::ceil(tiles / sms) * kb_total * (channels == 64 ? 0.28 : 0.42);
+        const double per_block = channels != 64 ? 0.42 : p.rows > kGroupedTokens ? 0.28 : 0.2875;
+        return (channels == 64 ? 2.9 : 3.2) + std::ceil(tiles / sms) * kb_total * per_block;
     }
     if (p.rows > kWeightStreamTokens) {
         // Weight-streaming kernel with several token tiles per channel slab. Fitted to launches of 65 to 1024 rows on

@@ -124,3 +124,13 @@ def test_decode_plans_match_the_measured_table():
         assert plan(rows, 12288, 2048)[0][3] == 1
         assert plan(rows, 2048, 2048)[0][3] in (3, 4) and plan(rows, 2048, 6144)[0][3] in (4, 5, 6)
         assert plan(rows, 4096, 2048)[0][3] in (2, 3, 4)
+
+
+@pytest.mark.parametrize("fmt", [I8, FP8])
+def test_group_plans_of_one_and_two_token_tiles(fmt):
+    """K groups, K = 2048: a single token tile goes to two splits of 64 tokens where the persistent kernel (128 tokens, unsplit) takes longer
+    in a decoder layer; two token tiles with as many CTAs stay there, and so do shorter and longer K."""
+    for rows in (97, 103, 112, 119, 128):
+        assert plan(rows, 4096, 2048, 128, 128, fmt)[0] == (5, 64, 128, 2)
+    for rows, n, k in ((129, 4096, 2048), (240, 2048, 2048), (256, 2048, 2048), (128, 4096, 1024), (128, 12288, 2048), (448, 2048, 6144), (1024, 512, 2048)):
+        assert plan(rows, n, k, 128, 128, fmt)[0] == (5, 128, 128, 1)
