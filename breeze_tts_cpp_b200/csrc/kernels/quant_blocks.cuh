@@ -401,8 +401,9 @@ template <Type F, class T> __device__ __forceinline__ uint64_t encode_words(uint
     return finite ? encode8<F, true>(v, inverse2) : encode8<F, false>(v, inverse2);
 }
 // Tail of the per-row producers: the CTA holds one row as packed storage values, thread t, item j owning columns
-// (j*Threads + t)*8 .. +7 (zeros past the end); one scale. `slots` holds one word per warp. Equals quantize_tail
-// (quant_codec.cuh) bit for bit with about a third of its instructions.
+// (j*Threads + t)*8 .. +7 (zeros past the end); one scale. `slots` holds one word per warp and is still being
+// read on return: a barrier has to come before it is written again. Equals quantize_tail (quant_codec.cuh)
+// bit for bit with about a third of its instructions.
 template <Type F, class T, int Threads, int Items>
 __device__ __forceinline__ void quantize_row_packed(const uint4 (&v)[Items], unsigned char *out, float *scale, int cols, uint32_t *slots,
                                                     bool store = true) {

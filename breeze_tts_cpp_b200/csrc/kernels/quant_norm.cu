@@ -68,6 +68,7 @@ rms_quantize(T *__restrict__ x, const T *__restrict__ update, const T *__restric
 #pragma unroll 1
     for (int pass = Packed && rehearse ? 0 : 1; pass < 2; ++pass) {
         const bool real = !Packed || pass;
+        if (Packed && rehearse && real) __syncthreads(); // the rehearsal's maxima have been read
         if (real) pdl_wait_upstream();
         uint4 value = make_uint4(0, 0, 0, 0);
         if (real && column < cols) {

@@ -53,3 +53,22 @@ def test_inputs_written_by_the_kernel_before(ctx_factory, mode, rows):
         ctx.quantized_norm(residual, update, gamma, norm_q, 1e-6)  # writes the residual back ...
         ctx.quantized_norm(residual, update, gamma, norm_again, 1e-6)  # ... in front of this one
         assert torch.equal(residual, kept) and torch.equal(norm_q.values, norm_again.values)
+
+
+@pytest.mark.parametrize("mode", ["int8", "fp8"])
+@pytest.mark.parametrize("rows", [1, 5, 64, 148])
+def test_norm_repeats_itself(ctx_factory, mode, rows):
+    """The rehearsal and the pass behind it share memory: a short batch, over and over, against the same rows in a batch too long for one."""
+    from breeze_tts_cpp_b200 import ops
+    ctx, fmt, k = ctx_factory(mode), ops.format_of(mode), 2048
+    g = torch.Generator(device="cuda").manual_seed(rows)
+    draw = lambda *shape: torch.randn(*shape, generator=g, device="cuda").to(torch.bfloat16)
+    x, update, gamma = draw(600, k), draw(600, k), draw(1, k)
+    torch.cuda.synchronize()  # gamma is a parameter
+    whole = ctx.quantized_norm(x.clone(), update, gamma, ops.RowScaledView.empty(600, k, fmt), 1e-6)
+    outs = [ops.RowScaledView.empty(rows, k, fmt) for _ in range(200)]
+    inputs = [x[:rows].clone() for _ in outs]
+    for kept, out in zip(inputs, outs):
+        ctx.quantized_norm(kept, update[:rows], gamma, out, 1e-6)
+    assert torch.equal(torch.stack([o.values for o in outs]), whole.values[:rows].expand(len(outs), -1, -1))
+    assert torch.equal(torch.stack([o.scales for o in outs]), whole.scales[:rows].expand(len(outs), -1, -1))
