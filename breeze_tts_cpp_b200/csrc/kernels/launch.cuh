@@ -4,7 +4,8 @@
 //   * it executes `pdl_launch_dependents()` early, and
 //   * it executes `pdl_wait_upstream()` before its first read of data a previous kernel may have
 //     written and before its first global write. Only parameters that are complete by contract are read
-//     earlier: announced weights with their scales (GEMMs) and RMSNorm weights.
+//     earlier: announced weights with their scales (GEMMs) and RMSNorm weights. A kernel whose inputs are pointers to const
+//     __restrict__ reads them by load_upstream16 and its kin (quant_codec.cuh): the compiler may move a plain load in front of the wait.
 // Because every kernel waits for its predecessor to finish before it finishes itself, ordering
 // stays transitive along the whole chain. Outside such a launch both instructions do nothing.
 #pragma once

@@ -78,13 +78,6 @@ __device__ __forceinline__ Words8 load_words8(const void *p) {
 __device__ __forceinline__ void store_words8(void *p, const Words8 &v) {
     asm volatile("st.global.v4.b64 [%0], {%1, %2, %3, %4};" ::"l"(p), "l"(v.w[0]), "l"(v.w[1]), "l"(v.w[2]), "l"(v.w[3]) : "memory");
 }
-// 16 bytes of what an upstream kernel wrote. The compiler may take a plain load through a pointer to const __restrict__ out of a loop,
-// wait on upstream or not; this one stays behind the wait.
-__device__ __forceinline__ uint4 load_upstream16(const void *p) {
-    uint4 r;
-    asm volatile("ld.global.v4.b32 {%0, %1, %2, %3}, [%4];" : "=r"(r.x), "=r"(r.y), "=r"(r.z), "=r"(r.w) : "l"(p) : "memory");
-    return r;
-}
 // 32 consecutive 16-bit elements (64 bytes, 32-byte aligned) as 16 packed words.
 __device__ __forceinline__ void load_row32(const void *p, uint32_t (&raw)[16]) {
 #pragma unroll

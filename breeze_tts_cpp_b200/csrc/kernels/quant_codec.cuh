@@ -56,17 +56,33 @@ __device__ __forceinline__ float rotation_sign(uint32_t column) {
     return ((h ^ (h >> 16)) & 1u) ? 1.f : -1.f;
 }
 
-// Eight consecutive 16-bit elements -> fp32. `aligned` selects one 128-bit load; otherwise (odd
+// 16 bytes, or one 16-bit element, of what an upstream kernel wrote. The compiler may take a plain load through a pointer to const
+// __restrict__ out of a loop, wait on upstream or not; these stay behind the wait.
+__device__ __forceinline__ uint4 load_upstream16(const void *p) {
+    uint4 r;
+    asm volatile("ld.global.v4.b32 {%0, %1, %2, %3}, [%4];" : "=r"(r.x), "=r"(r.y), "=r"(r.z), "=r"(r.w) : "l"(p) : "memory");
+    return r;
+}
+template <class T> __device__ __forceinline__ T load_upstream(const T *p) {
+    static_assert(sizeof(T) == 2);
+    union {
+        unsigned short bits;
+        T value;
+    } r{};
+    asm volatile("ld.global.b16 %0, [%1];" : "=h"(r.bits) : "l"(p) : "memory");
+    return r.value;
+}
+// Eight consecutive 16-bit elements of an upstream kernel -> fp32. `aligned` selects one 128-bit load; otherwise (odd
 // pointers, ragged row ends) elements are fetched one by one and missing ones read as zero.
 template <class T> __device__ __forceinline__ void load8(const T *p, int remaining, bool aligned, float (&v)[8]) {
     if (aligned && remaining >= 8) {
-        uint4 raw = *reinterpret_cast<const uint4 *>(p);
+        uint4 raw = load_upstream16(p);
         const T *e = reinterpret_cast<const T *>(&raw);
 #pragma unroll
         for (int i = 0; i < 8; ++i) v[i] = float(e[i]);
     } else {
 #pragma unroll
-        for (int i = 0; i < 8; ++i) v[i] = i < remaining ? float(p[i]) : 0.f;
+        for (int i = 0; i < 8; ++i) v[i] = i < remaining ? float(load_upstream(p + i)) : 0.f;
     }
 }
 

@@ -34,7 +34,7 @@ template <class T> __device__ __forceinline__ uint4 load_raw8(const T *p, int re
     if (aligned && remaining >= 8) return load_upstream16(p);
     T *e = reinterpret_cast<T *>(&raw);
     for (int i = 0; i < 8; ++i)
-        if (i < remaining) e[i] = p[i];
+        if (i < remaining) e[i] = load_upstream(p + i);
     return raw;
 }
 template <class T> __device__ __forceinline__ void store_raw8(T *p, uint4 raw, int remaining, bool aligned) {

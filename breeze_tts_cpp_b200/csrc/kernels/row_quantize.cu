@@ -52,7 +52,7 @@ row_quantize_cached(const T *__restrict__ x, unsigned char *__restrict__ q, floa
 #pragma unroll
         for (int j = 0; j < Items; ++j) {
             int column = ((j * parts + shard) * kThreads + int(threadIdx.x)) * 8;
-            raw[j] = column < cols ? *reinterpret_cast<const uint4 *>(source + column) : make_uint4(0, 0, 0, 0);
+            raw[j] = column < cols ? load_upstream16(source + column) : make_uint4(0, 0, 0, 0);
         }
 #pragma unroll
         for (int j = 0; j < Items; ++j) unpack8<T>(raw[j], v[j]);
@@ -122,7 +122,7 @@ row_quantize_warp_rows(const T *__restrict__ x, unsigned char *__restrict__ q, f
 #pragma unroll
     for (int j = 0; j < Loads; ++j) {
         const int column = (j * 32 + lane) * 8;
-        raw[j] = column < cols ? *reinterpret_cast<const uint4 *>(source + column) : make_uint4(0, 0, 0, 0);
+        raw[j] = column < cols ? load_upstream16(source + column) : make_uint4(0, 0, 0, 0);
     }
     uint32_t largest = 0u;
 #pragma unroll

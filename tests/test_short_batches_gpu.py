@@ -21,38 +21,47 @@ def test_gate_by_row_count(ctx_factory, mode, cols, rows):
         assert torch.equal(one.values[0], whole.values[row]) and float(one.scales[0]) == float(whole.scales[row])
 
 
-@pytest.mark.parametrize("mode", ["int8", "fp8"])
+@pytest.mark.parametrize("mode", ["int8", "fp8", "group_int8", "group_fp8"])
 @pytest.mark.parametrize("rows", [3, 64, 148])
-def test_inputs_written_by_the_kernel_before(ctx_factory, mode, rows):
+@pytest.mark.parametrize("aligned", [True, False])
+def test_inputs_written_by_the_kernel_before(ctx_factory, mode, rows, aligned):
+    """Stale values are settled in a producer's input, then the GEMM that writes it and the producer are queued behind a long kernel, so that the
+    producer starts while the GEMM runs. Unaligned rows take the producers' general forms."""
     from breeze_tts_cpp_b200 import ops
-    ctx = ctx_factory(mode)
-    fmt, k, n = ops.format_of(mode), 2048, 4096
+    ctx, k, n = ctx_factory(mode), 2048, 4096
+    fmt, (group, _, rotation) = ops.format_of(mode), ops.groups_of(mode)
     g = torch.Generator(device="cuda").manual_seed(rows)
     draw = lambda *shape: torch.randn(*shape, generator=g, device="cuda").to(torch.bfloat16)
-    w = ctx.quantize_rows(draw(n, k), ops.RowScaledView.empty(n, k, fmt))
-    ctx.prepare_quantized(rows, n, k, weight=w)
-    gamma, update = draw(1, k), torch.zeros(rows, k, dtype=torch.bfloat16, device="cuda")
-    torch.cuda.synchronize()
-    y = torch.empty(rows, n, dtype=torch.bfloat16, device="cuda")
-    q = lambda c: ops.RowScaledView.empty(rows, c, fmt)
-    for _ in range(8):
-        x = ctx.quantize_rows(draw(rows, k), q(k))
-        y.fill_(7.0)
-        torch.cuda.synchronize()
-        ctx.matmul(x, w, y)
-        rows_q, gate_q = q(n), q(n // 2)
-        ctx.quantize_rows(y, rows_q)
-        ctx.matmul(x, w, y)
-        ctx.quantized_gated(y, gate_q)
-        torch.cuda.synchronize()
-        again = ctx.quantize_rows(y, q(n)), ctx.quantized_gated(y, q(n // 2))
-        for one, two in zip((rows_q, gate_q), again):
-            assert torch.equal(one.values, two.values) and torch.equal(one.scales, two.scales)
-        residual = draw(rows, n)[:, :k].contiguous()
-        norm_q, norm_again, kept = q(k), q(k), residual.clone()
-        ctx.quantized_norm(residual, update, gamma, norm_q, 1e-6)  # writes the residual back ...
-        ctx.quantized_norm(residual, update, gamma, norm_again, 1e-6)  # ... in front of this one
-        assert torch.equal(residual, kept) and torch.equal(norm_q.values, norm_again.values)
+    q = lambda r, c: ops.RowScaledView.empty(r, c, fmt, group, rotation)
+    place = lambda c: torch.empty(rows * c + 1, dtype=torch.bfloat16, device="cuda")[0 if aligned else 1:][:rows * c].view(rows, c)
+    wide, square = (ctx.quantize_rows(draw(c, k), q(c, k)) for c in (n, k))
+    for w, c in ((wide, n), (square, k)):
+        ctx.prepare_quantized(rows, c, k, weight=w)
+    gamma, beta, residual, busy = draw(1, k), draw(1, k), draw(rows, k), draw(4096, 4096)
+    producers = [  # weight of the GEMM in front, its output's columns, the producer on that output -> tensors
+        (wide, n, lambda y: ctx.quantize_rows(y, q(rows, n))),
+        (wide, n, lambda y: ctx.quantized_gated(y, q(rows, n // 2))),
+        (square, k, lambda y: ctx.quantized_norm(kept[-1], y, gamma, q(rows, k), 1e-6)),
+        (square, k, lambda y: ctx.quantized_norm(y, residual, gamma, q(rows, k), 1e-6)),
+        (square, k, lambda y: ctx.layer_norm_quantize(y, q(rows, k), gamma, beta)),
+        (square, k, lambda y: ctx.layer_norm_quantize(residual, q(rows, k), gamma, beta, residual=y)),
+    ]
+    x = ctx.quantize_rows(draw(rows, k), q(rows, k))
+    for w, columns, produce in producers:
+        y, kept, got = place(columns), [], []
+        for settled in (False, True, False, False):
+            y.fill_(7.0)
+            kept.append(residual.clone())
+            torch.cuda.synchronize()
+            torch.mm(busy, busy)
+            ctx.matmul(x, w, y)
+            if settled:
+                torch.cuda.synchronize()
+            out = produce(y)
+            torch.cuda.synchronize()
+            got.append((out.values, out.scales, y.clone(), kept[-1]))
+        for other in got:
+            assert all(torch.equal(a, b) for a, b in zip(other, got[1]))
 
 
 @pytest.mark.parametrize("mode", ["int8", "fp8"])
