@@ -38,7 +38,7 @@ gated_quantize(const T *__restrict__ input, unsigned char *__restrict__ out, flo
     constexpr int kThreads = Threads; // shadows the file-wide default inside this kernel
     __shared__ float slots[kThreads / 32];
     pdl_launch_dependents();
-    // `rehearse` (short batches): once through on zeros before the wait, so that the code is in the instruction caches (rms_quantize).
+    // `rehearse` (kRehearsedRows): once through on zeros before the wait, without a global access.
 #pragma unroll 1
     for (int pass = Packed && rehearse ? 0 : 1; pass < 2; ++pass) {
         const bool real = !Packed || pass;
@@ -155,7 +155,7 @@ void launch_items(const T *x, unsigned char *q, float *s, int rows, int cols, in
         const int threads = blocks >= 8 * (kThreads / 32) * sms ? kThreads : 64;
         const int per_cta = 8 * (threads / 32);
         launch_pdl("quantized gated launch", gated_quantize_blocks<F, T, Kind>, dim3(unsigned((blocks + per_cta - 1) / per_cta)),
-                   dim3(unsigned(threads)), 0, stream, x, q, s, rows, cols, blocks, blocks <= 8 * kThreads / 32 * sms);
+                   dim3(unsigned(threads)), 0, stream, x, q, s, rows, cols, blocks, rows <= kRehearsedRows);
         return;
     }
     // K-group slabs of a row are independent, so short batches spread them over several CTAs. With
@@ -169,7 +169,7 @@ void launch_items(const T *x, unsigned char *q, float *s, int rows, int cols, in
     // as two such CTAs per multiprocessor hold the batch (200 rows: 3.4 -> 2.7 us), two groups on one half as wide up to five (301
     // rows 4.5 -> 3.9, 700 5.3 -> 4.9); beyond that 256 threads (1021 rows: 6.2 against 6.5 and 8.3).
     if (!group && aligned && chunks > 1 && chunks <= 4 && rows <= 5 * sms) {
-        const bool wide = rows <= 2 * sms, rehearse = rows <= sms;
+        const bool wide = rows <= 2 * sms, rehearse = rows <= kRehearsedRows;
         const int threads = chunks * (wide ? kThreads : kThreads / 2);
 #define B200Q_WIDE(N, I)                                                                                                   \
     launch_pdl("quantized gated launch", !Rotate ? gated_quantize<F, T, Kind, I, false, true, N> : gated_quantize<F, T, Kind, I, Rotate, false, N>, dim3(unsigned(rows)), dim3(N), 0, stream, x, \

@@ -62,9 +62,7 @@ rms_quantize(T *__restrict__ x, const T *__restrict__ update, const T *__restric
     const int row = blockIdx.x, column = threadIdx.x * 8;
     uint4 w = make_uint4(0, 0, 0, 0);
     if (column < cols) w = load_raw8(weight + column, cols - column, aligned); // a parameter: may precede the wait
-    // `rehearse` (short batches): once through on zeros before the wait, without a global access. A launch finds the instruction caches cold,
-    // and fetching the code while there is nothing else to do takes that off the chain's critical path (with the other two
-    // quantizers, 28 layers: 64 rows INT8 813 -> 809 us, 5 rows FP8 671 -> 661).
+    // `rehearse` (kRehearsedRows): once through on zeros before the wait, without a global access.
 #pragma unroll 1
     for (int pass = Packed && rehearse ? 0 : 1; pass < 2; ++pass) {
         const bool real = !Packed || pass;
@@ -240,15 +238,15 @@ void launch(T *x, const T *update, const T *weight, const T *update_scale, unsig
         const dim3 grid(unsigned((rows + per_cta - 1) / per_cta)), block(unsigned(64 * per_cta));
         if (update)
             launch_pdl("quantized norm launch", rms_quantize_blocks<F, T, true>, grid, block, 0, stream, x, update, weight, update_scale, q,
-                       s, rows, cols, eps, gemma, rows <= sms);
+                       s, rows, cols, eps, gemma, rows <= kRehearsedRows);
         else
             launch_pdl("quantized norm launch", rms_quantize_blocks<F, T, false>, grid, block, 0, stream, x, update, weight, update_scale,
-                       q, s, rows, cols, eps, gemma, rows <= sms);
+                       q, s, rows, cols, eps, gemma, rows <= kRehearsedRows);
         return;
     }
 #define B200Q_RUN(ADD, ROT)                                                                        \
     launch_pdl("quantized norm launch", aligned && !group && !ROT ? rms_quantize<F, T, ADD, false, true> : rms_quantize<F, T, ADD, ROT, false>, dim3(rows), dim3(kThreads), 0, stream, x, update,   \
-               weight, update_scale, q, s, rows, cols, eps, gemma, group, aligned, rows <= sms)
+               weight, update_scale, q, s, rows, cols, eps, gemma, group, aligned, rows <= kRehearsedRows)
     if (update) { if (rotation) B200Q_RUN(true, true); else B200Q_RUN(true, false); }
     else { if (rotation) B200Q_RUN(false, true); else B200Q_RUN(false, false); }
 #undef B200Q_RUN

@@ -169,7 +169,7 @@ row_quantize_blocks(const T *__restrict__ x, unsigned char *__restrict__ q, floa
         pdl_wait_upstream();
         return;
     }
-    // `rehearse` (short lists): once through on the masks before the wait, so that the code is in the instruction caches.
+    // `rehearse` (kRehearsedRows): once through on the masks before the wait, without a global access.
 #pragma unroll 1
     for (int pass = rehearse ? 0 : 1; pass < 2; ++pass) {
 #pragma unroll
@@ -248,7 +248,7 @@ void launch_typed(const T *x, unsigned char *q, float *scales, int rows, int col
         const int threads = blocks >= 8 * (kThreads / 32) * multiprocessors ? kThreads : 64;
         const int per_cta = 8 * (threads / 32);
         launch_pdl("row quantize launch", row_quantize_blocks<F, T>, dim3(unsigned((blocks + per_cta - 1) / per_cta)),
-                   dim3(unsigned(threads)), 0, stream, x, q, scales, rows, cols, stride, blocks, blocks <= 8 * kThreads / 32 * multiprocessors);
+                   dim3(unsigned(threads)), 0, stream, x, q, scales, rows, cols, stride, blocks, rows <= kRehearsedRows);
         return;
     }
     int parts = 1;
@@ -267,7 +267,7 @@ void launch_typed(const T *x, unsigned char *q, float *scales, int rows, int col
 #define B200Q_LAUNCH(I)                                                                            \
     launch_pdl("row quantize launch", aligned && !group && !Rotate ? row_quantize_cached<F, T, I, false, true>                   \
                                                                     : row_quantize_cached<F, T, I, Rotate, false>, dim3(grid), dim3(kThreads), 0, stream, x, q, \
-               scales, rows, cols, stride, group, parts, aligned, rows <= multiprocessors)
+               scales, rows, cols, stride, group, parts, aligned, rows <= kRehearsedRows)
     switch (items) {
     case 1: B200Q_LAUNCH(1); break;
     case 2: B200Q_LAUNCH(2); break;

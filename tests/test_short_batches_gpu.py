@@ -22,7 +22,7 @@ def test_gate_by_row_count(ctx_factory, mode, cols, rows):
 
 
 @pytest.mark.parametrize("mode", ["int8", "fp8", "group_int8", "group_fp8"])
-@pytest.mark.parametrize("rows", [3, 64, 148])
+@pytest.mark.parametrize("rows", [3, 64, 65, 148])
 @pytest.mark.parametrize("aligned", [True, False])
 def test_inputs_written_by_the_kernel_before(ctx_factory, mode, rows, aligned):
     """Stale values are settled in a producer's input, then the GEMM that writes it and the producer are queued behind a long kernel, so that the
@@ -65,7 +65,7 @@ def test_inputs_written_by_the_kernel_before(ctx_factory, mode, rows, aligned):
 
 
 @pytest.mark.parametrize("mode", ["int8", "fp8"])
-@pytest.mark.parametrize("rows", [1, 5, 64, 148])
+@pytest.mark.parametrize("rows", [1, 5, 64, 65, 148])
 def test_norm_repeats_itself(ctx_factory, mode, rows):
     """The rehearsal and the pass behind it share memory: a short batch, over and over, against the same rows in a batch too long for one."""
     from breeze_tts_cpp_b200 import ops
