@@ -117,10 +117,16 @@ double linear_cost(KernelProblem p, LinearPath path, Type format, const ChipMode
         const int tile = path.tokens <= 32 ? 0 : path.tokens <= 64 ? 1 : path.tokens <= 128 ? 2 : 3;
         static constexpr double kBase[2][4] = {{2.3, 2.5, 3.4, 6.2}, {2.7, 3.4, 5.6, 9.0}};
         static constexpr double kSlope[2][4] = {{0.17, 0.17, 0.17, 0.42}, {0.245, 0.31, 0.44, 0.9}};
-        // A second 64-token tile with up to eight rows exchanges next to nothing (67 rows: a decoder layer with QKV split in two 36.4 us, unsplit 37.3).
-        const double exchange64 = p.rows <= kWeightStreamTokens + 8 ? 0.25 + 0.15 * splits : 1.0 + 0.08 * splits;
-        const double exchange = splits == 1 ? 0.0 : group ? 0.25 + 0.2 * splits : path.tokens <= 64 ? exchange64 : 2.2;
-        const double contention = 0.012 * double(std::max<int64_t>(0, std::min(ctas, slots) - 48));
+        // Up to two token tiles with per-row scales a split costs more by its number of CTAs (those that are no power of two are placed later) and
+        // the grid's size less. Decoder layers of 87, 103, 119 and 127 rows (INT8) with QKV unsplit / in two splits of 64 tokens: 36.5 / 36.7,
+        // 38.0 / 37.9, 38.2 / 38.8 and 38.4 / 39.0 us called one by one, 33.7 / 33.3, 34.4 / 34.3, 35.8 / 35.2 and 36.1 / 35.3 in a graph.
+        // K = 2048 -> 512 in six splits / four: blocks of 87 and 103 rows in a graph 18.1 / 17.1 and 18.5 / 16.9.
+        const bool short_batch = !group && p.rows <= 2 * kWeightStreamTokens && path.tokens <= 64;
+        const double exchange = splits == 1 ? 0.0
+                                : group     ? 0.25 + 0.2 * splits
+                                : short_batch ? 0.3 + 0.24 * splits + (splits & (splits - 1) ? 0.15 : 0.0)
+                                              : path.tokens <= 64 ? 1.0 + 0.08 * splits : 2.2;
+        const double contention = (short_batch ? 0.006 : 0.012) * double(std::max<int64_t>(0, std::min(ctas, slots) - 48));
         const double waves = double((ctas + slots - 1) / slots);
         const double one = kBase[group][tile] + per_split * units * kSlope[group][tile] + exchange + contention;
         return one + (waves - 1.0) * (one - 1.0);

@@ -134,3 +134,17 @@ def test_group_plans_of_one_and_two_token_tiles(fmt):
         assert plan(rows, 4096, 2048, 128, 128, fmt)[0] == (5, 64, 128, 2)
     for rows, n, k in ((129, 4096, 2048), (240, 2048, 2048), (256, 2048, 2048), (128, 4096, 1024), (128, 12288, 2048), (448, 2048, 6144), (1024, 512, 2048)):
         assert plan(rows, n, k, 128, 128, fmt)[0] == (5, 128, 128, 1)
+
+
+@pytest.mark.parametrize("fmt", [I8, FP8])
+def test_row_plans_of_two_token_tiles(fmt):
+    """One scale per row, 65 to 128 rows: one rule for the whole range (QKV in two splits, unsplit from the third token tile on), and clusters
+    of a power of two."""
+    for rows in (65, 72, 73, 80, 96, 104, 112, 128):
+        assert plan(rows, 4096, 2048, 0, 0, fmt)[0] == (5, 64, 128, 2)
+        assert plan(rows, 2048, 2048, 0, 0, fmt)[0] == (5, 64, 128, 2)
+        assert plan(rows, 2048, 6144, 0, 0, fmt)[0] == (5, 64, 128, 4)
+        assert plan(rows, 512, 2048, 0, 0, fmt)[0] == (5, 64, 128, 4)
+        assert plan(rows, 256, 1024, 0, 0, fmt)[0] == (5, 64, 128, 1)
+    for rows in (129, 160, 256):
+        assert plan(rows, 4096, 2048, 0, 0, fmt)[0] == (5, 64, 128, 1)
