@@ -28,6 +28,15 @@ __device__ __forceinline__ void pdl_wait_upstream() {
 // 44.6, 48.3 and 58.6 against 43.8, 47.0 and 57.3; from 149 rows on no difference.
 constexpr int kRehearsedRows = 64;
 
+// Whether launches on `stream` are being recorded into a graph: they cost no host time then and follow one another without gaps.
+inline bool being_captured(cudaStream_t stream) {
+    if (!stream || stream == cudaStreamLegacy) return false; // never captured
+    cudaStreamCaptureStatus status = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(stream, &status) == cudaSuccess) return status != cudaStreamCaptureStatusNone;
+    (void)cudaGetLastError(); // the launch itself will say so
+    return false;
+}
+
 template <class... Params, class... Args>
 void launch_pdl(const char *what, void (*kernel)(Params...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream,
                 Args... args) {

@@ -2,6 +2,7 @@
 // launch. Drop-in for the reference launchers `launch_quant_linear` and `grouped_quant_gemm`
 // (src/ops/kernels/quant/quant_dispatch.cu:194-234, quant_grouped.cu:221-239).
 #include "kernels/quant_dispatch.h"
+#include "kernels/launch.cuh"
 #include "kernels/quant_linear_dense.h"
 #include "kernels/quant_linear_sm100.cuh"
 #include "kernels/quant_prefill_pair_sm100.cuh"
@@ -479,7 +480,8 @@ bool launch_dense_linear(LinearPath config, KernelProblem shape, int rotation, T
         (grouped ? shape.input_group != kBlockK || shape.weight_group != kBlockK || rotation != kBlockK : rotation != 0))
         return false;
     const int per_split = (kb_total + config.splits - 1) / config.splits;
-    if (!dense_pays(shape.rows, shape.reduction, per_split, grouped)) return false;
+    if (!dense_pays(shape.rows, shape.reduction, per_split, grouped) || (!dense_pays_captured(shape.rows, grouped) && being_captured(stream)))
+        return false;
     const DenseShape launch = dense_launch_shape(config.tokens, grouped, per_split, config.splits);
     if (!launch.fits) return false;
     DenseArgs args{};

@@ -124,4 +124,8 @@ inline bool dense_pays(int rows, int reduction, int kb_per_split, bool grouped) 
     while (spread < rows) spread *= 2;
     return spread <= 8 && int64_t(spread) * reduction <= 16384 && rows * kb_per_split <= 48;
 }
+// In a graph, where the quantizer's launch costs no host time. A decoder layer's four projections, captured, a projection in two launches
+// against one: INT8 5.3 -> 5.7 us at one row, 5.5 -> 6.0 at eight (1024 -> 1024 alone 4.1 -> 4.8); K groups FP8 6.0 -> 5.7 at one row, 6.1 ->
+// 5.9 at three, but 6.2 -> 6.7 at five, where the widest projection takes two launches whatever the rule.
+inline bool dense_pays_captured(int rows, bool grouped) { return grouped && rows <= 4; }
 } // namespace tts::b200

@@ -180,8 +180,8 @@ void b200q_linear_layer_destroy(b200q_linear_layer *);
  * max_rows, and the layer's activation scratch (QuantizationWorkspace) sized for max_rows. */
 int b200q_linear_layer_prepare(b200q_context *, b200q_linear_layer *, int32_t max_rows, char *error, size_t error_capacity);
 /* reference: Linear::forward(workspace, input, output, epilogue, quantized_output)
- * (src/layers/linear.h:66-68). quantized_output may be NULL. A few rows (about eight) are quantized inside the GEMM's launch, with the
- * same bytes and sums; the layer's scratch is then not written. */
+ * (src/layers/linear.h:66-68). quantized_output may be NULL. A few rows (about eight; in a graph capture K groups and four) are quantized
+ * inside the GEMM's launch, with the same bytes and sums; the layer's scratch is then not written. */
 int b200q_linear_layer_forward(b200q_context *, b200q_linear_layer *, const b200q_tensor *input, const b200q_tensor *output,
                                const b200q_epilogue *epilogue, const b200q_row_scaled *quantized_output, char *error,
                                size_t error_capacity);

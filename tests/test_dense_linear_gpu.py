@@ -80,3 +80,47 @@ def test_output_over_its_input(ctx_factory, mode):
     for _ in range(5):
         x = draw(4, 512)
         compare(x, out=x)
+
+
+def _kernels(run):
+    """Names of the library's kernels that `run` launches."""
+    from torch.profiler import ProfilerActivity, profile
+    torch.cuda.synchronize()
+    with profile(activities=[ProfilerActivity.CUDA]) as trace:
+        run()
+        torch.cuda.synchronize()
+    names = (e.name for e in trace.events())
+    return ["gemm" if "w8a8_tcgen05_gemm" in n else "quantize" for n in names if "w8a8_tcgen05" in n or "row_quantize" in n]
+
+
+@pytest.mark.parametrize("mode,rows,k,n,one", [
+    ("int8", 1, 2048, 2048, True), ("int8", 8, 2048, 2048, True), ("int8", 9, 2048, 2048, False), ("fp8", 2, 6144, 2048, True),
+    ("fp8", 4, 6144, 2048, False), ("int8", 3, 2048, 12288, True), ("int8", 4, 2048, 12288, False), ("int8", 1, 144, 64, False),
+    ("group_int8", 1, 2048, 4096, True), ("group_int8", 8, 6144, 2048, True), ("group_fp8", 21, 384, 512, True), ("group_fp8", 33, 384, 512, False)])
+def test_which_calls_are_one_launch(ctx_factory, mode, rows, k, n, one):
+    from breeze_tts_cpp_b200 import ops
+    ctx = ctx_factory(mode)
+    layer = ops.Linear(ctx, [torch.randn(n, k, device="cuda").to(torch.bfloat16)], max_rows=rows)
+    x, out = torch.randn(rows, k, device="cuda").to(torch.bfloat16), torch.empty(rows, n, dtype=torch.bfloat16, device="cuda")
+    layer.forward(x, out)
+    assert _kernels(lambda: layer.forward(x, out)) == (["gemm"] if one else ["quantize", "gemm"])
+
+
+@pytest.mark.parametrize("mode,rows,one", [("int8", 1, False), ("int8", 3, False), ("group_fp8", 4, True), ("group_fp8", 5, False)])
+def test_captured_calls(mode, rows, one):
+    from breeze_tts_cpp_b200 import ops
+    stream = torch.cuda.Stream()
+    with torch.cuda.stream(stream):
+        ctx = ops.Context(mode, stream=stream)
+        layer = ops.Linear(ctx, [torch.randn(512, 1024, device="cuda").to(torch.bfloat16)], max_rows=rows)
+        x, eager, replayed = torch.randn(rows, 1024, device="cuda").to(torch.bfloat16), *(torch.zeros(rows, 512, dtype=torch.bfloat16, device="cuda") for _ in range(2))
+        layer.forward(x, eager)
+        stream.synchronize()
+        graph = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(graph, stream=stream):
+            layer.forward(x, replayed)
+        assert _kernels(graph.replay) == (["gemm"] if one else ["quantize", "gemm"])
+    torch.cuda.synchronize()
+    assert torch.equal(eager.view(torch.int16), replayed.view(torch.int16))
+    del graph
+    ctx.close()
