@@ -475,7 +475,7 @@ bool launch_dense_linear(LinearPath config, KernelProblem shape, int rotation, T
     const bool grouped = shape.input_group || shape.weight_group;
     const int kb_total = shape.reduction / kBlockK;
     // Whole K blocks, K groups of 128 with their rotation or neither, rows that can be read in 16 (groups: 32) byte pieces.
-    if (config.kind != LinearKind::Tcgen05 || config.tokens > kDenseTokens || shape.rows > config.tokens || shape.reduction % kBlockK ||
+    if (config.kind != LinearKind::Tcgen05 || config.tokens > dense_tokens(grouped) || shape.rows > config.tokens || shape.reduction % kBlockK ||
         (x.type != Type::BF16 && x.type != Type::F16) || x.ld() % (grouped ? 16 : 8) || reinterpret_cast<uintptr_t>(x.data) % (grouped ? 32 : 16) ||
         (grouped ? shape.input_group != kBlockK || shape.weight_group != kBlockK || rotation != kBlockK : rotation != 0))
         return false;

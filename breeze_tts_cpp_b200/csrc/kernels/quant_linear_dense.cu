@@ -15,10 +15,10 @@ template <class Pick> auto by_instance(Type format, bool grouped, int tokens, Ty
         constexpr int BN = decltype(bn)::value;
         return input == Type::F16 ? pick(instance<F, G, BN, __half>()) : pick(instance<F, G, BN, __nv_bfloat16>());
     };
-    const auto tiled = [&](auto f, auto g) {
-        return tokens == 16 ? typed(f, g, std::integral_constant<int, 16>{}) : typed(f, g, std::integral_constant<int, 32>{});
+    const auto of = [&](auto f) { // 32 tokens for K groups only
+        if (!grouped) return typed(f, std::false_type{}, std::integral_constant<int, 16>{});
+        return tokens == 16 ? typed(f, std::true_type{}, std::integral_constant<int, 16>{}) : typed(f, std::true_type{}, std::integral_constant<int, 32>{});
     };
-    const auto of = [&](auto f) { return grouped ? tiled(f, std::true_type{}) : tiled(f, std::false_type{}); };
     return format == Type::I8 ? of(std::integral_constant<Type, Type::I8>{}) : of(std::integral_constant<Type, Type::FP8>{});
 }
 } // namespace
@@ -26,7 +26,7 @@ template <class Pick> auto by_instance(Type format, bool grouped, int tokens, Ty
 void raise_dense_limits() {
     for (Type format : {Type::I8, Type::FP8})
         for (bool grouped : {false, true})
-            for (int tokens : {16, 32})
+            for (int tokens : {dense_tokens(false), dense_tokens(grouped)})
                 for (Type input : {Type::BF16, Type::F16})
                     by_instance(format, grouped, tokens, input, [](auto *kernel) {
                         check(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(kSmemBudget)), "cudaFuncSetAttribute(shared memory)");

@@ -92,7 +92,7 @@ inline LaunchShape launch_shape(int bn, bool grouped, int kb_per_split, int spli
     return shape;
 }
 // The same kernel when it quantizes 16-bit activations itself: the ring holds weights only, every K block's token tile stays.
-constexpr int kDenseTokens = 32;
+constexpr int dense_tokens(bool grouped) { return grouped ? 32 : 16; } // widest tile; dense_pays takes at most eight rows with one scale per row
 struct DenseShape : LaunchShape {
     int token_offset = 0, largest_offset = 0;
 };
