@@ -81,3 +81,19 @@ def test_norm_repeats_itself(ctx_factory, mode, rows):
         ctx.quantized_norm(kept, update[:rows], gamma, out, 1e-6)
     assert torch.equal(torch.stack([o.values for o in outs]), whole.values[:rows].expand(len(outs), -1, -1))
     assert torch.equal(torch.stack([o.scales for o in outs]), whole.scales[:rows].expand(len(outs), -1, -1))
+
+
+@pytest.mark.parametrize("mode", ["int8", "group_fp8"])
+@pytest.mark.parametrize("cols,rows", [(256, 1), (512, 1184), (512, 1185), (768, 148), (768, 149), (2048, 148), (2048, 149)])
+def test_layer_norm_by_row_count(ctx_factory, mode, cols, rows):
+    """On both sides of the rehearsal's limits, the rows of a batch too long for one."""
+    from breeze_tts_cpp_b200 import ops
+    ctx, fmt, (group, _, rotation) = ctx_factory(mode), ops.format_of(mode), ops.groups_of(mode)
+    g = torch.Generator(device="cuda").manual_seed(rows + cols)
+    draw = lambda *shape: torch.randn(*shape, generator=g, device="cuda").to(torch.bfloat16)
+    x, residual, gamma, beta = draw(1300, cols), draw(1300, cols), draw(1, cols), draw(1, cols)
+    whole = ctx.layer_norm_quantize(x, ops.RowScaledView.empty(1300, cols, fmt, group, rotation), gamma, beta, residual=residual)
+    for _ in range(20):
+        part = ctx.layer_norm_quantize(x[:rows], ops.RowScaledView.empty(rows, cols, fmt, group, rotation), gamma, beta, residual=residual[:rows])
+        assert torch.equal(part.values, whole.values[:rows])
+        assert torch.equal(part.scales, whole.scales[:, :rows] if group else whole.scales[:rows])
