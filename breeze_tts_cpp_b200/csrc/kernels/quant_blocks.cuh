@@ -1,5 +1,5 @@
-// Rotation + quantization of 128-column K blocks with FOUR lanes per block, 32 consecutive columns per lane: what the
-// K-group modes (group 128, H128 rotation) run on every activation and weight.
+// Rotation + quantization of 128-column K blocks: what the K-group modes (group 128, H128 rotation) run on every activation and weight.
+// FOUR lanes per block, 32 consecutive columns per lane, and for long lists ONE lane per block (further down).
 //
 // Bound: instruction issue, then HBM. With eight columns per lane (quant_codec.cuh) a block takes four shuffle stages
 // of eight values per lane, a hash per column for its sign and scalar fp32 throughout: about 300 instructions per
@@ -271,8 +271,8 @@ __device__ __forceinline__ void rotate_quantize32(const uint32_t (&raw)[16], uns
 
 // ---------------------------------------------------------------- long lists of blocks: one lane per block
 // A warp takes 32 rows of one K group, a lane one row's whole 128 columns: no shuffle stage, signs that are the same for the warp, and
-// one scale, division and address per 128 columns instead of per 32. About 1280 instructions per 32 blocks against 1960 with four lanes
-// each. What that costs is warps (160 registers, three per scheduler), so the rows come by asynchronous copies, the next task's while
+// one scale, division and address per 128 columns instead of per 32. 1570 instructions per 32 blocks, loads included, against 1960 with
+// four lanes each. What that costs is warps (160 to 166 registers by type, three per scheduler), so the rows come by asynchronous copies, the next task's while
 // this one is computed.
 constexpr int kLaneBlockThreads = 64, kLaneBlockResident = 6; // CTAs per multiprocessor
 constexpr int kLaneBlockBytes = 32 * 256;                      // 32 rows of 128 16-bit columns, per warp and operand

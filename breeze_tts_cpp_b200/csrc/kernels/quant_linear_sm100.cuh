@@ -121,8 +121,9 @@ template <bool F16> __device__ __forceinline__ uint32_t relu2x16(uint32_t v) {
 }
 // Post-GEMM chain on eight consecutive channels of one row, already rounded to storage and packed, up to and
 // including ReLU; rounding points follow the reference's separate pass
-// (src/ops/kernels/sequence/sequence_internal.cuh:52-74), so GEMM + fused chain equals GEMM followed by that pass
-// bit for bit. Every step ends in a storage value, which is why the row can stay packed between them.
+// (src/ops/kernels/sequence/sequence_internal.cuh:52-74), so a kernel's GEMM + fused chain equals the same kernel's
+// GEMM followed by that pass bit for bit (FP8 plans of 128 tokens run another kernel when a chain follows, launch_quant_linear, and its fp32 sums
+// may round differently). Every step ends in a storage value, which is why the row can stay packed between them.
 // The gate is one more rounding step here instead of a launch and a pass over the output: modulated FP8 block of 4 x 93 x 512,
 // 23.7 -> 18.8 us.
 template <bool F16, bool Gate = true> __device__ __forceinline__ uint4 chain8(const FusedEpilogue &e, uint4 row, uint4 bias, uint4 gate, uint4 skip) {

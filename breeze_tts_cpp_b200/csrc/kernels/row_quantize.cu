@@ -150,8 +150,8 @@ row_quantize_warp_rows(const T *__restrict__ x, unsigned char *__restrict__ q, f
 
 // K-group mode with rotation (group 128): the blocks of all rows in one list, block i = K group i / rows of row i %
 // rows, four lanes per block, eight blocks per warp. A block's scale then belongs at scales[i], a warp's eight scales
-// share one 32-byte sector, and neither rows nor columns leave lanes idle. 12288 x 2048: 43.9 -> 19.6 us (3.9 TB/s), 1021 x
-// 2048 5.1 -> 3.1, 16 x 2048 1.7 -> 1.4. One set of eight per warp: looping over four with the next one's loads in flight
+// share one 32-byte sector, and neither rows nor columns leave lanes idle. Against eight columns per lane: 8192 x 2048 11.5 us, 1021 x
+// 2048 5.1 -> 3.1, 16 x 2048 1.7 -> 1.4; 12288 x 2048, which takes row_quantize_lanes now, 43.9 -> 19.6 (3.9 TB/s). One set of eight per warp: looping over four with the next one's loads in flight
 // took 24.9 us, resident warps hide more. What is left is issue (491 instructions per 32 columns, 57 % busy).
 template <Type F, class T>
 __global__ void __launch_bounds__(kThreads, 3)
@@ -185,7 +185,7 @@ row_quantize_blocks(const T *__restrict__ x, unsigned char *__restrict__ q, floa
 }
 
 // The same with one lane per block for long lists (lane_blocks_pay): persistent warps over tasks of 32 rows x one K group, neighbouring
-// warps on neighbouring groups. Bound by the fp32 pipe: 1280 of its operations per lane and block; 12288 x 2048 20.2 -> 18.5 us.
+// warps on neighbouring groups. Bound by the fp32 pipe and issue; 12288 x 2048 20.2 -> 18.5 us against four lanes per block.
 template <Type F, class T>
 __global__ void __launch_bounds__(kLaneBlockThreads, kLaneBlockResident)
 row_quantize_lanes(const T *__restrict__ x, unsigned char *__restrict__ q, float *__restrict__ scales, int rows, int cols, int stride,
